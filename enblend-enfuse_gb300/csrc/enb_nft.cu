@@ -10,15 +10,27 @@
 // every column of the feature image (0 on features, FLT_MAX elsewhere), then
 // along every row of that result, then sqrt.  Every float operation is the
 // reference's, in its order and rounding (no contraction into fused
-// multiply-adds), so the masks are bit-identical.  One thread walks one line
-// (the envelope is sequential); its envelope (vertex indices v, boundaries
-// z) lives in global scratch interleaved across the threads of a launch.
+// multiply-adds), so the masks are bit-identical.
+//
+// Columns of at most 4096 rows: q^2 and every other number of the column
+// envelope is an integer below 2^24, exact in float, so the envelope of a
+// 0 / FLT_MAX column is the distance to the nearest feature above or below
+// (FLT_MAX without one) and k_nft_near scans for it with bit masks, one warp
+// per 32 columns x 1/32 of the rows.  Taller columns round and keep the
+// sequential envelope (k_nft_columns, one thread a line).
+//
+// Rows: the sums round (q^2 beyond 2^24) and which vertex survives depends on
+// it, so the envelope stays the reference's sequential walk, one lane a line
+// (k_nft_envelope); the lookup of the surviving vertex of every pixel is
+// parallel over the pixels (k_nft_select, a binary search of the line's
+// boundaries) and ends in the mask.
 //
 // Wrap-around (--wrap horizontal): the reference transforms the image
 // doubled horizontally and keeps, for x < w/2, column w + x and, for the
 // other columns, column x (src/nearest.h:136-342).
 #include <cuda_runtime.h>
 #include <float.h>
+#include <limits.h>
 #include <math_constants.h>
 #include <stdint.h>
 
@@ -70,11 +82,9 @@ struct NftArgs {
     int w, h;
     float* inter;        // [2][h][ipitch]: column pass of the two transforms
     int64_t ipitch;
-    float* dist;         // [2][h][ipitch]: distances of the kept columns
     int* v;              // envelope scratch
     float* z;
     unsigned int* tally; // [2]: pixels only white covers, only black covers
-    int wrap;
 };
 
 // Whether (x, y) is a feature of transform t: covered by the white image
@@ -85,8 +95,9 @@ __device__ __forceinline__ bool nft_feature(const NftArgs& a, int t, int x, int 
     return t == 0 ? wv > bv : bv > wv;
 }
 
-// Column pass: thread (x, t) for x < w, t = blockIdx.y.  With wrap the
-// doubled image's columns repeat, so each column is transformed once.
+// Column pass of tall canvases: thread (x, t) for x < w, t = blockIdx.y.
+// With wrap the doubled image's columns repeat, so each column is
+// transformed once.
 __global__ void __launch_bounds__(128) k_nft_columns(const NftArgs a)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -107,88 +118,401 @@ __global__ void __launch_bounds__(128) k_nft_columns(const NftArgs a)
     atomicAdd(&a.tally[t], count);
 }
 
-// Row pass: thread (y, t).  The row has w samples, or 2w with wrap (the
-// column pass repeated); the kept samples are written as distances.
-__global__ void __launch_bounds__(128) k_nft_rows(const NftArgs a)
+// ---- columns of at most kNearRows rows --------------------------------------
+
+constexpr int kNearRows = 4096;
+constexpr uint16_t kNoFeature = 0xffff;
+constexpr int kNearWords = kNearRows / 32 / 32;  // feature words of a warp's rows
+
+struct NearArgs {
+    const uint8_t* white;
+    const uint8_t* black;
+    int64_t wpitch, bpitch;
+    int w, h, rows;      // rows: rows of one warp
+    uint16_t* g;         // [2][h][pitch]: rows to the nearest feature, kNoFeature
+    int64_t pitch;
+    unsigned int* tally; // [2]
+};
+
+// Distance in rows to the nearest feature of the column, for both
+// transforms.  A block covers 16 columns; half warp r takes the rows
+// [r * rows, (r + 1) * rows), a lane keeps its rows' features as bits, the
+// half warps exchange the last and first feature of their rows through shared
+// memory, and every distance follows from the bits (clz / ffs) and the
+// neighbours'.  16 columns and 512 threads fit three blocks on an SM, so that
+// the 6963 columns of a panorama are one wave (32 columns and 1024 threads
+// took 1.4 waves and 0.17 ms).  Bound by the instructions of the bit scans:
+// 6963x3072 takes 0.11 ms (128 MB); the sequential envelope took 6.0 ms.
+constexpr int kNearCols = 16;
+
+__global__ void __launch_bounds__(32 * kNearCols, 3) k_nft_near(const NearArgs a)
 {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    const int t = blockIdx.y;
-    if (y >= a.h) {
+    __shared__ int last[2][32][kNearCols], first[2][32][kNearCols];
+    const int lane = threadIdx.x % kNearCols, r = threadIdx.x / kNearCols;
+    const int x = blockIdx.x * kNearCols + lane, y0 = r * a.rows, y1 = min(a.h, y0 + a.rows);
+    uint32_t bits[2][kNearWords];
+    int lo[2] = {INT_MAX / 2, INT_MAX / 2}, hi[2] = {INT_MIN / 2, INT_MIN / 2};
+    unsigned int count[2] = {0u, 0u};
+#pragma unroll
+    for (int i = 0; i < kNearWords; ++i) {
+        bits[0][i] = bits[1][i] = 0u;
+        if (y0 + 32 * i < y1 && x < a.w) {
+#pragma unroll 16
+            for (int b = 0; b < 32; ++b) {
+                const int y = y0 + 32 * i + b;
+                if (y < y1) {
+                    const int wv = __ldg(&a.white[(int64_t)y * a.wpitch + x]), bv = __ldg(&a.black[(int64_t)y * a.bpitch + x]);
+                    bits[0][i] |= (wv > bv ? 1u : 0u) << b;
+                    bits[1][i] |= (bv > wv ? 1u : 0u) << b;
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const uint32_t v = bits[t][i];
+            if (v) {
+                lo[t] = min(lo[t], y0 + 32 * i + __ffs(v) - 1);
+                hi[t] = y0 + 32 * i + 31 - __clz(v);
+                count[t] += __popc(v);
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        first[t][r][lane] = lo[t];
+        last[t][r][lane] = hi[t];
+        const unsigned int n = __reduce_add_sync(0xffffffffu, count[t]);
+        if (threadIdx.x % 32 == 0 && n) {
+            atomicAdd(&a.tally[t], n);
+        }
+    }
+    __syncthreads();
+    if (x >= a.w) {
         return;
     }
-    const int n = a.wrap ? 2 * a.w : a.w;
-    const int64_t line = (int64_t)t * a.h + y, ss = 2 * (int64_t)a.h;
-    int* v = a.v + line;
-    float* z = a.z + line;
-    const float* row = a.inter + ((int64_t)t * a.h + y) * a.ipitch;
-    float* drow = a.dist + ((int64_t)t * a.h + y) * a.ipitch;
-    const int w = a.w, half = a.w / 2;
-    const auto f = [&](int q) { return row[q < w ? q : q - w]; };
-    if (a.wrap) {
-        // keep columns w/2 .. w + w/2 - 1 of the doubled row, as column q mod w
-        fh_line(n, f, [&](int q, float d) {
-            if (q >= half && q < w + half) {
-                drow[q < w ? q : q - w] = sqrtf(d);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        int above = INT_MIN / 2, below = INT_MAX / 2;  // nearest feature outside the warp's rows
+        for (int q = 0; q < r; ++q) {
+            above = max(above, last[t][q][lane]);
+        }
+        for (int q = r + 1; q < 32; ++q) {
+            below = min(below, first[t][q][lane]);
+        }
+        uint16_t* col = a.g + (int64_t)t * a.h * a.pitch + x;
+#pragma unroll
+        for (int i = 0; i < kNearWords; ++i) {
+            int next = below;  // first feature after this word
+#pragma unroll
+            for (int j = kNearWords - 1; j > i; --j) {
+                next = bits[t][j] ? y0 + 32 * j + __ffs(bits[t][j]) - 1 : next;
             }
-        }, v, z, ss);
-    } else {
-        fh_line(n, f, [&](int q, float d) { drow[q] = sqrtf(d); }, v, z, ss);
+            const int base = y0 + 32 * i;
+            const uint32_t v = bits[t][i];
+            for (int b = 0; b < 32 && base + b < y1; ++b) {
+                const uint32_t up = v & (0xffffffffu >> (31 - b)), down = v >> b;
+                const int u = up ? b - 31 + __clz(up) : base + b - above;
+                const int d = down ? __ffs(down) - 1 : next - base - b;
+                const int m = min(u, d);
+                col[(int64_t)(base + b) * a.pitch] = m < kNearRows ? (uint16_t)m : kNoFeature;
+            }
+            above = v ? base + 31 - __clz(v) : above;
+        }
     }
 }
 
-__global__ void __launch_bounds__(256) k_nft_mask(const float* __restrict__ dist, int64_t ipitch, int w, int h,
-                                                  uint8_t* __restrict__ mask, int64_t mpitch)
+// ---- rows -------------------------------------------------------------------
+
+// f(q) of a row, eight at a time: squared row distances as floats, or the
+// distances of k_nft_near.  The planes' pitches are multiples of 32 samples,
+// so a group of eight is aligned and lies inside the plane.
+struct RowsF32 {
+    typedef float T;
+    __device__ __forceinline__ static float one(const float* p) { return *p; }
+    struct Group {
+        float4 a, b;
+    };
+    __device__ __forceinline__ static Group load(const float* p)
+    {
+        return Group{__ldg(reinterpret_cast<const float4*>(p)), __ldg(reinterpret_cast<const float4*>(p) + 1)};
+    }
+    __device__ __forceinline__ static float get(const Group& g, int i)
+    {
+        const float v[8] = {g.a.x, g.a.y, g.a.z, g.a.w, g.b.x, g.b.y, g.b.z, g.b.w};
+        return v[i];
+    }
+};
+
+struct RowsU16 {
+    typedef uint16_t T;
+    typedef uint4 Group;
+    __device__ __forceinline__ static float of(uint32_t v)
+    {
+        return v == kNoFeature ? FLT_MAX : (float)(v * v);  // v < 4096: exact
+    }
+    __device__ __forceinline__ static float one(const uint16_t* p) { return of(*p); }
+    __device__ __forceinline__ static Group load(const uint16_t* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+    __device__ __forceinline__ static float get(const Group& g, int i)
+    {
+        const uint32_t w = i < 2 ? g.x : (i < 4 ? g.y : (i < 6 ? g.z : g.w));
+        return of((i & 1) ? w >> 16 : w & 0xffffu);
+    }
+};
+
+// One vertex of a line's envelope: its column and the start of its range.
+struct Vertex {
+    int v;
+    float z;
+};
+
+struct RowArgs {
+    const void* f;       // [2][h][pitch]
+    int64_t pitch;
+    int w, h, wrap;
+    Vertex* env;         // [2][h][n], n = w or 2 w
+    int* count;          // [2][h] vertices
+    uint8_t* mask;
+    int64_t mpitch;
+};
+
+// The first loop of the 1-D transform (src/openmp_vigra.h:300-330) of row y,
+// transform t: the envelope's vertices in order.  Lane l of a warp walks line
+// blockIdx.x * kLines + l; the top of the stack is in registers, the entries
+// just below it in a shared-memory ring (a pop there is one access), all of
+// it in global memory, where pops beyond the ring read it back.
+//   * Samples without a feature (FLT_MAX) after the first are skipped: such a
+//     vertex is pushed with a boundary of 0 or FLT_MAX / (2 d), and the next
+//     finite sample's intersection with it is -FLT_MAX / (2 d), which pops it
+//     before anything else is compared; left at the end of the line, its range
+//     starts beyond the line (or, over a first sample without a feature, gives
+//     the same FLT_MAX).
+//   * The division by 2 (q - v) of neighbours is an exact halving.
+// Bound by the dependent chain of a line (about 470 cycles a sample), so a
+// warp takes only kLines lines: fewer lanes diverge, and every SM holds
+// several warps.  6963x3072, both transforms: 1.02 ms with 4 or 8 lines a
+// warp, 1.18 / 1.11 / 1.24 ms with 2 / 16 / 32; the walk with the envelope in
+// interleaved global scratch and the second loop in the same thread took
+// 11.6 ms.  (Cutting the lines into 16 parts, each on an empty stack above a
+// vertex later proven unpopped, took 1.40 ms: the lanes of a warp then walk
+// unlike samples, and in the overlap of two footprints no vertex stands.)
+constexpr int kLines = 8, kRing = 32;
+
+template <class R>
+__global__ void __launch_bounds__(32) k_nft_envelope(const RowArgs a)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y;
-    if (x >= w) {
+    __shared__ int ring_v[kRing][kLines];
+    __shared__ float ring_f[kRing][kLines], ring_z[kRing][kLines];
+    const int lane = threadIdx.x;
+    const int line = blockIdx.x * kLines + lane;
+    if (lane >= kLines || line >= 2 * a.h) {
         return;
     }
-    const float d12 = dist[(int64_t)y * ipitch + x], d21 = dist[((int64_t)h + y) * ipitch + x];
-    mask[(int64_t)y * mpitch + x] = d12 < d21 ? 255 : 0;
+    typedef typename R::T T;
+    const T* row = static_cast<const T*>(a.f) + (int64_t)line * a.pitch;
+    const int n = a.wrap ? 2 * a.w : a.w;
+    Vertex* env = a.env + (int64_t)line * n;
+    // f(v) + v^2 as the reference adds it for a vertex of the stack (an integer square)
+    const auto lift = [](float f, int v) { return __fadd_rn(f, (float)(int)((unsigned)v * (unsigned)v)); };
+    int k = 0, low = 0;  // top of the stack, lowest entry in the ring
+    int vk = 0;
+    float fk = lift(R::one(row), 0), zk = -CUDART_INF_F;
+    const auto put = [&]() {
+        ring_v[k % kRing][lane] = vk;
+        ring_f[k % kRing][lane] = fk;
+        ring_z[k % kRing][lane] = zk;
+        env[k] = Vertex{vk, zk};
+    };
+    put();
+    for (int pass = 0; pass * a.w < n; ++pass) {
+        typename R::Group next = R::load(row);
+        for (int x0 = 0; x0 < a.w; x0 += 8) {
+            const typename R::Group g = next;
+            if (x0 + 8 < a.w) {
+                next = R::load(row + x0 + 8);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int q = pass * a.w + x0 + i;
+                const float f = R::get(g, i);
+                if (x0 + i >= a.w || q == 0 || f == FLT_MAX) {
+                    continue;
+                }
+                const float qf = (float)q;
+                const float sum = __fadd_rn(f, __fmul_rn(qf, qf));
+                float num = __fsub_rn(sum, fk);
+                float s = vk == q - 1 ? 0.5f * num : __fdiv_rn(num, (float)(2 * (q - vk)));
+                while (s <= zk) {
+                    --k;
+                    if (k >= low) {
+                        vk = ring_v[k % kRing][lane];
+                        fk = ring_f[k % kRing][lane];
+                        zk = ring_z[k % kRing][lane];
+                    } else {
+                        const Vertex e = env[k];
+                        vk = e.v;
+                        zk = e.z;
+                        fk = lift(R::one(row + (vk < a.w ? vk : vk - a.w)), vk);
+                        low = k;
+                        ring_v[k % kRing][lane] = vk;
+                        ring_f[k % kRing][lane] = fk;
+                        ring_z[k % kRing][lane] = zk;
+                    }
+                    s = __fdiv_rn(__fsub_rn(sum, fk), (float)(2 * (q - vk)));
+                }
+                ++k;
+                low = max(low, k - kRing + 1);
+                vk = q;
+                fk = lift(f, q);
+                zk = s;
+                put();
+            }
+        }
+    }
+    a.count[line] = k + 1;
+}
+
+// The second loop (src/openmp_vigra.h:333-351) and the comparison: pixel q of
+// row y takes the last vertex whose range starts before q.  A thread finds it
+// for the first of its eight columns by binary search and walks on from there.
+template <class R>
+__global__ void __launch_bounds__(128) k_nft_select(const RowArgs a)
+{
+    const int y = blockIdx.y;
+    const int x0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (x0 >= a.w) {
+        return;
+    }
+    typedef typename R::T T;
+    const int n = a.wrap ? 2 * a.w : a.w, half = a.w / 2;
+    float d[2][8];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int64_t line = (int64_t)t * a.h + y;
+        const T* row = static_cast<const T*>(a.f) + line * a.pitch;
+        const Vertex* env = a.env + line * n;
+        const int m = a.count[line];
+        int k = -1, v = 0;
+        float next = 0.0f, f = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int x = min(x0 + i, a.w - 1);
+            // the periodic transform keeps the doubled row's columns w/2 .. w + w/2 - 1
+            const int q = a.wrap && x < half ? x + a.w : x;
+            bool moved = false;
+            if (k < 0 || (a.wrap && x == half)) {
+                int lo = 0, hi = m;  // env[lo].z < q <= env[hi].z
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) / 2;
+                    if (env[mid].z < (float)q) {
+                        lo = mid;
+                    } else {
+                        hi = mid;
+                    }
+                }
+                k = lo;
+                moved = true;
+                next = k + 1 < m ? env[k + 1].z : CUDART_INF_F;
+            }
+            while (next < (float)q) {
+                ++k;
+                moved = true;
+                next = k + 1 < m ? env[k + 1].z : CUDART_INF_F;
+            }
+            if (moved) {
+                v = env[k].v;
+                f = R::one(row + (v < a.w ? v : v - a.w));
+            }
+            d[t][i] = __fsqrt_rn(__fadd_rn((float)((q - v) * (q - v)), f));
+        }
+    }
+    uint8_t* out = a.mask + (int64_t)y * a.mpitch + x0;
+    uint32_t o[2] = {0u, 0u};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        o[i / 4] |= (d[0][i] < d[1][i] ? 255u : 0u) << (8 * (i % 4));
+    }
+    if (x0 + 8 <= a.w && (reinterpret_cast<uintptr_t>(out) & 7) == 0) {
+        *reinterpret_cast<uint2*>(out) = make_uint2(o[0], o[1]);
+    } else {
+        for (int i = 0; i < 8 && x0 + i < a.w; ++i) {
+            out[i] = (uint8_t)(o[i / 4] >> (8 * (i % 4)));
+        }
+    }
 }
 
 }  // namespace
 
-size_t nft_scratch_bytes(int w, int h, int wrap)
-{
-    const int64_t ipitch = (w + 31) / 32 * 32;
-    const int64_t n_col = 2 * (int64_t)w * ((int64_t)h + 1), n_row = 2 * (int64_t)h * ((wrap ? 2 : 1) * (int64_t)w + 1);
-    const int64_t n_env = n_col > n_row ? n_col : n_row;
-    return (size_t)(4 * ipitch * h * sizeof(float) + n_env * (sizeof(int) + sizeof(float)) + 256);
-}
+// Scratch of one call: the row pass's source planes (16-bit distances, or
+// floats for tall columns), the envelopes and the vertex counts.
+struct NftLayout {
+    int64_t pitch, env, count, column_v, column_z, total;  // byte offsets
+    NftLayout(int w, int h, int wrap)
+    {
+        const auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
+        const bool tall = h > kNearRows;
+        pitch = (w + 31) / 32 * 32;
+        env = up(2 * pitch * h * (tall ? (int64_t)sizeof(float) : (int64_t)sizeof(uint16_t)));
+        count = up(env + 2 * (int64_t)h * (wrap ? 2 : 1) * w * (int64_t)sizeof(Vertex));
+        column_v = up(count + 2 * (int64_t)h * (int64_t)sizeof(int));
+        // the sequential column envelopes of tall canvases
+        column_z = up(column_v + (tall ? 2 * (int64_t)w * (h + 1) * (int64_t)sizeof(int) : 0));
+        total = up(column_z + (tall ? 2 * (int64_t)w * (h + 1) * (int64_t)sizeof(float) : 0));
+    }
+};
 
-// Stage 0: the column pass and the tallies; 1: the row pass; 2: the mask.
+size_t nft_scratch_bytes(int w, int h, int wrap) { return (size_t)NftLayout(w, h, wrap).total; }
+
+// Stage 0: the column pass and the tallies; 1: the row envelopes; 2: the
+// nearest vertices and the mask.
 cudaError_t launch_nft_stage(int stage, const BytePlane& white, const BytePlane& black, const BytePlane& mask,
                              int wrap, void* scratch, unsigned int* tally, cudaStream_t st)
 {
     const int w = white.w, h = white.h;
-    NftArgs a{};
-    a.white = white.p;
-    a.black = black.p;
-    a.wpitch = white.pitch;
-    a.bpitch = black.pitch;
-    a.w = w;
-    a.h = h;
-    a.wrap = wrap;
-    a.ipitch = (w + 31) / 32 * 32;
-    a.inter = static_cast<float*>(scratch);
-    a.dist = a.inter + 2 * a.ipitch * h;
-    const int64_t n_col = 2 * (int64_t)w * ((int64_t)h + 1), n_row = 2 * (int64_t)h * ((wrap ? 2 : 1) * (int64_t)w + 1);
-    const int64_t n_env = n_col > n_row ? n_col : n_row;
-    a.v = reinterpret_cast<int*>(a.dist + 2 * a.ipitch * h);
-    a.z = reinterpret_cast<float*>(a.v + n_env);
-    a.tally = tally;
+    const NftLayout l(w, h, wrap);
+    char* base = static_cast<char*>(scratch);
+    const bool tall = h > kNearRows;
+    const double sample = tall ? 4.0 : 2.0;
     if (stage == 0) {
-        note_launch("nft_columns", 2.0 * w * h * (2.0 + 4.0));
+        note_launch("nft_columns", 2.0 * w * h * (1.0 + sample));
+        if (!tall) {
+            const NearArgs a{white.p, black.p, white.pitch, black.pitch, w, h, (h + 31) / 32,
+                             reinterpret_cast<uint16_t*>(base), l.pitch, tally};
+            k_nft_near<<<(unsigned)((w + kNearCols - 1) / kNearCols), 32 * kNearCols, 0, st>>>(a);
+            return cudaGetLastError();
+        }
+        NftArgs a{};
+        a.white = white.p;
+        a.black = black.p;
+        a.wpitch = white.pitch;
+        a.bpitch = black.pitch;
+        a.w = w;
+        a.h = h;
+        a.ipitch = l.pitch;
+        a.inter = reinterpret_cast<float*>(base);
+        a.v = reinterpret_cast<int*>(base + l.column_v);
+        a.z = reinterpret_cast<float*>(base + l.column_z);
+        a.tally = tally;
         k_nft_columns<<<dim3((unsigned)((w + 127) / 128), 2), 128, 0, st>>>(a);
-    } else if (stage == 1) {
-        note_launch("nft_rows", 2.0 * w * h * 8.0);
-        k_nft_rows<<<dim3((unsigned)((h + 127) / 128), 2), 128, 0, st>>>(a);
+        return cudaGetLastError();
+    }
+    RowArgs a{base, l.pitch, w, h, wrap, reinterpret_cast<Vertex*>(base + l.env), reinterpret_cast<int*>(base + l.count),
+              mask.p, mask.pitch};
+    if (stage == 1) {
+        note_launch("nft_rows", 2.0 * w * h * (sample + (wrap ? 16.0 : 8.0)));
+        const unsigned blocks = (unsigned)((2 * h + kLines - 1) / kLines);
+        if (tall) {
+            k_nft_envelope<RowsF32><<<blocks, 32, 0, st>>>(a);
+        } else {
+            k_nft_envelope<RowsU16><<<blocks, 32, 0, st>>>(a);
+        }
     } else {
-        note_launch("nft_mask", (double)w * h * 9.0);
-        k_nft_mask<<<dim3((unsigned)((w + 255) / 256), (unsigned)h), 256, 0, st>>>(a.dist, a.ipitch, w, h, mask.p,
-                                                                               mask.pitch);
+        note_launch("nft_mask", 2.0 * w * h * (sample + 8.0) + (double)w * h);
+        const dim3 grid((unsigned)((w + 1023) / 1024), (unsigned)h);
+        if (tall) {
+            k_nft_select<RowsF32><<<grid, 128, 0, st>>>(a);
+        } else {
+            k_nft_select<RowsU16><<<grid, 128, 0, st>>>(a);
+        }
     }
     return cudaGetLastError();
 }

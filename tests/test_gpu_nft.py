@@ -122,3 +122,30 @@ def test_front_end_generates_seams(orc, tmp_path):
     got = np.load(out)
     assert np.array_equal(got[..., :3], acc)
     assert np.array_equal(got[..., 3], np.where(acc_alpha != 0, 65535, 0).astype(np.uint16))
+
+
+@pytest.mark.parametrize("h,w,wrap", [(2, 2, False), (31, 33, True), (32, 7, False), (33, 64, False), (1023, 65, True),
+                                      (1025, 31, False), (4095, 40, False), (4096, 33, True), (4097, 40, False),
+                                      (4100, 33, True), (40, 4097, False), (70, 9001, False), (36, 4500, True)])
+def test_nft_mask_scan_and_envelope_edges(ctx, orc, h, w, wrap):
+    """The column scan at the edges of its 32-row words, 32 warps and 4096 rows (the sequential envelope beyond),
+    and rows long enough that their squares round in float; sparse, dense and blocky footprints, some columns and
+    rows without any feature."""
+    import enbgpu
+    rng = np.random.default_rng(10000 * h + w)
+    yy, xx = np.mgrid[0:h, 0:w]
+    for case in range(4):
+        if case < 2:
+            p = (0.02, 0.7)[case]
+            wa, ba = [np.where(rng.random((h, w)) < p, 255, 0).astype(np.uint8) for _ in range(2)]
+        else:
+            wa = np.where(xx + (case - 2) * 0.05 * yy >= w / 3, 255, 0).astype(np.uint8)
+            ba = np.where((xx <= 2 * w / 3) & (yy >= h // 4), 255, 0).astype(np.uint8)
+        try:
+            want = orc.nft_mask(wa, ba, wrap)
+        except ValueError:
+            with pytest.raises(enbgpu.EnbError):
+                ctx.nft_mask(_dev(wa), _dev(ba), wrap=wrap)
+            continue
+        got = ctx.nft_mask(_dev(wa), _dev(ba), wrap=wrap).cpu().numpy()
+        assert np.array_equal(got, want), case

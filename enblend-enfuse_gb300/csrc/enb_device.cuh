@@ -81,13 +81,15 @@ __device__ __forceinline__ TD mask_to_fixed(float m, int frac)
 
 // fromRealPromote(lp * fl(m / D)) with D = 255 * 2^F (src/enfuse.h:601-620).
 //
-// For 0 < m < D the exact value t = lp*m/D has denominator 2D after adding
+// For 0 <= m <= D the exact value t = lp*m/D has denominator 2D after adding
 // 1/2, so its distance to the rounding boundary is either 0 or >= 1/(2D);
 // the double expression differs from t by < 2^-26, which is smaller.  Hence
 // round-half-away(t) is the reference's result unless t is exactly a
-// half-integer, in which case the double expression is evaluated as is.
+// half-integer, in which case the double expression is evaluated as is (out
+// of line: it is rare, and the callers repeat this per exposure and sample).
+// m = 0 and m = D need no case of their own: the quotient is 0 and |lp|.
 template <typename T, int F>
-__device__ __forceinline__ T mask_multiply(int32_t lp, int32_t m)
+static __device__ __noinline__ T mask_multiply_double(int32_t lp, int32_t m)
 {
     constexpr int32_t D = 255 << F;
     if (m == 0) {
@@ -96,20 +98,34 @@ __device__ __forceinline__ T mask_multiply(int32_t lp, int32_t m)
     if (m == D) {
         return (T)lp;  // coefficient exactly 1.0
     }
-    const uint32_t a = lp < 0 ? (uint32_t)(-(int64_t)lp) : (uint32_t)lp;
-    if (m > 0 && m < D && a < (1u << 24)) {
-        const uint64_t N = 2ull * (uint64_t)a * (uint64_t)m + (uint64_t)D;
-        const uint32_t hi = (uint32_t)(N >> (F + 1));
-        const uint32_t lo = (uint32_t)(N & ((1ull << (F + 1)) - 1));
-        const uint32_t q = hi / 255u;
-        const bool tie = lo == 0 && hi == q * 255u;
-        if (!tie) {
-            const int32_t r = lp < 0 ? -(int32_t)q : (int32_t)q;
-            return sizeof(T) == 2 ? (T)min(max(r, -32768), 32767) : (T)r;
-        }
-    }
     const double coeff = __ddiv_rn((double)m, (double)D);
     return frp_store<T>(__dmul_rn((double)lp, coeff));
+}
+
+template <typename T, int F>
+__device__ __forceinline__ T mask_multiply(int32_t lp, int32_t m)
+{
+    constexpr uint32_t D = 255u << F;
+    // 2 |lp| m + D fits 32 bits for Int16 levels with 9.7 masks, else 48 up to |lp| < 2^24
+    constexpr bool NARROW = sizeof(T) == 2 && F == 7;
+    constexpr uint32_t AMAX = NARROW ? 32768u : (1u << 24) - 1u;
+    const uint32_t a = lp < 0 ? 0u - (uint32_t)lp : (uint32_t)lp;
+    uint32_t hi, lo;
+    if (NARROW) {
+        const uint32_t N = a * (2u * (uint32_t)m) + D;
+        hi = N >> (F + 1);
+        lo = N & ((1u << (F + 1)) - 1u);
+    } else {
+        const uint64_t N = (uint64_t)a * (2u * (uint32_t)m) + D;
+        hi = (uint32_t)(N >> (F + 1));
+        lo = (uint32_t)N & ((1u << (F + 1)) - 1u);
+    }
+    const uint32_t q = hi / 255u;
+    const bool tie = lo == 0 && hi == q * 255u;
+    if (tie || (uint32_t)m > D || a > AMAX) {
+        return mask_multiply_double<T, F>(lp, m);
+    }
+    return (T)(lp < 0 ? 0u - q : q);
 }
 
 __host__ __device__ __forceinline__ int imod(int a, int m)

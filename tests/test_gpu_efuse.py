@@ -137,3 +137,35 @@ def test_fused_enfuse_host_buffers(ctx, orc, dt):
     out, oa = ctx.enfuse(imgs, params=enbgpu.enfuse_params(**W_ALL), seed=6)
     assert np.array_equal(out, ref["out"])
     assert np.array_equal(oa, ref["alpha"])
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16])
+@pytest.mark.parametrize("w,h,K,wrap,chans", [(65, 33, 2, False, 3), (64, 16, 5, False, 3), (129, 31, 16, False, 3),
+                                              (130, 47, 3, True, 3), (131, 49, 4, True, 4), (63, 95, 9, True, 3),
+                                              (257, 63, 3, False, 4), (66, 34, 4, True, 1)])
+def test_level_tiles_at_their_edges(ctx, dtype, w, h, K, wrap, chans):
+    """The level passes at tile edges, odd and periodic levels, one and four channels, many exposures, and output
+    rows that allow paired stores or not, against the per-operation passes: every sample of level 0 and the pixels."""
+    rng = np.random.default_rng(w * 1000 + h)
+    maxv = np.iinfo(dtype).max
+    shape = (h, w) if chans == 1 else (h, w, chans)
+    imgs = [rng.integers(0, maxv + 1, shape).astype(dtype) for _ in range(K)]
+    if chans == 4:
+        for im in imgs:
+            im[..., 3] = maxv
+    alphas = [np.where(rng.random((h, w)) < 0.9, 255, 0).astype(np.uint8) for _ in range(K)]
+    import enbgpu
+    prm = enbgpu.enfuse_params(saturation_weight=0.2, contrast_weight=0.5)
+    got = []
+    for plain in (False, True):
+        l0 = np.zeros((h, w, min(chans, 3)), np.int32)
+        out, alpha = ctx.enfuse(imgs, alphas, params=prm, wrap=wrap, seed=9, level0=l0, plain=plain)
+        got.append((l0, out, alpha))
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    # device rows one sample off the pair's alignment
+    pad = [torch.from_numpy(np.pad(im, [(0, 0), (0, 1)] + [(0, 0)] * (im.ndim - 2))).cuda()[:, :w] for im in imgs]
+    out = torch.from_numpy(np.zeros_like(np.pad(imgs[0], [(0, 0), (0, 1)] + [(0, 0)] * (imgs[0].ndim - 2)))).cuda()[:, :w]
+    ctx.enfuse(pad, [torch.from_numpy(a).cuda() for a in alphas], params=prm, wrap=wrap, seed=9, out=out)
+    ctx.synchronize()
+    assert np.array_equal(out.cpu().numpy(), got[0][1])

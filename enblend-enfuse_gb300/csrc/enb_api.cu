@@ -763,11 +763,11 @@ enb_status float_cutoffs(enb_ctx* ctx, const enb_enfuse_params* prm, double rang
 
 enb_status alpha_plane(enb_ctx* ctx, const enb_image* img, const enb_image* alpha, DevBuf& buf, BytePlane& out);
 
-enb_status enfuse_mask_float(enb_ctx* ctx, const enb_enfuse_params* prm, const enb_image* src,
-                             const enb_image* alpha, const FloatPlane& out)
+// Parameters of the float weight kernels (and ctx->tables for them).
+enb_status float_weight_params(enb_ctx* ctx, const enb_enfuse_params* prm, FloatWeightParams& wp)
 {
-    ENB_TRY(build_tables(ctx, prm, 1u));  // p log p tables of the entropy
-    FloatWeightParams wp{};
+    ENB_TRY(build_tables(ctx, prm, 1u));
+    wp = FloatWeightParams{};
     wp.use_exposure = prm->w_exposure > 0.0;
     wp.use_contrast = prm->w_contrast > 0.0;
     wp.use_saturation = prm->w_saturation > 0.0;
@@ -793,7 +793,14 @@ enb_status enfuse_mask_float(enb_ctx* ctx, const enb_enfuse_params* prm, const e
     const double inv_width = 1.0 / exposure_effective_width(prm->exp_function, prm->exp_width);
     wp.inv_hi = (float)inv_width;
     wp.inv_lo = (float)(inv_width - (double)wp.inv_hi);
-    ENB_TRY(float_cutoffs(ctx, prm, range, wp));
+    return float_cutoffs(ctx, prm, range, wp);
+}
+
+enb_status enfuse_mask_float(enb_ctx* ctx, const enb_enfuse_params* prm, const enb_image* src,
+                             const enb_image* alpha, const FloatPlane& out)
+{
+    FloatWeightParams wp;
+    ENB_TRY(float_weight_params(ctx, prm, wp));
     const PixelView pv = pixel_view(src);
     DevBuf abuf;
     BytePlane ap;
@@ -1264,6 +1271,68 @@ enb_status enfuse_fused(enb_ctx* ctx, const enb_enfuse_params* prm, int K, const
     return ENB_OK;
 }
 
+// enfuseMain of float images through the batched fuse's kernels
+// (enb_batch.cu): the exposures of a level share a launch and no Laplacian is
+// stored, with the values of the per-operation passes.  It keeps the
+// pyramids of every exposure at once; done is false when they do not fit the
+// device's memory (the per-operation passes, which keep one, then run).
+// 4 x 1601x1203 RGB, all weights: 22 launches and 0.66 ms, against 165
+// launches and 1.43 ms one operation at a time.
+enb_status enfuse_float(enb_ctx* ctx, const enb_enfuse_params* prm, int K, const enb_image* images,
+                        const enb_image* alphas, const enb_image* out, const enb_image* out_alpha,
+                        const enb_fuse_options& o, bool& done)
+{
+    done = false;
+    const int w = images[0].width, h = images[0].height;
+    FloatWeightParams wp;
+    ENB_TRY(float_weight_params(ctx, prm, wp));
+    if (out_alpha && out_alpha->data) {
+        ENB_CHECK(ctx, bytes_ok(out_alpha, w, h), "out_alpha: must be U8 of the image size");
+    }
+    BatchStackHost hs{};
+    hs.K = K;
+    hs.w = w;
+    hs.h = h;
+    hs.C = images[0].channels;
+    std::vector<DevBuf> abufs(K);
+    for (int k = 0; k < K; ++k) {
+        const PixelView v = pixel_view(&images[k]);
+        hs.img[k] = (const float*)v.p;
+        hs.ipitch[k] = v.pitch;
+        hs.istride[k] = v.stride;
+        const enb_image* al = alphas ? &alphas[k] : nullptr;
+        if (alpha_source(&images[k], al).mode != kAlphaOpaque) {
+            BytePlane ap;
+            ENB_TRY(alpha_plane(ctx, &images[k], al, abufs[k], ap));
+            hs.alpha[k] = ap.p;
+            hs.apitch[k] = ap.pitch;
+        }
+    }
+    const PixelView ov = pixel_view(out);
+    hs.out = (float*)out->data;
+    hs.opitch = ov.pitch;
+    hs.ostride = ov.stride;
+    if (out_alpha && out_alpha->data) {
+        hs.oalpha = (uint8_t*)out_alpha->data;
+        hs.oapitch = out_alpha->pitch;
+    }
+    const std::unique_ptr<BatchSingle, void (*)(BatchSingle*)> p(
+        batch_single_create(hs, wp, ctx->tables, o.levels, o.wrap != 0, o.hard_mask != 0), batch_single_destroy);
+    DevBuf work;
+    const cudaError_t e = work.alloc(batch_single_bytes(p.get()), ctx->stream);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return ENB_OK;
+    }
+    ENB_CUDA(ctx, e);
+    done = true;
+    batch_single_workspace(p.get(), work.p);
+    for (int i = 0; i < batch_single_steps(p.get()); ++i) {
+        ENB_LAUNCH(ctx, batch_single_launch(p.get(), i, ctx->stream));
+    }
+    return ENB_OK;
+}
+
 enb_status enfuse_device(enb_ctx* ctx, const enb_enfuse_params* prm, int K, const enb_image* images,
                          const enb_image* alphas, const enb_image* masks_in, const enb_image* out,
                          const enb_image* out_alpha, const enb_fuse_options& o, int32_t* level0)
@@ -1279,6 +1348,13 @@ enb_status enfuse_device(enb_ctx* ctx, const enb_enfuse_params* prm, int K, cons
         }
         if (uniform) {
             return enfuse_fused(ctx, prm, K, images, alphas, masks_in, out, out_alpha, o, level0, L);
+        }
+    }
+    if (!o.plain && dt == ENB_F32 && K <= kBatchMaxK && !masks_in && !level0) {
+        bool done = false;
+        ENB_TRY(enfuse_float(ctx, prm, K, images, alphas, out, out_alpha, o, done));
+        if (done) {
+            return ENB_OK;
         }
     }
     const int pdt = fixed_bits_image(dt), mdt = fixed_bits_mask(dt), mf = mask_frac(dt);
@@ -2181,38 +2257,6 @@ enb_status enb_enblend(enb_ctx* ctx, const enb_image* white, const enb_image* wh
 
 // ---- batched stacks ---------------------------------------------------------
 
-static enb_status float_weight_params(enb_ctx* ctx, const enb_enfuse_params* prm, FloatWeightParams& wp)
-{
-    ENB_TRY(build_tables(ctx, prm, 1u));
-    wp = FloatWeightParams{};
-    wp.use_exposure = prm->w_exposure > 0.0;
-    wp.use_contrast = prm->w_contrast > 0.0;
-    wp.use_saturation = prm->w_saturation > 0.0;
-    wp.use_entropy = prm->w_entropy > 0.0;
-    wp.contrast_window = prm->contrast_window;
-    wp.entropy_window = prm->entropy_window;
-    wp.gray_projector = prm->gray_projector;
-    wp.exp_function = prm->exp_function;
-    if (prm->gray_projector == ENB_GRAY_MIXER) {
-        const double sm = prm->mixer[0] + prm->mixer[1] + prm->mixer[2];
-        for (int i = 0; i < 3; ++i) {
-            wp.mixer[i] = prm->mixer[i] / sm;
-        }
-    }
-    wp.w_exposure = (float)prm->w_exposure;
-    wp.w_contrast = (float)prm->w_contrast;
-    wp.w_saturation = (float)prm->w_saturation;
-    wp.w_entropy = (float)prm->w_entropy;
-    const double range = float_range_of(prm);
-    wp.range = (float)range;
-    wp.opt_hi = (float)prm->exp_optimum;
-    wp.opt_lo = (float)(prm->exp_optimum - (double)wp.opt_hi);
-    const double inv_width = 1.0 / exposure_effective_width(prm->exp_function, prm->exp_width);
-    wp.inv_hi = (float)inv_width;
-    wp.inv_lo = (float)(inv_width - (double)wp.inv_hi);
-    return float_cutoffs(ctx, prm, range, wp);
-}
-
 // What the batched fuse's work depends on: the stacks' sizes, exposure
 // counts and channels, the parameters and the options (not the buffers).
 static std::string batch_geometry_key(const enb_enfuse_params* prm, int n, const enb_stack* stacks,
@@ -2272,10 +2316,10 @@ enb_status enb_fuse_stacks(enb_ctx* ctx, const enb_enfuse_params* prm, int n, co
         ENB_TRY(check_params(ctx, prm, st.images[0].width, st.images[0].height));
     }
     if (o.plain) {
-        // the plain per-stack path: enb_enfuse stack by stack
+        // the plain per-stack path: enb_enfuse stack by stack, one kernel
+        // per operation
         for (int i = 0; i < n; ++i) {
             enb_fuse_options so = o;
-            so.plain = 0;
             so.level0_out = nullptr;
             ENB_TRY(enb_enfuse(ctx, prm, stacks[i].K, stacks[i].images, stacks[i].alphas, nullptr, stacks[i].out,
                                stacks[i].out_alpha, &so));

@@ -71,6 +71,31 @@ struct BatchStack {
     int pitch[kMaxLevels], lw[kMaxLevels], lh[kMaxLevels];
 };
 
+// Where a launch's CTAs find their stack and tile: the host-built tables of a
+// batch, or the launch's own parameters and grid for one stack (blockIdx.x, y
+// the tile, blockIdx.z the exposure of a reduce).  A single stack's launches
+// follow each other by programmatic dependent launch: its small levels would
+// otherwise be mostly launch gaps.
+struct BatchTable {
+    const BatchStack* stacks;
+    const int4* jobs;
+    static constexpr bool kOne = false;
+    __device__ __forceinline__ const BatchStack& stack() const { return stacks[jobs[blockIdx.x].x]; }
+    __device__ __forceinline__ int2 tile() const { return make_int2(jobs[blockIdx.x].y, jobs[blockIdx.x].z); }
+    __device__ __forceinline__ int reduce_kind() const { return jobs[blockIdx.x].y; }
+    __device__ __forceinline__ int2 reduce_tile() const { return make_int2(jobs[blockIdx.x].z, jobs[blockIdx.x].w); }
+};
+
+struct BatchOne {
+    BatchStack s;
+    int kind0;  // kind of blockIdx.z 0
+    static constexpr bool kOne = true;
+    __device__ __forceinline__ const BatchStack& stack() const { return s; }
+    __device__ __forceinline__ int2 tile() const { return make_int2(blockIdx.x, blockIdx.y); }
+    __device__ __forceinline__ int reduce_kind() const { return kind0 + (int)blockIdx.z; }
+    __device__ __forceinline__ int2 reduce_tile() const { return tile(); }
+};
+
 namespace {
 
 __device__ __forceinline__ float* g_level(const BatchStack& s, int k, int l, int C)
@@ -166,23 +191,24 @@ __device__ __forceinline__ void batch_normalise(const BatchStack& s, const float
 
 // Weights of window sizes that the pair kernel does not take: one output
 // pixel per thread on 16x16 tiles (enb_fweights.cuh).
-template <int CW, int EW>
-__global__ void __launch_bounds__(256, 4) k_batch_weights(const BatchStack* __restrict__ stacks,
-                                                       const int4* __restrict__ jobs, FloatWeightParams wp,
+template <int CW, int EW, class J>
+__global__ void __launch_bounds__(256, 4) k_batch_weights(const __grid_constant__ J jobs, FloatWeightParams wp,
                                                        WeightTables tab, int hard, int C)
 {
     extern __shared__ __align__(16) unsigned char bsmem[];
-    const int4 job = jobs[blockIdx.x];
-    const BatchStack& s = stacks[job.x];
+    griddep_wait();
+    griddep_launch();
+    const int2 tile = jobs.tile();
+    const BatchStack& s = jobs.stack();
     const int halo = fweight_halo(wp);
     const FTile t = ftile_carve(bsmem, BWT + 2 * halo, wp.repeat_slots, wp.ent_cut);
     float* wk = reinterpret_cast<float*>(bsmem + align16(ftile_bytes(t.TW, t.slots, wp.ent_cut))) + threadIdx.x;  // [K][BWT * BWT]
     const int lx = threadIdx.x % BWT, ly = threadIdx.x / BWT;
-    const int x = job.y * BWT + lx, y = job.z * BWT + ly;
+    const int x = tile.x * BWT + lx, y = tile.y * BWT + ly;
     const bool inside = x < s.w && y < s.h;
     const int ci = (ly + halo) * t.TW + (lx + halo);
     const int K = s.K;
-    const int x0 = job.y * BWT - halo, y0 = job.z * BWT - halo;
+    const int x0 = tile.x * BWT - halo, y0 = tile.y * BWT - halo;
     uint8_t ua = 0;
     for (int k = 0; k < K; ++k) {
         const int opaque =
@@ -211,24 +237,25 @@ __global__ void __launch_bounds__(256, 4) k_batch_weights(const BatchStack* __re
 // until the normalisation replaces it.  Five CTAs per SM (48 registers;
 // the 42.6 KB tile of 5x5 windows fits five times): the warps hide the
 // kernel's latencies better than more registers would.
-template <int CW, int EW, int C>
-__global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const BatchStack* __restrict__ stacks,
-                                                            const int4* __restrict__ jobs, FloatWeightParams wp,
-                                                            WeightTables tab, int hard)
+template <int CW, int EW, int C, class J>
+__global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const __grid_constant__ J jobs, FloatWeightParams wp,
+                                                            WeightTables tab)
 {
     constexpr int HALO = fpair_halo(CW, EW), HX = fpair_halo_x(HALO);
     constexpr int TW = fpair_tw(CW, EW), TT = TW * fpair_th(CW, EW), NP = (TT + FPT - 1) / FPT;
     extern __shared__ __align__(16) unsigned char bsmem[];
-    const int4 job = jobs[blockIdx.x];
-    const BatchStack& s = stacks[job.x];
+    griddep_wait();
+    griddep_launch();
+    const int2 tile = jobs.tile();
+    const BatchStack& s = jobs.stack();
     const FTileP t0 = fpair_carve(bsmem, TW, TT, wp.repeat_slots, wp.ent_cut);
     const int px = threadIdx.x % (FPX / 2), py = threadIdx.x / (FPX / 2);
-    const int x = job.y * FPX + 2 * px, y = job.z * FPY + py;
+    const int x = tile.x * FPX + 2 * px, y = tile.y * FPY + py;
     const bool in0 = x < s.w && y < s.h, in1 = x + 1 < s.w && y < s.h;
     const int cx = HX + 2 * px, cy = HALO + py, ci = cy * TW + cx;
     const int K = s.K;
     const int64_t plane = (int64_t)s.pitch[0] * s.h, o = (int64_t)y * s.pitch[0] + x;
-    const int x0 = job.y * FPX - HX, y0 = job.z * FPY - HALO;
+    const int x0 = tile.x * FPX - HX, y0 = tile.y * FPY - HALO;
     uint8_t ua0 = 0, ua1 = 0;
     if (t0.slots) {
         fpair_clear_tables<C>(fpair_for_exposure(t0, 0));
@@ -291,13 +318,15 @@ __global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const BatchStack*
 // mask planes (float bits) of a 32x16 tile of a stack, two output pixels per
 // thread: src/enfuse.h:1382-1385 (sum in exposure order), :1399-1442 (hard
 // mask), :1526-1535 (soft mask), into Int32 9.15 masks.
-__global__ void __launch_bounds__(256) k_batch_normalise(const BatchStack* __restrict__ stacks,
-                                                         const int4* __restrict__ jobs, int hard)
+template <class J>
+__global__ void __launch_bounds__(256) k_batch_normalise(const __grid_constant__ J jobs, int hard)
 {
-    const int4 job = jobs[blockIdx.x];
-    const BatchStack& s = stacks[job.x];
+    griddep_wait();
+    griddep_launch();
+    const int2 tile = jobs.tile();
+    const BatchStack& s = jobs.stack();
     const int px = threadIdx.x % (FPX / 2), py = threadIdx.x / (FPX / 2);
-    const int x = job.y * FPX + 2 * px, y = job.z * FPY + py;
+    const int x = tile.x * FPX + 2 * px, y = tile.y * FPY + py;
     if (x >= s.w || y >= s.h) {
         return;
     }
@@ -397,28 +426,31 @@ constexpr int kBatchReduceSmem = ReduceSmem<3, true>::WORDS * 4;
 
 // Image jobs (kind < K) and mask jobs (kind >= K) of a level run as two
 // launches, each with the registers its path needs.
-template <int C>
-__global__ void __launch_bounds__(RTHREADS, 3) k_batch_reduce(const BatchStack* __restrict__ stacks,
-                                                              const int4* __restrict__ jobs, int l, int wrap)
+template <int C, class J>
+__global__ void __launch_bounds__(RTHREADS, 3) k_batch_reduce(const __grid_constant__ J jobs, int l, int wrap)
 {
     __shared__ __align__(16) unsigned char smem[kBatchReduceSmem];
-    const int4 job = jobs[blockIdx.x];
-    batch_reduce_tile<C, true>(stacks[job.x], job.y, l, job.z * RDW, job.w * RDH, wrap, smem);
+    griddep_wait();
+    griddep_launch();
+    const int2 tile = jobs.reduce_tile();
+    batch_reduce_tile<C, true>(jobs.stack(), jobs.reduce_kind(), l, tile.x * RDW, tile.y * RDH, wrap, smem);
 }
 
-__global__ void __launch_bounds__(RTHREADS, 4) k_batch_reduce_mask(const BatchStack* __restrict__ stacks,
-                                                                   const int4* __restrict__ jobs, int l, int wrap)
+template <class J>
+__global__ void __launch_bounds__(RTHREADS, 4) k_batch_reduce_mask(const __grid_constant__ J jobs, int l, int wrap)
 {
     __shared__ __align__(16) int32_t V[ReduceSmem<1, true>::NV][RDH][RVP];
-    const int4 job = jobs[blockIdx.x];
-    const BatchStack& s = stacks[job.x];
-    const int k = job.y - s.K;
+    griddep_wait();
+    griddep_launch();
+    const int2 tile = jobs.reduce_tile();
+    const BatchStack& s = jobs.stack();
+    const int k = jobs.reduce_kind() - s.K;
     const int sw = s.lw[l], sh = s.lh[l], dw = s.lw[l + 1], dh = s.lh[l + 1];
     using Src = PlanarSource<int32_t, 1, true, true>;
     const ReduceJob<Src, int32_t> rj{
         Src{m_level(s, k, l), s.pitch[l], (int64_t)s.pitch[l] * sh, s.u + s.off0[l], s.pitch[l]}, m_level(s, k, l + 1),
         s.pitch[l + 1], (int64_t)s.pitch[l + 1] * dh, s.u + s.off0[l + 1], s.pitch[l + 1]};
-    reduce_tile<Src, int32_t, 1, true, int32_t>(rj, job.z * RDW, job.w * RDH, sw, sh, dw, dh, wrap, V);
+    reduce_tile<Src, int32_t, 1, true, int32_t>(rj, tile.x * RDW, tile.y * RDH, sw, sh, dw, dh, wrap, V);
 }
 
 // ---------------------------------------------------------------------------
@@ -437,16 +469,12 @@ __device__ __forceinline__ void expand_quad_f(const float (*ss)[ESH][ESW], int q
     if (i >= 1 && i + 1 < sw && j >= 1 && j + 1 < sh) {
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            const float* a = &ss[c][qy][qx];
-            const float* b = &ss[c][qy + 1][qx];
-            const float* d = &ss[c][qy + 2][qx];
-            const float hea = a[0] + 6.0f * a[1] + a[2], heb = b[0] + 6.0f * b[1] + b[2],
-                        hec = d[0] + 6.0f * d[1] + d[2];
-            const float hoa = 4.0f * (a[1] + a[2]), hob = 4.0f * (b[1] + b[2]), hoc = 4.0f * (d[1] + d[2]);
-            e[0][c] = (hea + 6.0f * heb + hec) * 0.015625f;
-            e[1][c] = (hoa + 6.0f * hob + hoc) * 0.015625f;
-            e[2][c] = (heb + hec) * 0.0625f;
-            e[3][c] = (hob + hoc) * 0.0625f;
+            float v[4];
+            expand9_f(&ss[c][qy][qx], &ss[c][qy + 1][qx], &ss[c][qy + 2][qx], v);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                e[q][c] = v[q];
+            }
         }
         return;
     }
@@ -459,13 +487,7 @@ __device__ __forceinline__ void expand_quad_f(const float (*ss)[ESH][ESW], int q
         const float den = (float)(hden * vden);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            float num = 0.0f;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float* row = &ss[c][qy + a][qx];
-                num += (float)vw[a] * ((float)hw[0] * row[0] + (float)hw[1] * row[1] + (float)hw[2] * row[2]);
-            }
-            e[q][c] = __fdiv_rn(num, den);
+            e[q][c] = expand_border_f(&ss[c][qy][qx], &ss[c][qy + 1][qx], &ss[c][qy + 2][qx], vw, hw, den);
         }
     }
 }
@@ -694,19 +716,21 @@ __host__ __device__ constexpr int up0_stage_floats()
 // Level l of a stack (one 64x16 tile, 2x2 quads): level 0 converts the
 // result into the output pixels, levels >= 1 write the result level
 // (batch_up_tile's computation with the tiles streamed through the stages).
-template <int C, bool L0>
-__global__ void __launch_bounds__(256, 3) k_batch_up0(const BatchStack* __restrict__ stacks,
-                                                     const int4* __restrict__ jobs, int l, int wrap, float inv_d)
+// One stack's launch waits for its predecessor, which wrote C[l+1], only
+// after the exposures' sum: everything else is older (each launch of the
+// chain waits before it lets the next one start).
+template <int C, bool L0, class J>
+__global__ void __launch_bounds__(256, 3) k_batch_up0(const __grid_constant__ J jobs, int l, int wrap, float inv_d)
 {
     extern __shared__ __align__(16) float up0smem[];
-    const int4 job = jobs[blockIdx.x];
-    const BatchStack& s = stacks[job.x];
+    const int2 tile = jobs.tile();
+    const BatchStack& s = jobs.stack();
     if (L0) {
         l = 0;
     }
     const int K = s.K;
     const bool top = l == s.L - 1;
-    const int X0 = job.y * ETW, Y0 = job.z * ETH;
+    const int X0 = tile.x * ETW, Y0 = tile.y * ETH;
     const int dw = s.lw[l], dh = s.lh[l];
     const int sw = top ? 1 : s.lw[l + 1], sh = top ? 1 : s.lh[l + 1];
     const int I0 = X0 >> 1, J0 = Y0 >> 1;
@@ -726,8 +750,12 @@ __global__ void __launch_bounds__(256, 3) k_batch_up0(const BatchStack* __restri
         }
         up0_issue<C>(s, k, l, X0, Y0, dw, dh, g_tile(b), mask_tile(b));
     };
+    if (J::kOne && top) {
+        griddep_wait();  // the reduces that wrote this level
+        griddep_launch();
+    }
     // exposures 0 and 1 (with the window of C[1]) in flight before the first merge
-    if (!top) {
+    if (!top && !J::kOne) {
         stage_window_async<C>(rwin, r_level(s, l + 1, C), sp, splane, sw, sh, I0, J0, wrap);
     }
     issue(0);
@@ -779,6 +807,14 @@ __global__ void __launch_bounds__(256, 3) k_batch_up0(const BatchStack* __restri
             }
         }
         __syncthreads();  // this stage is refilled for exposure k + 3
+    }
+    if (J::kOne && !top) {
+        griddep_wait();
+        griddep_launch();
+        stage_window_async<C>(rwin, r_level(s, l + 1, C), sp, splane, sw, sh, I0, J0, wrap);
+        cp_async_commit();
+        cp_async_wait_all();
+        __syncthreads();
     }
     if (!active) {
         return;
@@ -963,6 +999,80 @@ void level_geometry(BatchStack& s, int64_t coarse_pixels)
 
 }  // namespace
 
+// Sizes, levels and buffers of a stack's images and output.
+static BatchStack stack_of(const BatchStackHost& h, int levels, int64_t coarse_pixels)
+{
+    BatchStack s;
+    std::memset(&s, 0, sizeof s);
+    s.K = h.K;
+    s.w = h.w;
+    s.h = h.h;
+    s.L = enb_num_levels(h.w, h.h, 1, levels);
+    for (int k = 0; k < h.K; ++k) {
+        s.img[k] = h.img[k];
+        s.ipitch[k] = h.ipitch[k];
+        s.istride[k] = h.istride[k];
+        s.alpha[k] = h.alpha[k];
+        s.apitch[k] = h.apitch[k];
+    }
+    s.out = h.out;
+    s.opitch = h.opitch;
+    s.ostride = h.ostride;
+    s.oalpha = h.oalpha;
+    s.oapitch = h.oapitch;
+    level_geometry(s, coarse_pixels);
+    return s;
+}
+
+static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+// Bytes of a stack's workspace, and the workspace's division.
+static size_t stack_bytes(const BatchStack& s, int C)
+{
+    return align256((size_t)s.K * s.s0 * 4) + align256((size_t)s.s0) + align256((size_t)s.K * C * s.s1 * 4) +
+           align256((size_t)s.K * s.s1) + align256((size_t)C * s.s1 * 4) + align256((size_t)s.K * C * s.s0 * 4);
+}
+
+static void stack_buffers(BatchStack& s, int C, char* q)
+{
+    s.m = (int32_t*)q;
+    q += align256((size_t)s.K * s.s0 * 4);
+    s.u = (uint8_t*)q;
+    q += align256((size_t)s.s0);
+    s.g = (float*)q;
+    q += align256((size_t)s.K * C * s.s1 * 4);
+    s.a = (uint8_t*)q;
+    q += align256((size_t)s.K * s.s1);
+    s.r = (float*)q;
+    q += align256((size_t)C * s.s1 * 4);
+    s.g0 = (float*)q;
+}
+
+// The weights step's kernel family, tile, hash slots and shared memory.
+struct WeightsStep {
+    bool pair;
+    int tx, ty, slots;
+    size_t smem;
+    WeightsStep(const FloatWeightParams& wp, int maxK)
+    {
+        pair = fpair_path(wp);
+        if (pair) {
+            const int cw = wp.use_contrast ? wp.contrast_window : 0, ew = wp.use_entropy ? wp.entropy_window : 0;
+            const int TT = fpair_tw(cw, ew) * fpair_th(cw, ew);
+            slots = fpair_slots(wp, TT);
+            smem = fpair_tile_bytes(TT, slots, wp.ent_cut);
+            tx = FPX;
+            ty = FPY;
+        } else {
+            // the tile, then the K weights of each output pixel
+            const int TW = BWT + 2 * fweight_halo(wp);
+            slots = fweight_slots(wp, TW);
+            smem = align16(ftile_bytes(TW, slots, wp.ent_cut)) + (size_t)maxK * BWT * BWT * sizeof(float);
+            tx = ty = BWT;
+        }
+    }
+};
+
 void batch_plan_destroy(BatchPlan* p)
 {
     if (!p) {
@@ -987,32 +1097,12 @@ cudaError_t batch_plan_create(const std::vector<BatchStackHost>& hs, const Float
     p->coarse_pixels = coarse_pixels;
     std::vector<BatchStack> stacks(hs.size());
     size_t bytes = 0;
-    auto align = [](size_t v) { return (v + 255) & ~(size_t)255; };
     std::vector<size_t> base(hs.size());
     for (size_t i = 0; i < hs.size(); ++i) {
-        BatchStack& s = stacks[i];
-        std::memset(&s, 0, sizeof s);
         const BatchStackHost& h = hs[i];
-        s.K = h.K;
-        s.w = h.w;
-        s.h = h.h;
-        s.L = enb_num_levels(h.w, h.h, 1, levels);
-        for (int k = 0; k < h.K; ++k) {
-            s.img[k] = h.img[k];
-            s.ipitch[k] = h.ipitch[k];
-            s.istride[k] = h.istride[k];
-            s.alpha[k] = h.alpha[k];
-            s.apitch[k] = h.apitch[k];
-        }
-        s.out = h.out;
-        s.opitch = h.opitch;
-        s.ostride = h.ostride;
-        s.oalpha = h.oalpha;
-        s.oapitch = h.oapitch;
-        level_geometry(s, coarse_pixels);
+        stacks[i] = stack_of(h, levels, coarse_pixels);
         base[i] = bytes;
-        bytes += align((size_t)s.K * s.s0 * 4) + align((size_t)s.s0) + align((size_t)s.K * p->C * s.s1 * 4) +
-                 align((size_t)s.K * s.s1) + align((size_t)p->C * s.s1 * 4) + align((size_t)s.K * p->C * s.s0 * 4);
+        bytes += stack_bytes(stacks[i], p->C);
         p->pixels += (double)h.K * h.w * h.h;
         p->maxK = std::max(p->maxK, h.K);
     }
@@ -1022,21 +1112,11 @@ cudaError_t batch_plan_create(const std::vector<BatchStackHost>& hs, const Float
         p->steps.push_back(BatchPlan::Step{kind, level, 0, 0, b});
         p->steps.back().job0 = (int64_t)jobs.size();
     };
-    // the tile, then the K weights of each output pixel
-    p->pair_weights = fpair_path(wp);
-    int wtx = BWT, wty = BWT;
-    if (p->pair_weights) {
-        const int cw = wp.use_contrast ? wp.contrast_window : 0, ew = wp.use_entropy ? wp.entropy_window : 0;
-        const int TT = fpair_tw(cw, ew) * fpair_th(cw, ew);
-        p->wp.repeat_slots = fpair_slots(wp, TT);
-        p->wsmem = fpair_tile_bytes(TT, p->wp.repeat_slots, p->wp.ent_cut);
-        wtx = FPX;
-        wty = FPY;
-    } else {
-        const int TW = BWT + 2 * fweight_halo(wp);
-        p->wp.repeat_slots = fweight_slots(wp, TW);
-        p->wsmem = align16(ftile_bytes(TW, p->wp.repeat_slots, p->wp.ent_cut)) + (size_t)p->maxK * BWT * BWT * sizeof(float);
-    }
+    const WeightsStep ws(wp, p->maxK);
+    p->pair_weights = ws.pair;
+    p->wp.repeat_slots = ws.slots;
+    p->wsmem = ws.smem;
+    const int wtx = ws.tx, wty = ws.ty;
     double b = 0.0;
     add_step(0, 0, 0.0);
     for (int i = 0; i < p->nstacks; ++i) {
@@ -1201,10 +1281,10 @@ cudaError_t batch_plan_create(const std::vector<BatchStackHost>& hs, const Float
         }
     }
     // device memory: workspace, stack table, jobs, coarse list, queue counter
-    const size_t o_st = align(bytes), o_jobs = o_st + align(sizeof(BatchStack) * stacks.size()),
-                 o_coarse = o_jobs + align(sizeof(int4) * std::max<size_t>(jobs.size(), 1)),
-                 o_queue = o_coarse + align(sizeof(CoarseItem) * std::max<size_t>(items.size(), 1)),
-                 total = o_queue + align(sizeof(int) * (size_t)(1 + p->nctrs));
+    const size_t o_st = align256(bytes), o_jobs = o_st + align256(sizeof(BatchStack) * stacks.size()),
+                 o_coarse = o_jobs + align256(sizeof(int4) * std::max<size_t>(jobs.size(), 1)),
+                 o_queue = o_coarse + align256(sizeof(CoarseItem) * std::max<size_t>(items.size(), 1)),
+                 total = o_queue + align256(sizeof(int) * (size_t)(1 + p->nctrs));
     cudaError_t e = cudaMalloc(&p->work, total);
     if (e != cudaSuccess) {
         delete p;
@@ -1212,19 +1292,7 @@ cudaError_t batch_plan_create(const std::vector<BatchStackHost>& hs, const Float
     }
     char* w = (char*)p->work;
     for (size_t i = 0; i < stacks.size(); ++i) {
-        BatchStack& s = stacks[i];
-        char* q = w + base[i];
-        s.m = (int32_t*)q;
-        q += align((size_t)s.K * s.s0 * 4);
-        s.u = (uint8_t*)q;
-        q += align((size_t)s.s0);
-        s.g = (float*)q;
-        q += align((size_t)s.K * p->C * s.s1 * 4);
-        s.a = (uint8_t*)q;
-        q += align((size_t)s.K * s.s1);
-        s.r = (float*)q;
-        q += align((size_t)p->C * s.s1 * 4);
-        s.g0 = (float*)q;
+        stack_buffers(stacks[i], p->C, w + base[i]);
     }
     p->dstacks = (BatchStack*)(w + o_st);
     p->djobs = (int4*)(w + o_jobs);
@@ -1254,58 +1322,81 @@ double batch_plan_pixels(const BatchPlan* p) { return p->pixels; }
 // Shared memory of an up tile: the windows of K exposures and of C[l+1].
 static size_t up_smem_bytes(int K, int C) { return (size_t)(K + 1) * C * ESH * ESW * sizeof(float); }
 
+// Launch of one step's kernel: plain for the tables of a batch, dependent for
+// one stack.
+template <class J, typename... KArgs, typename... Args>
+static cudaError_t launch_batch(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, Args&&... args)
+{
+    if (smem > 48 * 1024) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    }
+    if (J::kOne) {
+        return launch_pdl_smem(kernel, grid, dim3(block), smem, st, std::forward<Args>(args)...);
+    }
+    kernel<<<grid, block, smem, st>>>(std::forward<Args>(args)...);
+    return cudaGetLastError();
+}
+
+template <int C, class J>
+static cudaError_t launch_weights(const J& jobs, dim3 grid, bool pair, const FloatWeightParams& wp, const WeightTables& tab,
+                                  int hard, size_t smem, cudaStream_t st)
+{
+    cudaError_t e = cudaErrorInvalidValue;
+    if (pair) {
+        ENB_FPAIR_DISPATCH(wp, {
+            auto k = k_batch_weights_pair<CWV, EWV, C, J>;
+            // as many CTAs per SM as the shared memory holds
+            cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+            e = launch_batch<J>(k, grid, FPT, smem, st, jobs, wp, tab);
+        });
+        return e;
+    }
+    const int cw = wp.use_contrast ? wp.contrast_window : 5;
+    const int ew = wp.use_entropy ? wp.entropy_window : 5;
+    void (*k)(const J, FloatWeightParams, WeightTables, int, int) = k_batch_weights<0, 0, J>;
+    if (cw == 5 && ew == 5) {
+        k = k_batch_weights<5, 5, J>;
+    } else if (cw == 5 && ew == 3) {
+        k = k_batch_weights<5, 3, J>;
+    } else if (cw == 3 && ew == 3) {
+        k = k_batch_weights<3, 3, J>;
+    } else if (ew == 5) {
+        k = k_batch_weights<0, 5, J>;
+    } else if (ew == 3) {
+        k = k_batch_weights<0, 3, J>;
+    }
+    return launch_batch<J>(k, grid, BWT * BWT, smem, st, jobs, wp, tab, hard, C);
+}
+
+template <int C, class J>
+static cudaError_t launch_up(const J& jobs, dim3 grid, int l, int wrap, cudaStream_t st)
+{
+    const float inv_d = (float)(1.0 / (double)(255 << 15));
+    const size_t smem = ((size_t)kUp0Stages * up0_stage_floats<C>() + (size_t)C * ESH * ESW) * sizeof(float);
+    if (l == 0) {
+        return launch_batch<J>(k_batch_up0<C, true, J>, grid, 256, smem, st, jobs, 0, wrap, inv_d);
+    }
+    return launch_batch<J>(k_batch_up0<C, false, J>, grid, 256, smem, st, jobs, l, wrap, inv_d);
+}
+
 template <int C>
 static cudaError_t launch_step(const BatchPlan* p, const BatchPlan::Step& s, cudaStream_t st)
 {
-    const int4* jobs = p->djobs + s.job0;
-    const float inv_d = (float)(1.0 / (double)(255 << 15));
+    const BatchTable jobs{p->dstacks, p->djobs + s.job0};
+    const dim3 grid((unsigned)s.njobs);
     switch (s.kind) {
-    case 0: {
+    case 0:
         note_launch("batch_weights", s.bytes);
-        if (p->pair_weights) {
-            ENB_FPAIR_DISPATCH(p->wp, {
-                auto k = k_batch_weights_pair<CWV, EWV, C>;
-                if (p->wsmem > 48 * 1024) {
-                    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->wsmem);
-                }
-                // as many CTAs per SM as the shared memory holds
-                cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-                k<<<(unsigned)s.njobs, FPT, p->wsmem, st>>>(p->dstacks, jobs, p->wp, p->tab, p->hard);
-            });
-            break;
-        }
-        const int cw = p->wp.use_contrast ? p->wp.contrast_window : 5;
-        const int ew = p->wp.use_entropy ? p->wp.entropy_window : 5;
-        void (*k)(const BatchStack*, const int4*, FloatWeightParams, WeightTables, int, int) = k_batch_weights<0, 0>;
-        if (cw == 5 && ew == 5) {
-            k = k_batch_weights<5, 5>;
-        } else if (cw == 5 && ew == 3) {
-            k = k_batch_weights<5, 3>;
-        } else if (cw == 3 && ew == 3) {
-            k = k_batch_weights<3, 3>;
-        } else if (ew == 5) {
-            k = k_batch_weights<0, 5>;
-        } else if (ew == 3) {
-            k = k_batch_weights<0, 3>;
-        }
-        if (p->wsmem > 48 * 1024) {
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->wsmem);
-        }
-        k<<<(unsigned)s.njobs, BWT * BWT, p->wsmem, st>>>(p->dstacks, jobs, p->wp, p->tab, p->hard, C);
-        break;
-    }
+        return launch_weights<C>(jobs, grid, p->pair_weights, p->wp, p->tab, p->hard, p->wsmem, st);
     case 5:
         note_launch("batch_normalise", s.bytes);
-        k_batch_normalise<<<(unsigned)s.njobs, 256, 0, st>>>(p->dstacks, jobs, p->hard);
-        break;
+        return launch_batch<BatchTable>(k_batch_normalise<BatchTable>, grid, 256, 0, st, jobs, p->hard);
     case 1:
         note_launch("batch_reduce", s.bytes);
-        k_batch_reduce<C><<<(unsigned)s.njobs, RTHREADS, 0, st>>>(p->dstacks, jobs, s.level, p->wrap);
-        break;
+        return launch_batch<BatchTable>(k_batch_reduce<C, BatchTable>, grid, RTHREADS, 0, st, jobs, s.level, p->wrap);
     case 4:
         note_launch("batch_reduce_mask", s.bytes);
-        k_batch_reduce_mask<<<(unsigned)s.njobs, RTHREADS, 0, st>>>(p->dstacks, jobs, s.level, p->wrap);
-        break;
+        return launch_batch<BatchTable>(k_batch_reduce_mask<BatchTable>, grid, RTHREADS, 0, st, jobs, s.level, p->wrap);
     case 2: {
         note_launch("batch_coarse", 0.0);
         // the queue position and the step counters start at 0 on every run
@@ -1316,40 +1407,123 @@ static cudaError_t launch_step(const BatchPlan* p, const BatchPlan::Step& s, cud
         int sms = 0, dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int grid = std::max(1, std::min(p->nitems, 2 * sms));
+        const int grid2 = std::max(1, std::min(p->nitems, 2 * sms));
         const size_t smem = std::max((size_t)kBatchReduceSmem, up_smem_bytes(p->maxK, C));
-        if (smem > 48 * 1024) {
-            cudaFuncSetAttribute(k_batch_coarse<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        }
-        k_batch_coarse<C><<<grid, RTHREADS, smem, st>>>(p->dstacks, p->ditems, p->nitems, p->dqueue, p->dqueue + 1,
-                                                        p->err, p->wrap, inv_d);
-        break;
+        const float inv_d = (float)(1.0 / (double)(255 << 15));
+        return launch_batch<BatchTable>(k_batch_coarse<C>, dim3((unsigned)grid2), RTHREADS, smem, st,
+                                        (const BatchStack*)p->dstacks, (const CoarseItem*)p->ditems, p->nitems, p->dqueue,
+                                        p->dqueue + 1, p->err, p->wrap, inv_d);
     }
-    default: {
+    default:
         note_launch(s.level == 0 ? "batch_up0" : "batch_up", s.bytes);
-        if (s.level == 0) {
-            const size_t smem = ((size_t)kUp0Stages * up0_stage_floats<C>() + (size_t)C * ESH * ESW) * sizeof(float);
-            if (smem > 48 * 1024) {
-                cudaFuncSetAttribute(k_batch_up0<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            }
-            k_batch_up0<C, true><<<(unsigned)s.njobs, 256, smem, st>>>(p->dstacks, jobs, 0, p->wrap, inv_d);
-            break;
-        }
-        const size_t smem = ((size_t)kUp0Stages * up0_stage_floats<C>() + (size_t)C * ESH * ESW) * sizeof(float);
-        if (smem > 48 * 1024) {
-            cudaFuncSetAttribute(k_batch_up0<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        }
-        k_batch_up0<C, false><<<(unsigned)s.njobs, 256, smem, st>>>(p->dstacks, jobs, s.level, p->wrap, inv_d);
-        break;
+        return launch_up<C>(jobs, grid, s.level, p->wrap, st);
     }
-    }
-    return cudaGetLastError();
 }
 
 cudaError_t batch_plan_launch(const BatchPlan* p, int i, cudaStream_t st)
 {
     const BatchPlan::Step& s = p->steps[(size_t)i];
     return p->C == 1 ? launch_step<1>(p, s, st) : launch_step<3>(p, s, st);
+}
+
+// ---------------------------------------------------------------------------
+// one stack (enb_enfuse on float images)
+// ---------------------------------------------------------------------------
+//
+// The launches of a batch of one, without its tables, graph and plan: the
+// stack goes in the kernels' parameters.  Steps in order: the weights, their
+// normalisation (pair kernel only), per level the image and the mask reduces
+// (one launch where both fit the GPU at once), the merges from the top level
+// down to the output.
+
+struct BatchSingle {
+    BatchStack s;
+    int C, wrap, hard;
+    FloatWeightParams wp;
+    WeightTables tab;
+    WeightsStep ws;
+    struct Step {
+        int kind, level;  // 0 weights, 1 normalisation, 2 image reduce, 3 mask reduce, 4 both, 5 merge
+    };
+    std::vector<Step> steps;
+};
+
+// A launch of at most this many reduce tiles takes the image and the mask
+// pyramids of a level together: two CTAs an SM, so the level is one wave
+// either way and a launch is saved.
+constexpr int kJointReduceTiles = 304;
+
+BatchSingle* batch_single_create(const BatchStackHost& h, const FloatWeightParams& wp, const WeightTables& tab, int levels,
+                                 int wrap, int hard)
+{
+    BatchSingle* p = new BatchSingle{stack_of(h, levels, 0), h.C, wrap, hard, wp, tab, WeightsStep(wp, h.K), {}};
+    const BatchStack& s = p->s;
+    p->wp.repeat_slots = p->ws.slots;
+    p->steps.push_back({0, 0});
+    if (p->ws.pair) {
+        p->steps.push_back({1, 0});
+    }
+    for (int l = 0; l + 1 < s.L; ++l) {
+        const int64_t tiles = (int64_t)((s.lw[l + 1] + RDW - 1) / RDW) * ((s.lh[l + 1] + RDH - 1) / RDH);
+        if (2 * s.K * tiles <= kJointReduceTiles) {
+            p->steps.push_back({4, l});
+        } else {
+            p->steps.push_back({2, l});
+            p->steps.push_back({3, l});
+        }
+    }
+    for (int l = s.L - 1; l >= 0; --l) {
+        p->steps.push_back({5, l});
+    }
+    return p;
+}
+
+void batch_single_destroy(BatchSingle* p) { delete p; }
+size_t batch_single_bytes(const BatchSingle* p) { return stack_bytes(p->s, p->C); }
+void batch_single_workspace(BatchSingle* p, void* work) { stack_buffers(p->s, p->C, (char*)work); }
+int batch_single_steps(const BatchSingle* p) { return (int)p->steps.size(); }
+
+template <int C>
+static cudaError_t single_step(const BatchSingle* p, int i, cudaStream_t st)
+{
+    const BatchStack& s = p->s;
+    const int l = p->steps[(size_t)i].level, K = s.K;
+    const double px = (double)s.lw[l] * s.lh[l], up = l + 1 < s.L ? (double)s.lw[l + 1] * s.lh[l + 1] : 0.0;
+    const auto tiles = [](int w, int h, int tx, int ty, int z) {
+        return dim3((unsigned)((w + tx - 1) / tx), (unsigned)((h + ty - 1) / ty), (unsigned)z);
+    };
+    BatchOne jobs{s, 0};
+    const double img = K * (px * (4.0 * C + (l == 0 ? 0.0 : 1.0)) + up * (4.0 * C + 1.0)), msk = K * (px + up) * 4.0 + px + up;
+    switch (p->steps[(size_t)i].kind) {
+    case 0:
+        note_launch("batch_weights", K * px * (4.0 * s.istride[0] + 4.0 * C + 4.0) + px);
+        return launch_weights<C>(jobs, tiles(s.w, s.h, p->ws.tx, p->ws.ty, 1), p->ws.pair, p->wp, p->tab, p->hard, p->ws.smem, st);
+    case 1:
+        note_launch("batch_normalise", K * px * 12.0);
+        return launch_batch<BatchOne>(k_batch_normalise<BatchOne>, tiles(s.w, s.h, FPX, FPY, 1), 256, 0, st, jobs, p->hard);
+    case 2:
+        note_launch("batch_reduce", img);
+        return launch_batch<BatchOne>(k_batch_reduce<C, BatchOne>, tiles(s.lw[l + 1], s.lh[l + 1], RDW, RDH, K), RTHREADS, 0, st,
+                                      jobs, l, p->wrap);
+    case 3:
+        note_launch("batch_reduce_mask", msk);
+        jobs.kind0 = K;
+        return launch_batch<BatchOne>(k_batch_reduce_mask<BatchOne>, tiles(s.lw[l + 1], s.lh[l + 1], RDW, RDH, K), RTHREADS, 0, st,
+                                      jobs, l, p->wrap);
+    case 4:
+        note_launch("batch_reduce", img + msk);
+        return launch_batch<BatchOne>(k_batch_reduce<C, BatchOne>, tiles(s.lw[l + 1], s.lh[l + 1], RDW, RDH, 2 * K), RTHREADS, 0, st,
+                                      jobs, l, p->wrap);
+    default:
+        note_launch(l == 0 ? "batch_up0" : "batch_up",
+                    K * (px * (4.0 * C + 4.0) + up * 4.0 * C) + up * 4.0 * C + px * (l == 0 ? 4.0 * s.ostride + 1.0 : 4.0 * C));
+        return launch_up<C>(jobs, tiles(s.lw[l], s.lh[l], ETW, ETH, 1), l, p->wrap, st);
+    }
+}
+
+cudaError_t batch_single_launch(const BatchSingle* p, int i, cudaStream_t st)
+{
+    return p->C == 1 ? single_step<1>(p, i, st) : single_step<3>(p, i, st);
 }
 
 }  // namespace enb

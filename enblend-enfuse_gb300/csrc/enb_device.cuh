@@ -236,6 +236,32 @@ __device__ __forceinline__ void expand_vweights(int Y, int sh, int w[3], int& de
     den = w[0] + w[1] + w[2];
 }
 
+// The float expand (src/pyramid.h:875-1457, real division) of a 2x2 quad from
+// its 3x3 source neighbourhood, rows a, b, d of three samples each, inside
+// the level (the divisors 64 and 16 are powers of two), and of one pixel with
+// the border weights.  Every operation's rounding is spelled out: the
+// per-operation and the fused passes expand to the same bits.
+__device__ __forceinline__ void expand9_f(const float* a, const float* b, const float* d, float (&e)[4])
+{
+    const float hea = __fadd_rn(__fmaf_rn(6.0f, a[1], a[0]), a[2]), heb = __fadd_rn(__fmaf_rn(6.0f, b[1], b[0]), b[2]),
+                hec = __fadd_rn(__fmaf_rn(6.0f, d[1], d[0]), d[2]);
+    const float hoa = 4.0f * __fadd_rn(a[1], a[2]), hob = 4.0f * __fadd_rn(b[1], b[2]), hoc = 4.0f * __fadd_rn(d[1], d[2]);
+    e[0] = __fadd_rn(__fmaf_rn(6.0f, heb, hea), hec) * 0.015625f;
+    e[1] = __fadd_rn(__fmaf_rn(6.0f, hob, hoa), hoc) * 0.015625f;
+    e[2] = __fadd_rn(heb, hec) * 0.0625f;
+    e[3] = __fadd_rn(hob, hoc) * 0.0625f;
+}
+
+__device__ __forceinline__ float expand_border_f(const float* a, const float* b, const float* d, const int (&vw)[3],
+                                                 const int (&hw)[3], float den)
+{
+    const auto row = [&](const float* r) {
+        return __fmaf_rn((float)hw[2], r[2], __fmaf_rn((float)hw[1], r[1], __fmul_rn((float)hw[0], r[0])));
+    };
+    const float num = __fmaf_rn((float)vw[2], row(d), __fmaf_rn((float)vw[1], row(b), __fmul_rn((float)vw[0], row(a))));
+    return __fdiv_rn(num, den);
+}
+
 // Truncating division by a divisor d in [1, 256] known only at run time, as a
 // multiplication (division by invariant integers, Granlund & Montgomery
 // 1994): with l = ceil(log2 d) and m = floor(2^(31+l) / d) + 1 < 2^32,

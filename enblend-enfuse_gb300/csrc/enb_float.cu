@@ -112,23 +112,18 @@ __global__ void __launch_bounds__(256) k_f_expand(const float* __restrict__ src,
     if (interior) {
 #pragma unroll
         for (int ch = 0; ch < C; ++ch) {
-            const float* a = &ss[ch][qy][qx];
-            const float* b = &ss[ch][qy + 1][qx];
-            const float* c = &ss[ch][qy + 2][qx];
-            const float hea = a[0] + 6.0f * a[1] + a[2], heb = b[0] + 6.0f * b[1] + b[2],
-                        hec = c[0] + 6.0f * c[1] + c[2];
-            const float hoa = 4.0f * (a[1] + a[2]), hob = 4.0f * (b[1] + b[2]), hoc = 4.0f * (c[1] + c[2]);
+            float e[4];
+            expand9_f(&ss[ch][qy][qx], &ss[ch][qy + 1][qx], &ss[ch][qy + 2][qx], e);
             float* d0 = dst + (int64_t)ch * dplane + (int64_t)Y * dpitch + X;
-            // divisors 64 and 16 are powers of two: the products are exact divisions
-            f_combine<ADD>(d0, (hea + 6.0f * heb + hec) * 0.015625f);
+            f_combine<ADD>(d0, e[0]);
             if (has_x1) {
-                f_combine<ADD>(d0 + 1, (hoa + 6.0f * hob + hoc) * 0.015625f);
+                f_combine<ADD>(d0 + 1, e[1]);
             }
             if (has_y1) {
                 float* d1 = d0 + dpitch;
-                f_combine<ADD>(d1, (heb + hec) * 0.0625f);
+                f_combine<ADD>(d1, e[2]);
                 if (has_x1) {
-                    f_combine<ADD>(d1 + 1, (hob + hoc) * 0.0625f);
+                    f_combine<ADD>(d1 + 1, e[3]);
                 }
             }
         }
@@ -154,13 +149,8 @@ __global__ void __launch_bounds__(256) k_f_expand(const float* __restrict__ src,
             const float den = (float)(hden * vden);
 #pragma unroll
             for (int ch = 0; ch < C; ++ch) {
-                float num = 0.0f;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const float* row = &ss[ch][qy + a][qx];
-                    num += (float)vw[a] * ((float)hw[0] * row[0] + (float)hw[1] * row[1] + (float)hw[2] * row[2]);
-                }
-                f_combine<ADD>(dst + (int64_t)ch * dplane + (int64_t)YY * dpitch + XX, __fdiv_rn(num, den));
+                f_combine<ADD>(dst + (int64_t)ch * dplane + (int64_t)YY * dpitch + XX,
+                               expand_border_f(&ss[ch][qy][qx], &ss[ch][qy + 1][qx], &ss[ch][qy + 2][qx], vw, hw, den));
             }
         }
     }

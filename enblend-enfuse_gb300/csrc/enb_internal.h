@@ -333,6 +333,17 @@ int batch_plan_steps(const BatchPlan* p);
 double batch_plan_pixels(const BatchPlan* p);
 cudaError_t batch_plan_launch(const BatchPlan* p, int step, cudaStream_t st);
 
+// one float stack through the batch's kernels (enb_enfuse): its workspace of
+// batch_single_bytes goes in before the steps are launched in order
+struct BatchSingle;
+BatchSingle* batch_single_create(const BatchStackHost& h, const FloatWeightParams& wp, const WeightTables& tab, int levels,
+                                 int wrap, int hard);
+void batch_single_destroy(BatchSingle* p);
+size_t batch_single_bytes(const BatchSingle* p);
+void batch_single_workspace(BatchSingle* p, void* work);
+int batch_single_steps(const BatchSingle* p);
+cudaError_t batch_single_launch(const BatchSingle* p, int step, cudaStream_t st);
+
 // nearest-feature seam mask (enb_nft.cu): scratch bytes for a w x h
 // canvas, and the three stages (0 columns and tallies, 1 rows, 2 mask)
 size_t nft_scratch_bytes(int w, int h, int wrap);

@@ -365,7 +365,7 @@ typedef struct {
  * is replayed as a CUDA graph.  Each stack's result is that of enb_enfuse on
  * it (same FP32 arithmetic up to the order of float additions).  masks are
  * computed (no --load-masks); opt->plain = 1 runs enb_enfuse stack by stack
- * instead (for comparisons).  The workspace and graph of the last batch
+ * instead, one kernel per operation (for comparisons).  The workspace and graph of the last batch
  * geometry stay cached in the context. */
 enb_status enb_fuse_stacks(enb_ctx* ctx, const enb_enfuse_params* params, int n_stacks, const enb_stack* stacks,
                            const enb_fuse_options* opt);

@@ -341,3 +341,37 @@ def test_enblend_f32(ctx, orc, wrap, stride):
     assert np.array_equal(oa.cpu().numpy(), ref["alpha"])
     _close(l0.cpu().numpy().astype(np.float64), ref["level0"], 1e-5, 1e-6, "level 0")
     _close(out.cpu().numpy().astype(np.float64), ref["out"].astype(np.float64), 1e-5, 1e-6, "pixels")
+
+
+@pytest.mark.parametrize("h,w,K,chans,kw,opt", [
+    (65, 64, 2, 3, {}, {}), (33, 131, 5, 3, {}, {"wrap": True}), (130, 67, 16, 3, {}, {"hard_mask": True}),
+    (9, 40, 3, 3, {}, {}), (7, 9, 3, 3, {}, {}), (300, 411, 4, 3, {"contrast_window_size": 7}, {"levels": 2}),
+    (48, 90, 3, 3, {"entropy_window_size": 7}, {"wrap": True}), (75, 97, 4, 4, {}, {}), (75, 98, 4, 1, {}, {"wrap": True}),
+    (600, 900, 7, 3, {}, {})])
+def test_enfuse_f32_level_passes_equal_single_operations(ctx, h, w, K, chans, kw, opt):
+    """enb_enfuse of float images through the launches of a batch of one, against one kernel per operation: the same
+    bits for RGB, RGBA (alpha from the 4th component) and gray, alpha planes, odd and periodic levels, one level,
+    window sizes inside and outside the pair kernel, several exposures, device rows off any alignment."""
+    import enbgpu
+    rng = np.random.default_rng(h * 1000 + w)
+    imgs = [np.clip(rng.random((h, w) if chans == 1 else (h, w, chans)) * 1.2 - 0.1, 0, 1).astype(np.float32)
+            for _ in range(K)]
+    if chans == 4:
+        for im in imgs:
+            im[..., 3] = np.where(rng.random((h, w)) < 0.9, 1.0, 0.2)
+    p = enbgpu.enfuse_params(**{**dict(saturation_weight=0.2, contrast_weight=0.5, entropy_weight=0.3,
+                                       contrast_window_size=5, entropy_window_size=5, float_range=1.0), **kw})
+    pad = [torch.from_numpy(np.pad(im, [(0, 0), (1, 2)] + [(0, 0)] * (im.ndim - 2))).cuda()[:, 1:w + 1] for im in imgs]
+    for planes in (False, True) if chans != 4 else (False,):
+        alphas = [np.where(rng.random((h, w)) < 0.8, 255, 0).astype(np.uint8) for _ in range(K)] if planes else None
+        dal = [torch.from_numpy(a).cuda() for a in alphas] if planes else None
+        got = []
+        for plain in (False, True):
+            dout = torch.full_like(torch.from_numpy(imgs[0]), 7.0).cuda()
+            doa = torch.full((h, w), 9, dtype=torch.uint8, device="cuda")
+            ctx.enfuse(pad, dal, params=p, out=dout, out_alpha=doa, plain=plain, **opt)
+            got.append((dout.cpu().numpy(), doa.cpu().numpy()))
+        assert np.array_equal(got[0][1], got[1][1])
+        assert np.array_equal(got[0][0], got[1][0])
+        out, oa = ctx.enfuse(imgs, alphas, params=p, **opt)
+        assert np.array_equal(out, got[0][0]) and np.array_equal(oa, got[0][1])

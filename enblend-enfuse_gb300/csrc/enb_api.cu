@@ -2655,110 +2655,114 @@ enb_status enb_fuse_grad(enb_ctx* ctx, const enb_enfuse_params* prm, int K, cons
     }
     ENB_TRY(check_params(ctx, prm, w, h));
     const int L = enb_num_levels(w, h, 1, o.levels);
-    const int64_t fp = round_up(w, 32), plane = fp * h;
-    DevBuf planes, a255;
-    ENB_CUDA(ctx, planes.alloc((size_t)plane * 4 * K * 6 + 64, ctx->stream));
-    float* wk = (float*)planes.p;
-    float* ak = wk + plane * K;
-    float* mk = ak + plane * K;
-    float* gm = mk + plane * K;
-    float* gw = gm + plane * K;
-    float* ga = gw + plane * K;
-    double* dsc = (double*)(ga + plane * K);
-    const int64_t apitch = round_up(w, 128);
-    ENB_CUDA(ctx, a255.alloc((size_t)(apitch * h), ctx->stream));
-    ENB_CUDA(ctx, cudaMemsetAsync(a255.p, 255, (size_t)(apitch * h), ctx->stream));
-    ENB_CUDA(ctx, cudaMemsetAsync(dsc, 0, 6 * sizeof(double), ctx->stream));
-    const BytePlane alpha{(uint8_t*)a255.p, apitch, w, h};
-    enb_image aimg{};
-    aimg.data = a255.p;
-    aimg.pitch = apitch;
-    aimg.width = w;
-    aimg.height = h;
-    aimg.channels = 1;
-    aimg.pix_stride = 1;
-    aimg.dtype = ENB_U8;
-
-    // forward: weights, logits, masks
-    for (int k = 0; k < K; ++k) {
-        ENB_TRY(enfuse_mask_impl(ctx, prm, &images[k], &aimg, FloatPlane{wk + plane * k, fp, w, h}));
-        if (logits) {
-            ENB_CUDA(ctx, cudaMemcpy2DAsync(ak + plane * k, fp * 4, logits[k].data, logits[k].pitch, (size_t)w * 4, h,
-                                            cudaMemcpyDeviceToDevice, ctx->stream));
-        }
-    }
-    ENB_LAUNCH(ctx, launch_adj_norm(K, wk, logits ? ak : nullptr, mk, fp, plane, w, h, ctx->stream));
-    PyrHolder R(ctx), LP(ctx), M(ctx), GR(ctx), ACC(ctx);
-    ENB_TRY(pyramid_alloc(ctx, L, w, h, 3, ENB_F32, &R.p));
-    ENB_TRY(pyramid_alloc(ctx, L, w, h, 3, ENB_F32, &LP.p));
-    ENB_TRY(pyramid_alloc(ctx, L, w, h, 1, ENB_F32, &M.p));
-    auto build_lp = [&](int k) -> enb_status {
-        const PixelView iv = pixel_view(&images[k]);
-        ENB_LAUNCH(ctx, launch_adj_to_pyramid(FloatPixelView{(const float*)iv.p, iv.pitch, iv.w, iv.h, 3, iv.stride},
-                                              level_view(LP.p, 0), ctx->stream));
-        ENB_TRY(gaussian_levels(ctx, 0, LP.p, &alpha));
-        ENB_TRY(laplacian_levels(ctx, 0, LP.p));
-        return ENB_OK;
-    };
-    for (int k = 0; k < K; ++k) {
-        ENB_TRY(build_lp(k));
-        const PlanarView m0 = level_view(M.p, 0);
-        ENB_CUDA(ctx, cudaMemcpy2DAsync(m0.p, m0.pitch * 4, mk + plane * k, fp * 4, (size_t)w * 4, h,
-                                        cudaMemcpyDeviceToDevice, ctx->stream));
-        ENB_TRY(gaussian_levels(ctx, 0, M.p, &alpha));
-        for (int l = 0; l < L; ++l) {
-            ENB_LAUNCH(ctx, launch_adj_merge(level_view(LP.p, l), level_view(M.p, l), level_view(R.p, l), k == 0,
-                                             ctx->stream));
-        }
-    }
-    ENB_TRY(collapse_levels(ctx, 0, R.p));
-    ENB_TRY(pyramid_alloc(ctx, L, w, h, 3, ENB_F32, &GR.p));
-    const PixelView tv = pixel_view(target);
-    float* outp = nullptr;
-    int64_t opitch = 0;
-    int ostride = 3;
-    if (out) {
-        const PixelView ov = pixel_view(out);
-        outp = (float*)out->data;
-        opitch = ov.pitch;
-        ostride = ov.stride;
-        if (ov.stride == 4) {
-            ENB_LAUNCH(ctx, launch_alpha_component(alpha, out->data, ov.pitch, ENB_F32, ctx->stream));
-        }
-    }
-    ENB_LAUNCH(ctx, launch_adj_loss(level_view(R.p, 0), (const float*)target->data, tv.pitch, tv.stride, outp, opitch,
-                                    ostride, level_view(GR.p, 0), dsc, ctx->stream));
-
-    // backward: collapse, merge and mask pyramids per exposure
-    for (int l = 0; l + 1 < L; ++l) {
-        ENB_LAUNCH(ctx, launch_expand_T(level_view(GR.p, l), level_view(GR.p, l + 1), ctx->stream));
-    }
-    ENB_TRY(pyramid_alloc(ctx, L, w, h, 1, ENB_F32, &ACC.p));
-    for (int k = 0; k < K; ++k) {
-        ENB_TRY(build_lp(k));
-        for (int l = L - 1; l >= 0; --l) {
-            const PlanarView nxt = l + 1 < L ? level_view(ACC.p, l + 1) : PlanarView{};
-            ENB_LAUNCH(ctx, launch_adj_mask_level(level_view(GR.p, l), level_view(LP.p, l), l + 1 < L ? &nxt : nullptr,
-                                                  level_view(ACC.p, l), ctx->stream));
-        }
-        const PlanarView a0 = level_view(ACC.p, 0);
-        ENB_CUDA(ctx, cudaMemcpy2DAsync(gm + plane * k, fp * 4, a0.p, a0.pitch * 4, (size_t)w * 4, h,
-                                        cudaMemcpyDeviceToDevice, ctx->stream));
-    }
-    ENB_LAUNCH(ctx, launch_adj_norm_bw(K, wk, logits ? ak : nullptr, gm, gw, ga, fp, plane, w, h, ctx->stream));
     FloatWeightParams wp;
     ENB_TRY(float_weight_params(ctx, prm, wp));
-    const float inv_width = (float)(1.0 / exposure_effective_width(prm->exp_function, prm->exp_width));
+    AdjGeometry g{};
+    g.K = K;
+    g.L = L;
+    for (int l = 0; l < L; ++l) {
+        g.lw[l] = l == 0 ? w : (g.lw[l - 1] + 1) >> 1;
+        g.lh[l] = l == 0 ? h : (g.lh[l - 1] + 1) >> 1;
+        g.pitch[l] = (int)round_up(g.lw[l], 32);
+        g.off[l] = g.s;
+        g.s += (int64_t)g.pitch[l] * g.lh[l];
+    }
+    // one allocation: the sums, the exposures' table, the weights, the mask
+    // and image pyramids of every exposure, the result and its gradient
+    const int64_t plane = (int64_t)g.pitch[0] * h;
+    const int64_t o_table = 256, o_w = o_table + round_up(K * (int64_t)sizeof(AdjExposure), 256);
+    DevBuf mem;
+    ENB_CUDA(ctx, mem.alloc((size_t)(o_w + 4 * (K * plane + K * g.s + 3 * K * g.s + 6 * g.s)), ctx->stream));
+    double* dsc = (double*)mem.p;
+    g.exposures = (const AdjExposure*)((char*)mem.p + o_table);
+    g.w = (float*)((char*)mem.p + o_w);
+    g.m = g.w + K * plane;
+    g.g = g.m + K * g.s;
+    g.r = g.g + 3 * K * g.s;
+    g.gr = g.r + 3 * g.s;
+    std::vector<AdjExposure> table((size_t)K);
     for (int k = 0; k < K; ++k) {
         const PixelView iv = pixel_view(&images[k]);
-        ENB_LAUNCH(ctx, launch_adj_weights_bw(FloatPixelView{(const float*)iv.p, iv.pitch, iv.w, iv.h, 3, iv.stride},
-                                              gw + plane * k, fp, wp, inv_width, (float)prm->exp_width,
-                                              (float)prm->w_exposure, prm->contrast_window, dsc + 1, ctx->stream));
+        AdjExposure& e = table[(size_t)k];
+        e.img = (const float*)iv.p;
+        e.ipitch = iv.pitch;
+        e.stride = iv.stride;
+        if (logits) {
+            e.logit = (const float*)logits[k].data;
+            e.lpitch = logits[k].pitch / 4;
+        }
+        if (grad_logits) {
+            e.glogit = (float*)grad_logits[k].data;
+            e.gpitch = grad_logits[k].pitch / 4;
+        }
     }
-    if (grad_logits) {
+    ENB_CUDA(ctx, cudaMemcpyAsync((void*)g.exposures, table.data(), table.size() * sizeof(AdjExposure),
+                                  cudaMemcpyHostToDevice, ctx->stream));
+    ENB_CUDA(ctx, cudaMemsetAsync(dsc, 0, 6 * sizeof(double), ctx->stream));
+
+    // forward: weights and level 0, masks, pyramids, merge, loss
+    if (adj_weights_at_once(wp)) {
+        ENB_LAUNCH(ctx, launch_adj_weights(g, wp, ctx->tables, ctx->stream));
+    } else {
+        DevBuf a255;
+        const int64_t apitch = round_up(w, 128);
+        ENB_CUDA(ctx, a255.alloc((size_t)(apitch * h), ctx->stream));
+        ENB_CUDA(ctx, cudaMemsetAsync(a255.p, 255, (size_t)(apitch * h), ctx->stream));
         for (int k = 0; k < K; ++k) {
-            ENB_CUDA(ctx, cudaMemcpy2DAsync(grad_logits[k].data, grad_logits[k].pitch, ga + plane * k, fp * 4,
-                                            (size_t)w * 4, h, cudaMemcpyDeviceToDevice, ctx->stream));
+            const AdjExposure& e = table[(size_t)k];
+            ENB_LAUNCH(ctx, launch_f_enfuse_mask(FloatPixelView{e.img, e.ipitch, w, h, 3, e.stride},
+                                                 BytePlane{(uint8_t*)a255.p, apitch, w, h}, wp, ctx->tables,
+                                                 FloatPlane{g.w + k * plane, g.pitch[0], w, h}, ctx->stream));
+        }
+        ENB_LAUNCH(ctx, launch_adj_to_pyramid(g, ctx->stream));
+    }
+    ENB_LAUNCH(ctx, launch_adj_norm(g, logits != nullptr, ctx->stream));
+    for (int l = 0; l + 1 < L; ++l) {
+        ENB_LAUNCH(ctx, launch_adj_reduce(g, l, ctx->stream));
+    }
+    AdjLoss loss{};
+    const PixelView tv = pixel_view(target);
+    loss.target = (const float*)target->data;
+    loss.tpitch = tv.pitch;
+    loss.tstride = tv.stride;
+    loss.inv_n = (float)(1.0 / (3.0 * w * (double)h));
+    loss.sums = dsc;
+    if (out) {
+        const PixelView ov = pixel_view(out);
+        loss.out = (float*)out->data;
+        loss.opitch = ov.pitch;
+        loss.ostride = ov.stride;
+        if (ov.stride == 4) {
+            DevBuf a255;
+            const int64_t apitch = round_up(w, 128);
+            ENB_CUDA(ctx, a255.alloc((size_t)(apitch * h), ctx->stream));
+            ENB_CUDA(ctx, cudaMemsetAsync(a255.p, 255, (size_t)(apitch * h), ctx->stream));
+            ENB_LAUNCH(ctx, launch_alpha_component(BytePlane{(uint8_t*)a255.p, apitch, w, h}, out->data, ov.pitch, ENB_F32,
+                                                   ctx->stream));
+        }
+    }
+    for (int l = L - 1; l >= 0; --l) {
+        ENB_LAUNCH(ctx, launch_adj_up(g, l, loss, ctx->stream));
+    }
+
+    // backward: collapse, merge and mask pyramids, normalisation, weights
+    for (int l = 0; l + 1 < L; ++l) {
+        ENB_LAUNCH(ctx, launch_adj_expand_T(g, l, ctx->stream));
+    }
+    for (int l = L - 1; l >= 0; --l) {
+        ENB_LAUNCH(ctx, launch_adj_mask_level(g, l, ctx->stream));
+    }
+    ENB_LAUNCH(ctx, launch_adj_norm_bw(g, logits != nullptr, grad_logits != nullptr, ctx->stream));
+    const float inv_width = (float)(1.0 / exposure_effective_width(prm->exp_function, prm->exp_width));
+    if (prm->contrast_window == 3 || prm->contrast_window == 5) {
+        ENB_LAUNCH(ctx, launch_adj_weights_bw_pair(g, wp, inv_width, (float)prm->exp_width, (float)prm->w_exposure,
+                                                   prm->contrast_window, dsc + 1, ctx->stream));
+    } else {
+        for (int k = 0; k < K; ++k) {
+            const AdjExposure& e = table[(size_t)k];
+            ENB_LAUNCH(ctx, launch_adj_weights_bw(FloatPixelView{e.img, e.ipitch, w, h, 3, e.stride}, g.w + k * plane,
+                                                  g.pitch[0], wp, inv_width, (float)prm->exp_width, (float)prm->w_exposure,
+                                                  prm->contrast_window, dsc + 1, ctx->stream));
         }
     }
     double hs[6];

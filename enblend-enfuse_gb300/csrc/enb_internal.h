@@ -350,19 +350,54 @@ size_t nft_scratch_bytes(int w, int h, int wrap);
 cudaError_t launch_nft_stage(int stage, const BytePlane& white, const BytePlane& black, const BytePlane& mask,
                              int wrap, void* scratch, unsigned int* tally, cudaStream_t st);
 
-// adjoint of the float enfuse (enb_adjoint.cu)
-cudaError_t launch_adj_norm(int K, const float* w, const float* a, float* m, int64_t pitch, int64_t plane, int width,
-                            int height, cudaStream_t st);
-cudaError_t launch_adj_merge(const PlanarView& lp, const PlanarView& m, const PlanarView& r, int first, cudaStream_t st);
-// level 0 of an image pyramid in the adjoint's offset form (G - 1)
-cudaError_t launch_adj_to_pyramid(const FloatPixelView& img, const PlanarView& g, cudaStream_t st);
-cudaError_t launch_adj_loss(const PlanarView& c0, const float* tgt, int64_t tpitch, int tstride, float* out,
-                            int64_t opitch, int ostride, const PlanarView& g0, double* loss, cudaStream_t st);
-cudaError_t launch_expand_T(const PlanarView& fine, const PlanarView& coarse, cudaStream_t st);
-cudaError_t launch_adj_mask_level(const PlanarView& gr, const PlanarView& lp, const PlanarView* next,
-                                  const PlanarView& acc, cudaStream_t st);
-cudaError_t launch_adj_norm_bw(int K, const float* w, const float* a, const float* gm, float* gw, float* ga,
-                               int64_t pitch, int64_t plane, int width, int height, cudaStream_t st);
+// adjoint of the float enfuse (enb_adjoint.cu): K exposures' images and logits
+// (device table), and the level planes of all of them.  Levels are planes of
+// pitch[l] * lh[l] floats at off[l] (times the planes of a level); s is the
+// sum over the levels.
+struct AdjExposure {
+    const float* img;
+    int64_t ipitch;  // floats
+    const float* logit;  // or null
+    int64_t lpitch;
+    float* glogit;       // or null
+    int64_t gpitch;
+    int stride;
+};
+struct AdjGeometry {
+    int K, L;
+    int lw[kMaxLevels], lh[kMaxLevels], pitch[kMaxLevels];
+    int64_t off[kMaxLevels], s;
+    const AdjExposure* exposures;
+    float* w;   // K planes of level 0: weights, later dL/dw
+    float* m;   // K * s: mask pyramids, later their adjoints
+    float* g;   // K * 3 * s: image pyramids (G - 1)
+    float* r;   // 3 * s: C[l], l >= 1
+    float* gr;  // 3 * s: dL/dC[l]
+};
+struct AdjLoss {
+    const float* target;
+    int64_t tpitch;
+    int tstride;
+    float* out;  // or null
+    int64_t opitch;
+    int ostride;
+    float inv_n;
+    double* sums;
+};
+// Whether launch_adj_weights takes the parameters (else launch_f_enfuse_mask
+// per exposure and launch_adj_to_pyramid).
+bool adj_weights_at_once(const FloatWeightParams& wp);
+cudaError_t launch_adj_weights(const AdjGeometry& g, const FloatWeightParams& wp, const WeightTables& tab, cudaStream_t st);
+cudaError_t launch_adj_to_pyramid(const AdjGeometry& g, cudaStream_t st);
+cudaError_t launch_adj_norm(const AdjGeometry& g, bool logits, cudaStream_t st);
+cudaError_t launch_adj_reduce(const AdjGeometry& g, int l, cudaStream_t st);
+cudaError_t launch_adj_up(const AdjGeometry& g, int l, const AdjLoss& loss, cudaStream_t st);
+cudaError_t launch_adj_expand_T(const AdjGeometry& g, int l, cudaStream_t st);
+cudaError_t launch_adj_mask_level(const AdjGeometry& g, int l, cudaStream_t st);
+cudaError_t launch_adj_norm_bw(const AdjGeometry& g, bool logits, bool grad, cudaStream_t st);
+// contrast windows of 3 or 5, all exposures; else one exposure a launch
+cudaError_t launch_adj_weights_bw_pair(const AdjGeometry& g, const FloatWeightParams& wp, float inv_width, float width, float w_exp,
+                                       int cwin, double* d, cudaStream_t st);
 cudaError_t launch_adj_weights_bw(const FloatPixelView& img, const float* gw, int64_t gpitch, const FloatWeightParams& wp,
                                   float inv_width, float width, float w_exp, int cwin, double* d, cudaStream_t st);
 

@@ -16,6 +16,11 @@
 //               image dropped, x periodic when wrap (pyramid.h:166-573);
 //   no alpha:   clamp-to-edge replication in y (and x unless wrap), /256
 //               (pyramid.h:601-848).
+//   opaque:     the normalised convolution of a level without transparent
+//               pixels: the divisor is a product of two position factors, so
+//               no alpha is read, summed or written;
+//   zeros:      taps outside the image dropped, times a constant (the
+//               transposed expand, enb_adjoint.cu).
 // blockIdx.z selects one of up to two jobs of the same geometry (the white and
 // black pyramids of a level), so a level of both images is one launch.
 #pragma once
@@ -88,14 +93,26 @@ struct ReduceJobs {
     int ty0;  // first destination tile row of the launch
 };
 
+// What a reduce does at the borders and with alpha.
+enum ReduceMode { kReduceClamp = 0, kReduceAlpha = 1, kReduceOpaque = 2, kReduceZeros = 3 };
+
+// In-image weight sum of the 5-tap binomial centred at 2I (the opaque reduce's
+// divisor factor along one axis of n samples, not periodic).
+__host__ __device__ __forceinline__ int reduce_den1(int I, int n)
+{
+    const int x = 2 * I;
+    return 16 - (x < 1 ? 5 : 0) - (x + 1 >= n ? 4 : 0) - (x + 2 >= n ? 1 : 0);
+}
+
 // Phase 1 for one column item: vertical sums of destination rows r0..r0+7.
 // Border items load from clamped (always valid) positions and zero the taps
 // outside the image afterwards, so that no load waits behind a branch and
 // all 19 rows are in flight at once.
-template <class Src, int C, bool ALPHA, bool INTERIOR, typename AC>
+template <class Src, int C, int MODE, bool INTERIOR, typename AC>
 __device__ __forceinline__ void reduce_column(const Src& src, int gx, int gyb, int sw, int sh, int wrap,
                                               AC (*V)[RDH][RVP], int col, int r0)
 {
+    constexpr bool ALPHA = MODE == kReduceAlpha;
     constexpr int NV = C + (ALPHA ? 1 : 0);
     bool colok = true;
     if (!INTERIOR) {
@@ -123,7 +140,8 @@ __device__ __forceinline__ void reduce_column(const Src& src, int gx, int gyb, i
         }
 #pragma unroll
         for (int ch = 0; ch < C; ++ch) {
-            x[k][ch] = (ALPHA && !al) ? (AC)0 : v[ch];   // without alpha: clamp-to-edge
+            // without alpha: clamp-to-edge
+            x[k][ch] = (ALPHA && !al) || (MODE >= kReduceOpaque && !ok) ? (AC)0 : v[ch];
         }
         if (ALPHA) {
             x[k][NV - 1] = (AC)al;
@@ -191,14 +209,18 @@ __device__ __forceinline__ int32_t reduce_norm(int32_t s, int32_t den)
 __device__ __forceinline__ float reduce_norm(float s, float den) { return __fdiv_rn(s, den); }
 __device__ __forceinline__ int32_t reduce_256(int32_t s) { return s / 256; }
 __device__ __forceinline__ float reduce_256(float s) { return s * 0.00390625f; }
+// The transposed expand's scale: its taps are [1 4 6 4 1] / 8 along each axis.
+__device__ __forceinline__ int32_t reduce_zeros(int32_t s) { return s / 64; }
+__device__ __forceinline__ float reduce_zeros(float s) { return s * 0.015625f; }
 
 // One 64x16 destination tile at (X0, Y0) of a reduce job (RTHREADS threads;
 // V holds ReduceSmem<C, ALPHA>::WORDS 16-byte aligned words of the
 // accumulator type AC: int32 for fixed point, float for FP32 levels).
-template <class Src, typename TD, int C, bool ALPHA, typename AC = int32_t>
+template <class Src, typename TD, int C, int MODE, typename AC = int32_t>
 __device__ __forceinline__ void reduce_tile(const ReduceJob<Src, TD>& job, int X0, int Y0, int sw, int sh, int dw,
                                             int dh, int wrap, AC (*V)[RDH][RVP])
 {
+    constexpr bool ALPHA = MODE == kReduceAlpha;
     constexpr int NV = C + (ALPHA ? 1 : 0);
     const int gx0 = 2 * X0 - 2, gy0 = 2 * Y0 - 2;
     const int tid = threadIdx.x;
@@ -208,9 +230,9 @@ __device__ __forceinline__ void reduce_tile(const ReduceJob<Src, TD>& job, int X
         const int col = tid - g * RSW;
         const int gyb = gy0 + 2 * RGR * g;
         if (gx0 >= 0 && gy0 >= 0 && gx0 + RSW <= sw && gy0 + RSH <= sh) {
-            reduce_column<Src, C, ALPHA, true, AC>(job.src, gx0 + col, gyb, sw, sh, wrap, V, col, RGR * g);
+            reduce_column<Src, C, MODE, true, AC>(job.src, gx0 + col, gyb, sw, sh, wrap, V, col, RGR * g);
         } else {
-            reduce_column<Src, C, ALPHA, false, AC>(job.src, gx0 + col, gyb, sw, sh, wrap, V, col, RGR * g);
+            reduce_column<Src, C, MODE, false, AC>(job.src, gx0 + col, gyb, sw, sh, wrap, V, col, RGR * g);
         }
     }
     __syncthreads();
@@ -263,12 +285,26 @@ __device__ __forceinline__ void reduce_tile(const ReduceJob<Src, TD>& job, int X
             }
         }
     } else {
+        // opaque: 256 but for the destination pixels at the level's ends
+        AC den[4];
+        bool whole = MODE != kReduceOpaque;
+        if (MODE == kReduceOpaque) {
+            const int dy = reduce_den1(Y, sh);
+            whole = dy == 16;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int dx = wrap ? 16 : reduce_den1(Xb + q, sw);
+                den[q] = (AC)(dx * dy);
+                whole = whole && (dx == 16 || q >= n);
+            }
+        }
 #pragma unroll
         for (int ch = 0; ch < C; ++ch) {
             AC out[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                out[q] = reduce_256(s[ch][q]);
+                out[q] = whole ? (MODE == kReduceZeros ? reduce_zeros(s[ch][q]) : reduce_256(s[ch][q]))
+                               : (q < n ? reduce_norm(s[ch][q], den[q]) : (AC)0);
             }
             store4(job.dst + ch * job.dplane + o, out, n);
         }

@@ -97,3 +97,38 @@ def test_adjoint_rejects_entropy(ctx):
     dev = [torch.from_numpy(x).cuda() for x in imgs]
     with pytest.raises(enbgpu.EnbError):
         ctx.fuse_grad(dev, torch.from_numpy(target).cuda(), params=enbgpu.enfuse_params(entropy_weight=0.3))
+
+
+@pytest.mark.parametrize("K,h,w,cwin,chans,with_logits", [
+    (2, 33, 47, 5, 3, True), (3, 65, 64, 3, 3, True), (4, 16, 130, 5, 4, False), (5, 129, 67, 7, 3, True),
+    (9, 70, 95, 5, 3, True), (8, 7, 8, 3, 3, True), (2, 200, 33, 5, 4, True)])
+def test_adjoint_level_passes_at_their_edges(ctx, K, h, w, cwin, chans, with_logits):
+    """Odd levels, tile edges, one level, exposure counts around the register and staging limits, contrast windows
+    inside and outside the pair kernel, 4-sample pixels and missing logits; tolerances as above."""
+    import enbgpu
+    imgs, target = _scene(K=K, h=max(h, 32), w=max(w, 32), seed=K + h)
+    imgs, target = np.ascontiguousarray(imgs[:, :h, :w]), np.ascontiguousarray(target[:h, :w])
+    rng = np.random.default_rng(h)
+    logits = rng.normal(0.0, 0.3, imgs.shape[:3]) if with_logits else np.zeros(imgs.shape[:3])
+    theta = [0.5, 0.2, 1.0, 0.2, 0.5]
+    pix = lambda a: torch.from_numpy(np.concatenate([a, np.ones((h, w, 1), np.float32)], 2) if chans == 4 else a).cuda()
+    dev, out = [pix(x) for x in imgs], torch.zeros((h, w, chans), device="cuda")
+    lg = [torch.from_numpy(x.astype(np.float32)).cuda() for x in logits] if with_logits else None
+    gl = [torch.zeros((h, w), device="cuda") for _ in range(K)]
+    prm = enbgpu.enfuse_params(saturation_weight=0.2, contrast_weight=0.5, contrast_window_size=cwin, float_range=1.0)
+    r = ctx.fuse_grad(dev, torch.from_numpy(target).cuda(), params=prm, logits=lg, grad_logits=gl, out=out)
+    xl = torch.from_numpy(logits.astype(np.float32).astype(np.float64)).requires_grad_(True)
+    th = torch.tensor(theta, dtype=torch.float64, requires_grad=True)
+    t = torch.from_numpy(target.astype(np.float64))
+    ref = ar.fuse(torch.from_numpy(imgs.astype(np.float64)), xl, th, cwin=cwin)
+    loss = ((ref - t) ** 2).mean()
+    loss.backward()
+    assert abs(r["loss"] - loss.item()) <= 1e-5 * loss.item()
+    assert np.allclose(out.cpu().numpy()[..., :3], ref.detach().numpy(), rtol=1e-4, atol=1e-5)
+    if chans == 4:
+        assert (out[..., 3] == 1.0).all()
+    gt = np.array([r["d_exp_optimum"], r["d_exp_width"], r["d_w_exposure"], r["d_w_saturation"], r["d_w_contrast"]])
+    at = th.grad.numpy()
+    scale = max(np.abs(xl.grad.numpy()).max(), 1e-12)
+    assert np.all(np.abs(np.stack([g.cpu().numpy() for g in gl]) - xl.grad.numpy()) <= 1e-4 * scale)
+    assert np.all(np.abs(gt - at) <= 1e-4 * np.abs(at) + 1e-4 * np.abs(at).max()), (gt, at)

@@ -1260,10 +1260,8 @@ enb_status enfuse_fused(enb_ctx* ctx, const enb_enfuse_params* prm, int K, const
 
     ENB_LAUNCH(ctx, launch_ef_weights(eh, ctx->stream));
     for (int l = 0; l + 1 < L; ++l) {
-        ENB_LAUNCH(ctx, launch_ef_reduce(eh, l, 0, ctx->stream));
-        ENB_LAUNCH(ctx, launch_ef_reduce(eh, l, 1, ctx->stream));
+        ENB_LAUNCH(ctx, launch_ef_reduce(eh, l, ctx->stream));
     }
-    ENB_LAUNCH(ctx, launch_ef_top(eh, ctx->stream));
     for (int l = L - 2; l >= 1; --l) {
         ENB_LAUNCH(ctx, launch_ef_up(eh, l, ctx->stream));
     }

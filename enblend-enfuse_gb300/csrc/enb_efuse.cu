@@ -218,6 +218,36 @@ struct EfWindow {
             }
         }
     }
+    // R of the top level, sum_k fromRealPromote(G_k M_k / D), at the thread's
+    // taps, from the staged windows of the K image pyramids (one level of a
+    // few pixels, not worth a launch and a trip through memory)
+    template <typename T, typename TM, int C, int F>
+    __device__ __forceinline__ void top(int32_t (*ss)[ESH][ESW], const TM* const* m, int K, int32_t (&v)[C][2]) const
+    {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            v[c][0] = v[c][1] = 0;
+        }
+        for (int k = 0; k < K; ++k) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (f[u] == 0 || (u == 1 && !two)) {
+                    continue;
+                }
+                const int32_t mv = (int32_t)__ldg(&m[k][o[u]]);
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    const int32_t g = (&ss[k * C + c][0][0])[threadIdx.x + 256 * u] / f[u];
+                    v[c][u] += (int32_t)mask_multiply<T, F>(g, mv);
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            v[c][0] = (int32_t)cast_store<T>(v[c][0]);
+            v[c][1] = (int32_t)cast_store<T>(v[c][1]);
+        }
+    }
     // the windows of the K image pyramids, four exposures' loads in flight
     template <typename T, int C>
     __device__ __forceinline__ void stage(int32_t (*ss)[ESH][ESW], const T* const* g, int64_t cplane, int K) const
@@ -353,7 +383,7 @@ __device__ __forceinline__ void ld_pair(const T* p, int32_t& a, int32_t& b)
 }
 
 // ---------------------------------------------------------------------------
-// top level: R = sum_k fromRealPromote(G_k * M_k / D)
+// levels L-2 .. 1: Laplacians, mask products, accumulation and collapse
 // ---------------------------------------------------------------------------
 
 template <typename T, typename TM>
@@ -363,51 +393,35 @@ struct EfLevelArgs {
     const T* gc[kEfuseMaxK];  // level l + 1
     const TM* m[kEfuseMaxK];  // level l of the mask pyramids
     const T* rc;              // R[l + 1]
+    const TM* mc[kEfuseMaxK]; // level l + 1 of the mask pyramids
     T* r;                     // R[l]
     int64_t pitch, plane, cpitch, cplane;
 };
 
-template <typename T, typename TM, int F>
-__global__ void __launch_bounds__(256) k_ef_top(const __grid_constant__ EfLevelArgs<T, TM> a)
-{
-    griddep_wait();
-    griddep_launch();
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y;
-    if (x >= a.dw) {
-        return;
-    }
-    const int64_t o = (int64_t)y * a.pitch + x;
-    for (int c = 0; c < a.C; ++c) {
-        int32_t acc = 0;
-        for (int k = 0; k < a.K; ++k) {
-            acc += (int32_t)mask_multiply<T, F>((int32_t)a.g[k][c * a.plane + o], (int32_t)a.m[k][o]);
-        }
-        a.r[c * a.plane + o] = cast_store<T>(acc);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// levels L-2 .. 1: Laplacians, mask products, accumulation and collapse
-// ---------------------------------------------------------------------------
-
 // One 64x16 tile of level l (256 threads, one 2x2 quad each): the K coarse
 // windows of every channel are staged together (one barrier), the exposures'
 // products summed, and only then the launch waits for its predecessor, which
-// wrote R_l+1: every other input is older than that (each launch of the chain
-// waits before it lets the next one start), so that on the small levels the
-// sum overlaps the level before.  ss holds (K + 1) * C windows.
+// wrote R_l+1.  The first of these launches (FOLD) waits for the reduces
+// before it lets the next start, the others let theirs start at once: every
+// input but R_l+1 is complete by then, the small levels' sums run side by
+// side, and from level to level only the expansion of R remains.  ss holds
+// (K + 1) * C windows.
 // Bound by instructions, about a hundred per exposure, channel and quad; one
 // division table entry per quad serves every border expansion, so that the
 // small levels, all border, cost no more than the large ones.  The eight
 // levels of 9 x 6000x4000 u16 take 0.46 ms (3.2 TB/s; 1.28 ms with a staging
 // loop per window, per-position border weights and the wait up front), the six
 // of 3 x 1024x768 u8 75 us with event overhead (157 us).
-template <typename T, typename TM, int C, int F>
+// FOLD: level l + 1 is the top and its R is formed here.
+template <typename T, typename TM, int C, int F, bool FOLD>
 __global__ void __launch_bounds__(256, 3) k_ef_up(const __grid_constant__ EfLevelArgs<T, TM> a)
 {
     extern __shared__ __align__(16) int32_t ewin[];
     int32_t (*ss)[ESH][ESW] = reinterpret_cast<int32_t (*)[ESH][ESW]>(ewin);
+    if (FOLD) {
+        griddep_wait();  // the launch before wrote the top level
+    }
+    griddep_launch();
     const int K = a.K;
     const int X0 = blockIdx.x * ETW, Y0 = blockIdx.y * ETH;
     const int I0 = X0 >> 1, J0 = Y0 >> 1;
@@ -478,10 +492,13 @@ __global__ void __launch_bounds__(256, 3) k_ef_up(const __grid_constant__ EfLeve
         }
     }
     griddep_wait();
-    griddep_launch();
     {
         int32_t v[C][2];
-        win.load_written<T, C>(a.rc, a.cplane, v);
+        if constexpr (FOLD) {
+            win.top<T, TM, C, F>(ss, a.mc, K, v);
+        } else {
+            win.load_written<T, C>(a.rc, a.cplane, v);
+        }
         win.store<C>(ss + K * C, v);
     }
     __syncthreads();
@@ -530,6 +547,7 @@ struct EfOut0Args {
     int64_t mpitch;
     const T* g1[kEfuseMaxK];
     const T* r1;
+    const TM* mc[kEfuseMaxK];  // level 1 of the mask pyramids
     int64_t cpitch, cplane;
     const uint8_t* u0;
     int64_t upitch;
@@ -547,11 +565,15 @@ struct EfOut0Args {
 // pyramids and the output pixels in place of R_0 (stored in words of the
 // pair's size where the rows allow it).  9 x 6000x4000 u16: 1.21 ms
 // (2.5 TB/s), 2.73 ms before the changes named at k_ef_up.
-template <typename TIn, typename T, typename TM, int C, int S, int F>
+template <typename TIn, typename T, typename TM, int C, int S, int F, bool FOLD>
 __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOut0Args<TIn, T, TM> a)
 {
     extern __shared__ __align__(16) int32_t ewin[];
     int32_t (*ss)[ESH][ESW] = reinterpret_cast<int32_t (*)[ESH][ESW]>(ewin);
+    if (FOLD) {
+        griddep_wait();  // the launch before wrote the top level
+        griddep_launch();
+    }
     const int K = a.K;
     const int X0 = blockIdx.x * ETW, Y0 = blockIdx.y * ETH;
     const int I0 = X0 >> 1, J0 = Y0 >> 1;
@@ -638,7 +660,11 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
     griddep_launch();
     {
         int32_t v[C][2];
-        win.load_written<T, C>(a.r1, a.cplane, v);
+        if constexpr (FOLD) {
+            win.top<T, TM, C, F>(ss, a.mc, K, v);
+        } else {
+            win.load_written<T, C>(a.r1, a.cplane, v);
+        }
         win.store<C>(ss + K * C, v);
     }
     __syncthreads();
@@ -762,7 +788,33 @@ cudaError_t launch_ef_weights(const EfuseHost& h, cudaStream_t st)
     return h.dtype == ENB_U8 ? ef_weights_t<int16_t>(h, st) : ef_weights_t<int32_t>(h, st);
 }
 
-// Level-1 reduce of the K images straight from their pixels (PixelSourceV).
+// No exposure has alpha: the pyramids need no alpha planes (kReduceOpaque).
+static bool ef_opaque(const EfuseHost& h)
+{
+    bool opaque = true;
+    for (int k = 0; k < h.K; ++k) {
+        opaque = opaque && h.alpha[k].mode == kAlphaOpaque;
+    }
+    return opaque;
+}
+
+// The mask pyramids' jobs from level l to l + 1 (A: with the union alpha).
+template <typename TM, bool A>
+static ReduceJobsN<PlanarSource<TM, 1, A>, TM> ef_mask_jobs(const EfuseHost& h, int l)
+{
+    using Src = PlanarSource<TM, 1, A>;
+    ReduceJobsN<Src, TM> jobs{};
+    const int64_t ap = l == 0 ? h.upitch0 : h.apitch[l];
+    for (int k = 0; k < h.K; ++k) {
+        jobs.j[k] = ReduceJob<Src, TM>{Src{(const TM*)h.m[k][l], h.pitch[l], h.pitch[l] * h.lh[l], h.u[l], ap},
+                                       (TM*)h.m[k][l + 1], h.pitch[l + 1], h.pitch[l + 1] * h.lh[l + 1], h.u[l + 1],
+                                       h.apitch[l + 1]};
+    }
+    return jobs;
+}
+
+// Level 1 of the K image pyramids straight from the pixels (PixelSourceV) and
+// of the mask pyramids.
 struct EfReduce0 {
     const EfuseHost& h;
     cudaStream_t st;
@@ -771,6 +823,7 @@ struct EfReduce0 {
     void operator()()
     {
         using Src = PixelSourceV<TIn, C, S, AM, VEC>;
+        constexpr bool A = AM != 1;
         ReduceJobsN<Src, T> jobs{};
         for (int k = 0; k < h.K; ++k) {
             const AlphaSrc& al = h.alpha[k];
@@ -779,51 +832,39 @@ struct EfReduce0 {
                     al.mode == kAlphaPlane ? al.plane.pitch : 0, al.lo, al.hi, 7},
                 (T*)h.g[k][1], h.pitch[1], h.pitch[1] * h.lh[1], h.a[k][1], h.apitch[1]};
         }
-        err = launch_reduce_n<Src, T, C, true>(jobs, h.K, h.w, h.h, h.lw[1], h.lh[1], h.wrap, st);
+        err = launch_reduce_joint<Src, T, C, PlanarSource<T, 1, A>, T, A ? kReduceAlpha : kReduceOpaque>(
+            jobs, ef_mask_jobs<T, A>(h, 0), h.K, h.w, h.h, h.lw[1], h.lh[1], h.wrap, st);
     }
 };
 
-template <typename T, int C>
-static cudaError_t ef_reduce_images(const EfuseHost& h, int l, cudaStream_t st)
+template <typename T, int C, bool A>
+static cudaError_t ef_reduce_level(const EfuseHost& h, int l, cudaStream_t st)
 {
-    using Src = PlanarSource<T, C, true>;
+    using Src = PlanarSource<T, C, A>;
     ReduceJobsN<Src, T> jobs{};
     for (int k = 0; k < h.K; ++k) {
         jobs.j[k] = ReduceJob<Src, T>{Src{(const T*)h.g[k][l], h.pitch[l], h.pitch[l] * h.lh[l], h.a[k][l], h.apitch[l]},
                                       (T*)h.g[k][l + 1], h.pitch[l + 1], h.pitch[l + 1] * h.lh[l + 1], h.a[k][l + 1],
                                       h.apitch[l + 1]};
     }
-    return launch_reduce_n<Src, T, C, true>(jobs, h.K, h.lw[l], h.lh[l], h.lw[l + 1], h.lh[l + 1], h.wrap, st);
+    return launch_reduce_joint<Src, T, C, PlanarSource<T, 1, A>, T, A ? kReduceAlpha : kReduceOpaque>(
+        jobs, ef_mask_jobs<T, A>(h, l), h.K, h.lw[l], h.lh[l], h.lw[l + 1], h.lh[l + 1], h.wrap, st);
 }
 
-template <typename TM>
-static cudaError_t ef_reduce_masks(const EfuseHost& h, int l, cudaStream_t st)
-{
-    using Src = PlanarSource<TM, 1, true>;
-    ReduceJobsN<Src, TM> jobs{};
-    const int64_t ap = l == 0 ? h.upitch0 : h.apitch[l];
-    for (int k = 0; k < h.K; ++k) {
-        jobs.j[k] = ReduceJob<Src, TM>{Src{(const TM*)h.m[k][l], h.pitch[l], h.pitch[l] * h.lh[l], h.u[l], ap},
-                                       (TM*)h.m[k][l + 1], h.pitch[l + 1], h.pitch[l + 1] * h.lh[l + 1], h.u[l + 1],
-                                       h.apitch[l + 1]};
-    }
-    return launch_reduce_n<Src, TM, 1, true>(jobs, h.K, h.lw[l], h.lh[l], h.lw[l + 1], h.lh[l + 1], h.wrap, st);
-}
-
-cudaError_t launch_ef_reduce(const EfuseHost& h, int l, int masks, cudaStream_t st)
+// Level l + 1 of the K image pyramids and the K mask pyramids.
+cudaError_t launch_ef_reduce(const EfuseHost& h, int l, cudaStream_t st)
 {
     const double sp = (double)h.lw[l] * h.lh[l], dp = (double)h.lw[l + 1] * h.lh[l + 1];
     const double ps = h.dtype == ENB_U8 ? 2.0 : 4.0;
-    if (masks) {
-        note_launch(l == 0 ? "ef_reduce0_mask" : "ef_reduce_mask", h.K * (sp * ps + dp * ps + dp) + sp);
-        return h.dtype == ENB_U8 ? ef_reduce_masks<int16_t>(h, l, st) : ef_reduce_masks<int32_t>(h, l, st);
-    }
+    const bool opaque = ef_opaque(h);
+    const double as = opaque ? 0.0 : 1.0;
+    const double masks = h.K * (sp + dp) * ps + as * (sp + h.K * dp);
     if (l == 0) {
         double in = 0.0;
         for (int k = 0; k < h.K; ++k) {
             in += sp * (h.S * esz_b(h.dtype) + (h.alpha[k].mode == kAlphaPlane ? 1.0 : 0.0));
         }
-        note_launch("ef_reduce0", in + h.K * dp * (h.C * ps + 1.0));
+        note_launch("ef_reduce0", in + h.K * dp * (h.C * ps + as) + masks);
         const PixelView& v = h.img[0];
         bool vec = h.S == 4;
         for (int k = 0; k < h.K; ++k) {
@@ -857,59 +898,54 @@ cudaError_t launch_ef_reduce(const EfuseHost& h, int l, int masks, cudaStream_t 
 #undef ENB_EF_CASE
         return cudaErrorInvalidValue;
     }
-    note_launch("ef_reduce", h.K * (sp * (h.C * ps + 1.0) + dp * (h.C * ps + 1.0)));
+    note_launch("ef_reduce", h.K * (sp + dp) * (h.C * ps + as) + masks);
     if (h.dtype == ENB_U8) {
-        return h.C == 1 ? ef_reduce_images<int16_t, 1>(h, l, st) : ef_reduce_images<int16_t, 3>(h, l, st);
+        if (opaque) {
+            return h.C == 1 ? ef_reduce_level<int16_t, 1, false>(h, l, st) : ef_reduce_level<int16_t, 3, false>(h, l, st);
+        }
+        return h.C == 1 ? ef_reduce_level<int16_t, 1, true>(h, l, st) : ef_reduce_level<int16_t, 3, true>(h, l, st);
     }
-    return h.C == 1 ? ef_reduce_images<int32_t, 1>(h, l, st) : ef_reduce_images<int32_t, 3>(h, l, st);
+    if (opaque) {
+        return h.C == 1 ? ef_reduce_level<int32_t, 1, false>(h, l, st) : ef_reduce_level<int32_t, 3, false>(h, l, st);
+    }
+    return h.C == 1 ? ef_reduce_level<int32_t, 1, true>(h, l, st) : ef_reduce_level<int32_t, 3, true>(h, l, st);
 }
 
 template <typename T, typename TM>
 static EfLevelArgs<T, TM> level_args(const EfuseHost& h, int l)
 {
     EfLevelArgs<T, TM> a{};
-    const bool top = l == h.L - 1;
     a.K = h.K;
     a.C = h.C;
     a.dw = h.lw[l];
     a.dh = h.lh[l];
-    a.cw = top ? 1 : h.lw[l + 1];
-    a.ch = top ? 1 : h.lh[l + 1];
+    a.cw = h.lw[l + 1];
+    a.ch = h.lh[l + 1];
     a.wrap = h.wrap;
     a.mfrac = h.dtype == ENB_U8 ? 7 : 15;
     for (int k = 0; k < h.K; ++k) {
         a.g[k] = (const T*)h.g[k][l];
-        a.gc[k] = top ? nullptr : (const T*)h.g[k][l + 1];
+        a.gc[k] = (const T*)h.g[k][l + 1];
         a.m[k] = (const TM*)h.m[k][l];
+        a.mc[k] = (const TM*)h.m[k][l + 1];
     }
-    a.rc = top ? nullptr : (const T*)h.r[l + 1];
+    a.rc = (const T*)h.r[l + 1];
     a.r = (T*)h.r[l];
     a.pitch = h.pitch[l];
     a.plane = h.pitch[l] * h.lh[l];
-    a.cpitch = top ? 0 : h.pitch[l + 1];
-    a.cplane = top ? 0 : h.pitch[l + 1] * h.lh[l + 1];
+    a.cpitch = h.pitch[l + 1];
+    a.cplane = h.pitch[l + 1] * h.lh[l + 1];
     return a;
-}
-
-cudaError_t launch_ef_top(const EfuseHost& h, cudaStream_t st)
-{
-    const int l = h.L - 1;
-    const double px = (double)h.lw[l] * h.lh[l], ps = h.dtype == ENB_U8 ? 2.0 : 4.0;
-    note_launch("ef_top", px * (h.K * (h.C * ps + ps) + h.C * ps));
-    const dim3 g((unsigned)((h.lw[l] + 255) / 256), (unsigned)h.lh[l]);
-    if (h.dtype == ENB_U8) {
-        return launch_pdl(k_ef_top<int16_t, int16_t, 7>, g, dim3(256), st, level_args<int16_t, int16_t>(h, l));
-    }
-    return launch_pdl(k_ef_top<int32_t, int32_t, 15>, g, dim3(256), st, level_args<int32_t, int32_t>(h, l));
 }
 
 template <typename T, typename TM, int C, int F>
 static cudaError_t ef_up_t(const EfuseHost& h, int l, cudaStream_t st)
 {
     const size_t smem = win_smem(h.K, C);
-    allow_smem(k_ef_up<T, TM, C, F>, smem);
+    auto k = l + 2 == h.L ? k_ef_up<T, TM, C, F, true> : k_ef_up<T, TM, C, F, false>;
+    allow_smem(k, smem);
     const dim3 g((unsigned)((h.lw[l] + ETW - 1) / ETW), (unsigned)((h.lh[l] + ETH - 1) / ETH));
-    return launch_pdl_smem(k_ef_up<T, TM, C, F>, g, dim3(256), smem, st, level_args<T, TM>(h, l));
+    return launch_pdl_smem(k, g, dim3(256), smem, st, level_args<T, TM>(h, l));
 }
 
 cudaError_t launch_ef_up(const EfuseHost& h, int l, cudaStream_t st)
@@ -938,6 +974,7 @@ static cudaError_t ef_out0_t(const EfuseHost& h, cudaStream_t st)
         a.ipitch[k] = h.img[k].pitch;
         a.m0[k] = (const TM*)h.m[k][0];
         a.g1[k] = (const T*)h.g[k][1];
+        a.mc[k] = (const TM*)h.m[k][1];
     }
     a.mpitch = h.pitch[0];
     a.r1 = (const T*)h.r[1];
@@ -959,9 +996,10 @@ static cudaError_t ef_out0_t(const EfuseHost& h, cudaStream_t st)
     a.ovec = (uintptr_t)h.out % (size_t)PixelPair<TIn, S>::UNIT == 0 &&
              ((size_t)h.opitch * sizeof(TIn)) % (size_t)PixelPair<TIn, S>::UNIT == 0;
     const size_t smem = win_smem(h.K, C);
-    allow_smem(k_ef_out0<TIn, T, TM, C, S, F>, smem);
+    auto k = h.L == 2 ? k_ef_out0<TIn, T, TM, C, S, F, true> : k_ef_out0<TIn, T, TM, C, S, F, false>;
+    allow_smem(k, smem);
     const dim3 g((unsigned)((h.w + ETW - 1) / ETW), (unsigned)((h.h + ETH - 1) / ETH));
-    return launch_pdl_smem(k_ef_out0<TIn, T, TM, C, S, F>, g, dim3(256), smem, st, a);
+    return launch_pdl_smem(k, g, dim3(256), smem, st, a);
 }
 
 cudaError_t launch_ef_out0(const EfuseHost& h, cudaStream_t st)

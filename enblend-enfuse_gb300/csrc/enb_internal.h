@@ -303,8 +303,7 @@ struct EfuseHost {
     uint64_t seed;
 };
 cudaError_t launch_ef_weights(const EfuseHost& h, cudaStream_t st);
-cudaError_t launch_ef_reduce(const EfuseHost& h, int l, int masks, cudaStream_t st);
-cudaError_t launch_ef_top(const EfuseHost& h, cudaStream_t st);
+cudaError_t launch_ef_reduce(const EfuseHost& h, int l, cudaStream_t st);
 cudaError_t launch_ef_up(const EfuseHost& h, int l, cudaStream_t st);
 cudaError_t launch_ef_out0(const EfuseHost& h, cudaStream_t st);
 

@@ -381,24 +381,36 @@ struct ReduceJobsN {
     ReduceJob<Src, TD> j[kReduceMaxJobs];
 };
 
-template <class Src, typename TD, int C, bool ALPHA>
-__global__ void __launch_bounds__(RTHREADS, 3) k_reduce_n(const __grid_constant__ ReduceJobsN<Src, TD> jobs, int sw,
-                                                          int sh, int dw, int dh, int wrap)
+// One level of the K image pyramids (blockIdx.z < K, C channels) and of the K
+// mask pyramids in one launch: on the small levels the launches' latency is
+// what counts.  (Registers for one CTA an SM, so that all 19 rows of a column
+// item load at once, changed nothing on grids of less than a wave.)
+template <class SrcI, typename TI, int C, class SrcM, typename TM, int MODE>
+__global__ void __launch_bounds__(RTHREADS, 3) k_reduce_joint(const __grid_constant__ ReduceJobsN<SrcI, TI> img,
+                                                              const __grid_constant__ ReduceJobsN<SrcM, TM> msk, int K,
+                                                              int sw, int sh, int dw, int dh, int wrap)
 {
-    typedef typename ReduceAcc<TD>::type AC;
-    __shared__ __align__(16) AC V[ReduceSmem<C, ALPHA>::NV][RDH][RVP];
+    typedef typename ReduceAcc<TI>::type ACI;
+    typedef typename ReduceAcc<TM>::type ACM;
+    __shared__ __align__(16) ACI V[ReduceSmem<C, MODE == kReduceAlpha>::NV][RDH][RVP];
+    static_assert(sizeof(ACI) == sizeof(ACM), "the mask tile reuses the image tile's memory");
     griddep_wait();
     griddep_launch();
-    reduce_tile<Src, TD, C, ALPHA, AC>(jobs.j[blockIdx.z], blockIdx.x * RDW, blockIdx.y * RDH, sw, sh, dw, dh, wrap,
-                                       V);
+    const int z = blockIdx.z;
+    if (z < K) {
+        reduce_tile<SrcI, TI, C, MODE, ACI>(img.j[z], blockIdx.x * RDW, blockIdx.y * RDH, sw, sh, dw, dh, wrap, V);
+    } else {
+        reduce_tile<SrcM, TM, 1, MODE, ACM>(msk.j[z - K], blockIdx.x * RDW, blockIdx.y * RDH, sw, sh, dw, dh, wrap,
+                                            reinterpret_cast<ACM(*)[RDH][RVP]>(V));
+    }
 }
 
-template <class Src, typename TD, int C, bool ALPHA>
-inline cudaError_t launch_reduce_n(const ReduceJobsN<Src, TD>& jobs, int njobs, int sw, int sh, int dw, int dh,
-                                   int wrap, cudaStream_t st)
+template <class SrcI, typename TI, int C, class SrcM, typename TM, int MODE>
+inline cudaError_t launch_reduce_joint(const ReduceJobsN<SrcI, TI>& img, const ReduceJobsN<SrcM, TM>& msk, int K, int sw,
+                                       int sh, int dw, int dh, int wrap, cudaStream_t st)
 {
-    const dim3 g((unsigned)((dw + RDW - 1) / RDW), (unsigned)reduce_tile_rows(dh), (unsigned)njobs);
-    return launch_pdl(k_reduce_n<Src, TD, C, ALPHA>, g, dim3(RTHREADS), st, jobs, sw, sh, dw, dh, wrap);
+    const dim3 g((unsigned)((dw + RDW - 1) / RDW), (unsigned)reduce_tile_rows(dh), (unsigned)(2 * K));
+    return launch_pdl(k_reduce_joint<SrcI, TI, C, SrcM, TM, MODE>, g, dim3(RTHREADS), st, img, msk, K, sw, sh, dw, dh, wrap);
 }
 
 template <class Src, typename TD, int C, bool ALPHA>

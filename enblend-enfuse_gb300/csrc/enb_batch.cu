@@ -47,6 +47,7 @@ namespace enb {
 // Per-stack geometry and buffers (device table, one entry per stack).
 struct BatchStack {
     int K, w, h, L, Lc;  // exposures, size, levels, first level of the coarse kernel
+    int opaque;          // no exposure has alpha: the levels need no alpha planes
     int istride[kBatchMaxK];
     const float* img[kBatchMaxK];
     int64_t ipitch[kBatchMaxK];  // floats
@@ -72,29 +73,65 @@ struct BatchStack {
 };
 
 // Where a launch's CTAs find their stack and tile: the host-built tables of a
-// batch, or the launch's own parameters and grid for one stack (blockIdx.x, y
-// the tile, blockIdx.z the exposure of a reduce).  A single stack's launches
+// batch (BatchTable; the tables are restrict parameters of their own, or every
+// store would make the compiler read the stack's fields again), or the
+// launch's own parameters and grid for one stack (BatchOne; blockIdx.x, y the
+// tile, blockIdx.z the exposure of a reduce).  A single stack's launches
 // follow each other by programmatic dependent launch: its small levels would
 // otherwise be mostly launch gaps.
 struct BatchTable {
-    const BatchStack* stacks;
-    const int4* jobs;
     static constexpr bool kOne = false;
-    __device__ __forceinline__ const BatchStack& stack() const { return stacks[jobs[blockIdx.x].x]; }
-    __device__ __forceinline__ int2 tile() const { return make_int2(jobs[blockIdx.x].y, jobs[blockIdx.x].z); }
-    __device__ __forceinline__ int reduce_kind() const { return jobs[blockIdx.x].y; }
-    __device__ __forceinline__ int2 reduce_tile() const { return make_int2(jobs[blockIdx.x].z, jobs[blockIdx.x].w); }
 };
 
 struct BatchOne {
+    static constexpr bool kOne = true;
     BatchStack s;
     int kind0;  // kind of blockIdx.z 0
-    static constexpr bool kOne = true;
-    __device__ __forceinline__ const BatchStack& stack() const { return s; }
-    __device__ __forceinline__ int2 tile() const { return make_int2(blockIdx.x, blockIdx.y); }
-    __device__ __forceinline__ int reduce_kind() const { return kind0 + (int)blockIdx.z; }
-    __device__ __forceinline__ int2 reduce_tile() const { return tile(); }
 };
+
+// The job parameters of a launch.
+template <class J>
+struct BatchJobs {
+    const BatchStack* stacks;
+    const int4* jobs;
+    J one;
+};
+
+#define ENB_BATCH_JOBS(J) \
+    const BatchStack* __restrict__ stacks, const int4* __restrict__ jobs, const __grid_constant__ J one
+
+template <class J>
+__device__ __forceinline__ const BatchStack& job_stack(const BatchStack* stacks, const int4* jobs, const J& one)
+{
+    if constexpr (J::kOne) {
+        return one.s;
+    } else {
+        return stacks[jobs[blockIdx.x].x];
+    }
+}
+
+template <class J>
+__device__ __forceinline__ int2 job_tile(const int4* jobs)
+{
+    if constexpr (J::kOne) {
+        return make_int2(blockIdx.x, blockIdx.y);
+    } else {
+        const int4 j = jobs[blockIdx.x];
+        return make_int2(j.y, j.z);
+    }
+}
+
+// (kind, x, y) of a reduce tile
+template <class J>
+__device__ __forceinline__ int3 job_reduce(const int4* jobs, const J& one)
+{
+    if constexpr (J::kOne) {
+        return make_int3(one.kind0 + (int)blockIdx.z, blockIdx.x, blockIdx.y);
+    } else {
+        const int4 j = jobs[blockIdx.x];
+        return make_int3(j.y, j.z, j.w);
+    }
+}
 
 namespace {
 
@@ -122,7 +159,7 @@ __device__ __forceinline__ float* g0_level(const BatchStack& s, int k, int C)
 
 // Level 0 of an exposure's image pyramid (planar floats) with the input's
 // alpha plane, or opaque when there is none.
-template <int C>
+template <int C, bool A>
 struct Level0Source {
     const float* p;
     int64_t pitch, plane;
@@ -136,7 +173,7 @@ struct Level0Source {
         for (int c = 0; c < C; ++c) {
             v[c] = __ldg(&p[c * plane + o]);
         }
-        al = a ? (__ldg(&a[(int64_t)gy * apitch + gx]) != 0) : 1;
+        al = A && a ? (__ldg(&a[(int64_t)gy * apitch + gx]) != 0) : 1;
     }
 };
 
@@ -192,14 +229,14 @@ __device__ __forceinline__ void batch_normalise(const BatchStack& s, const float
 // Weights of window sizes that the pair kernel does not take: one output
 // pixel per thread on 16x16 tiles (enb_fweights.cuh).
 template <int CW, int EW, class J>
-__global__ void __launch_bounds__(256, 4) k_batch_weights(const __grid_constant__ J jobs, FloatWeightParams wp,
+__global__ void __launch_bounds__(256, 4) k_batch_weights(ENB_BATCH_JOBS(J), FloatWeightParams wp,
                                                        WeightTables tab, int hard, int C)
 {
     extern __shared__ __align__(16) unsigned char bsmem[];
     griddep_wait();
     griddep_launch();
-    const int2 tile = jobs.tile();
-    const BatchStack& s = jobs.stack();
+    const int2 tile = job_tile<J>(jobs);
+    const BatchStack& s = job_stack(stacks, jobs, one);
     const int halo = fweight_halo(wp);
     const FTile t = ftile_carve(bsmem, BWT + 2 * halo, wp.repeat_slots, wp.ent_cut);
     float* wk = reinterpret_cast<float*>(bsmem + align16(ftile_bytes(t.TW, t.slots, wp.ent_cut))) + threadIdx.x;  // [K][BWT * BWT]
@@ -236,18 +273,21 @@ __global__ void __launch_bounds__(256, 4) k_batch_weights(const __grid_constant_
 // pixel's weight waits in its exposure's level-0 mask plane (as float bits)
 // until the normalisation replaces it.  Five CTAs per SM (48 registers;
 // the 42.6 KB tile of 5x5 windows fits five times): the warps hide the
-// kernel's latencies better than more registers would.
+// kernel's latencies better than more registers would.  For the same reason the
+// tables come inside a struct, not as restrict parameters: reading the stack's
+// fields again after every store costs less than the registers that keep them
+// (16 stacks: 10.9 against 11.5 ms).
 template <int CW, int EW, int C, class J>
-__global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const __grid_constant__ J jobs, FloatWeightParams wp,
-                                                            WeightTables tab)
+__global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const __grid_constant__ BatchJobs<J> j,
+                                                               FloatWeightParams wp, WeightTables tab)
 {
     constexpr int HALO = fpair_halo(CW, EW), HX = fpair_halo_x(HALO);
     constexpr int TW = fpair_tw(CW, EW), TT = TW * fpair_th(CW, EW), NP = (TT + FPT - 1) / FPT;
     extern __shared__ __align__(16) unsigned char bsmem[];
     griddep_wait();
     griddep_launch();
-    const int2 tile = jobs.tile();
-    const BatchStack& s = jobs.stack();
+    const int2 tile = job_tile<J>(j.jobs);
+    const BatchStack& s = job_stack(j.stacks, j.jobs, j.one);
     const FTileP t0 = fpair_carve(bsmem, TW, TT, wp.repeat_slots, wp.ent_cut);
     const int px = threadIdx.x % (FPX / 2), py = threadIdx.x / (FPX / 2);
     const int x = tile.x * FPX + 2 * px, y = tile.y * FPY + py;
@@ -319,12 +359,12 @@ __global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const __grid_cons
 // thread: src/enfuse.h:1382-1385 (sum in exposure order), :1399-1442 (hard
 // mask), :1526-1535 (soft mask), into Int32 9.15 masks.
 template <class J>
-__global__ void __launch_bounds__(256) k_batch_normalise(const __grid_constant__ J jobs, int hard)
+__global__ void __launch_bounds__(256) k_batch_normalise(ENB_BATCH_JOBS(J), int hard)
 {
     griddep_wait();
     griddep_launch();
-    const int2 tile = jobs.tile();
-    const BatchStack& s = jobs.stack();
+    const int2 tile = job_tile<J>(jobs);
+    const BatchStack& s = job_stack(stacks, jobs, one);
     const int px = threadIdx.x % (FPX / 2), py = threadIdx.x / (FPX / 2);
     const int x = tile.x * FPX + 2 * px, y = tile.y * FPY + py;
     if (x >= s.w || y >= s.h) {
@@ -384,6 +424,45 @@ __global__ void __launch_bounds__(256) k_batch_normalise(const __grid_constant__
 // reduce of one image or mask tile (down sweep)
 // ---------------------------------------------------------------------------
 
+// One tile of exposure k's image pyramid; A: with its alpha.
+template <int C, bool NC, bool A>
+__device__ __forceinline__ void batch_reduce_image(const BatchStack& s, int k, int l, int X0, int Y0, int wrap,
+                                                   unsigned char* smem)
+{
+    constexpr int MODE = A ? kReduceAlpha : kReduceOpaque;
+    const int sw = s.lw[l], sh = s.lh[l], dw = s.lw[l + 1], dh = s.lh[l + 1];
+    float* dst = g_level(s, k, l + 1, C);
+    const int64_t dplane = (int64_t)s.pitch[l + 1] * dh;
+    float(*V)[RDH][RVP] = reinterpret_cast<float(*)[RDH][RVP]>(smem);
+    if (l == 0) {
+        using Src = Level0Source<C, A>;
+        const ReduceJob<Src, float> job{
+            Src{g0_level(s, k, C), s.pitch[0], (int64_t)s.pitch[0] * sh, s.alpha[k], s.apitch[k]}, dst, s.pitch[l + 1],
+            dplane, a_level(s, k, l + 1), s.pitch[l + 1]};
+        reduce_tile<Src, float, C, MODE, float>(job, X0, Y0, sw, sh, dw, dh, wrap, V);
+    } else {
+        using Src = PlanarSource<float, C, A, NC>;
+        const ReduceJob<Src, float> job{
+            Src{g_level(s, k, l, C), s.pitch[l], (int64_t)s.pitch[l] * sh, a_level(s, k, l), s.pitch[l]}, dst,
+            s.pitch[l + 1], dplane, a_level(s, k, l + 1), s.pitch[l + 1]};
+        reduce_tile<Src, float, C, MODE, float>(job, X0, Y0, sw, sh, dw, dh, wrap, V);
+    }
+}
+
+// One tile of exposure k's mask pyramid; A: with the union alpha.
+template <bool NC, bool A>
+__device__ __forceinline__ void batch_reduce_mask(const BatchStack& s, int k, int l, int X0, int Y0, int wrap,
+                                                  unsigned char* smem)
+{
+    const int sw = s.lw[l], sh = s.lh[l], dw = s.lw[l + 1], dh = s.lh[l + 1];
+    using Src = PlanarSource<int32_t, 1, A, NC>;
+    int32_t(*V)[RDH][RVP] = reinterpret_cast<int32_t(*)[RDH][RVP]>(smem);
+    const ReduceJob<Src, int32_t> job{
+        Src{m_level(s, k, l), s.pitch[l], (int64_t)s.pitch[l] * sh, s.u + s.off0[l], s.pitch[l]}, m_level(s, k, l + 1),
+        s.pitch[l + 1], (int64_t)s.pitch[l + 1] * dh, s.u + s.off0[l + 1], s.pitch[l + 1]};
+    reduce_tile<Src, int32_t, 1, A ? kReduceAlpha : kReduceOpaque, int32_t>(job, X0, Y0, sw, sh, dw, dh, wrap, V);
+}
+
 // Job kind k < K: exposure k's image; K <= kind < 2K: exposure kind-K's mask.
 // NC: the source levels are read through the read-only path (they were
 // written by an earlier launch); false inside the coarse kernel, which reads
@@ -392,33 +471,12 @@ template <int C, bool NC>
 __device__ __forceinline__ void batch_reduce_tile(const BatchStack& s, int kind, int l, int X0, int Y0, int wrap,
                                                   unsigned char* smem)
 {
-    const int sw = s.lw[l], sh = s.lh[l], dw = s.lw[l + 1], dh = s.lh[l + 1];
     if (kind < s.K) {
-        const int k = kind;
-        float* dst = g_level(s, k, l + 1, C);
-        const int64_t dplane = (int64_t)s.pitch[l + 1] * dh;
-        float(*V)[RDH][RVP] = reinterpret_cast<float(*)[RDH][RVP]>(smem);
-        if (l == 0) {
-            using Src = Level0Source<C>;
-            const ReduceJob<Src, float> job{
-                Src{g0_level(s, k, C), s.pitch[0], (int64_t)s.pitch[0] * sh, s.alpha[k], s.apitch[k]}, dst,
-                s.pitch[l + 1], dplane, a_level(s, k, l + 1), s.pitch[l + 1]};
-            reduce_tile<Src, float, C, true, float>(job, X0, Y0, sw, sh, dw, dh, wrap, V);
-        } else {
-            using Src = PlanarSource<float, C, true, NC>;
-            const ReduceJob<Src, float> job{
-                Src{g_level(s, k, l, C), s.pitch[l], (int64_t)s.pitch[l] * sh, a_level(s, k, l), s.pitch[l]}, dst,
-                s.pitch[l + 1], dplane, a_level(s, k, l + 1), s.pitch[l + 1]};
-            reduce_tile<Src, float, C, true, float>(job, X0, Y0, sw, sh, dw, dh, wrap, V);
-        }
+        s.opaque ? batch_reduce_image<C, NC, false>(s, kind, l, X0, Y0, wrap, smem)
+                 : batch_reduce_image<C, NC, true>(s, kind, l, X0, Y0, wrap, smem);
     } else {
-        const int k = kind - s.K;
-        using Src = PlanarSource<int32_t, 1, true, NC>;
-        int32_t(*V)[RDH][RVP] = reinterpret_cast<int32_t(*)[RDH][RVP]>(smem);
-        const ReduceJob<Src, int32_t> job{
-            Src{m_level(s, k, l), s.pitch[l], (int64_t)s.pitch[l] * sh, s.u + s.off0[l], s.pitch[l]},
-            m_level(s, k, l + 1), s.pitch[l + 1], (int64_t)s.pitch[l + 1] * dh, s.u + s.off0[l + 1], s.pitch[l + 1]};
-        reduce_tile<Src, int32_t, 1, true, int32_t>(job, X0, Y0, sw, sh, dw, dh, wrap, V);
+        s.opaque ? batch_reduce_mask<NC, false>(s, kind - s.K, l, X0, Y0, wrap, smem)
+                 : batch_reduce_mask<NC, true>(s, kind - s.K, l, X0, Y0, wrap, smem);
     }
 }
 
@@ -427,30 +485,26 @@ constexpr int kBatchReduceSmem = ReduceSmem<3, true>::WORDS * 4;
 // Image jobs (kind < K) and mask jobs (kind >= K) of a level run as two
 // launches, each with the registers its path needs.
 template <int C, class J>
-__global__ void __launch_bounds__(RTHREADS, 3) k_batch_reduce(const __grid_constant__ J jobs, int l, int wrap)
+__global__ void __launch_bounds__(RTHREADS, 3) k_batch_reduce(ENB_BATCH_JOBS(J), int l, int wrap)
 {
     __shared__ __align__(16) unsigned char smem[kBatchReduceSmem];
     griddep_wait();
     griddep_launch();
-    const int2 tile = jobs.reduce_tile();
-    batch_reduce_tile<C, true>(jobs.stack(), jobs.reduce_kind(), l, tile.x * RDW, tile.y * RDH, wrap, smem);
+    const int3 job = job_reduce(jobs, one);
+    batch_reduce_tile<C, true>(job_stack(stacks, jobs, one), job.x, l, job.y * RDW, job.z * RDH, wrap, smem);
 }
 
 template <class J>
-__global__ void __launch_bounds__(RTHREADS, 4) k_batch_reduce_mask(const __grid_constant__ J jobs, int l, int wrap)
+__global__ void __launch_bounds__(RTHREADS, 4) k_batch_reduce_mask(ENB_BATCH_JOBS(J), int l, int wrap)
 {
-    __shared__ __align__(16) int32_t V[ReduceSmem<1, true>::NV][RDH][RVP];
+    __shared__ __align__(16) unsigned char smem[ReduceSmem<1, true>::WORDS * 4];
     griddep_wait();
     griddep_launch();
-    const int2 tile = jobs.reduce_tile();
-    const BatchStack& s = jobs.stack();
-    const int k = jobs.reduce_kind() - s.K;
-    const int sw = s.lw[l], sh = s.lh[l], dw = s.lw[l + 1], dh = s.lh[l + 1];
-    using Src = PlanarSource<int32_t, 1, true, true>;
-    const ReduceJob<Src, int32_t> rj{
-        Src{m_level(s, k, l), s.pitch[l], (int64_t)s.pitch[l] * sh, s.u + s.off0[l], s.pitch[l]}, m_level(s, k, l + 1),
-        s.pitch[l + 1], (int64_t)s.pitch[l + 1] * dh, s.u + s.off0[l + 1], s.pitch[l + 1]};
-    reduce_tile<Src, int32_t, 1, true, int32_t>(rj, tile.x * RDW, tile.y * RDH, sw, sh, dw, dh, wrap, V);
+    const int3 job = job_reduce(jobs, one);
+    const BatchStack& s = job_stack(stacks, jobs, one);
+    const int k = job.x - s.K, X0 = job.y * RDW, Y0 = job.z * RDH;
+    s.opaque ? batch_reduce_mask<true, false>(s, k, l, X0, Y0, wrap, smem)
+             : batch_reduce_mask<true, true>(s, k, l, X0, Y0, wrap, smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -717,14 +771,15 @@ __host__ __device__ constexpr int up0_stage_floats()
 // result into the output pixels, levels >= 1 write the result level
 // (batch_up_tile's computation with the tiles streamed through the stages).
 // One stack's launch waits for its predecessor, which wrote C[l+1], only
-// after the exposures' sum: everything else is older (each launch of the
-// chain waits before it lets the next one start).
+// after the exposures' sum.  The top level's waits for the reduces before it
+// lets the next start, the others let theirs start at once: all but C[l+1]
+// is complete by then, and the sums of the small levels run side by side.
 template <int C, bool L0, class J>
-__global__ void __launch_bounds__(256, 3) k_batch_up0(const __grid_constant__ J jobs, int l, int wrap, float inv_d)
+__global__ void __launch_bounds__(256, 3) k_batch_up0(ENB_BATCH_JOBS(J), int l, int wrap, float inv_d)
 {
     extern __shared__ __align__(16) float up0smem[];
-    const int2 tile = jobs.tile();
-    const BatchStack& s = jobs.stack();
+    const int2 tile = job_tile<J>(jobs);
+    const BatchStack& s = job_stack(stacks, jobs, one);
     if (L0) {
         l = 0;
     }
@@ -750,9 +805,13 @@ __global__ void __launch_bounds__(256, 3) k_batch_up0(const __grid_constant__ J 
         }
         up0_issue<C>(s, k, l, X0, Y0, dw, dh, g_tile(b), mask_tile(b));
     };
-    if (J::kOne && top) {
-        griddep_wait();  // the reduces that wrote this level
-        griddep_launch();
+    if (J::kOne) {
+        if (top) {
+            griddep_wait();  // the reduces that wrote this level
+        }
+        if (!L0 || top) {
+            griddep_launch();
+        }
     }
     // exposures 0 and 1 (with the window of C[1]) in flight before the first merge
     if (!top && !J::kOne) {
@@ -810,7 +869,9 @@ __global__ void __launch_bounds__(256, 3) k_batch_up0(const __grid_constant__ J 
     }
     if (J::kOne && !top) {
         griddep_wait();
-        griddep_launch();
+        if (L0) {
+            griddep_launch();
+        }
         stage_window_async<C>(rwin, r_level(s, l + 1, C), sp, splane, sw, sh, I0, J0, wrap);
         cp_async_commit();
         cp_async_wait_all();
@@ -1020,6 +1081,10 @@ static BatchStack stack_of(const BatchStackHost& h, int levels, int64_t coarse_p
     s.ostride = h.ostride;
     s.oalpha = h.oalpha;
     s.oapitch = h.oapitch;
+    s.opaque = 1;
+    for (int k = 0; k < h.K; ++k) {
+        s.opaque = s.opaque && !h.alpha[k];
+    }
     level_geometry(s, coarse_pixels);
     return s;
 }
@@ -1338,7 +1403,7 @@ static cudaError_t launch_batch(void (*kernel)(KArgs...), dim3 grid, int block, 
 }
 
 template <int C, class J>
-static cudaError_t launch_weights(const J& jobs, dim3 grid, bool pair, const FloatWeightParams& wp, const WeightTables& tab,
+static cudaError_t launch_weights(const BatchJobs<J>& j, dim3 grid, bool pair, const FloatWeightParams& wp, const WeightTables& tab,
                                   int hard, size_t smem, cudaStream_t st)
 {
     cudaError_t e = cudaErrorInvalidValue;
@@ -1347,13 +1412,13 @@ static cudaError_t launch_weights(const J& jobs, dim3 grid, bool pair, const Flo
             auto k = k_batch_weights_pair<CWV, EWV, C, J>;
             // as many CTAs per SM as the shared memory holds
             cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-            e = launch_batch<J>(k, grid, FPT, smem, st, jobs, wp, tab);
+            e = launch_batch<J>(k, grid, FPT, smem, st, j, wp, tab);
         });
         return e;
     }
     const int cw = wp.use_contrast ? wp.contrast_window : 5;
     const int ew = wp.use_entropy ? wp.entropy_window : 5;
-    void (*k)(const J, FloatWeightParams, WeightTables, int, int) = k_batch_weights<0, 0, J>;
+    void (*k)(const BatchStack*, const int4*, const J, FloatWeightParams, WeightTables, int, int) = k_batch_weights<0, 0, J>;
     if (cw == 5 && ew == 5) {
         k = k_batch_weights<5, 5, J>;
     } else if (cw == 5 && ew == 3) {
@@ -1365,38 +1430,38 @@ static cudaError_t launch_weights(const J& jobs, dim3 grid, bool pair, const Flo
     } else if (ew == 3) {
         k = k_batch_weights<0, 3, J>;
     }
-    return launch_batch<J>(k, grid, BWT * BWT, smem, st, jobs, wp, tab, hard, C);
+    return launch_batch<J>(k, grid, BWT * BWT, smem, st, j.stacks, j.jobs, j.one, wp, tab, hard, C);
 }
 
 template <int C, class J>
-static cudaError_t launch_up(const J& jobs, dim3 grid, int l, int wrap, cudaStream_t st)
+static cudaError_t launch_up(const BatchJobs<J>& j, dim3 grid, int l, int wrap, cudaStream_t st)
 {
     const float inv_d = (float)(1.0 / (double)(255 << 15));
     const size_t smem = ((size_t)kUp0Stages * up0_stage_floats<C>() + (size_t)C * ESH * ESW) * sizeof(float);
     if (l == 0) {
-        return launch_batch<J>(k_batch_up0<C, true, J>, grid, 256, smem, st, jobs, 0, wrap, inv_d);
+        return launch_batch<J>(k_batch_up0<C, true, J>, grid, 256, smem, st, j.stacks, j.jobs, j.one, 0, wrap, inv_d);
     }
-    return launch_batch<J>(k_batch_up0<C, false, J>, grid, 256, smem, st, jobs, l, wrap, inv_d);
+    return launch_batch<J>(k_batch_up0<C, false, J>, grid, 256, smem, st, j.stacks, j.jobs, j.one, l, wrap, inv_d);
 }
 
 template <int C>
 static cudaError_t launch_step(const BatchPlan* p, const BatchPlan::Step& s, cudaStream_t st)
 {
-    const BatchTable jobs{p->dstacks, p->djobs + s.job0};
+    const BatchJobs<BatchTable> j{p->dstacks, p->djobs + s.job0, {}};
     const dim3 grid((unsigned)s.njobs);
     switch (s.kind) {
     case 0:
         note_launch("batch_weights", s.bytes);
-        return launch_weights<C>(jobs, grid, p->pair_weights, p->wp, p->tab, p->hard, p->wsmem, st);
+        return launch_weights<C>(j, grid, p->pair_weights, p->wp, p->tab, p->hard, p->wsmem, st);
     case 5:
         note_launch("batch_normalise", s.bytes);
-        return launch_batch<BatchTable>(k_batch_normalise<BatchTable>, grid, 256, 0, st, jobs, p->hard);
+        return launch_batch<BatchTable>(k_batch_normalise<BatchTable>, grid, 256, 0, st, j.stacks, j.jobs, j.one, p->hard);
     case 1:
         note_launch("batch_reduce", s.bytes);
-        return launch_batch<BatchTable>(k_batch_reduce<C, BatchTable>, grid, RTHREADS, 0, st, jobs, s.level, p->wrap);
+        return launch_batch<BatchTable>(k_batch_reduce<C, BatchTable>, grid, RTHREADS, 0, st, j.stacks, j.jobs, j.one, s.level, p->wrap);
     case 4:
         note_launch("batch_reduce_mask", s.bytes);
-        return launch_batch<BatchTable>(k_batch_reduce_mask<BatchTable>, grid, RTHREADS, 0, st, jobs, s.level, p->wrap);
+        return launch_batch<BatchTable>(k_batch_reduce_mask<BatchTable>, grid, RTHREADS, 0, st, j.stacks, j.jobs, j.one, s.level, p->wrap);
     case 2: {
         note_launch("batch_coarse", 0.0);
         // the queue position and the step counters start at 0 on every run
@@ -1416,7 +1481,7 @@ static cudaError_t launch_step(const BatchPlan* p, const BatchPlan::Step& s, cud
     }
     default:
         note_launch(s.level == 0 ? "batch_up0" : "batch_up", s.bytes);
-        return launch_up<C>(jobs, grid, s.level, p->wrap, st);
+        return launch_up<C>(j, grid, s.level, p->wrap, st);
     }
 }
 
@@ -1492,32 +1557,33 @@ static cudaError_t single_step(const BatchSingle* p, int i, cudaStream_t st)
     const auto tiles = [](int w, int h, int tx, int ty, int z) {
         return dim3((unsigned)((w + tx - 1) / tx), (unsigned)((h + ty - 1) / ty), (unsigned)z);
     };
-    BatchOne jobs{s, 0};
+    BatchJobs<BatchOne> j{nullptr, nullptr, BatchOne{s, 0}};
     const double img = K * (px * (4.0 * C + (l == 0 ? 0.0 : 1.0)) + up * (4.0 * C + 1.0)), msk = K * (px + up) * 4.0 + px + up;
     switch (p->steps[(size_t)i].kind) {
     case 0:
         note_launch("batch_weights", K * px * (4.0 * s.istride[0] + 4.0 * C + 4.0) + px);
-        return launch_weights<C>(jobs, tiles(s.w, s.h, p->ws.tx, p->ws.ty, 1), p->ws.pair, p->wp, p->tab, p->hard, p->ws.smem, st);
+        return launch_weights<C>(j, tiles(s.w, s.h, p->ws.tx, p->ws.ty, 1), p->ws.pair, p->wp, p->tab, p->hard, p->ws.smem, st);
     case 1:
         note_launch("batch_normalise", K * px * 12.0);
-        return launch_batch<BatchOne>(k_batch_normalise<BatchOne>, tiles(s.w, s.h, FPX, FPY, 1), 256, 0, st, jobs, p->hard);
+        return launch_batch<BatchOne>(k_batch_normalise<BatchOne>, tiles(s.w, s.h, FPX, FPY, 1), 256, 0, st, j.stacks, j.jobs, j.one,
+                                      p->hard);
     case 2:
         note_launch("batch_reduce", img);
         return launch_batch<BatchOne>(k_batch_reduce<C, BatchOne>, tiles(s.lw[l + 1], s.lh[l + 1], RDW, RDH, K), RTHREADS, 0, st,
-                                      jobs, l, p->wrap);
+                                      j.stacks, j.jobs, j.one, l, p->wrap);
     case 3:
         note_launch("batch_reduce_mask", msk);
-        jobs.kind0 = K;
+        j.one.kind0 = K;
         return launch_batch<BatchOne>(k_batch_reduce_mask<BatchOne>, tiles(s.lw[l + 1], s.lh[l + 1], RDW, RDH, K), RTHREADS, 0, st,
-                                      jobs, l, p->wrap);
+                                      j.stacks, j.jobs, j.one, l, p->wrap);
     case 4:
         note_launch("batch_reduce", img + msk);
         return launch_batch<BatchOne>(k_batch_reduce<C, BatchOne>, tiles(s.lw[l + 1], s.lh[l + 1], RDW, RDH, 2 * K), RTHREADS, 0, st,
-                                      jobs, l, p->wrap);
+                                      j.stacks, j.jobs, j.one, l, p->wrap);
     default:
         note_launch(l == 0 ? "batch_up0" : "batch_up",
                     K * (px * (4.0 * C + 4.0) + up * 4.0 * C) + up * 4.0 * C + px * (l == 0 ? 4.0 * s.ostride + 1.0 : 4.0 * C));
-        return launch_up<C>(jobs, tiles(s.lw[l], s.lh[l], ETW, ETH, 1), l, p->wrap, st);
+        return launch_up<C>(j, tiles(s.lw[l], s.lh[l], ETW, ETH, 1), l, p->wrap, st);
     }
 }
 

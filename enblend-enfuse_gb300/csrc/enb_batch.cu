@@ -1020,6 +1020,12 @@ struct BatchPlan {
     unsigned int* err = nullptr;   // the context's device error word
     int maxK = 1;
     bool pair_weights = false;  // the weights step runs k_batch_weights_pair
+    // the stack table on the host, and two pinned copies that rebinding
+    // uploads in turn, each guarded by the event of its last upload
+    std::vector<BatchStack> stacks;
+    BatchStack* pinned = nullptr;
+    cudaEvent_t uploaded[2] = {nullptr, nullptr};
+    int slot = 0;
     struct Step {
         int kind;  // 0 weights, 5 normalisation, 1 image reduce, 4 mask reduce, 2 coarse, 3 up
         int level;
@@ -1060,15 +1066,9 @@ void level_geometry(BatchStack& s, int64_t coarse_pixels)
 
 }  // namespace
 
-// Sizes, levels and buffers of a stack's images and output.
-static BatchStack stack_of(const BatchStackHost& h, int levels, int64_t coarse_pixels)
+// A stack's images, alpha planes and output.
+static void stack_pixels(BatchStack& s, const BatchStackHost& h)
 {
-    BatchStack s;
-    std::memset(&s, 0, sizeof s);
-    s.K = h.K;
-    s.w = h.w;
-    s.h = h.h;
-    s.L = enb_num_levels(h.w, h.h, 1, levels);
     for (int k = 0; k < h.K; ++k) {
         s.img[k] = h.img[k];
         s.ipitch[k] = h.ipitch[k];
@@ -1085,6 +1085,18 @@ static BatchStack stack_of(const BatchStackHost& h, int levels, int64_t coarse_p
     for (int k = 0; k < h.K; ++k) {
         s.opaque = s.opaque && !h.alpha[k];
     }
+}
+
+// Sizes, levels and buffers of a stack's images and output.
+static BatchStack stack_of(const BatchStackHost& h, int levels, int64_t coarse_pixels)
+{
+    BatchStack s;
+    std::memset(&s, 0, sizeof s);
+    s.K = h.K;
+    s.w = h.w;
+    s.h = h.h;
+    s.L = enb_num_levels(h.w, h.h, 1, levels);
+    stack_pixels(s, h);
     level_geometry(s, coarse_pixels);
     return s;
 }
@@ -1144,7 +1156,42 @@ void batch_plan_destroy(BatchPlan* p)
         return;
     }
     cudaFree(p->work);
+    for (cudaEvent_t e : p->uploaded) {
+        if (e) {
+            cudaEventSynchronize(e);
+            cudaEventDestroy(e);
+        }
+    }
+    cudaFreeHost(p->pinned);
     delete p;
+}
+
+cudaError_t batch_plan_rebind(BatchPlan* p, const std::vector<BatchStackHost>& hs, cudaStream_t st)
+{
+    const size_t n = p->stacks.size();
+    if (!p->pinned) {
+        cudaError_t e = cudaMallocHost((void**)&p->pinned, 2 * n * sizeof(BatchStack));
+        for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+            e = p->uploaded[i] ? cudaSuccess : cudaEventCreateWithFlags(&p->uploaded[i], cudaEventDisableTiming);
+        }
+        if (e != cudaSuccess) {
+            cudaFreeHost(p->pinned);
+            p->pinned = nullptr;
+            return e;
+        }
+    }
+    p->slot ^= 1;
+    cudaError_t e = cudaEventSynchronize(p->uploaded[p->slot]);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    BatchStack* to = p->pinned + (size_t)p->slot * n;
+    for (size_t i = 0; i < n; ++i) {
+        stack_pixels(p->stacks[i], hs[i]);
+        to[i] = p->stacks[i];
+    }
+    e = cudaMemcpyAsync(p->dstacks, to, n * sizeof(BatchStack), cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? cudaEventRecord(p->uploaded[p->slot], st) : e;
 }
 
 cudaError_t batch_plan_create(const std::vector<BatchStackHost>& hs, const FloatWeightParams& wp,
@@ -1377,6 +1424,7 @@ cudaError_t batch_plan_create(const std::vector<BatchStackHost>& hs, const Float
         batch_plan_destroy(p);
         return e;
     }
+    p->stacks = std::move(stacks);
     *out = p;
     return cudaSuccess;
 }

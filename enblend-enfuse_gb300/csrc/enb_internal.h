@@ -328,6 +328,8 @@ cudaError_t batch_plan_create(const std::vector<BatchStackHost>& stacks, const F
                               const WeightTables& tab, int levels, int wrap, int hard, int64_t coarse_pixels,
                               unsigned int* err, cudaStream_t st, BatchPlan** out);
 void batch_plan_destroy(BatchPlan* p);
+// The plan's stacks on other buffers (the same sizes, layouts and planes).
+cudaError_t batch_plan_rebind(BatchPlan* p, const std::vector<BatchStackHost>& stacks, cudaStream_t st);
 int batch_plan_steps(const BatchPlan* p);
 double batch_plan_pixels(const BatchPlan* p);
 cudaError_t batch_plan_launch(const BatchPlan* p, int step, cudaStream_t st);

@@ -173,3 +173,40 @@ def test_level_schedule_autotuner(ctx):
         assert torch.equal(a, b)
     with pytest.raises(Exception):
         ctx.tune_stacks(dev, params=p, candidates=[0])
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_batch_on_other_buffers(ctx, graph):
+    """Batches of one geometry on changing buffers: outputs, alpha planes and row pitches other than the call
+    before's, calls in a row without a wait, and another stream; each against the plain per-stack path."""
+    import enbgpu
+    shapes = [(37, 53, 3), (130, 67, 5), (64, 40, 2)]
+    p = _params()
+    sets = []
+    for i in range(4):
+        stacks = []
+        for st in _batch(seed=60 + 7 * i, shapes=shapes):
+            pad = 0 if i % 2 == 0 else 3
+            stacks.append([_dev(np.pad(x, [(0, 0), (0, pad), (0, 0)]))[:, :x.shape[1]] for x in st])
+        rng = np.random.default_rng(i)
+        alphas = [[_dev(np.where(rng.random(x.shape[:2]) < 0.9, 255, 0).astype(np.uint8)) for x in st] for st in stacks]
+        want = ctx.fuse_stacks(stacks, params=p, alphas=alphas, plain=True)
+        want_opaque = ctx.fuse_stacks(stacks, params=p, plain=True)
+        sets.append((stacks, alphas, [w.clone() for w in want], [w.clone() for w in want_opaque]))
+    side = torch.cuda.Stream()
+    for use_alpha in (True, False):
+        got = []
+        for i in (0, 1, 2, 3, 0, 3, 2, 2):
+            stacks, alphas, _, _ = sets[i]
+            outs = [torch.full(tuple(st[0].shape), -1.0, device="cuda") for st in stacks]
+            if len(got) == 4:
+                torch.cuda.synchronize()
+                ctx.set_stream(side.cuda_stream)
+            ctx.fuse_stacks(stacks, params=p, outs=outs, alphas=alphas if use_alpha else None, graph=graph)
+            got.append((i, outs))
+        ctx.synchronize()
+        ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        for i, outs in got:
+            for o, w in zip(outs, sets[i][2 if use_alpha else 3]):
+                assert torch.equal(o, w), i

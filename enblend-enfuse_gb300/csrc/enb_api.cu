@@ -1088,9 +1088,18 @@ enb_status enblend_fused(enb_ctx* ctx, const enb_image* white, const enb_image* 
             ch.wrap = wrap;
             ENB_LAUNCH(ctx, launch_coarse(ch, ctx->stream));
             up_from = first - 1;
+        } else if (NL >= 2 && up_late_level(level_view(rr.p, NL - 2))) {
+            // Up sweep (src/blend.h:81-121, src/pyramid.h:1758-1784): the small
+            // levels, the top's blend in the first of them
+            for (; up_from >= 0 && up_late_level(level_view(rr.p, up_from)); --up_from) {
+                const int j = up_from;
+                ENB_LAUNCH(ctx, launch_up_late(level_view(gw.p, j + 1), level_view(gb.p, j + 1), level_view(mg.p, j + 1),
+                                               level_view(rr.p, j + 1), level_view(mg.p, j), level_view(gw.p, j),
+                                               level_view(gb.p, j), level_view(rr.p, j), white_value, wrap, j == NL - 2,
+                                               ctx->stream));
+            }
         } else {
-            // Up sweep: top level blend, then Laplacian + blend + collapse per
-            // level (src/blend.h:81-121, src/pyramid.h:1758-1784).
+            // top level blend, then Laplacian + blend + collapse per level
             ENB_LAUNCH(ctx, launch_blend_into(level_view(mg.p, NL - 1), level_view(gw.p, NL - 1),
                                               level_view(gb.p, NL - 1), level_view(rr.p, NL - 1), white_value,
                                               ctx->stream));

@@ -151,176 +151,38 @@ __global__ void __launch_bounds__(256, 3) k_ef_weights(const __grid_constant__ E
 }
 
 // ---------------------------------------------------------------------------
-// staging and expansion of coarse windows
+// the top level and pixel pairs
 // ---------------------------------------------------------------------------
 
-// The coarse window of a 64x16 tile: the (ESH x ESW) taps from (I0 - 1,
-// J0 - 1) of each plane, one or two of them per thread.  Taps outside the
-// level are stored as 0 (and x is periodic when wrap), which makes the
-// interior numerators of expand9 those of the border positions
-// (expand_hweights / expand_vweights) too; the one other weight there, 4 at
-// the seam of a periodic level of odd width, goes into the stored tap, as no
-// other position reads it.  (Coarse levels are at least five pixels wide, so
-// the rule for a single periodic column does not arise.)
-struct EfWindow {
-    int64_t o[2];  // offset of the tap in a coarse plane
-    int32_t f[2];  // factor of the stored tap: 0, 1 or 4
-    bool two;
-    __device__ __forceinline__ EfWindow(int I0, int J0, int cw, int ch, int64_t cpitch, int dw, int wrap)
-    {
-        two = threadIdx.x + 256 < ESH * ESW;
+// R of the top level, sum_k fromRealPromote(G_k M_k / D), at the thread's
+// taps, from the staged windows of the K image pyramids (one level of a
+// few pixels, not worth a launch and a trip through memory)
+template <typename T, typename TM, int C, int F>
+__device__ __forceinline__ void ef_top(const TileWindow& win, int32_t (*ss)[ESH][ESW], const TM* const* m, int K,
+                                       int32_t (&v)[C][2])
+{
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        v[c][0] = v[c][1] = 0;
+    }
+    for (int k = 0; k < K; ++k) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            const int k = min((int)threadIdx.x + 256 * u, ESH * ESW - 1);
-            const int r = k / ESW, c = k - r * ESW;
-            const int j = J0 - 1 + r;
-            int i = I0 - 1 + c;
-            f[u] = wrap && (dw & 1) && (i == -1 || i == cw) ? 4 : 1;
-            if (wrap) {
-                i = imod(i, cw);
+            if (win.f[u] == 0 || (u == 1 && !win.two)) {
+                continue;
             }
-            f[u] = j >= 0 && j < ch && i >= 0 && i < cw ? f[u] : 0;
-            o[u] = (int64_t)min(max(j, 0), ch - 1) * cpitch + min(max(i, 0), cw - 1);
-        }
-    }
-    template <typename T, int C>
-    __device__ __forceinline__ void load(const T* __restrict__ p, int64_t cplane, int32_t (&v)[C][2]) const
-    {
+            const int32_t mv = (int32_t)__ldg(&m[k][win.o[u]]);
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                v[c][u] = (int32_t)__ldg(&p[c * cplane + o[u]]);
+            for (int c = 0; c < C; ++c) {
+                const int32_t g = (&ss[k * C + c][0][0])[threadIdx.x + 256 * u] / win.f[u];
+                v[c][u] += (int32_t)mask_multiply<T, F>(g, mv);
             }
         }
     }
-    // a plane that the launch before wrote: not through the read-only path,
-    // whose loads could be moved above the wait
-    template <typename T, int C>
-    __device__ __forceinline__ void load_written(const T* p, int64_t cplane, int32_t (&v)[C][2]) const
-    {
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                v[c][u] = (int32_t)__ldcg(&p[c * cplane + o[u]]);
-            }
-        }
-    }
-    template <int C>
-    __device__ __forceinline__ void store(int32_t (*ss)[ESH][ESW], const int32_t (&v)[C][2]) const
-    {
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            (&ss[c][0][0])[threadIdx.x] = v[c][0] * f[0];
-            if (two) {
-                (&ss[c][0][0])[threadIdx.x + 256] = v[c][1] * f[1];
-            }
-        }
-    }
-    // R of the top level, sum_k fromRealPromote(G_k M_k / D), at the thread's
-    // taps, from the staged windows of the K image pyramids (one level of a
-    // few pixels, not worth a launch and a trip through memory)
-    template <typename T, typename TM, int C, int F>
-    __device__ __forceinline__ void top(int32_t (*ss)[ESH][ESW], const TM* const* m, int K, int32_t (&v)[C][2]) const
-    {
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            v[c][0] = v[c][1] = 0;
-        }
-        for (int k = 0; k < K; ++k) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                if (f[u] == 0 || (u == 1 && !two)) {
-                    continue;
-                }
-                const int32_t mv = (int32_t)__ldg(&m[k][o[u]]);
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    const int32_t g = (&ss[k * C + c][0][0])[threadIdx.x + 256 * u] / f[u];
-                    v[c][u] += (int32_t)mask_multiply<T, F>(g, mv);
-                }
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            v[c][0] = (int32_t)cast_store<T>(v[c][0]);
-            v[c][1] = (int32_t)cast_store<T>(v[c][1]);
-        }
-    }
-    // the windows of the K image pyramids, four exposures' loads in flight
-    template <typename T, int C>
-    __device__ __forceinline__ void stage(int32_t (*ss)[ESH][ESW], const T* const* g, int64_t cplane, int K) const
-    {
-        constexpr int B = 4;
-        for (int k0 = 0; k0 < K; k0 += B) {
-            int32_t v[B][C][2];
-#pragma unroll
-            for (int u = 0; u < B; ++u) {
-                load<T, C>(g[min(k0 + u, K - 1)], cplane, v[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < B; ++u) {
-                if (k0 + u < K) {
-                    store<C>(ss + (k0 + u) * C, v[u]);
-                }
-            }
-        }
-    }
-};
-
-// Divisors of a quad's four expansions (divided by the (4,4) taps' common
-// factor, as in expand9), as entries of g_div_table.
-struct EfDivisors {
-    static constexpr bool value = false;
-    uint64_t d[4];
-    __device__ __forceinline__ EfDivisors(int X, int Y, int cw, int ch, int dw, int wrap)
-    {
-        int w[3], he, ho, ve, vo;
-        expand_hweights(X, cw, dw, wrap, w, he);
-        expand_hweights(X + 1, cw, dw, wrap, w, ho);
-        expand_vweights(Y, ch, w, ve);
-        expand_vweights(Y + 1, ch, w, vo);
-        ho >>= 2;
-        d[0] = __ldg(&g_div_table.e[he * ve]);
-        d[1] = __ldg(&g_div_table.e[ho * ve]);
-        d[2] = __ldg(&g_div_table.e[he * vo]);
-        d[3] = __ldg(&g_div_table.e[ho * vo]);
-    }
-};
-
-// All neighbourhoods of the tile lie inside the coarse level: the divisors
-// are 64, 16, 16 and 4.
-struct EfInside {
-    static constexpr bool value = true;
-};
-
-// Expansion of the quad at (qx, qy) of a staged window.
-template <bool NONNEG, class DIV>
-__device__ __forceinline__ void ef_expand(const int32_t (*s)[ESW], int qx, int qy, const DIV& div, int32_t e[4])
-{
-    int32_t v[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            v[r][c] = s[qy + r][qx + c];
-        }
-    }
-    if constexpr (DIV::value) {
-        expand9<NONNEG>(v, e);
-        return;
-    } else {
-    const int32_t ea = v[0][0] + 6 * v[0][1] + v[0][2], eb = v[1][0] + 6 * v[1][1] + v[1][2],
-                  ec = v[2][0] + 6 * v[2][1] + v[2][2];
-    const int32_t oa = v[0][1] + v[0][2], ob = v[1][1] + v[1][2], oc = v[2][1] + v[2][2];
-    const int32_t n[4] = {ea + 6 * eb + ec, oa + 6 * ob + oc, eb + ec, ob + oc};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint32_t a = !NONNEG && n[q] < 0 ? 0u - (uint32_t)n[q] : (uint32_t)n[q];
-        const uint32_t t = (uint32_t)(((uint64_t)a * (uint32_t)div.d[q]) >> (uint32_t)(div.d[q] >> 32));
-        e[q] = !NONNEG && n[q] < 0 ? -(int32_t)t : (int32_t)t;
-    }
+    for (int c = 0; c < C; ++c) {
+        v[c][0] = (int32_t)cast_store<T>(v[c][0]);
+        v[c][1] = (int32_t)cast_store<T>(v[c][1]);
     }
 }
 
@@ -455,7 +317,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_up(const __grid_constant__ EfLeve
     };
     int32_t m[4], g[C][4];
     fetch(0, m, g);
-    const EfWindow win(I0, J0, a.cw, a.ch, a.cpitch, a.dw, a.wrap);
+    const TileWindow win(I0, J0, a.cw, a.ch, a.cpitch, a.dw, a.wrap);
     win.stage<T, C>(ss, a.gc, a.cplane, K);
     const bool interior = interior_tile(X0, Y0, a.dw, a.dh, I0, J0, a.cw, a.ch);
     __syncthreads();
@@ -467,7 +329,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_up(const __grid_constant__ EfLeve
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 int32_t e[4];
-                ef_expand<true>(ss[k * C + c], qx, qy, div, e);
+                expand_window<true>(ss[k * C + c], qx, qy, div, e);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int32_t lp = (int32_t)cast_store<T>((int64_t)g[c][q] - e[q]);
@@ -486,16 +348,16 @@ __global__ void __launch_bounds__(256, 3) k_ef_up(const __grid_constant__ EfLeve
     };
     if (on) {
         if (interior) {
-            sum(EfInside());
+            sum(QuadInside());
         } else {
-            sum(EfDivisors(X, Y, a.cw, a.ch, a.dw, a.wrap));
+            sum(QuadDivisors(X, Y, a.cw, a.ch, a.dw, a.wrap));
         }
     }
     griddep_wait();
     {
         int32_t v[C][2];
         if constexpr (FOLD) {
-            win.top<T, TM, C, F>(ss, a.mc, K, v);
+            ef_top<T, TM, C, F>(win, ss, a.mc, K, v);
         } else {
             win.load_written<T, C>(a.rc, a.cplane, v);
         }
@@ -509,9 +371,9 @@ __global__ void __launch_bounds__(256, 3) k_ef_up(const __grid_constant__ EfLeve
     for (int c = 0; c < C; ++c) {
         int32_t e[4];
         if (interior) {
-            ef_expand<false>(ss[K * C + c], qx, qy, EfInside(), e);
+            expand_window<false>(ss[K * C + c], qx, qy, QuadInside(), e);
         } else {
-            ef_expand<false>(ss[K * C + c], qx, qy, EfDivisors(X, Y, a.cw, a.ch, a.dw, a.wrap), e);
+            expand_window<false>(ss[K * C + c], qx, qy, QuadDivisors(X, Y, a.cw, a.ch, a.dw, a.wrap), e);
         }
         T r[4];
 #pragma unroll
@@ -618,7 +480,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
     int32_t m[4];
     TIn px[4][S];
     fetch(0, m, px);
-    const EfWindow win(I0, J0, a.cw, a.ch, a.cpitch, a.w, a.wrap);
+    const TileWindow win(I0, J0, a.cw, a.ch, a.cpitch, a.w, a.wrap);
     win.stage<T, C>(ss, a.g1, a.cplane, K);
     const bool interior = interior_tile(X0, Y0, a.w, a.h, I0, J0, a.cw, a.ch);
     __syncthreads();
@@ -631,7 +493,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 int32_t e[4];
-                ef_expand<true>(ss[k * C + c], qx, qy, div, e);
+                expand_window<true>(ss[k * C + c], qx, qy, div, e);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     // copyToPyramidImage: v << 7 (src/fixmath.h:197-202)
@@ -651,9 +513,9 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
     };
     if (on) {
         if (interior) {
-            sum(EfInside());
+            sum(QuadInside());
         } else {
-            sum(EfDivisors(X, Y, a.cw, a.ch, a.w, a.wrap));
+            sum(QuadDivisors(X, Y, a.cw, a.ch, a.w, a.wrap));
         }
     }
     griddep_wait();
@@ -661,7 +523,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
     {
         int32_t v[C][2];
         if constexpr (FOLD) {
-            win.top<T, TM, C, F>(ss, a.mc, K, v);
+            ef_top<T, TM, C, F>(win, ss, a.mc, K, v);
         } else {
             win.load_written<T, C>(a.r1, a.cplane, v);
         }
@@ -676,9 +538,9 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
     for (int c = 0; c < C; ++c) {
         int32_t e[4];
         if (interior) {
-            ef_expand<false>(ss[K * C + c], qx, qy, EfInside(), e);
+            expand_window<false>(ss[K * C + c], qx, qy, QuadInside(), e);
         } else {
-            ef_expand<false>(ss[K * C + c], qx, qy, EfDivisors(X, Y, a.cw, a.ch, a.w, a.wrap), e);
+            expand_window<false>(ss[K * C + c], qx, qy, QuadDivisors(X, Y, a.cw, a.ch, a.w, a.wrap), e);
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {

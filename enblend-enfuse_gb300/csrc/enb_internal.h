@@ -269,6 +269,12 @@ cudaError_t launch_blend_into(const PlanarView& mask, const PlanarView& gw, cons
 cudaError_t launch_up_level(const PlanarView& gw1, const PlanarView& gb1, const PlanarView& r1,
                             const PlanarView& mask, const PlanarView& gw, const PlanarView& gb,
                             const PlanarView& r, int32_t white_value, int wrap, cudaStream_t st);
+// a small level, with the launches of the levels above in flight; top: level
+// l + 1 is the top, its R is formed here (r1 gives only its layout)
+bool up_late_level(const PlanarView& r);
+cudaError_t launch_up_late(const PlanarView& gw1, const PlanarView& gb1, const PlanarView& m1, const PlanarView& r1,
+                           const PlanarView& m, const PlanarView& gw, const PlanarView& gb, const PlanarView& r, int32_t wv,
+                           int wrap, bool top, cudaStream_t st);
 cudaError_t launch_out0(const PlanarView* gw1, const PlanarView* gb1, const PlanarView* r1, const Out0Host& h,
                         cudaStream_t st, int ty0 = 0, int nty = -1);
 cudaError_t launch_coarse(const CoarseHost& h, cudaStream_t st);

@@ -34,7 +34,7 @@ struct CoarseLevels {
 // planes; loads unrolled and independent of each other.
 template <int NP, typename T, bool NC, int NT>
 __device__ __forceinline__ void stage_coarse(int32_t (*ss)[ESH][ESW], const CoarseLevels& cl, int I0, int J0,
-                                             int wrap)
+                                             int dw, int wrap)
 {
     constexpr int N = ESH * ESW;
     constexpr int IT = (N + NT - 1) / NT;
@@ -45,6 +45,7 @@ __device__ __forceinline__ void stage_coarse(int32_t (*ss)[ESH][ESW], const Coar
             const int r = k / ESW, c = k - r * ESW;
             const int j = J0 - 1 + r;
             int i = I0 - 1 + c;
+            const int32_t f = wrap && (dw & 1) && (i == -1 || i == cl.w) ? 4 : 1;  // as TileWindow
             if (wrap) {
                 i = imod(i, cl.w);
             }
@@ -55,35 +56,9 @@ __device__ __forceinline__ void stage_coarse(int32_t (*ss)[ESH][ESW], const Coar
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
                 const int32_t v = (int32_t)ld_src<NC>(&reinterpret_cast<const T*>(cl.p[p])[o]);
-                ss[p][r][c] = in ? v : 0;
+                ss[p][r][c] = in ? v * f : 0;
             }
         }
-    }
-}
-
-// Expansion of the four destination pixels of the quad at tile position
-// (qx, qy) from one staged coarse plane (the 3x3 source neighbourhood), with
-// the border weights and divisors of expand_hweights / expand_vweights.
-__device__ __forceinline__ void expand_quad(const int32_t (*s)[ESW], int qx, int qy, int X, int Y, int sw, int sh,
-                                            int dw, int dh, int wrap, int32_t e[4])
-{
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int XX = X + (q & 1), YY = Y + (q >> 1);
-        e[q] = 0;
-        if (XX >= dw || YY >= dh) {
-            continue;
-        }
-        int vw[3], vden, hw[3], hden;
-        expand_vweights(YY, sh, vw, vden);
-        expand_hweights(XX, sw, dw, wrap, hw, hden);
-        int32_t num = 0;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const int32_t* row = &s[qy + a][qx];
-            num += vw[a] * (hw[0] * row[0] + hw[1] * row[1] + hw[2] * row[2]);
-        }
-        e[q] = div_den(num, hden * vden);
     }
 }
 
@@ -138,6 +113,146 @@ __device__ __forceinline__ void expand9(const int32_t (&v)[3][3], int32_t e[4])
         e[1] = n1 / 16;
         e[2] = n2 / 16;
         e[3] = n3 / 4;
+    }
+}
+
+// The coarse window of a 64x16 tile: the (ESH x ESW) taps from (I0 - 1,
+// J0 - 1) of each plane, one or two of them per thread.  Taps outside the
+// level are stored as 0 (and x is periodic when wrap), which makes the
+// interior numerators of expand9 those of the border positions
+// (expand_hweights / expand_vweights) too; the one other weight there, 4 at
+// the seam of a periodic level of odd width, goes into the stored tap, as no
+// other position reads it.  (Coarse levels are at least five pixels wide, so
+// the rule for a single periodic column does not arise.)
+struct TileWindow {
+    int64_t o[2];  // offset of the tap in a coarse plane
+    int32_t f[2];  // factor of the stored tap: 0, 1 or 4
+    bool two;
+    __device__ __forceinline__ TileWindow(int I0, int J0, int cw, int ch, int64_t cpitch, int dw, int wrap)
+    {
+        two = threadIdx.x + 256 < ESH * ESW;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int k = min((int)threadIdx.x + 256 * u, ESH * ESW - 1);
+            const int r = k / ESW, c = k - r * ESW;
+            const int j = J0 - 1 + r;
+            int i = I0 - 1 + c;
+            f[u] = wrap && (dw & 1) && (i == -1 || i == cw) ? 4 : 1;
+            if (wrap) {
+                i = imod(i, cw);
+            }
+            f[u] = j >= 0 && j < ch && i >= 0 && i < cw ? f[u] : 0;
+            o[u] = (int64_t)min(max(j, 0), ch - 1) * cpitch + min(max(i, 0), cw - 1);
+        }
+    }
+    template <typename T, int C>
+    __device__ __forceinline__ void load(const T* __restrict__ p, int64_t cplane, int32_t (&v)[C][2]) const
+    {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                v[c][u] = (int32_t)__ldg(&p[c * cplane + o[u]]);
+            }
+        }
+    }
+    // a plane that the launch before wrote: not through the read-only path,
+    // whose loads could be moved above the wait
+    template <typename T, int C>
+    __device__ __forceinline__ void load_written(const T* p, int64_t cplane, int32_t (&v)[C][2]) const
+    {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                v[c][u] = (int32_t)__ldcg(&p[c * cplane + o[u]]);
+            }
+        }
+    }
+    template <int C>
+    __device__ __forceinline__ void store(int32_t (*ss)[ESH][ESW], const int32_t (&v)[C][2]) const
+    {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            (&ss[c][0][0])[threadIdx.x] = v[c][0] * f[0];
+            if (two) {
+                (&ss[c][0][0])[threadIdx.x + 256] = v[c][1] * f[1];
+            }
+        }
+    }
+    // the windows of the K image pyramids, four exposures' loads in flight
+    template <typename T, int C>
+    __device__ __forceinline__ void stage(int32_t (*ss)[ESH][ESW], const T* const* g, int64_t cplane, int K) const
+    {
+        constexpr int B = 4;
+        for (int k0 = 0; k0 < K; k0 += B) {
+            int32_t v[B][C][2];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                load<T, C>(g[min(k0 + u, K - 1)], cplane, v[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                if (k0 + u < K) {
+                    store<C>(ss + (k0 + u) * C, v[u]);
+                }
+            }
+        }
+    }
+};
+
+// Divisors of a quad's four expansions (divided by the (4,4) taps' common
+// factor, as in expand9), as entries of g_div_table.
+struct QuadDivisors {
+    static constexpr bool value = false;
+    uint64_t d[4];
+    __device__ __forceinline__ QuadDivisors(int X, int Y, int cw, int ch, int dw, int wrap)
+    {
+        int w[3], he, ho, ve, vo;
+        expand_hweights(X, cw, dw, wrap, w, he);
+        expand_hweights(X + 1, cw, dw, wrap, w, ho);
+        expand_vweights(Y, ch, w, ve);
+        expand_vweights(Y + 1, ch, w, vo);
+        ho >>= 2;
+        d[0] = __ldg(&g_div_table.e[he * ve]);
+        d[1] = __ldg(&g_div_table.e[ho * ve]);
+        d[2] = __ldg(&g_div_table.e[he * vo]);
+        d[3] = __ldg(&g_div_table.e[ho * vo]);
+    }
+};
+
+// All neighbourhoods of the tile lie inside the coarse level: the divisors
+// are 64, 16, 16 and 4.
+struct QuadInside {
+    static constexpr bool value = true;
+};
+
+// Expansion of the quad at (qx, qy) of a staged window.
+template <bool NONNEG, class DIV>
+__device__ __forceinline__ void expand_window(const int32_t (*s)[ESW], int qx, int qy, const DIV& div, int32_t e[4])
+{
+    int32_t v[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            v[r][c] = s[qy + r][qx + c];
+        }
+    }
+    if constexpr (DIV::value) {
+        expand9<NONNEG>(v, e);
+        return;
+    } else {
+    const int32_t ea = v[0][0] + 6 * v[0][1] + v[0][2], eb = v[1][0] + 6 * v[1][1] + v[1][2],
+                  ec = v[2][0] + 6 * v[2][1] + v[2][2];
+    const int32_t oa = v[0][1] + v[0][2], ob = v[1][1] + v[1][2], oc = v[2][1] + v[2][2];
+    const int32_t n[4] = {ea + 6 * eb + ec, oa + 6 * ob + oc, eb + ec, ob + oc};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint32_t a = !NONNEG && n[q] < 0 ? 0u - (uint32_t)n[q] : (uint32_t)n[q];
+        const uint32_t t = (uint32_t)(((uint64_t)a * (uint32_t)div.d[q]) >> (uint32_t)(div.d[q] >> 32));
+        e[q] = !NONNEG && n[q] < 0 ? -(int32_t)t : (int32_t)t;
+    }
     }
 }
 
@@ -330,17 +445,18 @@ __device__ __forceinline__ void up_tile(const CoarseLevels& cl, const TM* __rest
             fb[c][q] = (int32_t)ld_src<NC>(&gb[c * plane + o]);
         }
     }
-    stage_coarse<3 * C, T, NC, NT>(ss, cl, I0, J0, wrap);
+    stage_coarse<3 * C, T, NC, NT>(ss, cl, I0, J0, w, wrap);
     __syncthreads();
     if (!active || X >= w || Y >= h) {
         return;
     }
+    const QuadDivisors div(X, Y, cl.w, cl.h, w, wrap);
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         int32_t ew[4], eb[4], er[4];
-        expand_quad(ss[c], qx, qy, X, Y, cl.w, cl.h, w, h, wrap, ew);
-        expand_quad(ss[C + c], qx, qy, X, Y, cl.w, cl.h, w, h, wrap, eb);
-        expand_quad(ss[2 * C + c], qx, qy, X, Y, cl.w, cl.h, w, h, wrap, er);
+        expand_window<true>(ss[c], qx, qy, div, ew);
+        expand_window<true>(ss[C + c], qx, qy, div, eb);
+        expand_window<false>(ss[2 * C + c], qx, qy, div, er);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int XX = X + (q & 1), YY = Y + (q >> 1);

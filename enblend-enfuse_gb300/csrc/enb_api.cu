@@ -1065,11 +1065,27 @@ enb_status enblend_fused(enb_ctx* ctx, const enb_image* white, const enb_image* 
                 }
             }
         }
-        for (int j = 1; j < first; ++j) {
+        int jt = first;  // local level from which one launch reduces the rest
+        if (first == NL) {
+            jt = enb_tail_level(gw.p->w, gw.p->h, NL);
+        }
+        for (int j = 1; j < first && j <= jt; ++j) {
             const BytePlane sa = awc.level(j - 1), da = awc.level(j), sb = abc.level(j - 1), db = abc.level(j);
             ENB_LAUNCH(ctx, launch_reduce_img2_mask(wrap, level_view(gw.p, j - 1), sa, level_view(gw.p, j), da,
                                                     level_view(gb.p, j - 1), sb, level_view(gb.p, j), db,
                                                     level_view(mg.p, j - 1), level_view(mg.p, j), ctx->stream));
+        }
+        if (jt < first) {
+            PlanarView tw[kMaxLevels], tb[kMaxLevels], tm[kMaxLevels];
+            BytePlane taw[kMaxLevels], tab[kMaxLevels];
+            for (int j = jt; j < NL; ++j) {
+                tw[j - jt] = level_view(gw.p, j);
+                tb[j - jt] = level_view(gb.p, j);
+                tm[j - jt] = level_view(mg.p, j);
+                taw[j - jt] = awc.level(j);
+                tab[j - jt] = abc.level(j);
+            }
+            ENB_LAUNCH(ctx, launch_reduce_img2_mask_tail(wrap, NL - jt, tw, taw, tb, tab, tm, ctx->stream));
         }
         int up_from = NL - 2;
         if (first < NL) {
@@ -1270,8 +1286,12 @@ enb_status enfuse_fused(enb_ctx* ctx, const enb_enfuse_params* prm, int K, const
     eh.opitch = pixel_view(out).pitch;
 
     ENB_LAUNCH(ctx, launch_ef_weights(eh, ctx->stream));
-    for (int l = 0; l + 1 < L; ++l) {
+    const int tail = ef_tail_level(eh);
+    for (int l = 0; l + 1 < L && l < tail; ++l) {
         ENB_LAUNCH(ctx, launch_ef_reduce(eh, l, ctx->stream));
+    }
+    if (tail < L) {
+        ENB_LAUNCH(ctx, launch_ef_reduce_tail(eh, tail, ctx->stream));
     }
     for (int l = L - 2; l >= 1; --l) {
         ENB_LAUNCH(ctx, launch_ef_up(eh, l, ctx->stream));

@@ -773,6 +773,47 @@ cudaError_t launch_ef_reduce(const EfuseHost& h, int l, cudaStream_t st)
     return h.C == 1 ? ef_reduce_level<int32_t, 1, true>(h, l, st) : ef_reduce_level<int32_t, 3, true>(h, l, st);
 }
 
+// The levels after l of all pyramids in one launch.
+template <typename T, int C, bool A>
+static cudaError_t ef_tail(const EfuseHost& h, int l, cudaStream_t st)
+{
+    constexpr int M = A ? kReduceAlpha : kReduceOpaque;
+    TailJobs<T, T> j{};
+    j.g.n = h.L - l;
+    j.images = h.K;
+    for (int i = 0; i < j.g.n; ++i) {
+        j.g.w[i] = h.lw[l + i];
+        j.g.h[i] = h.lh[l + i];
+        j.g.pitch[i] = h.pitch[l + i];
+        j.g.apitch[i] = h.apitch[l + i];
+        j.u[i] = h.u[l + i];
+        for (int k = 0; k < h.K; ++k) {
+            j.img[k][i] = (T*)h.g[k][l + i];
+            j.a[k][i] = h.a[k][l + i];
+            j.msk[k][i] = (T*)h.m[k][l + i];
+        }
+    }
+    return launch_reduce_tail<T, C, T, M, M>(j, h.K, h.wrap, st);
+}
+
+int ef_tail_level(const EfuseHost& h) { return tail_level(h.lw, h.lh, h.L); }
+
+cudaError_t launch_ef_reduce_tail(const EfuseHost& h, int l, cudaStream_t st)
+{
+    note_launch("ef_reduce_tail", 0.0);
+    const bool opaque = ef_opaque(h);
+    if (h.dtype == ENB_U8) {
+        if (h.C == 1) {
+            return opaque ? ef_tail<int16_t, 1, false>(h, l, st) : ef_tail<int16_t, 1, true>(h, l, st);
+        }
+        return opaque ? ef_tail<int16_t, 3, false>(h, l, st) : ef_tail<int16_t, 3, true>(h, l, st);
+    }
+    if (h.C == 1) {
+        return opaque ? ef_tail<int32_t, 1, false>(h, l, st) : ef_tail<int32_t, 1, true>(h, l, st);
+    }
+    return opaque ? ef_tail<int32_t, 3, false>(h, l, st) : ef_tail<int32_t, 3, true>(h, l, st);
+}
+
 template <typename T, typename TM>
 static EfLevelArgs<T, TM> level_args(const EfuseHost& h, int l)
 {

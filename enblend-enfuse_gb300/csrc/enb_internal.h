@@ -224,6 +224,11 @@ cudaError_t launch_reduce_img2_mask(int wrap, const PlanarView& s0, const BytePl
                                     const BytePlane& da0, const PlanarView& s1, const BytePlane& sa1,
                                     const PlanarView& d1, const BytePlane& da1, const PlanarView& ms,
                                     const PlanarView& md, cudaStream_t st);
+// the levels after 0 of n given ones (the last of the down sweep) in one launch;
+// enb_tail_level: the first such level of L
+int enb_tail_level(const int* lw, const int* lh, int L);
+cudaError_t launch_reduce_img2_mask_tail(int wrap, int n, const PlanarView* s0, const BytePlane* a0, const PlanarView* s1,
+                                         const BytePlane* a1, const PlanarView* ms, cudaStream_t st);
 cudaError_t launch_reduce2(int wrap, const PlanarView& s0, const BytePlane* sa0, const PlanarView& d0,
                            const BytePlane* da0, const PlanarView& s1, const BytePlane* sa1, const PlanarView& d1,
                            const BytePlane* da1, cudaStream_t st);
@@ -310,6 +315,9 @@ struct EfuseHost {
 };
 cudaError_t launch_ef_weights(const EfuseHost& h, cudaStream_t st);
 cudaError_t launch_ef_reduce(const EfuseHost& h, int l, cudaStream_t st);
+// the levels after l (ef_tail_level; L: none) in one launch
+int ef_tail_level(const EfuseHost& h);
+cudaError_t launch_ef_reduce_tail(const EfuseHost& h, int l, cudaStream_t st);
 cudaError_t launch_ef_up(const EfuseHost& h, int l, cudaStream_t st);
 cudaError_t launch_ef_out0(const EfuseHost& h, cudaStream_t st);
 

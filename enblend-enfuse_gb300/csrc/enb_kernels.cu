@@ -688,6 +688,56 @@ cudaError_t launch_reduce_img2_mask(int wrap, const PlanarView& s0, const BytePl
     return cudaGetLastError();
 }
 
+int enb_tail_level(const int* lw, const int* lh, int L) { return tail_level(lw, lh, L); }
+
+template <typename T, typename TM, int C>
+static cudaError_t reduce_img2_mask_tail_t(int wrap, int n, const PlanarView* s0, const BytePlane* a0, const PlanarView* s1,
+                                           const BytePlane* a1, const PlanarView* ms, cudaStream_t st)
+{
+    TailJobs<T, TM> j{};
+    j.g.n = n;
+    j.images = 2;
+    for (int i = 0; i < n; ++i) {
+        j.g.w[i] = s0[i].w;
+        j.g.h[i] = s0[i].h;
+        j.g.pitch[i] = s0[i].pitch;
+        j.g.apitch[i] = a0[i].pitch;
+        j.img[0][i] = (T*)s0[i].p;
+        j.img[1][i] = (T*)s1[i].p;
+        j.a[0][i] = a0[i].p;
+        j.a[1][i] = a1[i].p;
+        j.msk[0][i] = (TM*)ms[i].p;
+    }
+    return launch_reduce_tail<T, C, TM, kReduceAlpha, kReduceClamp>(j, 1, wrap, st);
+}
+
+cudaError_t launch_reduce_img2_mask_tail(int wrap, int n, const PlanarView* s0, const BytePlane* a0, const PlanarView* s1,
+                                         const BytePlane* a1, const PlanarView* ms, cudaStream_t st)
+{
+    // one geometry and row pitch a level for all three pyramids and both alphas
+    bool same = n >= 2 && n <= kTailLevels && (int64_t)s0[0].w * s0[0].h <= kTailPixels;
+    for (int i = 0; i < n; ++i) {
+        same = same && s0[i].pitch == s1[i].pitch && s0[i].pitch == ms[i].pitch && a0[i].pitch == a1[i].pitch &&
+               s0[i].plane == s0[i].pitch * s0[i].h && s1[i].plane == s0[i].plane;
+    }
+    if (!same) {
+        return cudaErrorInvalidValue;
+    }
+    note("reduce_tail", 0.0);
+#define ENB_RIT(T, TM, CC) return reduce_img2_mask_tail_t<T, TM, CC>(wrap, n, s0, a0, s1, a1, ms, st)
+    if (s0[0].dtype == ENB_I16) {
+        if (s0[0].C == 1) {
+            ENB_RIT(int16_t, int16_t, 1);
+        }
+        ENB_RIT(int16_t, int16_t, 3);
+    }
+    if (s0[0].C == 1) {
+        ENB_RIT(int32_t, int32_t, 1);
+    }
+    ENB_RIT(int32_t, int32_t, 3);
+#undef ENB_RIT
+}
+
 template <typename T, int C>
 static void expand_dispatch(int add, int wrap, const PlanarView& s, const PlanarView& d, cudaStream_t st)
 {

@@ -172,6 +172,12 @@ __device__ __forceinline__ void store4(float* p, const float (&v)[4], int n)
     }
 }
 
+// A reduced value as the pyramid's type.
+template <typename T>
+__device__ __forceinline__ T reduce_store(int32_t v) { return cast_store<T>(v); }
+template <typename T>
+__device__ __forceinline__ T reduce_store(float v) { return v; }
+
 template <typename TD>
 __device__ __forceinline__ void store4(TD* p, const int32_t (&v)[4], int n)
 {
@@ -411,6 +417,174 @@ inline cudaError_t launch_reduce_joint(const ReduceJobsN<SrcI, TI>& img, const R
 {
     const dim3 g((unsigned)((dw + RDW - 1) / RDW), (unsigned)reduce_tile_rows(dh), (unsigned)(2 * K));
     return launch_pdl(k_reduce_joint<SrcI, TI, C, SrcM, TM, MODE>, g, dim3(RTHREADS), st, img, msk, K, sw, sh, dw, dh, wrap);
+}
+
+// ---- the last levels in one launch -------------------------------------------
+
+// A level of at most this many pixels and the ones below it (four at most: the
+// top level's short side is at least 5) are reduced by one CTA per pyramid,
+// from shared memory: each had been a launch of a few CTAs, 4 to 5 us of
+// latency, where all of them take 7 us in one launch (1024 threads, 512 and
+// 256 the same within half a microsecond).
+constexpr int kTailPixels = 4096, kTailLevels = 6, kTailThreads = 1024;
+
+struct TailGeometry {
+    int n;  // levels, the source first
+    int w[kTailLevels], h[kTailLevels];
+    int64_t pitch[kTailLevels], apitch[kTailLevels];
+};
+
+// The pyramids of a launch: jobs image pyramids of C planes, then as many mask
+// pyramids (masks of them), level pointers from the source on; planes are
+// pitch * h apart.  a: alpha planes of each image pyramid, u: of the masks.
+template <typename TI, typename TM>
+struct TailJobs {
+    TailGeometry g;
+    int images;
+    TI* img[kReduceMaxJobs][kTailLevels];
+    uint8_t* a[kReduceMaxJobs][kTailLevels];
+    TM* msk[kReduceMaxJobs][kTailLevels];
+    uint8_t* u[kTailLevels];
+};
+
+// Words of shared memory: the level being reduced and its column sums.
+template <int NV>
+constexpr int tail_words()
+{
+    return NV * (kTailPixels + kTailPixels / 2 + 256);
+}
+
+template <typename T, int C, int MODE>
+__device__ __forceinline__ void reduce_tail(const TailGeometry& g, T* const* p, uint8_t* const* ap, int wrap,
+                                            typename ReduceAcc<T>::type* smem)
+{
+    typedef typename ReduceAcc<T>::type AC;
+    constexpr bool A = MODE == kReduceAlpha;
+    constexpr int NV = C + (A ? 1 : 0);
+    AC* lev = smem;                              // [NV][h][w]
+    AC* sums = smem + NV * kTailPixels;          // [NV][dh][w]
+    {
+        const int w = g.w[0], n = w * g.h[0];
+        const int64_t plane = g.pitch[0] * g.h[0];
+#pragma unroll 4
+        for (int i = threadIdx.x; i < n; i += kTailThreads) {
+            const int y = i / w, x = i - y * w;
+            const int64_t o = (int64_t)y * g.pitch[0] + x;
+            const int al = A ? __ldg(&ap[0][(int64_t)y * g.apitch[0] + x]) != 0 : 1;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const AC v = (AC)__ldg(&p[0][c * plane + o]);
+                lev[c * n + i] = al ? v : (AC)0;
+            }
+            if (A) {
+                lev[(NV - 1) * n + i] = (AC)al;
+            }
+        }
+    }
+    __syncthreads();
+    for (int l = 0; l + 1 < g.n; ++l) {
+        const int sw = g.w[l], sh = g.h[l], dw = g.w[l + 1], dh = g.h[l + 1], n = sw * sh, m = dh * sw;
+        for (int i = threadIdx.x; i < m; i += kTailThreads) {
+            const int J = i / sw, x = i - J * sw;
+            int r[5];
+            bool ok[5];
+#pragma unroll
+            for (int t = 0; t < 5; ++t) {
+                const int y = 2 * J - 2 + t;
+                ok[t] = MODE == kReduceClamp || (y >= 0 && y < sh);
+                r[t] = min(max(y, 0), sh - 1) * sw + x;
+            }
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                AC v[5];
+#pragma unroll
+                for (int t = 0; t < 5; ++t) {
+                    v[t] = ok[t] ? lev[c * n + r[t]] : (AC)0;
+                }
+                sums[c * m + i] = v[0] + (AC)4 * v[1] + (AC)6 * v[2] + (AC)4 * v[3] + v[4];
+            }
+        }
+        __syncthreads();
+        const int d = dw * dh;
+        const int64_t dplane = g.pitch[l + 1] * dh;
+        for (int i = threadIdx.x; i < d; i += kTailThreads) {
+            const int Y = i / dw, X = i - Y * dw;
+            int q[5];
+            bool ok[5];
+#pragma unroll
+            for (int t = 0; t < 5; ++t) {
+                const int x = 2 * X - 2 + t;
+                ok[t] = MODE == kReduceClamp || wrap || (x >= 0 && x < sw);
+                q[t] = Y * sw + (wrap ? imod(x, sw) : min(max(x, 0), sw - 1));
+            }
+            AC s[NV];
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                AC v[5];
+#pragma unroll
+                for (int t = 0; t < 5; ++t) {
+                    v[t] = ok[t] ? sums[c * m + q[t]] : (AC)0;
+                }
+                s[c] = v[0] + (AC)4 * v[1] + (AC)6 * v[2] + (AC)4 * v[3] + v[4];
+            }
+            const AC den = A ? s[NV - 1]
+                             : (MODE == kReduceOpaque ? (AC)((wrap ? 16 : reduce_den1(X, sw)) * reduce_den1(Y, sh)) : (AC)256);
+            const int64_t o = (int64_t)Y * g.pitch[l + 1] + X;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const AC v = A && den <= (AC)0 ? (AC)0 : (den == (AC)256 ? reduce_256(s[c]) : reduce_norm(s[c], den));
+                const T tv = reduce_store<T>(v);
+                p[l + 1][c * dplane + o] = tv;
+                lev[c * d + i] = (AC)tv;
+            }
+            if (A) {
+                ap[l + 1][(int64_t)Y * g.apitch[l + 1] + X] = den > (AC)0 ? 255 : 0;
+                lev[(NV - 1) * d + i] = den > (AC)0 ? (AC)1 : (AC)0;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+template <typename TI, int C, typename TM, int MODE, int MMODE>
+__global__ void __launch_bounds__(kTailThreads) k_reduce_tail(const __grid_constant__ TailJobs<TI, TM> jobs, int wrap)
+{
+    extern __shared__ __align__(16) int32_t tsmem[];
+    griddep_wait();
+    griddep_launch();
+    const int z = blockIdx.x;
+    if (z < jobs.images) {
+        reduce_tail<TI, C, MODE>(jobs.g, jobs.img[z], jobs.a[z], wrap,
+                                 reinterpret_cast<typename ReduceAcc<TI>::type*>(tsmem));
+    } else {
+        reduce_tail<TM, 1, MMODE>(jobs.g, jobs.msk[z - jobs.images], jobs.u, wrap,
+                                  reinterpret_cast<typename ReduceAcc<TM>::type*>(tsmem));
+    }
+}
+
+// images image pyramids and masks mask pyramids.
+template <typename TI, int C, typename TM, int MODE, int MMODE>
+inline cudaError_t launch_reduce_tail(const TailJobs<TI, TM>& jobs, int masks, int wrap, cudaStream_t st)
+{
+    auto k = k_reduce_tail<TI, C, TM, MODE, MMODE>;
+    const size_t smem = sizeof(int32_t) * (size_t)tail_words<C + (MODE == kReduceAlpha ? 1 : 0)>();
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    return launch_pdl_smem(k, dim3((unsigned)(jobs.images + masks)), dim3(kTailThreads), smem, st, jobs, wrap);
+}
+
+// First level l >= 1 whose reduces go into a tail launch, L without one: at
+// most kTailPixels pixels and at least two levels below it.
+inline int tail_level(const int* lw, const int* lh, int L)
+{
+    for (int l = 1; l + 2 < L; ++l) {
+        if ((int64_t)lw[l] * lh[l] <= kTailPixels) {
+            return L - l <= kTailLevels ? l : L;
+        }
+    }
+    return L;
 }
 
 template <class Src, typename TD, int C, bool ALPHA>

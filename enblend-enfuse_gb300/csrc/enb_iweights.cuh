@@ -163,9 +163,14 @@ __device__ __noinline__ static int32_t entropy_round(const uint16_t* v, int n, c
 __device__ __forceinline__ float saturation_weight(const WeightParams& wp, uint32_t d, uint32_t S)
 {
     const float fd = (float)d, fS = (float)S;
-    const float q1 = __fdiv_rn(fd, fS);
-    const float rem = __fmaf_rn(-q1, fS, fd);       // exact remainder
-    const float q2 = __fdiv_rn(rem, fS);
+    // q1 is within two ulps of d / S; its remainder is a multiple of ulp(q1)
+    // of at most 19 bits, so exact; q2's relative error of a few 2^-23 is far
+    // below the margin of the test
+    float rS;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(rS) : "f"(fS));
+    const float q1 = __fmul_rn(fd, rS);
+    const float rem = __fmaf_rn(-q1, fS, fd);
+    const float q2 = __fmul_rn(rem, rS);
     const float p_hi = __fmul_rn(wp.w_sat_hi, q1);
     const float e1 = __fmaf_rn(wp.w_sat_hi, q1, -p_hi);
     const float p_lo = __fadd_rn(e1, __fadd_rn(__fmul_rn(wp.w_sat_hi, q2), __fmul_rn(wp.w_sat_lo, q1)));
@@ -567,6 +572,268 @@ __device__ __forceinline__ float saturation_of(const WeightParams& wp, uint32_t 
     const uint32_t sum = mx + mn;
     const uint32_t S = sum <= wp.maxv ? sum : 2u * wp.maxv - sum;
     return saturation_weight(wp, mx - mn, S);
+}
+
+// ---- quads: 2x2 output pixels per thread -------------------------------------
+
+// stddev_round out of line (ties, windows with transparent pixels).
+static __device__ __noinline__ int32_t stddev_round_any(int64_t S, int64_t Q, int n) { return stddev_round(S, Q, n); }
+
+// stddev_round of an opaque CW x CW window (CW <= 7) of 16-bit samples: there
+// S < 2^22, num < 2^44 and n Q < 2^44, so the squares of the rounding test are
+// products of 32-bit integers, (2m -+ 1)^2 nn = (m^2 -+ m) 4 nn + nn, and the
+// reference's double expression is off by less than one in units of 4 num: S^2
+// is exact, its division by n costs 2^-51 n Q, the difference and the division
+// by n - 1 2^-50 num each, the square root and the sum with 0.5 2^-50 num
+// together.  4 num and the boundaries are integers, so only an exact tie needs
+// that expression (frequent near-ties in dark, nearly flat windows had made
+// its FP64 instructions 6% of the time).  The estimate only has to come within
+// one of m.
+template <int CW>
+__device__ __forceinline__ uint32_t stddev_round_full(uint32_t S, uint64_t Q)
+{
+    constexpr uint32_t n = CW * CW, nn = n * (n - 1);
+    static_assert(CW <= 7, "num and n Q stay below 2^45 and 2^48");
+    const int64_t num4 = 4 * (int64_t)(n * Q - (uint64_t)S * S);
+    // num4 < 2^46 as a float from two 32-bit halves (the 64-bit conversion runs
+    // at a fraction of the rate)
+    const float f4 = fmaf((float)(uint32_t)(num4 >> 20), 1048576.0f, (float)((uint32_t)num4 & 0xfffffu));
+    float est;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(est) : "f"(f4 * (0.25f / (float)nn)));
+    uint32_t m = (uint32_t)(est + 0.5f);
+    const auto lower = [](uint32_t v) { return (int64_t)((uint64_t)(v * v - v) * (4u * nn) + nn); };  // (2v - 1)^2 nn
+    if (m > 0 && lower(m) > num4) {
+        --m;
+    } else if (lower(m + 1) <= num4) {
+        ++m;
+    }
+    if (m == 0 || num4 != lower(m)) {
+        return m;
+    }
+    return (uint32_t)stddev_round_any((int64_t)S, (int64_t)Q, (int)n);
+}
+
+// Opaque pixels of the CW x CW windows of the 2x2 pixels at (cx, cy).
+template <int CW>
+__device__ __forceinline__ void opaque_quad(const uint8_t* a, int TW, int cx, int cy, int (&n)[4])
+{
+    constexpr int B = CW / 2;
+    n[0] = n[1] = n[2] = n[3] = 0;
+#pragma unroll
+    for (int dy = 0; dy <= CW; ++dy) {
+        const uint8_t* row = a + (cy + dy - B) * TW + cx - B;
+        int mid = 0;
+#pragma unroll
+        for (int c = 1; c < CW; ++c) {
+            mid += row[c];
+        }
+        const int l = mid + row[0], r = mid + row[CW];
+        n[0] += dy < CW ? l : 0;
+        n[1] += dy < CW ? r : 0;
+        n[2] += dy > 0 ? l : 0;
+        n[3] += dy > 0 ? r : 0;
+    }
+}
+
+// The rounded window deviations of the 2x2 pixels at (cx, cy), cx even: g[q]
+// of (q & 1, q >> 1).  The windows share all but one row and one column: a
+// column's sums over the common rows are formed once.  OPAQUE: every window
+// that counts is opaque; else transparent pixels have gray 0 in the tile, and
+// their flags a give each window's number of pixels.
+template <int CW, bool OPAQUE>
+__device__ __forceinline__ void contrast_quad(const int32_t* gray, const uint8_t* a, int TW, int cx, int cy, uint32_t (&g)[4])
+{
+    constexpr int B = CW / 2, NC = CW + 1;
+    int n[4] = {CW * CW, CW * CW, CW * CW, CW * CW};
+    if (!OPAQUE) {
+        opaque_quad<CW>(a, TW, cx, cy, n);
+    }
+    const auto round = [&](int q, uint32_t s, uint64_t sq) {
+        return OPAQUE || n[q] == CW * CW ? stddev_round_full<CW>(s, sq)
+                                         : (uint32_t)stddev_round_any((int64_t)s, (int64_t)sq, n[q]);
+    };
+    uint32_t S[2][NC];
+    uint64_t Q[2][NC];
+#pragma unroll
+    for (int dy = 0; dy <= CW; ++dy) {
+        const int32_t* row = gray + (cy + dy - B) * TW + cx - B;
+        uint32_t v[NC];
+        if constexpr ((B & 1) == 0) {
+#pragma unroll
+            for (int c = 0; c < NC / 2; ++c) {
+                const int2 p = reinterpret_cast<const int2*>(row)[c];
+                v[2 * c] = (uint32_t)p.x;
+                v[2 * c + 1] = (uint32_t)p.y;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                v[c] = (uint32_t)row[c];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const uint64_t q = (uint64_t)v[c] * v[c];
+            if (dy == 0) {
+                S[0][c] = v[c];
+                Q[0][c] = q;
+            } else if (dy == 1) {
+                S[1][c] = v[c];  // the common rows until the last
+                Q[1][c] = q;
+            } else if (dy < CW) {
+                S[1][c] += v[c];
+                Q[1][c] += q;
+            } else {
+                S[0][c] += S[1][c];
+                Q[0][c] += Q[1][c];
+                S[1][c] += v[c];
+                Q[1][c] += q;
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        uint32_t s0 = 0u;
+        uint64_t q0 = 0ull;
+#pragma unroll
+        for (int c = 0; c < CW; ++c) {
+            s0 += S[r][c];
+            q0 += Q[r][c];
+        }
+        g[2 * r] = round(2 * r, s0, q0);
+        g[2 * r + 1] = round(2 * r + 1, s0 - S[r][0] + S[r][CW], q0 - Q[r][0] + Q[r][CW]);
+    }
+}
+
+// The p log p tables of full W x W windows in shared memory: fx[1], the second
+// differences h[j] = g(j) - 2 g(j-1) + g(j-2) of g(len) = fx[len + 1] - fx[1]
+// (g(0) = g(-1) = 0) and max / log(bins) in 2^-40 fixed point.
+struct EntropyTables {
+    long long one, h[5];
+    long long g[26];
+    unsigned long long scale[26];
+};
+
+template <int W>
+__device__ __forceinline__ void entropy_tables_load(EntropyTables& e, const WeightTables& tab)
+{
+    constexpr int M = W * W;
+    const long long* fx = tab.plogp_fx + (int64_t)M * (M + 1);
+    const int i = threadIdx.x;
+    if (i <= M) {
+        e.scale[i] = tab.scale_fx[i];
+        e.g[i] = i < M ? fx[i + 1] - fx[1] : 0;  // g(len), len <= M - 1
+    }
+    if (i == 0) {
+        e.one = fx[1];
+    }
+    if (i >= 1 && i <= 4) {
+        const auto g = [&](int len) { return len > 0 ? fx[len + 1] - fx[1] : 0ll; };
+        e.h[i] = g(i) - 2 * g(i - 1) + (i > 1 ? g(i - 2) : 0ll);
+    }
+}
+
+// H * max in 2^-32 fixed point (entropy_fx_round before its rounding) of a
+// full window from the boundaries of its sorted keys (as
+// entropy_from_boundaries; 0 for a single bin).  With e_1 the keys equal to
+// their predecessor and e_j = e_1 & e_1 >> 1 & ..., popc(e_j) = sum over the
+// runs of max(len - j + 1, 0), and g(len) = sum_j (len - j + 1) h_j: the same
+// integer sum in as many steps as the longest run, not one per run.
+template <int M>
+__device__ __forceinline__ uint64_t entropy_scaled(uint32_t bnd, const EntropyTables& t)
+{
+    const int bins = __popc(bnd) + 1;
+    if (bins <= 1) {
+        return 0ull;
+    }
+    long long acc = (long long)bins * t.one;
+    uint32_t eq = ~bnd & (((1u << M) - 1u) & ~1u), e = eq;
+#pragma unroll
+    for (int j = 1; j <= 4; ++j) {
+        if (e == 0u) {
+            break;
+        }
+        acc += (long long)__popc(e) * t.h[j];
+        e &= eq >> j;
+    }
+    if (e != 0u) {  // a run of more than four: run by run
+        acc = (long long)bins * t.one;
+        while (eq) {
+            const int s0 = __ffs(eq) - 1;
+            const int len = __ffs(~(eq >> s0)) - 1;
+            acc += t.g[len];
+            eq &= ~(((1u << len) - 1u) << s0);
+        }
+    }
+    return __umul64hi((unsigned long long)(-acc), t.scale[bins]);
+}
+
+// Boundary masks of two windows sorted in the halves of k (as in entropy_pair).
+template <int M>
+__device__ __forceinline__ void pair_boundaries(const uint32_t (&k)[M], uint32_t& b0, uint32_t& b1)
+{
+    uint32_t lo = 0u, hi = 0u;  // boundaries 1..15 and 16.., both windows' halves together
+#pragma unroll
+    for (int i = 1; i < M; ++i) {
+        const uint32_t d = k[i] - k[i - 1];
+        uint32_t nz;
+        asm("min.u16x2 %0, %1, %2;" : "=r"(nz) : "r"(d), "r"(0x00010001u));
+        if (i < 16) {
+            lo += nz << i;
+        } else {
+            hi += nz << (i - 16);
+        }
+    }
+    b0 = (lo & 0xffffu) | (hi << 16);
+    b1 = (lo >> 16) | (hi & 0xffff0000u);
+}
+
+// Least H * max (2^-32 fixed point) over the channel's windows of the 2x2
+// pixels at (cx, cy), cx even: v[q] is lowered.  Horizontally adjacent windows
+// are the halves of the words, vertically adjacent ones share all but one
+// row: the W - 1 common rows are sorted once (the network's comparators per
+// quad: 207 instead of 280 for W = 5).
+template <int W>
+__device__ __forceinline__ void entropy_quad(const uint16_t* plane, int TW, int cx, int cy, const EntropyTables& t,
+                                             uint64_t (&v)[4])
+{
+    constexpr int B = W / 2;
+    uint32_t r[W + 1][W];
+#pragma unroll
+    for (int dy = 0; dy <= W; ++dy) {
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(plane + (cy + dy - B) * TW + cx - 2);
+        const uint32_t w0 = row[0], w1 = row[1], w2 = row[2];  // columns cx-2 .. cx+3
+        const uint32_t m01 = __byte_perm(w0, w1, 0x5432), m12 = __byte_perm(w1, w2, 0x5432);
+        if constexpr (W == 5) {
+            r[dy][0] = w0;
+            r[dy][1] = m01;
+            r[dy][2] = w1;
+            r[dy][3] = m12;
+            r[dy][4] = w2;
+        } else {
+            r[dy][0] = m01;
+            r[dy][1] = w1;
+            r[dy][2] = m12;
+        }
+        sort_row(r[dy], CeU16x2());
+    }
+    uint32_t common[(W - 1) * W], k[W * W];
+    if constexpr (W == 5) {
+        uint32_t a[10], b[10];
+        merge_sorted(r[1], r[2], a, CeU16x2());
+        merge_sorted(r[3], r[4], b, CeU16x2());
+        merge_sorted(a, b, common, CeU16x2());
+    } else {
+        merge_sorted(r[1], r[2], common, CeU16x2());
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        merge_sorted(r[q == 0 ? 0 : W], common, k, CeU16x2());
+        uint32_t b0, b1;
+        pair_boundaries<W * W>(k, b0, b1);
+        v[2 * q] = min(v[2 * q], entropy_scaled<W * W>(b0, t));
+        v[2 * q + 1] = min(v[2 * q + 1], entropy_scaled<W * W>(b1, t));
+    }
 }
 
 // Whether the pair path can weight a tile whose pixels are all opaque and

@@ -58,6 +58,64 @@ __device__ __forceinline__ void st_px(TIn* p, const TIn (&o)[S])
     }
 }
 
+// N (2 or 4) horizontally adjacent pixels (the first at a multiple of N) of an
+// interleaved image as N*S*sizeof(TIn) / UNIT words of UNIT bytes (UNIT: the
+// largest power of two, at most 16, dividing the run's size; the caller
+// checks that the image's base and row pitch are multiples of it).
+template <int U> struct PairWord;
+template <> struct PairWord<2> { typedef uint16_t type; };
+template <> struct PairWord<4> { typedef uint32_t type; };
+template <> struct PairWord<8> { typedef uint2 type; };
+template <> struct PairWord<16> { typedef uint4 type; };
+
+template <typename TIn, int S, int N>
+struct PixelRun {
+    static constexpr int BYTES = N * S * (int)sizeof(TIn);
+    static constexpr int UNIT = (BYTES % 16 == 0) ? 16 : (BYTES % 8 == 0) ? 8 : (BYTES % 4 == 0) ? 4 : 2;
+    static constexpr int NW = BYTES / UNIT;
+    typedef typename PairWord<UNIT>::type W;
+    __device__ __forceinline__ static void load(const TIn* p, TIn (&px)[N][S])
+    {
+        union {
+            W w[NW];
+            TIn s[N * S];
+        } u;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            u.w[i] = __ldg(reinterpret_cast<const W*>(p) + i);
+        }
+#pragma unroll
+        for (int i = 0; i < N * S; ++i) {
+            px[i / S][i % S] = u.s[i];
+        }
+    }
+    __device__ __forceinline__ static void store(TIn* p, const TIn (&px)[N][S])
+    {
+        union {
+            W w[NW];
+            TIn s[N * S];
+        } u;
+#pragma unroll
+        for (int i = 0; i < N * S; ++i) {
+            u.s[i] = px[i / S][i % S];
+        }
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            reinterpret_cast<W*>(p)[i] = u.w[i];
+        }
+    }
+};
+
+template <typename TIn, int S>
+using PixelPair = PixelRun<TIn, S, 2>;
+
+// Whether an image's base and row pitch (bytes) allow RUN's words.
+template <class RUN>
+inline bool run_aligned(const void* p, size_t pitch)
+{
+    return (uintptr_t)p % (size_t)RUN::UNIT == 0 && pitch % (size_t)RUN::UNIT == 0;
+}
+
 // Alpha of an interleaved pixel: 8-bit plane (AM 0), opaque (AM 1) or the
 // thresholded 4th component (AM 2, src/assemble.h:240-253).
 template <int AM, typename TIn, int S>

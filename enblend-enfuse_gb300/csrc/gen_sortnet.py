@@ -1,7 +1,9 @@
 """Generate enb_sortnet.cuh: Batcher's odd-even merge sorting networks for the
 local-entropy windows (3x3 = 9 and 5x5 = 25 keys), padded to 16 and 32 keys
 and pruned of every comparator that touches a padding position (padding keys
-are the maximum key, so such comparators never exchange).
+are the maximum key, so such comparators never exchange); and his odd-even
+merges of two sorted lists, from which the windows of vertically adjacent
+pixels are sorted with their common rows sorted once.
 
 Usage: python gen_sortnet.py > enb_sortnet.cuh
 """
@@ -35,6 +37,40 @@ def check(pairs, live):
             if v[a] > v[b]:
                 v[a], v[b] = v[b], v[a]
         assert v == sorted(v)
+
+
+def merge(a, b, pairs):
+    """Odd-even merge of the sorted wire lists a and b (Batcher 1968; Knuth
+    5.3.4 for any lengths): appends its comparators to pairs, returns the
+    wires in ascending order of their keys."""
+    if not a or not b:
+        return a + b
+    if len(a) == 1 and len(b) == 1:
+        pairs.append((a[0], b[0]))
+        return [a[0], b[0]]
+    v, w = merge(a[0::2], b[0::2], pairs), merge(a[1::2], b[1::2], pairs)
+    out = [v[0]]
+    for i in range(max(len(w), len(v) - 1)):
+        if i < len(w) and i + 1 < len(v):
+            pairs.append((w[i], v[i + 1]))
+        out += w[i:i + 1] + v[i + 1:i + 2]
+    return out
+
+
+def check_merge(m, n, pairs, out):
+    # the 0-1 principle: every pair of sorted 0-1 lists
+    for i in range(m + 1):
+        for j in range(n + 1):
+            v = [0] * i + [1] * (m - i) + [0] * j + [1] * (n - j)
+            for a, b in pairs:
+                if v[a] > v[b]:
+                    v[a], v[b] = v[b], v[a]
+            r = [v[x] for x in out]
+            assert r == sorted(r)
+
+
+SORT = {3: [(0, 1), (1, 2), (0, 1)],
+        5: [(0, 1), (3, 4), (2, 4), (2, 3), (0, 3), (0, 2), (1, 4), (1, 3), (1, 2)]}
 
 
 def main():
@@ -78,6 +114,40 @@ def main():
         print("{")
         for a, b in pairs:
             print(f"    ce(k[{a}], k[{b}]);")
+        print("}")
+    for n in (3, 5):
+        check(SORT[n], n)
+        print()
+        print(f"// Sorts k[0..{n - 1}] ascending ({len(SORT[n])} comparators).")
+        print("template <class CE = CeU32>")
+        print(f"__device__ __forceinline__ void sort_row(uint32_t (&k)[{n}], CE ce = CE())")
+        print("{")
+        for a, b in SORT[n]:
+            print(f"    ce(k[{a}], k[{b}]);")
+        print("}")
+    for m, n in ((3, 3), (3, 6), (5, 5), (10, 10), (5, 20)):
+        pairs = []
+        out = merge(list(range(m)), list(range(m, m + n)), pairs)
+        check_merge(m, n, pairs, out)
+        print()
+        print(f"// Merges the sorted lists a and b into o ({len(pairs)} comparators).")
+        print("template <class CE = CeU32>")
+        print(f"__device__ __forceinline__ void merge_sorted(const uint32_t (&a)[{m}], const uint32_t (&b)[{n}], "
+              f"uint32_t (&o)[{m + n}], CE ce = CE())")
+        print("{")
+        print(f"    uint32_t k[{m + n}];")
+        print("#pragma unroll")
+        print(f"    for (int i = 0; i < {m}; ++i) {{")
+        print("        k[i] = a[i];")
+        print("    }")
+        print("#pragma unroll")
+        print(f"    for (int i = 0; i < {n}; ++i) {{")
+        print(f"        k[{m} + i] = b[i];")
+        print("    }")
+        for x, y in pairs:
+            print(f"    ce(k[{x}], k[{y}]);")
+        for i, x in enumerate(out):
+            print(f"    o[{i}] = k[{x}];")
         print("}")
     print()
     print("}  // namespace enb")

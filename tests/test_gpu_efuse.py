@@ -169,3 +169,40 @@ def test_level_tiles_at_their_edges(ctx, dtype, w, h, K, wrap, chans):
     ctx.enfuse(pad, [torch.from_numpy(a).cuda() for a in alphas], params=prm, wrap=wrap, seed=9, out=out)
     ctx.synchronize()
     assert np.array_equal(out.cpu().numpy(), got[0][1])
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16])
+@pytest.mark.parametrize("con,ent", [(0, 0), (5, 0), (3, 0), (0, 5), (0, 3), (5, 5), (3, 5), (5, 3), (3, 3)])
+@pytest.mark.parametrize("chans", [3, 4])
+def test_weight_kernels_against_single_operations(ctx, dtype, con, ent, chans):
+    """The RGB weight kernels (points, 2x2 quads) against the per-image kernel behind the plain passes: few distinct
+    values (long runs of equal keys), random and flat samples, saturated and black ones, alpha holes and edges in
+    planes and in the 4th component, images smaller than a tile, ragged rows; level 0 and pixels bit for bit."""
+    import enbgpu
+    rng = np.random.default_rng(100 * con + 10 * ent + chans)
+    maxv = np.iinfo(dtype).max
+    prm = enbgpu.enfuse_params(saturation_weight=0.2, contrast_weight=0.5 if con else 0.0, entropy_weight=0.3 if ent else 0.0,
+                               contrast_window_size=con or 5, entropy_window_size=ent or 3)
+    for (w, h, K) in [(9, 11, 2), (33, 31, 3), (67, 64, 4), (130, 35, 2)]:
+        shape = (h, w, chans)
+        kinds = [rng.integers(0, maxv + 1, shape), rng.integers(0, 3, shape) * (maxv // 2), rng.integers(0, 25, shape),
+                 np.full(shape, maxv), maxv - rng.integers(0, 300, shape) % (maxv // 4)]
+        imgs = [np.ascontiguousarray(kinds[(i + w) % len(kinds)].astype(dtype)) for i in range(K)]
+        for im in imgs:
+            im[h // 2:, : w // 3] = 0
+        for alpha in ("none", "planes") if chans == 3 else ("channel", "planes"):
+            alphas = None
+            if chans == 4:
+                for im in imgs:
+                    im[..., 3] = np.where(rng.random((h, w)) < (0.9 if alpha == "channel" else 2.0), maxv, maxv // 3)
+                    im[: h // 4, w // 2:, 3] = 0 if alpha == "channel" else maxv
+            if alpha == "planes":
+                alphas = [np.where((np.add.outer(np.arange(h), 2 * np.arange(w)) > 12) & (rng.random((h, w)) < 0.97), 255, 0)
+                          .astype(np.uint8) for _ in range(K)]
+            got = []
+            for plain in (False, True):
+                l0 = np.zeros((h, w, 3), np.int32)
+                out, oa = ctx.enfuse(imgs, alphas, params=prm, seed=9, level0=l0, plain=plain)
+                got.append((l0, out, oa))
+            for a, b in zip(*got):
+                assert np.array_equal(a, b), (w, h, alpha)

@@ -444,34 +444,51 @@ struct AlphaChain {
 };
 
 // Reduce chain of a pyramid whose level 0 is filled (gaussianPyramid,
-// src/pyramid.h:1500-1530 with alpha, :1590-1610 without).
-enb_status gaussian_levels(enb_ctx* ctx, int wrap, enb_pyramid* p, const BytePlane* alpha0)
+// src/pyramid.h:1500-1530 with alpha, :1590-1610 without).  px: level 1 is
+// reduced from these pixels (laplacian_takes_pixels, with alpha), level 0 is
+// not read.
+enb_status gaussian_levels(enb_ctx* ctx, int wrap, enb_pyramid* p, const BytePlane* alpha0,
+                           const PixelView* px = nullptr, int frac = 0)
 {
-    if (p->levels <= 1) {
-        return ENB_OK;
-    }
-    if (!alpha0) {
-        for (int l = 1; l < p->levels; ++l) {
-            ENB_CHECK(ctx, p->w[l - 1] > 1 && p->h[l - 1] > 1, "reduce: src image too small in reduce");
-            ENB_LAUNCH(ctx, launch_reduce(wrap, level_view(p, l - 1), nullptr, level_view(p, l), nullptr, ctx->stream));
-        }
+    const int L = p->levels;
+    if (L <= 1) {
         return ENB_OK;
     }
     AlphaChain ac;
-    ENB_CUDA(ctx, ac.alloc(p->levels, p->w[0], p->h[0], ctx->stream));
-    for (int l = 1; l < p->levels; ++l) {
+    if (alpha0) {
+        ENB_CUDA(ctx, ac.alloc(L, p->w[0], p->h[0], ctx->stream));
+    }
+    PlanarView lv[kMaxLevels];
+    BytePlane la[kMaxLevels];
+    for (int l = 0; l < L; ++l) {
+        lv[l] = level_view(p, l);
+        if (alpha0) {
+            la[l] = l == 0 ? *alpha0 : ac.level(l);
+        }
+    }
+    const int tail = pyramid_tail_level(p->w, p->h, L, p->dtype);
+    for (int l = 1; l < L; ++l) {
         ENB_CHECK(ctx, p->w[l - 1] > 1 && p->h[l - 1] > 1, "reduce: src image too small in reduce");
-        const BytePlane src_a = l == 1 ? *alpha0 : ac.level(l - 1);
-        const BytePlane dst_a = ac.level(l);
-        ENB_LAUNCH(ctx, launch_reduce(wrap, level_view(p, l - 1), &src_a, level_view(p, l), &dst_a, ctx->stream));
+        if (l == 1 && px) {
+            AlphaSrc a{};
+            a.mode = kAlphaPlane;
+            a.plane = *alpha0;
+            ENB_LAUNCH(ctx, launch_reduce0_alpha(*px, a, frac, lv[1], la[1], wrap, ctx->stream));
+        } else if (l <= tail) {
+            ENB_LAUNCH(ctx, launch_reduce(wrap, lv[l - 1], alpha0 ? &la[l - 1] : nullptr, lv[l], alpha0 ? &la[l] : nullptr,
+                                          ctx->stream));
+        } else if (l + 1 == L) {  // the sizes of all levels are checked
+            ENB_LAUNCH(ctx, launch_reduce_tail_levels(wrap, L - tail, lv + tail, alpha0 ? la + tail : nullptr, ctx->stream));
+        }
     }
     return ENB_OK;
 }
 
-enb_status laplacian_levels(enb_ctx* ctx, int wrap, enb_pyramid* p)
+// first: the level to start from, the ones below it done by a launch_laplacian0.
+enb_status laplacian_levels(enb_ctx* ctx, int wrap, enb_pyramid* p, int first = 0)
 {
-    for (int l = 0; l + 1 < p->levels; ++l) {
-        ENB_LAUNCH(ctx, launch_expand(0, wrap, level_view(p, l + 1), level_view(p, l), ctx->stream));
+    for (int l = first; l + 1 < p->levels; ++l) {
+        ENB_LAUNCH(ctx, launch_expand(0, wrap, level_view(p, l + 1), level_view(p, l), ctx->stream, l > 0));
     }
     return ENB_OK;
 }
@@ -479,8 +496,20 @@ enb_status laplacian_levels(enb_ctx* ctx, int wrap, enb_pyramid* p)
 enb_status collapse_levels(enb_ctx* ctx, int wrap, enb_pyramid* p)
 {
     for (int l = p->levels - 2; l >= 0; --l) {
-        ENB_LAUNCH(ctx, launch_expand(1, wrap, level_view(p, l + 1), level_view(p, l), ctx->stream));
+        ENB_LAUNCH(ctx, launch_expand(1, wrap, level_view(p, l + 1), level_view(p, l), ctx->stream, l + 2 < p->levels));
     }
+    return ENB_OK;
+}
+
+enb_status blend_levels(enb_ctx* ctx, const enb_pyramid* m, const enb_pyramid* white, enb_pyramid* black, int32_t wv)
+{
+    PlanarView mv[kMaxLevels], wv_[kMaxLevels], bv[kMaxLevels];
+    for (int l = 0; l < black->levels; ++l) {
+        mv[l] = level_view(m, l);
+        wv_[l] = level_view(white, l);
+        bv[l] = level_view(black, l);
+    }
+    ENB_LAUNCH(ctx, launch_blend(black->levels, mv, wv_, bv, wv, ctx->stream));
     return ENB_OK;
 }
 
@@ -951,10 +980,7 @@ enb_status enblend_plain(enb_ctx* ctx, const enb_image* white, const enb_image* 
     ENB_LAUNCH(ctx, launch_union_alpha(wa, ua, 0, ctx->stream));
 
     // Blend, collapse, copy out (src/enblend.h:468-510).
-    for (int l = 0; l < L; ++l) {
-        ENB_LAUNCH(ctx, launch_blend(level_view(mg.p, l), level_view(wl.p, l), level_view(bl.p, l), 255 << mf,
-                                     ctx->stream));
-    }
+    ENB_TRY(blend_levels(ctx, mg.p, wl.p, bl.p, 255 << mf));
     ENB_TRY(collapse_levels(ctx, wrap, bl.p));
     if (level0) {
         ENB_LAUNCH(ctx, launch_copy_level0(level_view(bl.p, 0), level0, ctx->stream));
@@ -1965,7 +1991,8 @@ enb_status enb_blend(enb_ctx* ctx, const enb_image* mask, const enb_image* white
                        mask->height == black->height && (black->channels == 1 || black->channels == 3),
               "blend: size/channel mismatch");
     ENB_CHECK(ctx, white_value > 0, "blend: white value must be positive");
-    ENB_LAUNCH(ctx, launch_blend(planar_view(mask), planar_view(white), planar_view(black), white_value, ctx->stream));
+    const PlanarView m = planar_view(mask), w = planar_view(white), b = planar_view(black);
+    ENB_LAUNCH(ctx, launch_blend(1, &m, &w, &b, white_value, ctx->stream));
     return ENB_OK;
 }
 
@@ -2107,8 +2134,26 @@ enb_status enb_gaussian_pyramid_noalloc(enb_ctx* ctx, int wrap, const enb_image*
 enb_status enb_laplacian_pyramid(enb_ctx* ctx, int wrap, const enb_image* src, const enb_image* alpha, int frac,
                                  enb_pyramid* pyr)
 {
-    ENB_TRY(enb_gaussian_pyramid(ctx, wrap, src, alpha, frac, pyr));
-    return laplacian_levels(ctx, wrap != 0, pyr);
+    if (!ctx || !pyr) {
+        return ENB_ERR_INVALID;
+    }
+    // Level 0 is written once, as the pixels' difference from the expanded
+    // level 1, where the conversions allow it; what does not pass here is
+    // refused (or built level by level) by enb_gaussian_pyramid.
+    const int L = pyr->levels;
+    const bool direct = L > 1 && pyr->w[L - 2] > 1 && pyr->h[L - 2] > 1 && pixels_ok(src) && src->width == pyr->w[0] &&
+                        src->height == pyr->h[0] && src->channels == pyr->C && frac >= 0 && alpha &&
+                        bytes_ok(alpha, src->width, src->height) &&
+                        laplacian_takes_pixels(src->dtype, pyr->C, pixel_view(src).stride, pyr->dtype, frac);
+    if (!direct) {
+        ENB_TRY(enb_gaussian_pyramid(ctx, wrap, src, alpha, frac, pyr));
+        return laplacian_levels(ctx, wrap != 0, pyr);
+    }
+    const BytePlane a = byte_plane(alpha);
+    const PixelView px = pixel_view(src);
+    ENB_TRY(gaussian_levels(ctx, wrap != 0, pyr, &a, &px, frac));
+    ENB_LAUNCH(ctx, launch_laplacian0(px, frac, wrap != 0, level_view(pyr, 1), level_view(pyr, 0), ctx->stream));
+    return laplacian_levels(ctx, wrap != 0, pyr, 1);
 }
 
 enb_status enb_collapse_pyramid(enb_ctx* ctx, int wrap, enb_pyramid* pyr)
@@ -2129,10 +2174,8 @@ enb_status enb_blend_pyramids(enb_ctx* ctx, const enb_pyramid* mask_gp, const en
               "blend_pyramids: level count mismatch");
     for (int l = 0; l < black_lp->levels; ++l) {
         ENB_CHECK(ctx, mask_gp->w[l] == black_lp->w[l] && mask_gp->h[l] == black_lp->h[l], "blend_pyramids: size mismatch");
-        ENB_LAUNCH(ctx, launch_blend(level_view(mask_gp, l), level_view(white_lp, l), level_view(black_lp, l),
-                                     white_value, ctx->stream));
     }
-    return ENB_OK;
+    return blend_levels(ctx, mask_gp, white_lp, black_lp, white_value);
 }
 
 enb_status enb_enfuse_mask(enb_ctx* ctx, const enb_enfuse_params* prm, const enb_image* src, const enb_image* alpha,

@@ -232,9 +232,21 @@ cudaError_t launch_reduce_img2_mask_tail(int wrap, int n, const PlanarView* s0, 
 cudaError_t launch_reduce2(int wrap, const PlanarView& s0, const BytePlane* sa0, const PlanarView& d0,
                            const BytePlane* da0, const PlanarView& s1, const BytePlane* sa1, const PlanarView& d1,
                            const BytePlane* da1, cudaStream_t st);
+// The last levels of one pyramid from level pyramid_tail_level (L: none) on,
+// n of them with the source, in one launch (fixed point; alpha planes or null).
+int pyramid_tail_level(const int* lw, const int* lh, int L, int dtype);
+cudaError_t launch_reduce_tail_levels(int wrap, int n, const PlanarView* levels, const BytePlane* alpha, cudaStream_t st);
+// chained: the launch before on the stream is another of the same pyramid's
+// expands, the level below (subtracting) or above (adding)
 cudaError_t launch_expand(int add, int wrap, const PlanarView& src, const PlanarView& dst,
-                          cudaStream_t st);
-cudaError_t launch_blend(const PlanarView& mask, const PlanarView& white, const PlanarView& black,
+                          cudaStream_t st, bool chained = false);
+// level 0 of a Laplacian pyramid from the pixels and Gaussian level 1, for the
+// formats whose converted values fit the level
+bool laplacian_takes_pixels(int px_dtype, int C, int stride, int dtype, int frac);
+cudaError_t launch_laplacian0(const PixelView& px, int frac, int wrap, const PlanarView& g1, const PlanarView& l0,
+                              cudaStream_t st);
+// n levels of one type and channel count
+cudaError_t launch_blend(int n, const PlanarView* mask, const PlanarView* white, const PlanarView* black,
                          int32_t white_value, cudaStream_t st);
 cudaError_t launch_mask_mul_acc(const PlanarView& lp, const PlanarView& mask, int32_t divisor,
                                 const PlanarView& result, int accumulate, cudaStream_t st);

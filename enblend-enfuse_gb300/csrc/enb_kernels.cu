@@ -15,6 +15,8 @@
 #include "enb_entropy.cuh"
 #include "enb_iweights.cuh"
 #include "enb_reduce.cuh"
+#include "enb_pixels.cuh"
+#include "enb_tiles.cuh"
 
 namespace enb {
 
@@ -23,10 +25,11 @@ namespace enb {
 // ---------------------------------------------------------------------------
 
 template <typename TS, typename TD>
-__global__ void __launch_bounds__(256) k_to_fixed(const TS* __restrict__ src, int64_t spitch, int stride, int C,
-                                                  TD* __restrict__ dst, int64_t dpitch, int64_t dplane,
-                                                  int w, int h, int frac)
+__global__ void __launch_bounds__(256) k_to_fixed(const TS* src, int64_t spitch, int stride, int C, TD* dst,
+                                                  int64_t dpitch, int64_t dplane, int w, int h, int frac)
 {
+    griddep_wait();
+    griddep_launch();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= w) {
@@ -105,105 +108,144 @@ __global__ void __launch_bounds__(256) k_alpha_extract(AlphaSrc a, uint8_t* __re
 // even Y and (1,1) at odd Y, divided by the product of the in-image weight
 // sums (64 or 16 inside the image; 56, 49, 14, 8, ... at the borders).  One
 // thread handles the 2x2 destination quad of one source pixel.
+//
+// The levels of a pyramid are a chain of these launches, most of them far
+// below a wave, so the launch latency and the two load latencies counted:
+// a launch of the chain loads what the one before it does not write (the
+// destination samples; the source too when it subtracts, as level l + 1 is
+// only replaced by the next launch) and waits after that.  Border tiles share
+// the interior's arithmetic (TileWindow, QuadDivisors), where a quad at a
+// border had computed its weights and divided per sample.  The eight adding
+// launches of a 1921x1081 Int32 pyramid went from 92 to 60 us with event
+// overhead, the sixteen subtracting ones of two pyramids from 167 to 121 us.
 
-template <typename T, bool ADD>
-__device__ __forceinline__ void expand_combine(T* d, int32_t e)
-{
-    if (ADD) {
-        *d = sat_store<T>((int32_t)*d + e);
-    } else {
-        *d = cast_store<T>((int64_t)*d - e);
+// The destination's samples before the operation: the level itself, or (for
+// level 0 of a Laplacian pyramid) the pixels it is the conversion of, which
+// saves writing and reading the converted level.  PAIR: a pixel pair is read
+// as words (PixelPair), the image's base and pitch being multiples of theirs.
+struct FineLevel {
+    template <typename T, int C>
+    __device__ __forceinline__ void load(const T* d, int64_t o, int64_t o1, int64_t plane, int, int, int, bool pair,
+                                         bool x1, int32_t (&f)[C][4]) const
+    {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const T *p = d + c * plane + o, *q = d + c * plane + o1;
+            if (pair) {
+                ld2<T, false>(p, f[c][0], f[c][1]);
+                ld2<T, false>(q, f[c][2], f[c][3]);
+            } else {
+                f[c][0] = (int32_t)p[0];
+                f[c][2] = (int32_t)q[0];
+                f[c][1] = x1 ? (int32_t)p[1] : 0;
+                f[c][3] = x1 ? (int32_t)q[1] : 0;
+            }
+        }
     }
-}
+};
 
-template <typename T, int C, bool ADD>
-__global__ void __launch_bounds__(256) k_expand(const T* __restrict__ src, int64_t spitch, int64_t splane, int sw,
-                                                int sh, T* __restrict__ dst, int64_t dpitch, int64_t dplane, int dw,
-                                                int dh, int wrap)
+template <typename TIn, int S, bool PAIR>
+struct FinePixels {
+    const TIn* p;
+    int64_t pitch;
+    int frac;
+    template <typename T, int C>
+    __device__ __forceinline__ void load(const T*, int64_t, int64_t, int64_t, int X, int Y, int Y1, bool, bool x1,
+                                         int32_t (&f)[C][4]) const
+    {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const TIn* row = p + (int64_t)(r ? Y1 : Y) * pitch + (int64_t)X * S;
+            TIn px[2][S];
+            if (PAIR && x1) {
+                PixelPair<TIn, S>::load(row, px);
+            } else {
+                ld_px<TIn, S, false>(row, px[0]);
+                ld_px<TIn, S, false>(x1 ? row + S : row, px[1]);
+            }
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                f[c][2 * r] = (int32_t)px[0][c] << frac;
+                f[c][2 * r + 1] = (int32_t)px[1][c] << frac;
+            }
+        }
+    }
+};
+
+template <typename T>
+struct ExpandArgs {
+    const T* src;
+    T* dst;
+    int64_t spitch, splane, dpitch, dplane;
+    int sw, sh, dw, dh, wrap;
+    int pairs;    // destination rows hold aligned pairs
+    int chained;  // the launch before on the stream is another of the chain
+};
+
+template <typename T, int C, bool ADD, class FINE>
+__global__ void __launch_bounds__(256) k_expand(const __grid_constant__ ExpandArgs<T> a, const FINE fine)
 {
     __shared__ int32_t ss[C][ESH][ESW];
-    const int X0 = blockIdx.x * ETW, Y0 = blockIdx.y * ETH;
-    const int I0 = X0 >> 1, J0 = Y0 >> 1;
-    const int tid = threadIdx.x;
-
-    for (int k = tid; k < ESH * ESW; k += 256) {
-        const int r = k / ESW, c = k - r * ESW;
-        const int j = J0 - 1 + r;
-        int i = I0 - 1 + c;
-        if (wrap) {
-            i = imod(i, sw);
-        }
-        const bool in = j >= 0 && j < sh && i >= 0 && i < sw;
-#pragma unroll
-        for (int ch = 0; ch < C; ++ch) {
-            ss[ch][r][c] = in ? (int32_t)src[(int64_t)ch * splane + (int64_t)j * spitch + i] : 0;
-        }
+    if (!a.chained) {
+        griddep_wait();
     }
+    griddep_launch();
+    const int X0 = blockIdx.x * ETW, Y0 = blockIdx.y * ETH, I0 = X0 >> 1, J0 = Y0 >> 1;
+    const int qx = threadIdx.x % 32, qy = threadIdx.x / 32;
+    const int X = 2 * (I0 + qx), Y = 2 * (J0 + qy);
+    const bool on = X < a.dw && Y < a.dh, y1 = Y + 1 < a.dh;
+    const int Xc = min(X, a.dw - 1), Yc = min(Y, a.dh - 1), Y1 = min(Y + 1, a.dh - 1);
+    const bool x1 = Xc == X && X + 1 < a.dw, pair = a.pairs && x1;
+    const int64_t o = (int64_t)Yc * a.dpitch + Xc, o1 = (int64_t)Y1 * a.dpitch + Xc;
+    const TileWindow win(I0, J0, a.sw, a.sh, a.spitch, a.dw, a.wrap);
+    int32_t v[C][2], f[C][4];
+    if (!ADD) {
+        win.load_written<T, C>(a.src, a.splane, v);
+    }
+    fine.template load<T, C>(a.dst, o, o1, a.dplane, Xc, Yc, Y1, pair, x1, f);
+    griddep_wait();
+    if (ADD) {
+        win.load_written<T, C>(a.src, a.splane, v);
+    }
+    win.store<C>(ss, v);
     __syncthreads();
-
-    const int qx = tid % 32, qy = tid / 32;
-    const int i = I0 + qx, j = J0 + qy;
-    const int X = 2 * i, Y = 2 * j;
-    if (X >= dw || Y >= dh) {
-        return;
-    }
-    const bool has_x1 = X + 1 < dw, has_y1 = Y + 1 < dh;
-    const bool interior = i >= 1 && i + 1 < sw && j >= 1 && j + 1 < sh;
-
-    if (interior) {
+    const auto body = [&](const auto& div) {
 #pragma unroll
-        for (int ch = 0; ch < C; ++ch) {
-            const int32_t* a = &ss[ch][qy][qx];
-            const int32_t* b = &ss[ch][qy + 1][qx];
-            const int32_t* c = &ss[ch][qy + 2][qx];
-            const int32_t hea = a[0] + 6 * a[1] + a[2], heb = b[0] + 6 * b[1] + b[2], hec = c[0] + 6 * c[1] + c[2];
-            const int32_t hoa = 4 * (a[1] + a[2]), hob = 4 * (b[1] + b[2]), hoc = 4 * (c[1] + c[2]);
-            T* d0 = reinterpret_cast<T*>(dst) + (int64_t)ch * dplane + (int64_t)Y * dpitch + X;
-            expand_combine<T, ADD>(d0, (hea + 6 * heb + hec) / 64);
-            if (has_x1) {
-                expand_combine<T, ADD>(d0 + 1, (hoa + 6 * hob + hoc) / 64);
+        for (int c = 0; c < C; ++c) {
+            int32_t e[4];
+            expand_window<false>(ss[c], qx, qy, div, e);
+            T r[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                r[q] = ADD ? (T)sat_store<T>(f[c][q] + e[q]) : cast_store<T>((int64_t)f[c][q] - e[q]);
             }
-            if (has_y1) {
-                T* d1 = d0 + dpitch;
-                expand_combine<T, ADD>(d1, (heb + hec) / 16);
-                if (has_x1) {
-                    expand_combine<T, ADD>(d1 + 1, (hob + hoc) / 16);
+            T *p = a.dst + c * a.dplane + o, *q = a.dst + c * a.dplane + o1;
+            if (pair) {
+                st2<T>(p, r[0], r[1]);
+                if (y1) {
+                    st2<T>(q, r[2], r[3]);
+                }
+            } else {
+                p[0] = r[0];
+                if (x1) {
+                    p[1] = r[1];
+                }
+                if (y1) {
+                    q[0] = r[2];
+                    if (x1) {
+                        q[1] = r[3];
+                    }
                 }
             }
         }
+    };
+    if (!on) {
         return;
     }
-
-    // Border quads: per-position weights and divisors.
-#pragma unroll
-    for (int oy = 0; oy < 2; ++oy) {
-        const int YY = Y + oy;
-        if (YY >= dh) {
-            continue;
-        }
-        int vw[3], vden;
-        expand_vweights(YY, sh, vw, vden);
-#pragma unroll
-        for (int ox = 0; ox < 2; ++ox) {
-            const int XX = X + ox;
-            if (XX >= dw) {
-                continue;
-            }
-            int hw[3], hden;
-            expand_hweights(XX, sw, dw, wrap, hw, hden);
-            const int den = hden * vden;
-#pragma unroll
-            for (int ch = 0; ch < C; ++ch) {
-                int32_t num = 0;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const int32_t* row = &ss[ch][qy + a][qx];
-                    num += vw[a] * (hw[0] * row[0] + hw[1] * row[1] + hw[2] * row[2]);
-                }
-                T* d = reinterpret_cast<T*>(dst) + (int64_t)ch * dplane + (int64_t)YY * dpitch + XX;
-                expand_combine<T, ADD>(d, div_den(num, den));
-            }
-        }
+    if (interior_tile(X0, Y0, a.dw, a.dh, I0, J0, a.sw, a.sh)) {
+        body(QuadInside{});
+    } else {
+        body(QuadDivisors(X, Y, a.sw, a.sh, a.dw, a.wrap));
     }
 }
 
@@ -211,35 +253,87 @@ __global__ void __launch_bounds__(256) k_expand(const T* __restrict__ src, int64
 // Merge operators
 // ---------------------------------------------------------------------------
 
-// CartesianBlendFunctor (src/blend.h:41-76) in place on the black level,
+// CartesianBlendFunctor (src/blend.h:41-76) in place on the black levels,
 // evaluated by blend_sample (exact integer rounding, double only at ties).
-template <typename T, typename TM, int C>
-__global__ void __launch_bounds__(256) k_blend(const TM* __restrict__ mask, int64_t mpitch,
-                                               const T* __restrict__ white, int64_t wpitch, int64_t wplane,
-                                               T* __restrict__ black, int64_t bpitch, int64_t bplane, int w,
-                                               int h, int32_t white_value)
+// All levels in one launch, a run of four pixels a thread: the pass is bound by
+// memory (nothing is read where the mask is 0, white is copied where it is
+// full), and one launch a level and one pixel a thread took 77 us where this
+// takes 24 (nine levels of 1921x1081 Int32, with event overhead).
+struct BlendLevel {
+    const void *m, *w;
+    void* b;
+    int64_t mpitch, wpitch, wplane, bpitch, bplane;
+    int width, h;
+    int runs;        // a row's runs of four pixels
+    unsigned first;  // block
+};
+
+struct BlendLevels {
+    BlendLevel l[kMaxLevels];
+    int n;
+    int32_t white_value;
+};
+
+template <typename T>
+__device__ __forceinline__ void load4(const T* p, int32_t (&v)[4], int n)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y;
-    if (x >= w) {
-        return;
-    }
-    const int32_t m = (int32_t)mask[(int64_t)y * mpitch + x];
-    if (m <= 0) {
-        return;
-    }
-    if (m >= white_value) {
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            black[(int64_t)c * bplane + (int64_t)y * bpitch + x] = white[(int64_t)c * wplane + (int64_t)y * wpitch + x];
+    if (n == 4 && ((uintptr_t)p & (4 * sizeof(T) - 1)) == 0) {
+        if (sizeof(T) == 4) {
+            const int4 t = *reinterpret_cast<const int4*>(p);
+            v[0] = t.x;
+            v[1] = t.y;
+            v[2] = t.z;
+            v[3] = t.w;
+        } else {
+            const int2 t = *reinterpret_cast<const int2*>(p);
+            v[0] = (int32_t)(int16_t)(t.x & 0xffff);
+            v[1] = t.x >> 16;
+            v[2] = (int32_t)(int16_t)(t.y & 0xffff);
+            v[3] = t.y >> 16;
         }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            v[q] = q < n ? (int32_t)p[q] : 0;
+        }
+    }
+}
+
+template <typename T, typename TM, int C>
+__global__ void __launch_bounds__(256) k_blend(const __grid_constant__ BlendLevels a)
+{
+    griddep_wait();
+    griddep_launch();
+    int l = 0;
+    while (l + 1 < a.n && blockIdx.x >= a.l[l + 1].first) {
+        ++l;
+    }
+    const BlendLevel& b = a.l[l];
+    const unsigned i = (blockIdx.x - b.first) * 256 + threadIdx.x;
+    const int y = (int)(i / (unsigned)b.runs), x = 4 * (int)(i - (unsigned)y * (unsigned)b.runs);
+    if (y >= b.h) {
         return;
     }
+    const int n = min(4, b.width - x);
+    int32_t m[4];
+    load4((const TM*)b.m + (int64_t)y * b.mpitch + x, m, n);
+    if (max(max(m[0], m[1]), max(m[2], m[3])) <= 0) {
+        return;
+    }
+    const bool white = min(min(m[0], m[1]), min(m[2], m[3])) >= a.white_value;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-        T* b = &black[(int64_t)c * bplane + (int64_t)y * bpitch + x];
-        *b = (T)blend_sample<T>(m, white_value, (int32_t)white[(int64_t)c * wplane + (int64_t)y * wpitch + x],
-                                (int32_t)*b);
+        T* p = (T*)b.b + c * b.bplane + (int64_t)y * b.bpitch + x;
+        int32_t w[4], k[4];
+        load4((const T*)b.w + c * b.wplane + (int64_t)y * b.wpitch + x, w, n);
+        if (!white) {
+            load4(p, k, n);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                w[q] = blend_sample<T>(m[q], a.white_value, w[q], k[q]);
+            }
+        }
+        store4(p, w, n);
     }
 }
 
@@ -290,11 +384,13 @@ __global__ void __launch_bounds__(256) k_mask_mul_acc_generic(const T* __restric
 // ---------------------------------------------------------------------------
 
 template <typename TS, typename TD>
-__global__ void __launch_bounds__(256) k_from_fixed(const TS* __restrict__ src, int64_t spitch, int64_t splane, int C,
-                                                    const uint8_t* __restrict__ alpha, int64_t apitch,
-                                                    TD* __restrict__ dst, int64_t dpitch, int dstride, int w, int h,
-                                                    int frac, int dither, uint64_t seed, int32_t maxv)
+__global__ void __launch_bounds__(256) k_from_fixed(const TS* src, int64_t spitch, int64_t splane, int C,
+                                                    const uint8_t* alpha, int64_t apitch, TD* dst, int64_t dpitch,
+                                                    int dstride, int w, int h, int frac, int dither, uint64_t seed,
+                                                    int32_t maxv)
 {
+    griddep_wait();
+    griddep_launch();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= w || !alpha[(int64_t)y * apitch + x]) {
@@ -484,17 +580,17 @@ cudaError_t launch_to_fixed(const PixelView& s, const PlanarView& d, int frac, c
     note("to_fixed", npix(s.w, s.h) * s.C * esz(s.dtype) + planar_bytes(d));
     const dim3 g = row_grid(s.w, s.h);
     if (s.dtype == ENB_U8 && d.dtype == ENB_I16) {
-        k_to_fixed<uint8_t, int16_t><<<g, 256, 0, st>>>((const uint8_t*)s.p, s.pitch, s.stride, s.C, (int16_t*)d.p,
-                                                        d.pitch, d.plane, s.w, s.h, frac);
+        (void)launch_pdl(k_to_fixed<uint8_t, int16_t>, g, dim3(256), st,
+                         (const uint8_t*)s.p, s.pitch, s.stride, s.C, (int16_t*)d.p, d.pitch, d.plane, s.w, s.h, frac);
     } else if (s.dtype == ENB_U8 && d.dtype == ENB_I32) {
-        k_to_fixed<uint8_t, int32_t><<<g, 256, 0, st>>>((const uint8_t*)s.p, s.pitch, s.stride, s.C, (int32_t*)d.p,
-                                                        d.pitch, d.plane, s.w, s.h, frac);
+        (void)launch_pdl(k_to_fixed<uint8_t, int32_t>, g, dim3(256), st,
+                         (const uint8_t*)s.p, s.pitch, s.stride, s.C, (int32_t*)d.p, d.pitch, d.plane, s.w, s.h, frac);
     } else if (s.dtype == ENB_U16 && d.dtype == ENB_I32) {
-        k_to_fixed<uint16_t, int32_t><<<g, 256, 0, st>>>((const uint16_t*)s.p, s.pitch, s.stride, s.C,
-                                                         (int32_t*)d.p, d.pitch, d.plane, s.w, s.h, frac);
+        (void)launch_pdl(k_to_fixed<uint16_t, int32_t>, g, dim3(256), st,
+                         (const uint16_t*)s.p, s.pitch, s.stride, s.C, (int32_t*)d.p, d.pitch, d.plane, s.w, s.h, frac);
     } else if (s.dtype == ENB_U16 && d.dtype == ENB_I16) {
-        k_to_fixed<uint16_t, int16_t><<<g, 256, 0, st>>>((const uint16_t*)s.p, s.pitch, s.stride, s.C,
-                                                         (int16_t*)d.p, d.pitch, d.plane, s.w, s.h, frac);
+        (void)launch_pdl(k_to_fixed<uint16_t, int16_t>, g, dim3(256), st,
+                         (const uint16_t*)s.p, s.pitch, s.stride, s.C, (int16_t*)d.p, d.pitch, d.plane, s.w, s.h, frac);
     } else {
         return cudaErrorInvalidValue;
     }
@@ -688,6 +784,53 @@ cudaError_t launch_reduce_img2_mask(int wrap, const PlanarView& s0, const BytePl
     return cudaGetLastError();
 }
 
+template <typename T, int C>
+static cudaError_t reduce_tail_t(int wrap, int n, const PlanarView* s, const BytePlane* al, cudaStream_t st)
+{
+    TailJobs<T, T> j{};
+    j.g.n = n;
+    j.images = 1;
+    for (int i = 0; i < n; ++i) {
+        j.g.w[i] = s[i].w;
+        j.g.h[i] = s[i].h;
+        j.g.pitch[i] = s[i].pitch;
+        j.img[0][i] = (T*)s[i].p;
+        if (al) {
+            j.g.apitch[i] = al[i].pitch;
+            j.a[0][i] = al[i].p;
+        }
+    }
+    return al ? launch_reduce_tail<T, C, T, kReduceAlpha, kReduceClamp>(j, 0, wrap, st)
+              : launch_reduce_tail<T, C, T, kReduceClamp, kReduceClamp>(j, 0, wrap, st);
+}
+
+// A pyramid of the caller's may be of any shape and depth: the level's row of
+// column sums has to fit, and the last kTailLevels levels are enough.
+int pyramid_tail_level(const int* lw, const int* lh, int L, int dtype)
+{
+    int l = L > kTailLevels ? L - kTailLevels : 1;
+    while (l < L && ((int64_t)lw[l] * lh[l] > kTailPixels || lw[l] > 512)) {
+        ++l;
+    }
+    return dtype != ENB_F32 && l + 2 < L ? l : L;
+}
+
+cudaError_t launch_reduce_tail_levels(int wrap, int n, const PlanarView* s, const BytePlane* al, cudaStream_t st)
+{
+    bool fits = n >= 2 && n <= kTailLevels && s[0].dtype != ENB_F32;
+    for (int i = 0; i < n && fits; ++i) {
+        fits = (int64_t)s[i].w * s[i].h <= kTailPixels && s[i].w <= 512 && s[i].plane == s[i].pitch * s[i].h;
+    }
+    if (!fits) {
+        return cudaErrorInvalidValue;
+    }
+    note("reduce_tail", 0.0);
+    if (s[0].dtype == ENB_I16) {
+        return s[0].C == 1 ? reduce_tail_t<int16_t, 1>(wrap, n, s, al, st) : reduce_tail_t<int16_t, 3>(wrap, n, s, al, st);
+    }
+    return s[0].C == 1 ? reduce_tail_t<int32_t, 1>(wrap, n, s, al, st) : reduce_tail_t<int32_t, 3>(wrap, n, s, al, st);
+}
+
 int enb_tail_level(const int* lw, const int* lh, int L) { return tail_level(lw, lh, L); }
 
 template <typename T, typename TM, int C>
@@ -738,20 +881,24 @@ cudaError_t launch_reduce_img2_mask_tail(int wrap, int n, const PlanarView* s0, 
 #undef ENB_RIT
 }
 
-template <typename T, int C>
-static void expand_dispatch(int add, int wrap, const PlanarView& s, const PlanarView& d, cudaStream_t st)
+template <typename T>
+static ExpandArgs<T> expand_args(const PlanarView& s, const PlanarView& d, int wrap, bool chained)
 {
-    const dim3 g = grid2d(d.w, d.h, ETW, ETH);
-    if (add) {
-        k_expand<T, C, true><<<g, 256, 0, st>>>((const T*)s.p, s.pitch, s.plane, s.w, s.h, (T*)d.p, d.pitch, d.plane,
-                                                d.w, d.h, wrap);
-    } else {
-        k_expand<T, C, false><<<g, 256, 0, st>>>((const T*)s.p, s.pitch, s.plane, s.w, s.h, (T*)d.p, d.pitch, d.plane,
-                                                 d.w, d.h, wrap);
-    }
+    const bool pairs = (uintptr_t)d.p % (2 * sizeof(T)) == 0 && d.pitch % 2 == 0 && d.plane % 2 == 0;
+    return ExpandArgs<T>{(const T*)s.p, (T*)d.p, s.pitch, s.plane, d.pitch, d.plane, s.w, s.h,
+                         d.w, d.h, wrap, pairs, chained};
 }
 
-cudaError_t launch_expand(int add, int wrap, const PlanarView& s, const PlanarView& d, cudaStream_t st)
+template <typename T, int C>
+static cudaError_t expand_dispatch(int add, int wrap, const PlanarView& s, const PlanarView& d, bool chained,
+                                   cudaStream_t st)
+{
+    const ExpandArgs<T> a = expand_args<T>(s, d, wrap, chained);
+    return launch_pdl(add ? k_expand<T, C, true, FineLevel> : k_expand<T, C, false, FineLevel>,
+                      grid2d(d.w, d.h, ETW, ETH), dim3(256), st, a, FineLevel{});
+}
+
+cudaError_t launch_expand(int add, int wrap, const PlanarView& s, const PlanarView& d, cudaStream_t st, bool chained)
 {
     if (s.dtype != d.dtype || s.C != d.C) {
         return cudaErrorInvalidValue;
@@ -761,54 +908,100 @@ cudaError_t launch_expand(int add, int wrap, const PlanarView& s, const PlanarVi
     }
     note(add ? "expand_add" : "expand_sub", planar_bytes(s) + 2.0 * planar_bytes(d));
     if (s.dtype == ENB_I16) {
-        if (s.C == 1) {
-            expand_dispatch<int16_t, 1>(add, wrap, s, d, st);
-        } else {
-            expand_dispatch<int16_t, 3>(add, wrap, s, d, st);
-        }
-    } else {
-        if (s.C == 1) {
-            expand_dispatch<int32_t, 1>(add, wrap, s, d, st);
-        } else {
-            expand_dispatch<int32_t, 3>(add, wrap, s, d, st);
-        }
+        return s.C == 1 ? expand_dispatch<int16_t, 1>(add, wrap, s, d, chained, st)
+                        : expand_dispatch<int16_t, 3>(add, wrap, s, d, chained, st);
     }
-    return cudaGetLastError();
+    return s.C == 1 ? expand_dispatch<int32_t, 1>(add, wrap, s, d, chained, st)
+                    : expand_dispatch<int32_t, 3>(add, wrap, s, d, chained, st);
 }
 
-template <typename T, typename TM, int C>
-static void blend_dispatch(const PlanarView& m, const PlanarView& wt, const PlanarView& b, int32_t wv,
-                           cudaStream_t st)
+template <typename TIn, typename T, int C, int S>
+static cudaError_t laplacian0_dispatch(const PixelView& px, int frac, int wrap, const PlanarView& g1, const PlanarView& l0,
+                                       cudaStream_t st)
 {
-    k_blend<T, TM, C><<<row_grid(b.w, b.h), 256, 0, st>>>((const TM*)m.p, m.pitch, (const T*)wt.p, wt.pitch, wt.plane,
-                                                          (T*)b.p, b.pitch, b.plane, b.w, b.h, wv);
+    const ExpandArgs<T> a = expand_args<T>(g1, l0, wrap, false);
+    const dim3 g = grid2d(l0.w, l0.h, ETW, ETH);
+    const TIn* p = (const TIn*)px.p;
+    if (run_aligned<PixelPair<TIn, S>>(p, (size_t)px.pitch * sizeof(TIn))) {
+        return launch_pdl(k_expand<T, C, false, FinePixels<TIn, S, true>>, g, dim3(256), st, a,
+                          FinePixels<TIn, S, true>{p, px.pitch, frac});
+    }
+    return launch_pdl(k_expand<T, C, false, FinePixels<TIn, S, false>>, g, dim3(256), st, a,
+                      FinePixels<TIn, S, false>{p, px.pitch, frac});
 }
 
-cudaError_t launch_blend(const PlanarView& m, const PlanarView& wt, const PlanarView& b, int32_t wv,
-                         cudaStream_t st)
+bool laplacian_takes_pixels(int px_dtype, int C, int stride, int dtype, int frac)
 {
-    if (wt.dtype != b.dtype || wt.C != b.C) {
+    const bool value = (px_dtype == ENB_U8 && dtype == ENB_I16 && frac <= 7) ||
+                       (px_dtype == ENB_U16 && dtype == ENB_I32 && frac <= 15);
+    return value && ((C == 1 && stride == 1) || (C == 3 && (stride == 3 || stride == 4)));
+}
+
+cudaError_t launch_laplacian0(const PixelView& px, int frac, int wrap, const PlanarView& g1, const PlanarView& l0,
+                              cudaStream_t st)
+{
+    if (g1.dtype != l0.dtype || g1.C != l0.C || px.C != l0.C ||
+        !laplacian_takes_pixels(px.dtype, px.C, px.stride, l0.dtype, frac)) {
         return cudaErrorInvalidValue;
     }
-    if (b.dtype == ENB_F32) {
-        return m.dtype == ENB_I32 ? launch_f_blend(m, wt, b, wv, st) : cudaErrorInvalidValue;
+    note("laplacian0", npix(px.w, px.h) * px.stride * esz(px.dtype) + planar_bytes(g1) + planar_bytes(l0));
+    if (px.dtype == ENB_U8) {
+        return px.C == 1 ? laplacian0_dispatch<uint8_t, int16_t, 1, 1>(px, frac, wrap, g1, l0, st)
+               : px.stride == 3 ? laplacian0_dispatch<uint8_t, int16_t, 3, 3>(px, frac, wrap, g1, l0, st)
+                                : laplacian0_dispatch<uint8_t, int16_t, 3, 4>(px, frac, wrap, g1, l0, st);
     }
-    note("blend", planar_bytes(m) + planar_bytes(wt) + 2.0 * planar_bytes(b));
-    const bool m16 = m.dtype == ENB_I16;
-    if (b.dtype == ENB_I16) {
-        if (b.C == 1) {
-            m16 ? blend_dispatch<int16_t, int16_t, 1>(m, wt, b, wv, st) : blend_dispatch<int16_t, int32_t, 1>(m, wt, b, wv, st);
-        } else {
-            m16 ? blend_dispatch<int16_t, int16_t, 3>(m, wt, b, wv, st) : blend_dispatch<int16_t, int32_t, 3>(m, wt, b, wv, st);
+    return px.C == 1 ? laplacian0_dispatch<uint16_t, int32_t, 1, 1>(px, frac, wrap, g1, l0, st)
+           : px.stride == 3 ? laplacian0_dispatch<uint16_t, int32_t, 3, 3>(px, frac, wrap, g1, l0, st)
+                            : laplacian0_dispatch<uint16_t, int32_t, 3, 4>(px, frac, wrap, g1, l0, st);
+}
+
+cudaError_t launch_blend(int n, const PlanarView* m, const PlanarView* wt, const PlanarView* b, int32_t wv,
+                         cudaStream_t st)
+{
+    double bytes = 0.0;
+    for (int i = 0; i < n; ++i) {
+        if (wt[i].dtype != b[0].dtype || wt[i].C != b[0].C || b[i].dtype != b[0].dtype || b[i].C != b[0].C ||
+            m[i].dtype != m[0].dtype) {
+            return cudaErrorInvalidValue;
         }
-    } else {
-        if (b.C == 1) {
-            m16 ? blend_dispatch<int32_t, int16_t, 1>(m, wt, b, wv, st) : blend_dispatch<int32_t, int32_t, 1>(m, wt, b, wv, st);
-        } else {
-            m16 ? blend_dispatch<int32_t, int16_t, 3>(m, wt, b, wv, st) : blend_dispatch<int32_t, int32_t, 3>(m, wt, b, wv, st);
-        }
+        bytes += planar_bytes(m[i]) + planar_bytes(wt[i]) + 2.0 * planar_bytes(b[i]);
     }
-    return cudaGetLastError();
+    if (n < 1 || n > kMaxLevels) {
+        return cudaErrorInvalidValue;
+    }
+    if (b[0].dtype == ENB_F32) {
+        for (int i = 0; i < n; ++i) {
+            const cudaError_t e = m[i].dtype == ENB_I32 ? launch_f_blend(m[i], wt[i], b[i], wv, st) : cudaErrorInvalidValue;
+            if (e != cudaSuccess) {
+                return e;
+            }
+        }
+        last_launch() = LaunchInfo{"blend", bytes, n};
+        return cudaSuccess;
+    }
+    BlendLevels a{};
+    a.n = n;
+    a.white_value = wv;
+    unsigned blocks = 0;
+    for (int i = 0; i < n; ++i) {
+        const int runs = (b[i].w + 3) / 4;
+        a.l[i] = BlendLevel{m[i].p, wt[i].p, b[i].p, m[i].pitch, wt[i].pitch, wt[i].plane,
+                            b[i].pitch, b[i].plane, b[i].w, b[i].h, runs, blocks};
+        blocks += (unsigned)(((int64_t)runs * b[i].h + 255) / 256);
+    }
+    note("blend", bytes);
+    const dim3 g(blocks), t(256);
+    const bool m16 = m[0].dtype == ENB_I16;
+    if (b[0].dtype == ENB_I16) {
+        if (b[0].C == 1) {
+            return launch_pdl(m16 ? k_blend<int16_t, int16_t, 1> : k_blend<int16_t, int32_t, 1>, g, t, st, a);
+        }
+        return launch_pdl(m16 ? k_blend<int16_t, int16_t, 3> : k_blend<int16_t, int32_t, 3>, g, t, st, a);
+    }
+    if (b[0].C == 1) {
+        return launch_pdl(m16 ? k_blend<int32_t, int16_t, 1> : k_blend<int32_t, int32_t, 1>, g, t, st, a);
+    }
+    return launch_pdl(m16 ? k_blend<int32_t, int16_t, 3> : k_blend<int32_t, int32_t, 3>, g, t, st, a);
 }
 
 template <typename T, typename TM, int C>
@@ -869,23 +1062,23 @@ cudaError_t launch_from_fixed(const PlanarView& s, const BytePlane& a, void* dst
     const dim3 g = row_grid(s.w, s.h);
     if (s.dtype == ENB_I16) {
         if (ddtype == ENB_U8) {
-            k_from_fixed<int16_t, uint8_t><<<g, 256, 0, st>>>((const int16_t*)s.p, s.pitch, s.plane, s.C, a.p, a.pitch,
-                                                              (uint8_t*)dst, dpitch, dstride, s.w, s.h, frac, dither,
-                                                              seed, 255);
+            (void)launch_pdl(k_from_fixed<int16_t, uint8_t>, g, dim3(256), st,
+                             (const int16_t*)s.p, s.pitch, s.plane, s.C, a.p, a.pitch, (uint8_t*)dst, dpitch, dstride,
+                             s.w, s.h, frac, dither, seed, 255);
         } else {
-            k_from_fixed<int16_t, uint16_t><<<g, 256, 0, st>>>((const int16_t*)s.p, s.pitch, s.plane, s.C, a.p, a.pitch,
-                                                               (uint16_t*)dst, dpitch, dstride, s.w, s.h, frac, dither,
-                                                               seed, 65535);
+            (void)launch_pdl(k_from_fixed<int16_t, uint16_t>, g, dim3(256), st,
+                             (const int16_t*)s.p, s.pitch, s.plane, s.C, a.p, a.pitch, (uint16_t*)dst, dpitch, dstride,
+                             s.w, s.h, frac, dither, seed, 65535);
         }
     } else {
         if (ddtype == ENB_U8) {
-            k_from_fixed<int32_t, uint8_t><<<g, 256, 0, st>>>((const int32_t*)s.p, s.pitch, s.plane, s.C, a.p, a.pitch,
-                                                              (uint8_t*)dst, dpitch, dstride, s.w, s.h, frac, dither,
-                                                              seed, 255);
+            (void)launch_pdl(k_from_fixed<int32_t, uint8_t>, g, dim3(256), st,
+                             (const int32_t*)s.p, s.pitch, s.plane, s.C, a.p, a.pitch, (uint8_t*)dst, dpitch, dstride,
+                             s.w, s.h, frac, dither, seed, 255);
         } else {
-            k_from_fixed<int32_t, uint16_t><<<g, 256, 0, st>>>((const int32_t*)s.p, s.pitch, s.plane, s.C, a.p, a.pitch,
-                                                               (uint16_t*)dst, dpitch, dstride, s.w, s.h, frac, dither,
-                                                               seed, 65535);
+            (void)launch_pdl(k_from_fixed<int32_t, uint16_t>, g, dim3(256), st,
+                             (const int32_t*)s.p, s.pitch, s.plane, s.C, a.p, a.pitch, (uint16_t*)dst, dpitch, dstride,
+                             s.w, s.h, frac, dither, seed, 65535);
         }
     }
     return cudaGetLastError();

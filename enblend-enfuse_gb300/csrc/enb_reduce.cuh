@@ -587,14 +587,4 @@ inline int tail_level(const int* lw, const int* lh, int L)
     return L;
 }
 
-template <class Src, typename TD, int C, bool ALPHA>
-inline void launch_reduce_tiles(const Src& src, int sw, int sh, TD* dst, int64_t dpitch, int64_t dplane, int dw,
-                                int dh, uint8_t* da, int64_t dapitch, int wrap, cudaStream_t st)
-{
-    ReduceJobs<Src, TD> jobs{};
-    jobs.j[0] = ReduceJob<Src, TD>{src, dst, dpitch, dplane, da, dapitch};
-    jobs.j[1] = jobs.j[0];
-    launch_reduce_jobs<Src, TD, C, ALPHA>(jobs, 1, sw, sh, dw, dh, wrap, st);
-}
-
 }  // namespace enb

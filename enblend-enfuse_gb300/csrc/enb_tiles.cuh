@@ -122,8 +122,8 @@ __device__ __forceinline__ void expand9(const int32_t (&v)[3][3], int32_t e[4])
 // interior numerators of expand9 those of the border positions
 // (expand_hweights / expand_vweights) too; the one other weight there, 4 at
 // the seam of a periodic level of odd width, goes into the stored tap, as no
-// other position reads it.  (Coarse levels are at least five pixels wide, so
-// the rule for a single periodic column does not arise.)
+// other position reads it.  A single periodic column is its own left
+// neighbour and has no right one.
 struct TileWindow {
     int64_t o[2];  // offset of the tap in a coarse plane
     int32_t f[2];  // factor of the stored tap: 0, 1 or 4
@@ -139,7 +139,7 @@ struct TileWindow {
             int i = I0 - 1 + c;
             f[u] = wrap && (dw & 1) && (i == -1 || i == cw) ? 4 : 1;
             if (wrap) {
-                i = imod(i, cw);
+                i = cw == 1 && i > 0 ? cw : imod(i, cw);
             }
             f[u] = j >= 0 && j < ch && i >= 0 && i < cw ? f[u] : 0;
             o[u] = (int64_t)min(max(j, 0), ch - 1) * cpitch + min(max(i, 0), cw - 1);

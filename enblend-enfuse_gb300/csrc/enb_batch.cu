@@ -267,16 +267,19 @@ __global__ void __launch_bounds__(256, 4) k_batch_weights(ENB_BATCH_JOBS(J), Flo
     }
 }
 
-// Weights, normalisation, level 0 of the image pyramids and of the mask
-// pyramids, and the union alpha of a 32x16 tile of a stack, two output
-// pixels per thread (enb_fpair.cuh).  The exposures' tiles come in turn; a
-// pixel's weight waits in its exposure's level-0 mask plane (as float bits)
-// until the normalisation replaces it.  Five CTAs per SM (48 registers;
-// the 42.6 KB tile of 5x5 windows fits five times): the warps hide the
-// kernel's latencies better than more registers would.  For the same reason the
-// tables come inside a struct, not as restrict parameters: reading the stack's
-// fields again after every store costs less than the registers that keep them
-// (16 stacks: 10.9 against 11.5 ms).
+// Weights and level 0 of the image pyramid of a 32x16 tile of an exposure, two
+// output pixels per thread (enb_fpair.cuh).  A pixel's weight waits in its
+// exposure's level-0 mask plane (as float bits) until k_batch_normalise
+// replaces it.  Five CTAs per SM (48 registers; the 42.6 KB tile of 5x5
+// windows fits five times): the warps hide the kernel's latencies better than
+// more registers would.  For the same reason the tables come inside a struct,
+// not as restrict parameters: reading the stack's fields again after every
+// store costs less than the registers that keep them (16 stacks: 10.9 against
+// 11.5 ms).  A block is one exposure of a tile (blockIdx.z, in a batch
+// blockIdx.y, where those past a stack's exposures leave at once): a tile's
+// exposures in turn made blocks several times as long, and a single stack's
+// last wave of them kept the chip busy to 73 % (with the search for repeats of
+// fpair_load, 4x1601x1203: 0.39 to 0.24 ms; 16 stacks: 10.9 to 9.4 ms).
 template <int CW, int EW, int C, class J>
 __global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const __grid_constant__ BatchJobs<J> j,
                                                                FloatWeightParams wp, WeightTables tab)
@@ -286,77 +289,48 @@ __global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const __grid_cons
     extern __shared__ __align__(16) unsigned char bsmem[];
     griddep_wait();
     griddep_launch();
-    const int2 tile = job_tile<J>(j.jobs);
+    const int k = J::kOne ? (int)blockIdx.z : (int)blockIdx.y;
     const BatchStack& s = job_stack(j.stacks, j.jobs, j.one);
-    const FTileP t0 = fpair_carve(bsmem, TW, TT, wp.repeat_slots, wp.ent_cut);
+    if (k >= s.K) {
+        return;
+    }
+    const int2 tile = job_tile<J>(j.jobs);
+    const FTileP t = fpair_carve(bsmem, TW, TT, wp.repeat_slots, wp.ent_cut);
     const int px = threadIdx.x % (FPX / 2), py = threadIdx.x / (FPX / 2);
     const int x = tile.x * FPX + 2 * px, y = tile.y * FPY + py;
     const bool in0 = x < s.w && y < s.h, in1 = x + 1 < s.w && y < s.h;
     const int cx = HX + 2 * px, cy = HALO + py, ci = cy * TW + cx;
-    const int K = s.K;
     const int64_t plane = (int64_t)s.pitch[0] * s.h, o = (int64_t)y * s.pitch[0] + x;
-    const int x0 = tile.x * FPX - HX, y0 = tile.y * FPY - HALO;
-    uint8_t ua0 = 0, ua1 = 0;
-    if (t0.slots) {
-        fpair_clear_tables<C>(fpair_for_exposure(t0, 0));
-        __syncthreads();
+    const int opaque = fpair_load<NP, C, TW, TT>(t, wp, s.img[k], s.ipitch[k], s.istride[k], s.w, s.h, s.alpha[k],
+                                                 s.apitch[k], tile.x * FPX - HX, tile.y * FPY - HALO);
+    float w0, w1;
+    fpair_weights<CW, EW, C>(t, wp, tab, cx, cy, x, y, s.w, s.h, opaque != 0, w0, w1);
+    if (!in0) {
+        return;
     }
-    for (int k = 0; k < K; ++k) {
-        const FTileP t = fpair_for_exposure(t0, k);
-        const int opaque = fpair_load<NP, C, TW, TT>(t, wp, s.img[k], s.ipitch[k], s.istride[k], s.w, s.h, s.alpha[k],
-                                                     s.apitch[k], x0, y0);
-        if (in0) {
-            float w0, w1;
-            fpair_weights<CW, EW, C>(t, wp, tab, cx, cy, x, y, s.w, s.h, opaque != 0, w0, w1);
-            int32_t* m0 = m_level(s, k, 0) + o;
-            float* g0 = g0_level(s, k, C) + o;
-            if (in1) {
-                // x is even and rows start on 128-byte boundaries
-                *reinterpret_cast<int2*>(m0) = make_int2(__float_as_int(w0), __float_as_int(w1));
+    int32_t* m0 = m_level(s, k, 0) + o;
+    float* g0 = g0_level(s, k, C) + o;
+    if (in1) {
+        // x is even and rows start on 128-byte boundaries
+        *reinterpret_cast<int2*>(m0) = make_int2(__float_as_int(w0), __float_as_int(w1));
 #pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    // level 0 of the exposure's image pyramid: the log mapping, once
-                    *reinterpret_cast<float2*>(g0 + c * plane) =
-                        make_float2(to_pyramid_value(t.raw[c * TT + ci]), to_pyramid_value(t.raw[c * TT + ci + 1]));
-                }
-            } else {
-                m0[0] = __float_as_int(w0);
+        for (int c = 0; c < C; ++c) {
+            // level 0 of the exposure's image pyramid: the log mapping, once
+            *reinterpret_cast<float2*>(g0 + c * plane) =
+                make_float2(to_pyramid_value(t.raw[c * TT + ci]), to_pyramid_value(t.raw[c * TT + ci + 1]));
+        }
+    } else {
+        m0[0] = __float_as_int(w0);
 #pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    g0[c * plane] = to_pyramid_value(t.raw[c * TT + ci]);
-                }
-            }
-        }
-        ua0 |= t.a[ci];
-        ua1 |= t.a[ci + 1];
-        if (t.slots && k + 1 < K) {
-            // the tables for exposure k + 1 (the load of exposure k has ended
-            // with a barrier; exposure k - 1's row masks were read before
-            // the previous barrier)
-            fpair_clear_tables<C>(fpair_for_exposure(t0, k + 1));
-        }
-        __syncthreads();  // the next exposure's load overwrites the tile; its tables are empty
-    }
-    // the union alpha; k_batch_normalise turns the weights into masks
-    if (in0) {
-        const uint8_t u0 = ua0 ? 255 : 0, u1 = ua1 ? 255 : 0;
-        s.u[s.off0[0] + o] = u0;
-        if (in1) {
-            s.u[s.off0[0] + o + 1] = u1;
-        }
-        if (s.oalpha) {
-            uint8_t* oa = s.oalpha + (int64_t)y * s.oapitch + x;
-            oa[0] = u0;
-            if (in1) {
-                oa[1] = u1;
-            }
+        for (int c = 0; c < C; ++c) {
+            g0[c * plane] = to_pyramid_value(t.raw[c * TT + ci]);
         }
     }
 }
 
-// Normalisation of the weights that k_batch_weights_pair left in the level-0
-// mask planes (float bits) of a 32x16 tile of a stack, two output pixels per
-// thread: src/enfuse.h:1382-1385 (sum in exposure order), :1399-1442 (hard
+// Union alpha, and normalisation of the weights that k_batch_weights_pair left
+// in the level-0 mask planes (float bits), of a 32x16 tile of a stack, two
+// output pixels per thread: src/enfuse.h:1382-1385 (sum in exposure order), :1399-1442 (hard
 // mask), :1526-1535 (soft mask), into Int32 9.15 masks.
 template <class J>
 __global__ void __launch_bounds__(256) k_batch_normalise(ENB_BATCH_JOBS(J), int hard)
@@ -378,6 +352,26 @@ __global__ void __launch_bounds__(256) k_batch_normalise(ENB_BATCH_JOBS(J), int 
         // x is even and rows start on 128-byte boundaries
         return pair ? __ldcg(reinterpret_cast<const float2*>(m)) : make_float2(__int_as_float(__ldcg(m)), 0.0f);
     };
+    int u0 = 0, u1 = 0;  // the union alpha
+    for (int k = 0; k < K && !(u0 && u1); ++k) {
+        const uint8_t* a = s.alpha[k] ? s.alpha[k] + (int64_t)y * s.apitch[k] + x : nullptr;
+        u0 |= a ? a[0] : 1;
+        u1 |= a ? (pair ? a[1] : 0) : 1;
+    }
+    u0 = u0 ? 255 : 0;
+    u1 = u1 ? 255 : 0;
+    uint8_t* u = s.u + s.off0[0] + o;
+    u[0] = (uint8_t)u0;
+    if (pair) {
+        u[1] = (uint8_t)u1;
+    }
+    if (s.oalpha) {
+        uint8_t* oa = s.oalpha + (int64_t)y * s.oapitch + x;
+        oa[0] = (uint8_t)u0;
+        if (pair) {
+            oa[1] = (uint8_t)u1;
+        }
+    }
     const auto put = [&](int k, float m0, float m1) {
         int32_t* m = m_level(s, k, 0) + o;
         if (pair) {
@@ -1500,7 +1494,8 @@ static cudaError_t launch_step(const BatchPlan* p, const BatchPlan::Step& s, cud
     switch (s.kind) {
     case 0:
         note_launch("batch_weights", s.bytes);
-        return launch_weights<C>(j, grid, p->pair_weights, p->wp, p->tab, p->hard, p->wsmem, st);
+        return launch_weights<C>(j, dim3(grid.x, p->pair_weights ? (unsigned)p->maxK : 1u), p->pair_weights, p->wp, p->tab,
+                                 p->hard, p->wsmem, st);
     case 5:
         note_launch("batch_normalise", s.bytes);
         return launch_batch<BatchTable>(k_batch_normalise<BatchTable>, grid, 256, 0, st, j.stacks, j.jobs, j.one, p->hard);
@@ -1610,7 +1605,7 @@ static cudaError_t single_step(const BatchSingle* p, int i, cudaStream_t st)
     switch (p->steps[(size_t)i].kind) {
     case 0:
         note_launch("batch_weights", K * px * (4.0 * s.istride[0] + 4.0 * C + 4.0) + px);
-        return launch_weights<C>(j, tiles(s.w, s.h, p->ws.tx, p->ws.ty, 1), p->ws.pair, p->wp, p->tab, p->hard, p->ws.smem, st);
+        return launch_weights<C>(j, tiles(s.w, s.h, p->ws.tx, p->ws.ty, p->ws.pair ? K : 1), p->ws.pair, p->wp, p->tab, p->hard, p->ws.smem, st);
     case 1:
         note_launch("batch_normalise", K * px * 12.0);
         return launch_batch<BatchOne>(k_batch_normalise<BatchOne>, tiles(s.w, s.h, FPX, FPY, 1), 256, 0, st, j.stacks, j.jobs, j.one,

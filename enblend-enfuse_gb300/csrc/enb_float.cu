@@ -267,19 +267,15 @@ __global__ void __launch_bounds__(FPT, 4) k_f_enfuse_mask_pair(FloatPixelView im
     constexpr int TW = fpair_tw(CW, EW), TT = TW * fpair_th(CW, EW), NP = (TT + 255) / 256;
     extern __shared__ __align__(16) unsigned char fsmem[];
     const FTileP t = fpair_carve(fsmem, TW, TT, wp.repeat_slots, wp.ent_cut);
-    if (t.slots) {
-        fpair_clear_tables<C>(t);
-        __syncthreads();
-    }
     const int opaque = fpair_load<NP, C, TW, TT>(t, wp, img.p, img.pitch, img.stride, img.w, img.h, alpha, apitch,
                                                  blockIdx.x * FPX - HX, blockIdx.y * FPY - HALO);
     const int px = threadIdx.x % (FPX / 2), py = threadIdx.x / (FPX / 2);
     const int x = blockIdx.x * FPX + 2 * px, y = blockIdx.y * FPY + py;
+    float w0, w1;
+    fpair_weights<CW, EW, C>(t, wp, tab, HX + 2 * px, HALO + py, x, y, img.w, img.h, opaque != 0, w0, w1);
     if (x >= img.w || y >= img.h) {
         return;
     }
-    float w0, w1;
-    fpair_weights<CW, EW, C>(t, wp, tab, HX + 2 * px, HALO + py, x, y, img.w, img.h, opaque != 0, w0, w1);
     float* o = out + (int64_t)y * opitch + x;
     o[0] = w0;
     if (x + 1 < img.w) {

@@ -49,9 +49,9 @@ struct FTileP {
     float* gray;      // [TT]
     float* raw;       // [3][TT]
     float* eraw;      // [3][TT]: the entropy cutoff's clamped samples, else raw
-    uint32_t* table;     // [3][slots] repeat hash
-    uint64_t* markrow;   // [3][FPMAXROWS] of the exposure being weighted: bit x of row y: pixel (x, y)
-                         // has a repeat mark in that channel (two such buffers, by exposure parity)
+    uint16_t* table;     // [2][3][slots]: tile pixels by hashed sample (fpair_load)
+    uint64_t* markrow;   // [3][FPMAXROWS]: bit x of row y: pixel (x, y) has a repeat mark in that channel
+    uint32_t* listed;    // windows in the list of fpair_weights
     uint8_t* a;          // [TT] opaque flags
     int TW, TT, slots;
 };
@@ -61,7 +61,7 @@ constexpr int FPMAXROWS = FPY + 6;
 
 __host__ __device__ inline size_t fpair_tile_bytes(int TT, int slots, int ent_cut)
 {
-    return (size_t)TT * (8 + 4 + 12 + (ent_cut ? 12 : 0)) + (size_t)slots * 12 + (size_t)2 * 3 * FPMAXROWS * 8 +
+    return (size_t)TT * (8 + 4 + 12 + (ent_cut ? 12 : 0)) + (size_t)slots * 12 + (size_t)3 * FPMAXROWS * 8 + 16 +
            align16_sz((size_t)TT);
 }
 
@@ -97,45 +97,47 @@ __device__ __forceinline__ FTileP fpair_carve(unsigned char* smem, int TW, int T
     t.gray = reinterpret_cast<float*>(t.cnt + TT);
     t.raw = t.gray + TT;
     t.eraw = ent_cut ? t.raw + 3 * TT : t.raw;
-    t.table = reinterpret_cast<uint32_t*>(t.raw + (ent_cut ? 6 : 3) * TT);
-    t.markrow = reinterpret_cast<uint64_t*>(t.table + 3 * slots);
-    t.a = reinterpret_cast<uint8_t*>(t.markrow + 2 * 3 * FPMAXROWS);
+    t.table = reinterpret_cast<uint16_t*>(t.raw + (ent_cut ? 6 : 3) * TT);
+    t.markrow = reinterpret_cast<uint64_t*>(t.table + 2 * 3 * slots);
+    t.listed = reinterpret_cast<uint32_t*>(t.markrow + 3 * FPMAXROWS);
+    t.a = reinterpret_cast<uint8_t*>(t.listed + 4);
     return t;
 }
 
-// Tile t with the row-mask buffer of exposure k.
-__device__ __forceinline__ FTileP fpair_for_exposure(FTileP t, int k)
-{
-    t.markrow += (k & 1) * 3 * FPMAXROWS;
-    return t;
-}
-
-// Empties the C hash tables of the repeat marks and the row masks of t
-// (t.markrow: the buffer to be filled next).  The tables are used only while
-// a tile is loaded; the row masks are read while its windows are weighted,
-// so the kernels alternate two row-mask buffers and empty the one that no
-// thread reads.
-template <int C>
-__device__ __forceinline__ void fpair_clear_tables(const FTileP& t)
-{
-    uint4* t4 = reinterpret_cast<uint4*>(t.table);
-    const uint4 pad = make_uint4(kEntropyPad, kEntropyPad, kEntropyPad, kEntropyPad);
-    for (int i = threadIdx.x; i < C * t.slots / 4; i += FPT) {
-        t4[i] = pad;
-    }
-    if (threadIdx.x < 3 * FPMAXROWS) {
-        t.markrow[threadIdx.x] = 0ull;
-    }
-}
-
-// Records a repeat mark of channel c at tile pixel p in its counters and in
-// the channel's row mask (the owner of p only).
+// Records the repeat mark of channel c at tile pixel p in its counters and in
+// the channel's row mask (32-bit: the 64-bit operation would be a loop over the
+// lanes that meet in a row).  Only the thread that owns p calls it.
 template <int TW>
 __device__ __forceinline__ void fpair_mark(const FTileP& t, int p, int c)
 {
     t.cnt[p] |= 1ull << (kCntMark + 5 * c);
-    const int r = p / TW;
-    atomicOr(reinterpret_cast<unsigned long long*>(&t.markrow[c * FPMAXROWS + r]), 1ull << (p - r * TW));
+    const int y = p / TW, x = p - y * TW;
+    atomicOr(reinterpret_cast<uint32_t*>(&t.markrow[c * FPMAXROWS + y]) + (x >> 5), 1u << (x & 31));
+}
+
+// Whether tile pixel p has an equal opaque sample within R of it in both
+// directions (eraw: of the channel).
+template <int TW, int TT>
+__device__ __forceinline__ bool fpair_repeat_near(const float* eraw, const uint8_t* a, int p, int R)
+{
+    const int py = p / TW, px = p - py * TW;
+    const int y1 = min(py + R, TT / TW - 1), x0 = max(px - R, 0), x1 = min(px + R, TW - 1);
+    const uint32_t key = float_key(eraw[p]);
+    for (int y = max(py - R, 0); y <= y1; ++y) {
+        for (int x = x0; x <= x1; ++x) {
+            const int i = y * TW + x;
+            if (float_key(eraw[i]) == key && i != p && a[i]) {
+                return true;
+            }
+        }
+    }
+    return false;
+}
+
+// Slot of a sample in the given round's table (multiplicative hashing).
+__device__ __forceinline__ uint32_t fpair_slot(uint32_t key, int round, int shift)
+{
+    return dup_hash(round == 0 ? key : (round == 1 ? key * 0x9E3779B1u ^ key >> 15 : key * 0x85EBCA6Bu ^ key >> 13), shift);
 }
 
 // A thread's NP tile pixels (pixel p = threadIdx.x + j * FPT) as fetched
@@ -176,33 +178,22 @@ __device__ __forceinline__ void fpair_fetch(FpairFetch<NP>& f, const float* img,
     }
 }
 
-// Writes the thread's fetched pixels into tile t and, with hash slots,
-// issues the first probe of each of their repeat-mark keys (old: the
-// probed slots' previous contents; kEntropyPad where no key was inserted
-// or the slot was empty).  The tables must be empty.  Returns 1 when every
-// one of the pixels that lies in the image is opaque.
-//
-// Repeat marks: every opaque sample that is no clip value goes into its
-// channel's hash table (open addressing, linear probing); an insertion
-// that meets its own key marks its pixel.  Of every set of equal samples
-// all but the first inserted are marked, so a window holding two equal
-// samples holds a marked one.  Only the thread that owns a pixel writes
-// its counters.  slots: a power of two >= 2 TT, so every probe sequence
-// meets an empty slot.
+// Writes the thread's fetched pixels into tile t and, with hash slots, the
+// first round of the search for repeats: the pixel's number goes into its
+// sample's slot (opaque samples that are no clip value; bit j * 3 + c of pend
+// each).  Returns 1 when every one of the pixels that lies in the image is
+// opaque.
 template <int NP, int C, int TT>
 __device__ __forceinline__ int fpair_store(const FTileP& t, const FloatWeightParams& wp, const FpairFetch<NP>& f,
-                                           uint32_t (&old)[NP][3])
+                                           uint32_t& pend)
 {
     const int slots = t.slots;
     const int shift = slots ? 32 - (31 - __clz(slots)) : 0;
     int mine = 1;
+    pend = 0;
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
         const int p = (int)threadIdx.x + j * FPT;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            old[j][c] = kEntropyPad;
-        }
         if (j * FPT + FPT <= TT || p < TT) {
             const bool a = (f.fl >> j) & 1u;
             float rgb[3] = {f.v[j][0], f.v[j][1], f.v[j][2]};
@@ -224,11 +215,10 @@ __device__ __forceinline__ int fpair_store(const FTileP& t, const FloatWeightPar
                 if (slots && a) {
 #pragma unroll
                     for (int c = 0; c < C; ++c) {
-                        // clip values are counted per window, not hashed
+                        // clip values are counted per window, not searched
                         if (rgb[c] != 0.0f && rgb[c] != 1.0f) {
-                            const uint32_t key = float_key(rgb[c]);
-                            old[j][c] = atomicCAS(&t.table[(uint32_t)c * (uint32_t)slots + dup_hash(key, shift)],
-                                                  kEntropyPad, key);
+                            t.table[c * slots + (int)fpair_slot(float_key(rgb[c]), 0, shift)] = (uint16_t)p;
+                            pend |= 1u << (j * 3 + c);
                         }
                     }
                 }
@@ -239,68 +229,104 @@ __device__ __forceinline__ int fpair_store(const FTileP& t, const FloatWeightPar
     return mine;
 }
 
-// Completes the repeat marks of the thread's pixels of tile t from the first
-// probes' results (fpair_store): a probe that met its own key marks the
-// pixel; keys whose slot held another key probe on, one after the other.
-template <int NP, int C, int TW, int TT>
-__device__ __forceinline__ void fpair_hash_finish(const FTileP& t, const uint32_t (&old)[NP][3])
-{
-    const int slots = t.slots;
-    const int shift = 32 - (31 - __clz(slots));
-    uint32_t pend = 0;  // bit j * 3 + c: key (j, c) found its slot taken
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-        const int p = (int)threadIdx.x + j * FPT;
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            if (old[j][c] != kEntropyPad) {
-                if (old[j][c] == float_key(t.eraw[c * TT + p])) {
-                    fpair_mark<TW>(t, p, c);
-                } else {
-                    pend |= 1u << (j * 3 + c);
-                }
-            }
-        }
-    }
-    while (pend) {
-        const int b = __ffs(pend) - 1;
-        pend &= pend - 1u;
-        const int j = b / 3, c = b - 3 * j;
-        const int p = (int)threadIdx.x + j * FPT;
-        const uint32_t key = float_key(t.eraw[c * TT + p]);
-        uint32_t* tab = t.table + c * slots;
-        uint32_t h = dup_hash(key, shift);
-        for (int probe = 1; probe < slots; ++probe) {
-            h = (h + 1u) & (uint32_t)(slots - 1);
-            const uint32_t o = atomicCAS(&tab[h], kEntropyPad, key);
-            if (o == kEntropyPad) {
-                break;
-            }
-            if (o == key) {
-                fpair_mark<TW>(t, p, c);
-                break;
-            }
-        }
-    }
-}
-
-// Loads tile t whole (fetch, store, repeat marks) as the first step of a
-// kernel; the tables must be empty since the block's previous barrier.
-// Ends with a barrier; returns nonzero when every tile pixel inside the
-// image is opaque (then every window that is evaluated, which lies inside
-// the image, is opaque).
+// Loads tile t whole.  Begins after the block's previous use of the tile and
+// ends with a barrier; returns nonzero when every tile pixel inside the image
+// is opaque (then every window that is evaluated, which lies inside the image,
+// is opaque).
+//
+// Repeat marks: of every set of equal opaque samples in a window all but at
+// most one are marked, so a window holding two equal samples holds a marked
+// one.  The search is by rounds: every pixel writes its number into its
+// sample's slot, and after a barrier reads the slot back.  It finds itself
+// (done), a pixel of an equal sample, which marks it if a window can hold both,
+// or one of another sample, and enters the next round with another hash: 16 %
+// of the samples after the first, under 1 % after the second (2048 slots, 720
+// pixels).  Where the slot's pixel is equal but too far, and after the third
+// round, the pixel's surroundings decide.  Equal samples meet in every round
+// until one of them wins the slot.  No slot is read that this round did not
+// write, so the tables need no clearing.
+//
+// What bounds it: the shared-memory accesses, random by nature, and the chain
+// of the rounds.  16 stacks of 512 to 4096 px: the weights take 9.4 ms, 7.0
+// without the search; an exact table by compare-and-swap with linear probing,
+// cleared per exposure, marks for repeats anywhere in the tile, and each
+// thread's own windows with repeats evaluated in calls took 10.9 ms (a 4x1601x1203
+// bracket: 0.39 ms, now 0.24).  Tables of 1024 slots in six blocks an SM: 11.1 ms.
+// The rare paths are inlined: with calls to them the kernel takes 10 % longer,
+// executed or not.
 template <int NP, int C, int TW, int TT>
 __device__ __forceinline__ int fpair_load(const FTileP& t, const FloatWeightParams& wp, const float* img, int64_t pitch,
                                           int stride, int w, int h, const uint8_t* alpha, int64_t apitch, int x0, int y0)
 {
     FpairFetch<NP> f;
     fpair_fetch<NP, C, TW, TT>(f, img, pitch, stride, w, h, alpha, apitch, x0, y0);
-    uint32_t old[NP][3];
-    const int mine = fpair_store<NP, C, TT>(t, wp, f, old);
-    if (t.slots) {
-        fpair_hash_finish<NP, C, TW, TT>(t, old);
+    if (t.slots && threadIdx.x < 3 * FPMAXROWS) {
+        t.markrow[threadIdx.x] = 0ull;
+        *t.listed = 0u;
     }
-    return __syncthreads_and(mine);
+    uint32_t pend;
+    const int opaque = __syncthreads_and(fpair_store<NP, C, TT>(t, wp, f, pend));
+    if (t.slots) {
+        const int slots = t.slots, shift = 32 - (31 - __clz(slots)), R = wp.entropy_window - 1;
+        // bit j * 3 + c, a pixel of the thread: it goes on to the next round; its
+        // slot holds an equal one; its surroundings decide
+        uint32_t lost = 0, same = 0, far = 0;
+#pragma unroll
+        for (int b = 0; b < 3 * NP; ++b) {
+            if (b % 3 < C && ((pend >> b) & 1u)) {
+                const int c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
+                const uint32_t key = float_key(t.eraw[c * TT + p]);
+                const int q = t.table[c * slots + (int)fpair_slot(key, 0, shift)];
+                if (q != p) {
+                    if (float_key(t.eraw[c * TT + q]) == key) {
+                        same |= 1u << b;
+                    } else {
+                        t.table[(3 + c) * slots + (int)fpair_slot(key, 1, shift)] = (uint16_t)p;
+                        lost |= 1u << b;
+                    }
+                }
+            }
+        }
+        for (; same; same &= same - 1u) {
+            const int b = __ffs((int)same) - 1, c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
+            const int q = t.table[c * slots + (int)fpair_slot(float_key(t.eraw[c * TT + p]), 0, shift)];
+            const int dy = p / TW - q / TW, dx = p % TW - q % TW;
+            if (dy * dy <= R * R && dx * dx <= R * R) {
+                fpair_mark<TW>(t, p, c);
+            } else {
+                far |= 1u << b;
+            }
+        }
+        if (__syncthreads_or((int)lost)) {
+            for (pend = lost, lost = 0; pend; pend &= pend - 1u) {
+                const int b = __ffs((int)pend) - 1, c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
+                const uint32_t key = float_key(t.eraw[c * TT + p]);
+                const int q = t.table[(3 + c) * slots + (int)fpair_slot(key, 1, shift)];
+                if (q != p) {
+                    if (float_key(t.eraw[c * TT + q]) == key) {
+                        far |= 1u << b;
+                    } else {
+                        t.table[c * slots + (int)fpair_slot(key, 2, shift)] = (uint16_t)p;
+                        lost |= 1u << b;
+                    }
+                }
+            }
+            if (__syncthreads_or((int)lost)) {
+                for (; lost; lost &= lost - 1u) {
+                    const int b = __ffs((int)lost) - 1, c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
+                    far |= t.table[c * slots + (int)fpair_slot(float_key(t.eraw[c * TT + p]), 2, shift)] != p ? 1u << b : 0u;
+                }
+            }
+        }
+        for (; far; far &= far - 1u) {
+            const int b = __ffs((int)far) - 1, c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
+            if (fpair_repeat_near<TW, TT>(t.eraw + c * TT, t.a, p, R)) {
+                fpair_mark<TW>(t, p, c);
+            }
+        }
+        __syncthreads();
+    }
+    return opaque;
 }
 
 // The W x W window counters of the pair at (cx, cy), cx even: column sums
@@ -498,15 +524,15 @@ __device__ __forceinline__ float f_saturation_term(const FloatWeightParams& wp, 
 }
 
 // H of a window channel with repeat marks (rare), from its bins: every
-// repeated key of the window has a marked tap (of equal samples all but the
-// first inserted are marked), so the bins are the two clip bins (m1 taps at
+// repeated key of the window has a marked tap (of equal samples all but at
+// most one are marked), so the bins are the two clip bins (m1 taps at
 // 1.0, m0 at 0.0), one bin per distinct key of the marked taps, sized by
 // comparing that key with the window's taps, and singletons for the other
 // opaque taps: the same bin sizes, hence the same sum of p log p terms and
 // the same H, as sorting the window's keys.  (x0, y0): the window's top-left
 // tile pixel; raw, markrow: the channel's samples and row masks.
 template <int EW>
-__device__ __noinline__ float fpair_entropy_marked(const float* raw, const uint8_t* a, const uint64_t* markrow, int TW,
+__device__ __forceinline__ float fpair_entropy_marked(const float* raw, const uint8_t* a, const uint64_t* markrow, int TW,
                                                    int x0, int y0, int n, int m1, int m0, const long long* fx,
                                                    const float* scale_logb)
 {
@@ -558,36 +584,63 @@ __device__ __noinline__ float fpair_entropy_marked(const float* raw, const uint8
     return fminf(__fmul_rn(-(float)acc * 1.3877787807814457e-17f, scale_logb[bins]), 1.0f);
 }
 
-// min over the channels of H * range for the entropy window of tile pixel ci
-// with the window's counter sums cs (low and high halves).
+// A listed window: its pixel's number in the tile's output pixels, channel,
+// opaque taps and taps at 1.0 and 0.0.
+__device__ __forceinline__ uint32_t fpair_listed(int pix, int ch, int n, int m1, int m0)
+{
+    return (uint32_t)pix | (uint32_t)ch << 9 | (uint32_t)n << 11 | (uint32_t)m1 << 16 | (uint32_t)m0 << 21;
+}
+
+// min over the channels of H * range for the entropy window of output pixel
+// pix with the window's counter sums cs (low and high halves), as far as the
+// channels are unmarked; a marked one goes to the list, its bit into marked.
 template <int EW, int C>
 __device__ __forceinline__ float fpair_entropy(const FTileP& t, const FloatWeightParams& wp, const WeightTables& tab,
-                                               int ci, uint2 cs)
+                                               int pix, uint2 cs, uint32_t& marked)
 {
     constexpr int M = EW * EW;
     const int n = (int)((cs.y >> (kCntOpaque - 32)) & 31u);
     float emin = 3.402823466e38f;
 #pragma unroll
     for (int ch = 0; ch < C; ++ch) {
-        float H;
         const int m1 = (int)((cs.x >> (5 * ch)) & 31u), m0 = (int)((cs.x >> (15 + 5 * ch)) & 31u);
         if ((cs.y >> (kCntMark - 32 + 5 * ch)) & 31u) {
-            const int cy = ci / t.TW, cx = ci - cy * t.TW;
-            H = fpair_entropy_marked<EW>(t.eraw + ch * t.TT, t.a, t.markrow + ch * FPMAXROWS, t.TW, cx - EW / 2,
-                                         cy - EW / 2, n, m1, m0, tab.plogp_fx + (int64_t)n * (M + 1), tab.scale_logb);
+            marked |= 1u << ch;
+            reinterpret_cast<uint32_t*>(t.table)[atomicAdd(t.listed, 1u)] = fpair_listed(pix, ch, n, m1, m0);
         } else {
-            H = __ldg(&tab.clip_h[(n * (M + 1) + m1) * (M + 1) + m0]);
+            emin = fminf(emin, __fmul_rn(__ldg(&tab.clip_h[(n * (M + 1) + m1) * (M + 1) + m0]), wp.range));
         }
-        emin = fminf(emin, __fmul_rn(H, wp.range));
     }
     return emin;
+}
+
+// H of the listed windows, by all threads of the block, into the words after
+// the list.  (cx0, cy0): the tile position of output pixel 0.
+template <int EW>
+__device__ __forceinline__ void fpair_entropy_list(const FTileP& t, const WeightTables& tab, int cx0, int cy0)
+{
+    constexpr int M = EW * EW;
+    const uint32_t* list = reinterpret_cast<const uint32_t*>(t.table);
+    float* H = reinterpret_cast<float*>(t.table) + 3 * FPX * FPY;
+    const int total = (int)*t.listed;
+    for (int i = threadIdx.x; i < total; i += FPT) {
+        const uint32_t e = list[i];
+        const int pix = (int)(e & 511u), ch = (int)(e >> 9) & 3, n = (int)(e >> 11) & 31;
+        H[ch * FPX * FPY + pix] =
+            fpair_entropy_marked<EW>(t.eraw + ch * t.TT, t.a, t.markrow + ch * FPMAXROWS, t.TW, cx0 + pix % FPX - EW / 2,
+                                     cy0 + pix / FPX - EW / 2, n, (int)(e >> 16) & 31, (int)(e >> 21) & 31,
+                                     tab.plogp_fx + (int64_t)n * (M + 1), tab.scale_logb);
+    }
 }
 
 // The enfuseMask weights (w0, w1) of the output pixels (x, y), (x + 1, y) at
 // tile position (cx, cy): exposure, + contrast, + saturation, + entropy, in
 // the reference's order of the float adds (src/enfuse.h:1119-1120,
 // 1133-1134, 1208-1209); 0 for pixels that are transparent or outside the
-// image.  opaque: as fpair_load returned.
+// image.  opaque: as fpair_load returned.  With entropy all threads of the block
+// take part: the windows with repeats go to a list (in the tables' memory, free
+// after the load) that all threads then work through, where each thread's own
+// windows had left most lanes and warps of the few tiles with repeats idle.
 template <int CW, int EW, int C>
 __device__ __forceinline__ void fpair_weights(const FTileP& t, const FloatWeightParams& wp, const WeightTables& tab,
                                               int cx, int cy, int x, int y, int w, int h, bool opaque, float& w0,
@@ -596,7 +649,7 @@ __device__ __forceinline__ void fpair_weights(const FTileP& t, const FloatWeight
     const int TT = t.TT, ci = cy * t.TW + cx;
     const bool a[2] = {t.a[ci] != 0, t.a[ci + 1] != 0};
     float res[2] = {0.0f, 0.0f};
-    if (!a[0] && !a[1]) {
+    if (EW == 0 && !a[0] && !a[1]) {
         w0 = w1 = 0.0f;
         return;
     }
@@ -641,11 +694,35 @@ __device__ __forceinline__ void fpair_weights(const FTileP& t, const FloatWeight
         const bool rows = y >= B && y < h - B;
         const bool need0 = a[0] && rows && x >= B && x < w - B;
         const bool need1 = a[1] && rows && x + 1 >= B && x + 1 < w - B;
+        constexpr int HX = fpair_halo_x(fpair_halo(CW, EW)), HALO = fpair_halo(CW, EW);
+        const int pix = (cy - HALO) * FPX + cx - HX;
+        uint32_t m0 = 0, m1 = 0;
+        float e0 = 0.0f, e1 = 0.0f;
         if (need0 || need1) {
             uint2 cl, cr;
             fpair_counts<EW>(t.cnt, t.TW, cx, cy, cl, cr);
-            const float e0 = need0 ? fpair_entropy<EW, C>(t, wp, tab, ci, cl) : 0.0f;
-            const float e1 = need1 ? fpair_entropy<EW, C>(t, wp, tab, ci + 1, cr) : 0.0f;
+            if (need0) {
+                e0 = fpair_entropy<EW, C>(t, wp, tab, pix, cl, m0);
+            }
+            if (need1) {
+                e1 = fpair_entropy<EW, C>(t, wp, tab, pix + 1, cr, m1);
+            }
+        }
+        if (__syncthreads_or((int)(m0 | m1))) {
+            fpair_entropy_list<EW>(t, tab, HX, HALO);
+            __syncthreads();
+            const float* H = reinterpret_cast<const float*>(t.table) + 3 * FPX * FPY + pix;
+#pragma unroll
+            for (int ch = 0; ch < C; ++ch) {
+                if ((m0 >> ch) & 1u) {
+                    e0 = fminf(e0, __fmul_rn(H[ch * FPX * FPY], wp.range));
+                }
+                if ((m1 >> ch) & 1u) {
+                    e1 = fminf(e1, __fmul_rn(H[ch * FPX * FPY + 1], wp.range));
+                }
+            }
+        }
+        if (need0 || need1) {
             res[0] = __fadd_rn(__fmul_rn(wp.w_entropy, e0), res[0]);
             res[1] = __fadd_rn(__fmul_rn(wp.w_entropy, e1), res[1]);
         }

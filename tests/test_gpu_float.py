@@ -375,3 +375,33 @@ def test_enfuse_f32_level_passes_equal_single_operations(ctx, h, w, K, chans, kw
         assert np.array_equal(got[0][0], got[1][0])
         out, oa = ctx.enfuse(imgs, alphas, params=p, **opt)
         assert np.array_equal(out, got[0][0]) and np.array_equal(oa, got[0][1])
+
+
+@pytest.mark.parametrize("ew", [3, 5])
+@pytest.mark.parametrize("filled", [False, True])
+def test_enfuse_mask_f32_repeats_by_distance(ctx, orc, ew, filled):
+    """Single pairs of equal samples in images of distinct ones, at every
+    offset from touching to just outside a window's reach, across tile edges,
+    and with a third equal sample far away in the tile; filled: a transparent
+    pixel repeats the pair's sample beside it (it counts in no window)."""
+    import enbgpu
+    rng = np.random.default_rng(500 + ew)
+    offsets = [(dy, dx) for dy in range(ew + 1) for dx in range(-ew, ew + 1) if (dy, dx) > (0, 0)]
+    cell, cols = 15, 9
+    h, w = cell * -(-len(offsets) // cols) + 12, cell * cols + 12
+    img = ((rng.permutation(h * w * 3).reshape(h, w, 3) + 0.5) / (h * w * 3) * 0.8 + 0.1).astype(np.float32)
+    assert np.unique(img).size == img.size
+    alpha = np.full((h, w), 255, np.uint8)
+    for i, (dy, dx) in enumerate(offsets):
+        y, x, c = 6 + cell * (i // cols), 8 + cell * (i % cols), i % 3
+        img[y + dy, x + dx, c] = img[y, x, c]
+        if i % 4 == 0:
+            img[y + 9, x, c] = img[y, x, c]
+        if filled:
+            img[y, x - 7, c] = img[y, x + 1 if dx != 1 or dy else x - 1, c] = img[y, x, c]
+            alpha[y, x - 7] = alpha[y, x + 1 if dx != 1 or dy else x - 1] = 0
+    kw = dict(exposure_weight=1.0, entropy_weight=0.5, entropy_window_size=ew)
+    ref = orc.enfuse_mask_f(img, alpha, orc.params(**kw), 1.0)
+    out = torch.zeros((h, w), dtype=torch.float32, device="cuda")
+    ctx.enfuse_mask(_dev(img), _dev(alpha), out, enbgpu.enfuse_params(float_range=1.0, **kw))
+    _close(out.cpu().numpy().astype(np.float64), ref.astype(np.float64), WEIGHT_RTOL, 1e-7 * np.abs(ref).max(), f"repeats {ew}")

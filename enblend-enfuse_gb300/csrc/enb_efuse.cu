@@ -6,9 +6,9 @@
 // level by level and adds the product into the result pyramid, and finally
 // collapses it: the result pyramid is read and written once per exposure and
 // every level of every pyramid is materialised.  Here
-//   * one pass computes the weights of all K exposures per 16x16 tile, their
-//     sum, the normalised (or hard) masks as level 0 of the mask pyramids and
-//     the union alpha;
+//   * one pass (enb_efweights.cu) computes the weights of all K exposures,
+//     their sum, the normalised (or hard) masks as level 0 of the mask pyramids
+//     and the union alpha;
 //   * level 0 of no image pyramid is stored: the level-1 reduce reads the
 //     interleaved pixels and converts them to fixed point on the fly; each
 //     reduce launch covers the K exposures (blockIdx.z);

@@ -215,9 +215,6 @@ cudaError_t launch_float_to_fixed(const FloatPlane& src, const PlanarView& dst, 
 cudaError_t launch_alpha_extract(const AlphaSrc& a, const BytePlane& dst, cudaStream_t st);
 cudaError_t launch_reduce(int wrap, const PlanarView& src, const BytePlane* src_alpha,
                           const PlanarView& dst, const BytePlane* dst_alpha, cudaStream_t st);
-// The same reduce of two levels of equal geometry and type (the white and
-// black pyramids of one level) as one launch; falls back to two launches when
-// the geometries differ.
 // white and black images with alpha and the seam mask without, one level of
 // the enblend down sweep in one launch (integer pyramids)
 cudaError_t launch_reduce_img2_mask(int wrap, const PlanarView& s0, const BytePlane& sa0, const PlanarView& d0,
@@ -229,9 +226,6 @@ cudaError_t launch_reduce_img2_mask(int wrap, const PlanarView& s0, const BytePl
 int enb_tail_level(const int* lw, const int* lh, int L);
 cudaError_t launch_reduce_img2_mask_tail(int wrap, int n, const PlanarView* s0, const BytePlane* a0, const PlanarView* s1,
                                          const BytePlane* a1, const PlanarView* ms, cudaStream_t st);
-cudaError_t launch_reduce2(int wrap, const PlanarView& s0, const BytePlane* sa0, const PlanarView& d0,
-                           const BytePlane* da0, const PlanarView& s1, const BytePlane* sa1, const PlanarView& d1,
-                           const BytePlane* da1, cudaStream_t st);
 // The last levels of one pyramid from level pyramid_tail_level (L: none) on,
 // n of them with the source, in one launch (fixed point; alpha planes or null).
 int pyramid_tail_level(const int* lw, const int* lh, int L, int dtype);

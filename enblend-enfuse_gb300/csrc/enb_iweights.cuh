@@ -2,7 +2,7 @@
 // 962-1212 with integer pixels): the gray projectors, the rounding of the
 // window statistics, a shared-memory tile of one exposure and the weight of
 // one pixel of it.  Used by the per-image weight kernel (enb_kernels.cu) and
-// by the fused enfuse (enb_efuse.cu).
+// by the fused enfuse (enb_efweights.cu).
 #pragma once
 
 #include <stdint.h>

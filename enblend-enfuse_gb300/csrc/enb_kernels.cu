@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256) k_alpha_extract(AlphaSrc a, uint8_t* __re
     dst[(int64_t)y * dpitch + x] = alpha_at(a, x, y) ? 255 : 0;
 }
 
-// Reduce (src/pyramid.h:166-848): k_reduce_tiles in enb_reduce.cuh.
+// Reduce (src/pyramid.h:166-848): k_reduce in enb_reduce.cuh.
 
 // ---------------------------------------------------------------------------
 // Expand (src/pyramid.h:875-1457)
@@ -390,7 +390,6 @@ __global__ void __launch_bounds__(256) k_from_fixed(const TS* src, int64_t spitc
                                                     int32_t maxv)
 {
     griddep_wait();
-    griddep_launch();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= w || !alpha[(int64_t)y * apitch + x]) {
@@ -644,91 +643,41 @@ cudaError_t launch_alpha_extract(const AlphaSrc& a, const BytePlane& d, cudaStre
     return cudaGetLastError();
 }
 
-template <typename TS, typename TD, int C>
-static void reduce_dispatch(int wrap, int n, const PlanarView* const* s, const BytePlane* const* sa,
-                            const PlanarView* const* d, const BytePlane* const* da, cudaStream_t st)
+template <typename T, int C>
+static void reduce_dispatch(int wrap, const PlanarView& s, const BytePlane* sa, const PlanarView& d, const BytePlane* da,
+                            cudaStream_t st)
 {
-    if (sa[0]) {
-        using Src = PlanarSource<TS, C, true>;
-        ReduceJobs<Src, TD> jobs{};
-        for (int i = 0; i < 2; ++i) {
-            const int k = i < n ? i : 0;
-            jobs.j[i] = ReduceJob<Src, TD>{Src{(const TS*)s[k]->p, s[k]->pitch, s[k]->plane, sa[k]->p, sa[k]->pitch},
-                                           (TD*)d[k]->p, d[k]->pitch, d[k]->plane, da[k]->p, da[k]->pitch};
-        }
-        launch_reduce_jobs<Src, TD, C, true>(jobs, n, s[0]->w, s[0]->h, d[0]->w, d[0]->h, wrap, st);
+    if (sa) {
+        using Src = PlanarSource<T, C, true>;
+        ReduceJobs<Src, T> jobs{};
+        jobs.j[0] = ReduceJob<Src, T>{Src{(const T*)s.p, s.pitch, s.plane, sa->p, sa->pitch}, (T*)d.p, d.pitch, d.plane,
+                                      da->p, da->pitch};
+        launch_reduce_jobs<Src, T, C, true>(jobs, 1, s.w, s.h, d.w, d.h, wrap, st);
     } else {
-        using Src = PlanarSource<TS, C, false>;
-        ReduceJobs<Src, TD> jobs{};
-        for (int i = 0; i < 2; ++i) {
-            const int k = i < n ? i : 0;
-            jobs.j[i] = ReduceJob<Src, TD>{Src{(const TS*)s[k]->p, s[k]->pitch, s[k]->plane, nullptr, 0},
-                                           (TD*)d[k]->p, d[k]->pitch, d[k]->plane, nullptr, 0};
-        }
-        launch_reduce_jobs<Src, TD, C, false>(jobs, n, s[0]->w, s[0]->h, d[0]->w, d[0]->h, wrap, st);
+        using Src = PlanarSource<T, C, false>;
+        ReduceJobs<Src, T> jobs{};
+        jobs.j[0] = ReduceJob<Src, T>{Src{(const T*)s.p, s.pitch, s.plane, nullptr, 0}, (T*)d.p, d.pitch, d.plane,
+                                      nullptr, 0};
+        launch_reduce_jobs<Src, T, C, false>(jobs, 1, s.w, s.h, d.w, d.h, wrap, st);
     }
-}
-
-static cudaError_t reduce_jobs(int wrap, int n, const PlanarView* const* s, const BytePlane* const* sa,
-                               const PlanarView* const* d, const BytePlane* const* da, cudaStream_t st)
-{
-    double bytes = 0.0;
-    for (int i = 0; i < n; ++i) {
-        if (s[i]->dtype != d[i]->dtype || s[i]->C != d[i]->C || (sa[i] == nullptr) != (da[i] == nullptr)) {
-            return cudaErrorInvalidValue;
-        }
-        bytes += planar_bytes(*s[i]) + planar_bytes(*d[i]) +
-                 (sa[i] ? npix(s[i]->w, s[i]->h) + npix(d[i]->w, d[i]->h) : 0.0);
-    }
-    note(sa[0] ? "reduce_alpha" : "reduce", bytes);
-    if (s[0]->dtype == ENB_F32) {
-        if (s[0]->C == 1) {
-            reduce_dispatch<float, float, 1>(wrap, n, s, sa, d, da, st);
-        } else {
-            reduce_dispatch<float, float, 3>(wrap, n, s, sa, d, da, st);
-        }
-    } else if (s[0]->dtype == ENB_I16) {
-        if (s[0]->C == 1) {
-            reduce_dispatch<int16_t, int16_t, 1>(wrap, n, s, sa, d, da, st);
-        } else {
-            reduce_dispatch<int16_t, int16_t, 3>(wrap, n, s, sa, d, da, st);
-        }
-    } else {
-        if (s[0]->C == 1) {
-            reduce_dispatch<int32_t, int32_t, 1>(wrap, n, s, sa, d, da, st);
-        } else {
-            reduce_dispatch<int32_t, int32_t, 3>(wrap, n, s, sa, d, da, st);
-        }
-    }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_reduce(int wrap, const PlanarView& s, const BytePlane* sa, const PlanarView& d,
                           const BytePlane* da, cudaStream_t st)
 {
-    const PlanarView* sv[1] = {&s};
-    const PlanarView* dv[1] = {&d};
-    const BytePlane* sav[1] = {sa};
-    const BytePlane* dav[1] = {da};
-    return reduce_jobs(wrap, 1, sv, sav, dv, dav, st);
-}
-
-cudaError_t launch_reduce2(int wrap, const PlanarView& s0, const BytePlane* sa0, const PlanarView& d0,
-                           const BytePlane* da0, const PlanarView& s1, const BytePlane* sa1, const PlanarView& d1,
-                           const BytePlane* da1, cudaStream_t st)
-{
-    const bool same = s0.w == s1.w && s0.h == s1.h && d0.w == d1.w && d0.h == d1.h && s0.dtype == s1.dtype &&
-                      s0.C == s1.C && d0.dtype == d1.dtype && d0.C == d1.C && (sa0 == nullptr) == (sa1 == nullptr) &&
-                      (da0 == nullptr) == (da1 == nullptr);
-    if (!same) {
-        const cudaError_t e = launch_reduce(wrap, s0, sa0, d0, da0, st);
-        return e != cudaSuccess ? e : launch_reduce(wrap, s1, sa1, d1, da1, st);
+    if (s.dtype != d.dtype || s.C != d.C || (sa == nullptr) != (da == nullptr)) {
+        return cudaErrorInvalidValue;
     }
-    const PlanarView* sv[2] = {&s0, &s1};
-    const PlanarView* dv[2] = {&d0, &d1};
-    const BytePlane* sav[2] = {sa0, sa1};
-    const BytePlane* dav[2] = {da0, da1};
-    return reduce_jobs(wrap, 2, sv, sav, dv, dav, st);
+    note(sa ? "reduce_alpha" : "reduce",
+         planar_bytes(s) + planar_bytes(d) + (sa ? npix(s.w, s.h) + npix(d.w, d.h) : 0.0));
+    if (s.dtype == ENB_F32) {
+        s.C == 1 ? reduce_dispatch<float, 1>(wrap, s, sa, d, da, st) : reduce_dispatch<float, 3>(wrap, s, sa, d, da, st);
+    } else if (s.dtype == ENB_I16) {
+        s.C == 1 ? reduce_dispatch<int16_t, 1>(wrap, s, sa, d, da, st) : reduce_dispatch<int16_t, 3>(wrap, s, sa, d, da, st);
+    } else {
+        s.C == 1 ? reduce_dispatch<int32_t, 1>(wrap, s, sa, d, da, st) : reduce_dispatch<int32_t, 3>(wrap, s, sa, d, da, st);
+    }
+    return cudaGetLastError();
 }
 
 template <typename T, typename TM, int C>

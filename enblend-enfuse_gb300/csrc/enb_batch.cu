@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_weights(ENB_BATCH_JOBS(J), Flo
 // blockIdx.y, where those past a stack's exposures leave at once): a tile's
 // exposures in turn made blocks several times as long, and a single stack's
 // last wave of them kept the chip busy to 73 % (with the search for repeats of
-// fpair_load, 4x1601x1203: 0.39 to 0.24 ms; 16 stacks: 10.9 to 9.4 ms).
+// fpair_load, 4x1601x1203: 0.39 to 0.23 ms; 16 stacks: 10.9 to 8.9 ms).
 template <int CW, int EW, int C, class J>
 __global__ void __launch_bounds__(FPT, 5) k_batch_weights_pair(const __grid_constant__ BatchJobs<J> j,
                                                                FloatWeightParams wp, WeightTables tab)

@@ -115,25 +115,6 @@ __device__ __forceinline__ void fpair_mark(const FTileP& t, int p, int c)
     atomicOr(reinterpret_cast<uint32_t*>(&t.markrow[c * FPMAXROWS + y]) + (x >> 5), 1u << (x & 31));
 }
 
-// Whether tile pixel p has an equal opaque sample within R of it in both
-// directions (eraw: of the channel).
-template <int TW, int TT>
-__device__ __forceinline__ bool fpair_repeat_near(const float* eraw, const uint8_t* a, int p, int R)
-{
-    const int py = p / TW, px = p - py * TW;
-    const int y1 = min(py + R, TT / TW - 1), x0 = max(px - R, 0), x1 = min(px + R, TW - 1);
-    const uint32_t key = float_key(eraw[p]);
-    for (int y = max(py - R, 0); y <= y1; ++y) {
-        for (int x = x0; x <= x1; ++x) {
-            const int i = y * TW + x;
-            if (float_key(eraw[i]) == key && i != p && a[i]) {
-                return true;
-            }
-        }
-    }
-    return false;
-}
-
 // Slot of a sample in the given round's table (multiplicative hashing).
 __device__ __forceinline__ uint32_t fpair_slot(uint32_t key, int round, int shift)
 {
@@ -238,22 +219,23 @@ __device__ __forceinline__ int fpair_store(const FTileP& t, const FloatWeightPar
 // most one are marked, so a window holding two equal samples holds a marked
 // one.  The search is by rounds: every pixel writes its number into its
 // sample's slot, and after a barrier reads the slot back.  It finds itself
-// (done), a pixel of an equal sample, which marks it if a window can hold both,
-// or one of another sample, and enters the next round with another hash: 16 %
-// of the samples after the first, under 1 % after the second (2048 slots, 720
-// pixels).  Where the slot's pixel is equal but too far, and after the third
-// round, the pixel's surroundings decide.  Equal samples meet in every round
-// until one of them wins the slot.  No slot is read that this round did not
-// write, so the tables need no clearing.
+// (done), a pixel of an equal sample (marked), or one of another sample, and
+// enters the next round with another hash: 16 % of the samples after the
+// first, under 1 % after the second (2048 slots, 720 pixels); what the third
+// leaves is marked, which costs its windows time but changes nothing.  Equal
+// samples meet in every round until one of them wins the slot.  No slot is
+// read that this round did not write, so the tables need no clearing.
 //
 // What bounds it: the shared-memory accesses, random by nature, and the chain
-// of the rounds.  16 stacks of 512 to 4096 px: the weights take 9.4 ms, 7.0
+// of the rounds.  16 stacks of 512 to 4096 px: the weights take 8.9 ms, 7.0
 // without the search; an exact table by compare-and-swap with linear probing,
-// cleared per exposure, marks for repeats anywhere in the tile, and each
-// thread's own windows with repeats evaluated in calls took 10.9 ms (a 4x1601x1203
-// bracket: 0.39 ms, now 0.24).  Tables of 1024 slots in six blocks an SM: 11.1 ms.
-// The rare paths are inlined: with calls to them the kernel takes 10 % longer,
-// executed or not.
+// cleared per exposure, and each thread's own windows with repeats evaluated
+// in calls took 10.9 ms (a 4x1601x1203 bracket: 0.39 ms, now 0.23; the same
+// in 65,536 levels, all passes: 1.87 and 0.83).  Marking only samples with an
+// equal one within a window's reach: 9.4 ms, the test of the surroundings
+// costs more than the windows it spares.  Tables of 1024 slots in six blocks
+// an SM: 11.1 ms.  The rare paths are inlined: with calls to them the kernel
+// takes 10 % longer, executed or not.
 template <int NP, int C, int TW, int TT>
 __device__ __forceinline__ int fpair_load(const FTileP& t, const FloatWeightParams& wp, const float* img, int64_t pitch,
                                           int stride, int w, int h, const uint8_t* alpha, int64_t apitch, int x0, int y0)
@@ -267,10 +249,10 @@ __device__ __forceinline__ int fpair_load(const FTileP& t, const FloatWeightPara
     uint32_t pend;
     const int opaque = __syncthreads_and(fpair_store<NP, C, TT>(t, wp, f, pend));
     if (t.slots) {
-        const int slots = t.slots, shift = 32 - (31 - __clz(slots)), R = wp.entropy_window - 1;
+        const int slots = t.slots, shift = 32 - (31 - __clz(slots));
         // bit j * 3 + c, a pixel of the thread: it goes on to the next round; its
-        // slot holds an equal one; its surroundings decide
-        uint32_t lost = 0, same = 0, far = 0;
+        // slot holds an equal one
+        uint32_t lost = 0, same = 0;
 #pragma unroll
         for (int b = 0; b < 3 * NP; ++b) {
             if (b % 3 < C && ((pend >> b) & 1u)) {
@@ -287,16 +269,6 @@ __device__ __forceinline__ int fpair_load(const FTileP& t, const FloatWeightPara
                 }
             }
         }
-        for (; same; same &= same - 1u) {
-            const int b = __ffs((int)same) - 1, c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
-            const int q = t.table[c * slots + (int)fpair_slot(float_key(t.eraw[c * TT + p]), 0, shift)];
-            const int dy = p / TW - q / TW, dx = p % TW - q % TW;
-            if (dy * dy <= R * R && dx * dx <= R * R) {
-                fpair_mark<TW>(t, p, c);
-            } else {
-                far |= 1u << b;
-            }
-        }
         if (__syncthreads_or((int)lost)) {
             for (pend = lost, lost = 0; pend; pend &= pend - 1u) {
                 const int b = __ffs((int)pend) - 1, c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
@@ -304,7 +276,7 @@ __device__ __forceinline__ int fpair_load(const FTileP& t, const FloatWeightPara
                 const int q = t.table[(3 + c) * slots + (int)fpair_slot(key, 1, shift)];
                 if (q != p) {
                     if (float_key(t.eraw[c * TT + q]) == key) {
-                        far |= 1u << b;
+                        same |= 1u << b;
                     } else {
                         t.table[c * slots + (int)fpair_slot(key, 2, shift)] = (uint16_t)p;
                         lost |= 1u << b;
@@ -314,15 +286,13 @@ __device__ __forceinline__ int fpair_load(const FTileP& t, const FloatWeightPara
             if (__syncthreads_or((int)lost)) {
                 for (; lost; lost &= lost - 1u) {
                     const int b = __ffs((int)lost) - 1, c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
-                    far |= t.table[c * slots + (int)fpair_slot(float_key(t.eraw[c * TT + p]), 2, shift)] != p ? 1u << b : 0u;
+                    same |= t.table[c * slots + (int)fpair_slot(float_key(t.eraw[c * TT + p]), 2, shift)] != p ? 1u << b : 0u;
                 }
             }
         }
-        for (; far; far &= far - 1u) {
-            const int b = __ffs((int)far) - 1, c = b % 3, p = (int)threadIdx.x + (b / 3) * FPT;
-            if (fpair_repeat_near<TW, TT>(t.eraw + c * TT, t.a, p, R)) {
-                fpair_mark<TW>(t, p, c);
-            }
+        for (; same; same &= same - 1u) {
+            const int b = __ffs((int)same) - 1;
+            fpair_mark<TW>(t, (int)threadIdx.x + (b / 3) * FPT, b % 3);
         }
         __syncthreads();
     }

@@ -100,8 +100,8 @@ struct AdjWindow {
     {
 #pragma unroll
         for (int c = 0; c < P; ++c) {
-            v[c][0] = __ldg(&p[c * plane + o[0]]);
-            v[c][1] = __ldg(&p[c * plane + o[1]]);
+            v[c][0] = ld_dep(&p[c * plane + o[0]]);
+            v[c][1] = ld_dep(&p[c * plane + o[1]]);
         }
     }
     template <int P>
@@ -167,14 +167,14 @@ struct AdjQuad {
     __device__ __forceinline__ void load(const float* p, float (&v)[4]) const
     {
         if (pair) {  // X is even and rows start on 128-byte boundaries
-            const float2 a = __ldg(reinterpret_cast<const float2*>(p + off)), b = __ldg(reinterpret_cast<const float2*>(p + off2));
+            const float2 a = ld_dep(reinterpret_cast<const float2*>(p + off)), b = ld_dep(reinterpret_cast<const float2*>(p + off2));
             v[0] = a.x;
             v[1] = a.y;
             v[2] = b.x;
             v[3] = b.y;
         } else {
-            v[0] = v[1] = __ldg(p + off);
-            v[2] = v[3] = __ldg(p + off2);
+            v[0] = v[1] = ld_dep(p + off);
+            v[2] = v[3] = ld_dep(p + off2);
         }
     }
     __device__ __forceinline__ void store(float* p, const float (&v)[4]) const
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(256) k_adj_to_pyramid(const __grid_constant__ 
 // exp(a_k) of a pixel's logit, 1 without logits.
 __device__ __forceinline__ float exp_logit(const AdjExposure& e, int x, int y)
 {
-    return e.logit ? expf(__ldg(&e.logit[(int64_t)y * e.lpitch + x])) : 1.0f;
+    return e.logit ? expf(ld_dep(&e.logit[(int64_t)y * e.lpitch + x])) : 1.0f;
 }
 
 // w~_k = w_k exp(a_k), m_k = w~_k / S (S = sum_k w~_k; 1/K where S == 0) as
@@ -488,7 +488,7 @@ struct ExpandTSource {
         const int64_t o = (int64_t)gy * pitch + gx;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            v[c] = __ldg(&p[c * plane + o]) * f;
+            v[c] = ld_dep(&p[c * plane + o]) * f;
         }
         al = 1;
     }

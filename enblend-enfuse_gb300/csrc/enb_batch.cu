@@ -171,9 +171,9 @@ struct Level0Source {
         const int64_t o = (int64_t)gy * pitch + gx;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            v[c] = __ldg(&p[c * plane + o]);
+            v[c] = ld_dep(&p[c * plane + o]);
         }
-        al = A && a ? (__ldg(&a[(int64_t)gy * apitch + gx]) != 0) : 1;
+        al = A && a ? (ld_dep(&a[(int64_t)gy * apitch + gx]) != 0) : 1;
     }
 };
 
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256) k_batch_normalise(ENB_BATCH_JOBS(J), int 
     const auto wt = [&](int k) {
         const int32_t* m = m_level(s, k, 0) + o;
         // x is even and rows start on 128-byte boundaries
-        return pair ? __ldcg(reinterpret_cast<const float2*>(m)) : make_float2(__int_as_float(__ldcg(m)), 0.0f);
+        return pair ? ld_dep(reinterpret_cast<const float2*>(m)) : make_float2(__int_as_float(ld_dep(m)), 0.0f);
     };
     int u0 = 0, u1 = 0;  // the union alpha
     for (int k = 0; k < K && !(u0 && u1); ++k) {
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(256) k_batch_normalise(ENB_BATCH_JOBS(J), int 
 // ---------------------------------------------------------------------------
 
 // One tile of exposure k's image pyramid; A: with its alpha.
-template <int C, bool NC, bool A>
+template <int C, bool EARLIER, bool A>
 __device__ __forceinline__ void batch_reduce_image(const BatchStack& s, int k, int l, int X0, int Y0, int wrap,
                                                    unsigned char* smem)
 {
@@ -435,7 +435,7 @@ __device__ __forceinline__ void batch_reduce_image(const BatchStack& s, int k, i
             dplane, a_level(s, k, l + 1), s.pitch[l + 1]};
         reduce_tile<Src, float, C, MODE, float>(job, X0, Y0, sw, sh, dw, dh, wrap, V);
     } else {
-        using Src = PlanarSource<float, C, A, NC>;
+        using Src = PlanarSource<float, C, A, EARLIER>;
         const ReduceJob<Src, float> job{
             Src{g_level(s, k, l, C), s.pitch[l], (int64_t)s.pitch[l] * sh, a_level(s, k, l), s.pitch[l]}, dst,
             s.pitch[l + 1], dplane, a_level(s, k, l + 1), s.pitch[l + 1]};
@@ -444,12 +444,12 @@ __device__ __forceinline__ void batch_reduce_image(const BatchStack& s, int k, i
 }
 
 // One tile of exposure k's mask pyramid; A: with the union alpha.
-template <bool NC, bool A>
+template <bool EARLIER, bool A>
 __device__ __forceinline__ void batch_reduce_mask(const BatchStack& s, int k, int l, int X0, int Y0, int wrap,
                                                   unsigned char* smem)
 {
     const int sw = s.lw[l], sh = s.lh[l], dw = s.lw[l + 1], dh = s.lh[l + 1];
-    using Src = PlanarSource<int32_t, 1, A, NC>;
+    using Src = PlanarSource<int32_t, 1, A, EARLIER>;
     int32_t(*V)[RDH][RVP] = reinterpret_cast<int32_t(*)[RDH][RVP]>(smem);
     const ReduceJob<Src, int32_t> job{
         Src{m_level(s, k, l), s.pitch[l], (int64_t)s.pitch[l] * sh, s.u + s.off0[l], s.pitch[l]}, m_level(s, k, l + 1),
@@ -458,19 +458,18 @@ __device__ __forceinline__ void batch_reduce_mask(const BatchStack& s, int k, in
 }
 
 // Job kind k < K: exposure k's image; K <= kind < 2K: exposure kind-K's mask.
-// NC: the source levels are read through the read-only path (they were
-// written by an earlier launch); false inside the coarse kernel, which reads
-// levels it wrote itself.
-template <int C, bool NC>
+// EARLIER: the source levels were written by an earlier launch; false inside
+// the coarse kernel, which reads levels it wrote itself.
+template <int C, bool EARLIER>
 __device__ __forceinline__ void batch_reduce_tile(const BatchStack& s, int kind, int l, int X0, int Y0, int wrap,
                                                   unsigned char* smem)
 {
     if (kind < s.K) {
-        s.opaque ? batch_reduce_image<C, NC, false>(s, kind, l, X0, Y0, wrap, smem)
-                 : batch_reduce_image<C, NC, true>(s, kind, l, X0, Y0, wrap, smem);
+        s.opaque ? batch_reduce_image<C, EARLIER, false>(s, kind, l, X0, Y0, wrap, smem)
+                 : batch_reduce_image<C, EARLIER, true>(s, kind, l, X0, Y0, wrap, smem);
     } else {
-        s.opaque ? batch_reduce_mask<NC, false>(s, kind - s.K, l, X0, Y0, wrap, smem)
-                 : batch_reduce_mask<NC, true>(s, kind - s.K, l, X0, Y0, wrap, smem);
+        s.opaque ? batch_reduce_mask<EARLIER, false>(s, kind - s.K, l, X0, Y0, wrap, smem)
+                 : batch_reduce_mask<EARLIER, true>(s, kind - s.K, l, X0, Y0, wrap, smem);
     }
 }
 
@@ -651,7 +650,7 @@ __device__ __forceinline__ void batch_up_tile(const BatchStack& s, int l, int X0
                 const int XX = min(X + (q & 1), dw - 1), YY = min(Y + (q >> 1), dh - 1);
                 coeff[q] = __fmul_rn((float)ld_src<false>(&mk[(int64_t)YY * dp + XX]), inv_d);
                 if (l == 0) {
-                    g[q] = __ldg(&g0_level(s, k, C)[(int64_t)c * gplane + (int64_t)YY * dp + XX]);
+                    g[q] = ld_dep(&g0_level(s, k, C)[(int64_t)c * gplane + (int64_t)YY * dp + XX]);
                 } else {
                     g[q] = ld_src<false>(&gk[(int64_t)YY * dp + XX]);
                 }

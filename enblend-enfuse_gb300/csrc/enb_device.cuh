@@ -163,16 +163,26 @@ static inline dim3 grid2d(int w, int h, int tw, int th)
     return dim3((unsigned)((w + tw - 1) / tw), (unsigned)((h + th - 1) / th));
 }
 
-// Global load through the read-only path (NC: no thread of the launch writes
-// the data) or a load cached in L2 only (the data was written earlier in the
-// same launch, possibly by another SM, and is read only after the barrier or
-// the release/acquire counter that follows the write; L2 is coherent across
-// SMs, the SMs' L1 caches are not).
-template <bool NC, typename T>
+// Global load in a kernel of a chain of dependent launches (griddep_wait):
+// pyramid levels, masks, and the caller's pixels, which the launch before may
+// have written as its output.  That launch can still be writing when this one
+// starts, so the data is not read-only for the kernel's lifetime, as __ldg
+// (ld.global.nc) promises: the compiler may move such a load above the wait,
+// and its cache is not kept coherent.  An ordinary load stays behind the wait
+// and sees what it makes visible.  __ldg is for the tables, which no launch in
+// flight writes, and for kernels launched without overlap.
+template <typename T>
+__device__ __forceinline__ T ld_dep(const T* p) { return *p; }
+
+// The same (EARLIER: an earlier launch wrote the data), or a load cached in L2
+// only (the data was written earlier in the same launch, possibly by another
+// SM, and is read only after the barrier or the release/acquire counter that
+// follows the write; L2 is coherent across SMs, the SMs' L1 caches are not).
+template <bool EARLIER, typename T>
 __device__ __forceinline__ T ld_src(const T* p)
 {
-    if (NC) {
-        return __ldg(p);
+    if (EARLIER) {
+        return ld_dep(p);
     }
     return __ldcg(p);
 }

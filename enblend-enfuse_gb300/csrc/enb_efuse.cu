@@ -54,7 +54,7 @@ __device__ __forceinline__ void ef_top(const TileWindow& win, int32_t (*ss)[ESH]
             if (win.f[u] == 0 || (u == 1 && !win.two)) {
                 continue;
             }
-            const int32_t mv = (int32_t)__ldg(&m[k][win.o[u]]);
+            const int32_t mv = (int32_t)ld_dep(&m[k][win.o[u]]);
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const int32_t g = (&ss[k * C + c][0][0])[threadIdx.x + 256 * u] / win.f[u];
@@ -69,8 +69,7 @@ __device__ __forceinline__ void ef_top(const TileWindow& win, int32_t (*ss)[ESH]
     }
 }
 
-// Two adjacent samples of a planar level or mask (x even), as ld2 of the
-// enblend tiles through the read-only path.
+// Two adjacent samples of a planar level or mask (x even).
 template <typename T>
 __device__ __forceinline__ void ld_pair(const T* p, int32_t& a, int32_t& b)
 {
@@ -139,12 +138,12 @@ __global__ void __launch_bounds__(256, 3) k_ef_up(const __grid_constant__ EfLeve
                 ld_pair<T>(a.g[k] + c * a.plane + off2, g[c][2], g[c][3]);
             }
         } else {  // the last column of an odd level: only pixels 0 and 2 exist
-            m[0] = m[1] = (int32_t)__ldg(&a.m[k][off]);
-            m[2] = m[3] = (int32_t)__ldg(&a.m[k][off2]);
+            m[0] = m[1] = (int32_t)ld_dep(&a.m[k][off]);
+            m[2] = m[3] = (int32_t)ld_dep(&a.m[k][off2]);
 #pragma unroll
             for (int c = 0; c < C; ++c) {
-                g[c][0] = g[c][1] = (int32_t)__ldg(&a.g[k][c * a.plane + off]);
-                g[c][2] = g[c][3] = (int32_t)__ldg(&a.g[k][c * a.plane + off2]);
+                g[c][0] = g[c][1] = (int32_t)ld_dep(&a.g[k][c * a.plane + off]);
+                g[c][2] = g[c][3] = (int32_t)ld_dep(&a.g[k][c * a.plane + off2]);
             }
         }
     };
@@ -192,7 +191,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_up(const __grid_constant__ EfLeve
         if constexpr (FOLD) {
             ef_top<T, TM, C, F>(win, ss, a.mc, K, v);
         } else {
-            win.load_written<T, C>(a.rc, a.cplane, v);
+            win.load<T, C>(a.rc, a.cplane, v);
         }
         win.store<C>(ss + K * C, v);
     }
@@ -301,11 +300,11 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int x = q & 1 ? X1 : Xc, y = q & 2 ? Y1 : Yc;
-                m[q] = (int32_t)__ldg(&a.m0[k][(int64_t)y * a.mpitch + x]);
+                m[q] = (int32_t)ld_dep(&a.m0[k][(int64_t)y * a.mpitch + x]);
                 const TIn* p = a.img[k] + (int64_t)y * a.ipitch[k] + (int64_t)x * S;
 #pragma unroll
                 for (int s = 0; s < S; ++s) {
-                    px[q][s] = __ldg(&p[s]);
+                    px[q][s] = ld_dep(&p[s]);
                 }
             }
         }
@@ -358,7 +357,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
         if constexpr (FOLD) {
             ef_top<T, TM, C, F>(win, ss, a.mc, K, v);
         } else {
-            win.load_written<T, C>(a.r1, a.cplane, v);
+            win.load<T, C>(a.r1, a.cplane, v);
         }
         win.store<C>(ss + K * C, v);
     }
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_out0(const __grid_constant__ EfOu
         // copyFromPyramidImageIf (src/fixmath.h:2158-2294): the dither rule
         // where the union alpha is set, 0 elsewhere; an RGBA result's 4th
         // component is the union alpha
-        const bool set = __ldg(&a.u0[(int64_t)y * a.upitch + x]) != 0;
+        const bool set = ld_dep(&a.u0[(int64_t)y * a.upitch + x]) != 0;
         const uint32_t pixbits = mix32((uint32_t)pix ^ a.key);
 #pragma unroll
         for (int c = 0; c < C; ++c) {

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(256, 3) k_ef_weights(const __grid_constant__ E
         if (a.min[k]) {
             // --load-masks: the loaded weight replaces enfuseMask (src/enfuse.h:1288-1331)
             const float* mrow = a.min[k] + (int64_t)y * a.mipitch[k];
-            wk[k * 256] = make_float2(in0 ? __ldg(&mrow[x]) : 0.0f, in1 ? __ldg(&mrow[x + 1]) : 0.0f);
+            wk[k * 256] = make_float2(in0 ? ld_dep(&mrow[x]) : 0.0f, in1 ? ld_dep(&mrow[x + 1]) : 0.0f);
             ua0 |= in0 ? (uint32_t)alpha_at(a.alpha[k], x, y) : 0u;
             ua1 |= in1 ? (uint32_t)alpha_at(a.alpha[k], x + 1, y) : 0u;
             continue;
@@ -229,7 +229,7 @@ __device__ __forceinline__ void ef_load_run(const PixelView& img, int vec, int x
         const bool in = row && x + i >= 0 && x + i < img.w;
 #pragma unroll
         for (int s = 0; s < S; ++s) {
-            px[i][s] = in ? __ldg(p + i * S + s) : (TIn)0;
+            px[i][s] = in ? ld_dep(p + i * S + s) : (TIn)0;
         }
     }
 }

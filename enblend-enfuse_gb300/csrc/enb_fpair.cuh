@@ -151,9 +151,9 @@ __device__ __forceinline__ void fpair_fetch(FpairFetch<NP>& f, const float* img,
             const float* px = img + (int64_t)gy * pitch + (int64_t)gx * stride;
 #pragma unroll
             for (int ch = 0; ch < C; ++ch) {
-                f.v[j][ch] = __ldg(&px[ch]);
+                f.v[j][ch] = ld_dep(&px[ch]);
             }
-            const bool a = alpha ? __ldg(&alpha[(int64_t)gy * apitch + gx]) != 0 : true;
+            const bool a = alpha ? ld_dep(&alpha[(int64_t)gy * apitch + gx]) != 0 : true;
             f.fl |= (a ? 1u : 0u) << j | 1u << (8 + j);
         }
     }

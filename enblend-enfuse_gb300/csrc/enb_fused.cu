@@ -45,9 +45,8 @@ namespace enb {
 
 // Top level: R = blend(M, Gw, Gb) (the top Laplacian level is the Gaussian).
 template <typename T, typename TM, int C>
-__global__ void __launch_bounds__(256) k_blend_into(const TM* __restrict__ mask, int64_t mpitch,
-                                                    const T* __restrict__ gw, const T* __restrict__ gb,
-                                                    T* __restrict__ r, int64_t pitch, int64_t plane, int w, int h,
+__global__ void __launch_bounds__(256) k_blend_into(const TM* mask, int64_t mpitch, const T* gw, const T* gb,
+                                                    T* r, int64_t pitch, int64_t plane, int w, int h,
                                                     int32_t white_value)
 {
     griddep_wait();
@@ -70,9 +69,8 @@ __global__ void __launch_bounds__(256) k_blend_into(const TM* __restrict__ mask,
 // ---------------------------------------------------------------------------
 
 template <typename T, typename TM, int C>
-__global__ void __launch_bounds__(256) k_up_level(CoarseLevels cl, const TM* __restrict__ mask, int64_t mpitch,
-                                                  const T* __restrict__ gw, const T* __restrict__ gb,
-                                                  T* __restrict__ r, int64_t pitch, int64_t plane, int w, int h,
+__global__ void __launch_bounds__(256) k_up_level(CoarseLevels cl, const TM* mask, int64_t mpitch,
+                                                  const T* gw, const T* gb, T* r, int64_t pitch, int64_t plane, int w, int h,
                                                   int32_t white_value, int wrap)
 {
     __shared__ int4 sbuf[C][ESH][ESW];
@@ -123,7 +121,7 @@ __global__ void __launch_bounds__(256, 2) k_up_late(const __grid_constant__ UpLa
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int64_t row = win.o[u] / a.cpitch, col = win.o[u] - row * a.cpitch;
-            m1[u] = (int32_t)__ldg(&a.m1[row * a.mpitch1 + col]);
+            m1[u] = (int32_t)ld_dep(&a.m1[row * a.mpitch1 + col]);
         }
     }
     const auto quad = [&](const auto* p, int64_t o, int64_t o2, int32_t (&v)[4]) {
@@ -132,8 +130,8 @@ __global__ void __launch_bounds__(256, 2) k_up_late(const __grid_constant__ UpLa
             ld2<P, true>(p + o, v[0], v[1]);
             ld2<P, true>(p + o2, v[2], v[3]);
         } else {
-            v[0] = v[1] = (int32_t)__ldg(p + o);
-            v[2] = v[3] = (int32_t)__ldg(p + o2);
+            v[0] = v[1] = (int32_t)ld_dep(p + o);
+            v[2] = v[3] = (int32_t)ld_dep(p + o2);
         }
     };
     int32_t fm[4], fw[C][4], fb[C][4];
@@ -173,7 +171,7 @@ __global__ void __launch_bounds__(256, 2) k_up_late(const __grid_constant__ UpLa
             }
         }
     } else {
-        win.load_written<T, C>(a.r1, a.cplane, vr);
+        win.load<T, C>(a.r1, a.cplane, vr);
     }
     __syncthreads();  // the expansions above have read ss
     win.store<C>(ss, vr);
@@ -338,7 +336,7 @@ __device__ __forceinline__ void out0_border_tile(const CoarseLevels& cl, const O
         const int XX = min(X + (q & 1), a.w - 1), YY = min(Y + (q >> 1), a.h - 1);
         ld_px<TIn, S, VEC>(reinterpret_cast<const TIn*>(a.white) + (int64_t)YY * a.wpitch + (int64_t)XX * S, wp[q]);
         ld_px<TIn, S, VEC>(reinterpret_cast<const TIn*>(a.black) + (int64_t)YY * a.bpitch + (int64_t)XX * S, bp[q]);
-        mk[q] = (int32_t)__ldg(&a.mask[(int64_t)YY * a.mpitch + XX]) << MF;
+        mk[q] = (int32_t)ld_dep(&a.mask[(int64_t)YY * a.mpitch + XX]) << MF;
     }
     if (a.has_coarse) {
         stage_coarse<3 * C, T, true, 256>(ss, cl, I0, J0, a.w, a.wrap);
@@ -442,8 +440,8 @@ __global__ void __launch_bounds__(256, 3) k_out0(CoarseLevels cl, Out0Args a)
         ld_px<TIn, S, VEC>(b0 + a.bpitch, bp[2]);
         ld_px<TIn, S, VEC>(b0 + a.bpitch + S, bp[3]);
         const uint8_t* m0 = a.mask + (int64_t)Y * a.mpitch + X;
-        const int32_t mk[4] = {(int32_t)__ldg(m0) << MF, (int32_t)__ldg(m0 + 1) << MF,
-                               (int32_t)__ldg(m0 + a.mpitch) << MF, (int32_t)__ldg(m0 + a.mpitch + 1) << MF};
+        const int32_t mk[4] = {(int32_t)ld_dep(m0) << MF, (int32_t)ld_dep(m0 + 1) << MF,
+                               (int32_t)ld_dep(m0 + a.mpitch) << MF, (int32_t)ld_dep(m0 + a.mpitch + 1) << MF};
         stage_coarse4_interior<C, T, true, 256>(sbuf, cl, I0, J0);
         __syncthreads();
         out0_quad<TIn, T, C, S, AM, VEC>(a, PackedTaps{sbuf}, X, Y, qx, qy, wp, bp, mk);
@@ -674,8 +672,8 @@ __global__ void __launch_bounds__(256, 3) k_out0_tma(const __grid_constant__ Out
         int X0, Y0;
         origin(t, X0, Y0);
         const uint8_t* m0 = a.mask + (int64_t)(Y0 + 2 * qy) * a.mpitch + X0 + 2 * qx;
-        return (uint32_t)__ldg(m0) | (uint32_t)__ldg(m0 + 1) << 8 | (uint32_t)__ldg(m0 + a.mpitch) << 16 |
-               (uint32_t)__ldg(m0 + a.mpitch + 1) << 24;
+        return (uint32_t)ld_dep(m0) | (uint32_t)ld_dep(m0 + 1) << 8 | (uint32_t)ld_dep(m0 + a.mpitch) << 16 |
+               (uint32_t)ld_dep(m0 + a.mpitch + 1) << 24;
     };
     int t = blockIdx.x;
     uint32_t mreg = 0;

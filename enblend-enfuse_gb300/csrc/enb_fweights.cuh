@@ -294,10 +294,10 @@ __device__ __forceinline__ void ftile_fetch_px(float (&rgb)[3], uint8_t& a, cons
 #pragma unroll
         for (int ch = 0; ch < 3; ++ch) {
             if (ch < C) {
-                rgb[ch] = __ldg(&px[ch]);
+                rgb[ch] = ld_dep(&px[ch]);
             }
         }
-        a = alpha ? (__ldg(&alpha[(int64_t)gy * apitch + gx]) != 0) : 1;
+        a = alpha ? (ld_dep(&alpha[(int64_t)gy * apitch + gx]) != 0) : 1;
     }
 }
 

@@ -132,8 +132,8 @@ struct FineLevel {
         for (int c = 0; c < C; ++c) {
             const T *p = d + c * plane + o, *q = d + c * plane + o1;
             if (pair) {
-                ld2<T, false>(p, f[c][0], f[c][1]);
-                ld2<T, false>(q, f[c][2], f[c][3]);
+                ld2<T, true>(p, f[c][0], f[c][1]);
+                ld2<T, true>(q, f[c][2], f[c][3]);
             } else {
                 f[c][0] = (int32_t)p[0];
                 f[c][2] = (int32_t)q[0];
@@ -200,12 +200,12 @@ __global__ void __launch_bounds__(256) k_expand(const __grid_constant__ ExpandAr
     const TileWindow win(I0, J0, a.sw, a.sh, a.spitch, a.dw, a.wrap);
     int32_t v[C][2], f[C][4];
     if (!ADD) {
-        win.load_written<T, C>(a.src, a.splane, v);
+        win.load<T, C>(a.src, a.splane, v);
     }
     fine.template load<T, C>(a.dst, o, o1, a.dplane, Xc, Yc, Y1, pair, x1, f);
     griddep_wait();
     if (ADD) {
-        win.load_written<T, C>(a.src, a.splane, v);
+        win.load<T, C>(a.src, a.splane, v);
     }
     win.store<C>(ss, v);
     __syncthreads();

@@ -20,13 +20,13 @@ template <typename TIn, int S, bool VEC>
 __device__ __forceinline__ void ld_px(const TIn* p, TIn (&o)[S])
 {
     if (VEC && S == 4 && sizeof(TIn) == 2) {
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+        const uint2 v = ld_dep(reinterpret_cast<const uint2*>(p));
         o[0] = (TIn)(v.x & 0xffffu);
         o[1] = (TIn)(v.x >> 16);
         o[2] = (TIn)(v.y & 0xffffu);
         o[S - 1] = (TIn)(v.y >> 16);
     } else if (VEC && S == 4 && sizeof(TIn) == 1) {
-        const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(p));
+        const uint32_t v = ld_dep(reinterpret_cast<const uint32_t*>(p));
         o[0] = (TIn)(v & 0xffu);
         o[1] = (TIn)((v >> 8) & 0xffu);
         o[2] = (TIn)((v >> 16) & 0xffu);
@@ -34,7 +34,7 @@ __device__ __forceinline__ void ld_px(const TIn* p, TIn (&o)[S])
     } else {
 #pragma unroll
         for (int c = 0; c < S; ++c) {
-            o[c] = __ldg(&p[c]);
+            o[c] = ld_dep(&p[c]);
         }
     }
 }
@@ -82,7 +82,7 @@ struct PixelRun {
         } u;
 #pragma unroll
         for (int i = 0; i < NW; ++i) {
-            u.w[i] = __ldg(reinterpret_cast<const W*>(p) + i);
+            u.w[i] = ld_dep(reinterpret_cast<const W*>(p) + i);
         }
 #pragma unroll
         for (int i = 0; i < N * S; ++i) {
@@ -123,7 +123,7 @@ __device__ __forceinline__ int pixel_alpha(const TIn (&px)[S], const uint8_t* ap
                                            uint32_t alo, uint32_t ahi)
 {
     if (AM == 0) {
-        return __ldg(&ap[(int64_t)y * apitch + x]) != 0;
+        return ld_dep(&ap[(int64_t)y * apitch + x]) != 0;
     }
     if (AM == 1) {
         return 1;

@@ -43,11 +43,11 @@ constexpr int RVP = 148;                 // padded row of column sums
 // phase 2 (8 threads at a stride of 8 words) then hit 32 distinct banks.
 __device__ __forceinline__ int rphys(int c) { return c + ((c >> 5) << 2); }
 
-// Planar pyramid level (+ an 8-bit alpha plane when A); NC: read-only load
-// path (the level is not written by the launch).  Samples are delivered in
+// Planar pyramid level (+ an 8-bit alpha plane when A); EARLIER: an earlier
+// launch wrote the level (ld_src).  Samples are delivered in
 // the accumulator type of the reduce (int32 for fixed point, float for the
 // FP32 pyramids of float images).
-template <typename TS, int C, bool A, bool NC = true>
+template <typename TS, int C, bool A, bool EARLIER = true>
 struct PlanarSource {
     const TS* p;
     int64_t pitch, plane;   // elements
@@ -59,9 +59,9 @@ struct PlanarSource {
         const int64_t o = (int64_t)gy * pitch + gx;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            v[c] = (AC)ld_src<NC>(&p[c * plane + o]);
+            v[c] = (AC)ld_src<EARLIER>(&p[c * plane + o]);
         }
-        al = A ? (ld_src<NC>(&a[(int64_t)gy * apitch + gx]) != 0) : 1;
+        al = A ? (ld_src<EARLIER>(&a[(int64_t)gy * apitch + gx]) != 0) : 1;
     }
 };
 
@@ -73,7 +73,7 @@ struct ByteSource {
     template <typename AC>
     __device__ __forceinline__ void load(int gy, int gx, AC (&v)[1], int& al) const
     {
-        v[0] = (int32_t)__ldg(&p[(int64_t)gy * pitch + gx]) << frac;
+        v[0] = (int32_t)ld_dep(&p[(int64_t)gy * pitch + gx]) << frac;
         al = 1;
     }
 };
@@ -470,10 +470,10 @@ __device__ __forceinline__ void reduce_tail(const TailGeometry& g, T* const* p, 
         for (int i = threadIdx.x; i < n; i += kTailThreads) {
             const int y = i / w, x = i - y * w;
             const int64_t o = (int64_t)y * g.pitch[0] + x;
-            const int al = A ? __ldg(&ap[0][(int64_t)y * g.apitch[0] + x]) != 0 : 1;
+            const int al = A ? ld_dep(&ap[0][(int64_t)y * g.apitch[0] + x]) != 0 : 1;
 #pragma unroll
             for (int c = 0; c < C; ++c) {
-                const AC v = (AC)__ldg(&p[0][c * plane + o]);
+                const AC v = (AC)ld_dep(&p[0][c * plane + o]);
                 lev[c * n + i] = al ? v : (AC)0;
             }
             if (A) {

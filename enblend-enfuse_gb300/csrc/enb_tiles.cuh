@@ -2,8 +2,8 @@
 // coarse-level cluster kernel of the enblend blend: staging of the coarse
 // neighbourhood of a 64x16 destination tile, the expansion (src/pyramid.h
 // SKIPSM expand, 1227-1411) of its quads, and the per-tile Laplacian + blend
-// + collapse step.  NC selects the read-only load path (data no thread of the
-// launch writes) or plain loads (levels written earlier in the same launch);
+// + collapse step.  EARLIER: the levels were written by an earlier launch, else
+// earlier in the same launch (ld_src);
 // NT is the CTA's thread count.
 #pragma once
 
@@ -32,7 +32,7 @@ struct CoarseLevels {
 
 // Stage the 34x10 coarse neighbourhoods of a 64x16 destination tile for NP
 // planes; loads unrolled and independent of each other.
-template <int NP, typename T, bool NC, int NT>
+template <int NP, typename T, bool EARLIER, int NT>
 __device__ __forceinline__ void stage_coarse(int32_t (*ss)[ESH][ESW], const CoarseLevels& cl, int I0, int J0,
                                              int dw, int wrap)
 {
@@ -55,7 +55,7 @@ __device__ __forceinline__ void stage_coarse(int32_t (*ss)[ESH][ESW], const Coar
             const int64_t o = (int64_t)min(max(j, 0), cl.h - 1) * cl.pitch + min(max(i, 0), cl.w - 1);
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
-                const int32_t v = (int32_t)ld_src<NC>(&reinterpret_cast<const T*>(cl.p[p])[o]);
+                const int32_t v = (int32_t)ld_src<EARLIER>(&reinterpret_cast<const T*>(cl.p[p])[o]);
                 ss[p][r][c] = in ? v * f : 0;
             }
         }
@@ -66,7 +66,7 @@ __device__ __forceinline__ void stage_coarse(int32_t (*ss)[ESH][ESW], const Coar
 // one int4 per tap ({Gw, Gb, R, 0}): a quad's nine taps of all three planes
 // are then nine 16-byte shared loads (a warp's loads are 512 contiguous
 // bytes, four wavefronts, no bank conflicts).
-template <int C, typename T, bool NC, int NT>
+template <int C, typename T, bool EARLIER, int NT>
 __device__ __forceinline__ void stage_coarse4_interior(int4 (*s4)[ESH][ESW], const CoarseLevels& cl, int I0, int J0)
 {
     constexpr int N = ESH * ESW;
@@ -84,8 +84,8 @@ __device__ __forceinline__ void stage_coarse4_interior(int4 (*s4)[ESH][ESW], con
             const int o = r * (int)cl.pitch + c;
 #pragma unroll
             for (int ch = 0; ch < C; ++ch) {
-                s4[ch][r][c] = make_int4((int32_t)ld_src<NC>(&base[ch][o]), (int32_t)ld_src<NC>(&base[C + ch][o]),
-                                         (int32_t)ld_src<NC>(&base[2 * C + ch][o]), 0);
+                s4[ch][r][c] = make_int4((int32_t)ld_src<EARLIER>(&base[ch][o]), (int32_t)ld_src<EARLIER>(&base[C + ch][o]),
+                                         (int32_t)ld_src<EARLIER>(&base[2 * C + ch][o]), 0);
             }
         }
     }
@@ -146,26 +146,13 @@ struct TileWindow {
         }
     }
     template <typename T, int C>
-    __device__ __forceinline__ void load(const T* __restrict__ p, int64_t cplane, int32_t (&v)[C][2]) const
+    __device__ __forceinline__ void load(const T* p, int64_t cplane, int32_t (&v)[C][2]) const
     {
 #pragma unroll
         for (int c = 0; c < C; ++c) {
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                v[c][u] = (int32_t)__ldg(&p[c * cplane + o[u]]);
-            }
-        }
-    }
-    // a plane that the launch before wrote: not through the read-only path,
-    // whose loads could be moved above the wait
-    template <typename T, int C>
-    __device__ __forceinline__ void load_written(const T* p, int64_t cplane, int32_t (&v)[C][2]) const
-    {
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                v[c][u] = (int32_t)__ldcg(&p[c * cplane + o[u]]);
+                v[c][u] = (int32_t)ld_dep(&p[c * cplane + o[u]]);
             }
         }
     }
@@ -343,15 +330,15 @@ __device__ __forceinline__ int quad_kind(const int32_t (&m)[4], int32_t W)
 }
 
 // Two horizontally adjacent samples of a planar level (even x: 4- or 8-byte aligned).
-template <typename T, bool NC>
+template <typename T, bool EARLIER>
 __device__ __forceinline__ void ld2(const T* p, int32_t& a, int32_t& b)
 {
     if (sizeof(T) == 4) {
-        const int2 v = ld_src<NC>(reinterpret_cast<const int2*>(p));
+        const int2 v = ld_src<EARLIER>(reinterpret_cast<const int2*>(p));
         a = v.x;
         b = v.y;
     } else {
-        const int v = ld_src<NC>(reinterpret_cast<const int*>(p));
+        const int v = ld_src<EARLIER>(reinterpret_cast<const int*>(p));
         a = (int32_t)(int16_t)(v & 0xffff);
         b = v >> 16;
     }
@@ -381,9 +368,9 @@ __device__ __forceinline__ bool interior_tile(int X0, int Y0, int w, int h, int 
 // R_l = fromPromote(blend(M_l, Gw_l - E(Gw_{l+1}), Gb_l - E(Gb_{l+1})) + E(R_{l+1}))
 // on the tile at (X0, Y0), quads on threads 0..255 (threads NT > 256 only
 // take part in the staging and the barrier).  sbuf: C*ESH*ESW int4.
-template <typename T, typename TM, int C, bool NC, int NT>
-__device__ __forceinline__ void up_tile(const CoarseLevels& cl, const TM* __restrict__ mask, int64_t mpitch,
-                                        const T* __restrict__ gw, const T* __restrict__ gb, T* __restrict__ r,
+template <typename T, typename TM, int C, bool EARLIER, int NT>
+__device__ __forceinline__ void up_tile(const CoarseLevels& cl, const TM* mask, int64_t mpitch,
+                                        const T* gw, const T* gb, T* r,
                                         int64_t pitch, int64_t plane, int w, int h, int32_t white_value, int wrap,
                                         int X0, int Y0, int4 (*sbuf)[ESH][ESW])
 {
@@ -401,17 +388,17 @@ __device__ __forceinline__ void up_tile(const CoarseLevels& cl, const TM* __rest
         const int64_t o0 = (int64_t)Y * pitch + X;
         int32_t fw[C][4], fb[C][4], fm[4];
         if (active) {
-            ld2<TM, NC>(mask + (int64_t)Y * mpitch + X, fm[0], fm[1]);
-            ld2<TM, NC>(mask + (int64_t)(Y + 1) * mpitch + X, fm[2], fm[3]);
+            ld2<TM, EARLIER>(mask + (int64_t)Y * mpitch + X, fm[0], fm[1]);
+            ld2<TM, EARLIER>(mask + (int64_t)(Y + 1) * mpitch + X, fm[2], fm[3]);
 #pragma unroll
             for (int c = 0; c < C; ++c) {
-                ld2<T, NC>(gw + c * plane + o0, fw[c][0], fw[c][1]);
-                ld2<T, NC>(gw + c * plane + o0 + pitch, fw[c][2], fw[c][3]);
-                ld2<T, NC>(gb + c * plane + o0, fb[c][0], fb[c][1]);
-                ld2<T, NC>(gb + c * plane + o0 + pitch, fb[c][2], fb[c][3]);
+                ld2<T, EARLIER>(gw + c * plane + o0, fw[c][0], fw[c][1]);
+                ld2<T, EARLIER>(gw + c * plane + o0 + pitch, fw[c][2], fw[c][3]);
+                ld2<T, EARLIER>(gb + c * plane + o0, fb[c][0], fb[c][1]);
+                ld2<T, EARLIER>(gb + c * plane + o0 + pitch, fb[c][2], fb[c][3]);
             }
         }
-        stage_coarse4_interior<C, T, NC, NT>(sbuf, cl, I0, J0);
+        stage_coarse4_interior<C, T, EARLIER, NT>(sbuf, cl, I0, J0);
         __syncthreads();
         if (active) {
             const int kind = quad_kind(fm, white_value);
@@ -438,14 +425,14 @@ __device__ __forceinline__ void up_tile(const CoarseLevels& cl, const TM* __rest
     for (int q = 0; q < 4; ++q) {
         const int XX = min(X + (q & 1), w - 1), YY = min(Y + (q >> 1), h - 1);
         const int64_t o = (int64_t)YY * pitch + XX;
-        fm[q] = (int32_t)ld_src<NC>(&mask[(int64_t)YY * mpitch + XX]);
+        fm[q] = (int32_t)ld_src<EARLIER>(&mask[(int64_t)YY * mpitch + XX]);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            fw[c][q] = (int32_t)ld_src<NC>(&gw[c * plane + o]);
-            fb[c][q] = (int32_t)ld_src<NC>(&gb[c * plane + o]);
+            fw[c][q] = (int32_t)ld_src<EARLIER>(&gw[c * plane + o]);
+            fb[c][q] = (int32_t)ld_src<EARLIER>(&gb[c * plane + o]);
         }
     }
-    stage_coarse<3 * C, T, NC, NT>(ss, cl, I0, J0, w, wrap);
+    stage_coarse<3 * C, T, EARLIER, NT>(ss, cl, I0, J0, w, wrap);
     __syncthreads();
     if (!active || X >= w || Y >= h) {
         return;

@@ -1395,11 +1395,14 @@ enb_status enfuse_device(enb_ctx* ctx, const enb_enfuse_params* prm, int K, cons
     const int w = images[0].width, h = images[0].height, C = images[0].channels, dt = images[0].dtype;
     const int L = enb_num_levels(w, h, 1, o.levels);
     if (!o.plain && dt != ENB_F32 && K <= kEfuseMaxK && L >= 2 && pixel_view(out).stride == pixel_view(&images[0]).stride) {
-        // one alpha mode for all exposures (the level-1 reduce is compiled per mode)
+        // one alpha mode and one number of samples a pixel for all exposures
+        // (the kernels are compiled per mode and step every image by it)
         bool uniform = true;
         const int m0 = alpha_source(&images[0], alphas ? &alphas[0] : nullptr).mode;
+        const int s0 = pixel_view(&images[0]).stride;
         for (int k = 1; k < K; ++k) {
-            uniform = uniform && alpha_source(&images[k], alphas ? &alphas[k] : nullptr).mode == m0;
+            uniform = uniform && alpha_source(&images[k], alphas ? &alphas[k] : nullptr).mode == m0 &&
+                      pixel_view(&images[k]).stride == s0;
         }
         if (uniform) {
             return enfuse_fused(ctx, prm, K, images, alphas, masks_in, out, out_alpha, o, level0, L);

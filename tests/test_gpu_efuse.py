@@ -206,3 +206,23 @@ def test_weight_kernels_against_single_operations(ctx, dtype, con, ent, chans):
                 got.append((l0, out, oa))
             for a, b in zip(*got):
                 assert np.array_equal(a, b), (w, h, alpha)
+
+
+@pytest.mark.parametrize("dt", [np.uint8, np.uint16])
+@pytest.mark.parametrize("samples", [(3, 4, 3), (4, 3, 4)])
+@pytest.mark.parametrize("windows", [0, 5])
+def test_exposures_of_rgb_and_rgba_mixed(ctx, dt, samples, windows):
+    """A stack of RGB and RGBA images, all with alpha planes: the same result as the stack of their RGB samples, whose
+    exposures all have one layout (bit for bit, as every pass is in integers)."""
+    h, w = 45, 70
+    imgs = _stack(dt, h, w, len(samples), seed=61)
+    rng = np.random.default_rng(61)
+    alphas = [np.where(rng.random((h, w)) < 0.9, 255, 0).astype(np.uint8) for _ in samples]
+    kw = W_ALL if windows else dict(exposure_weight=1.0, saturation_weight=0.2)
+    l0, out, oa = _run(ctx, imgs, kw, seed=3, alphas=[_dev(a) for a in alphas])
+    mixed = [x if s == 3 else np.concatenate([x, rng.integers(0, 256, (h, w, 1)).astype(dt)], axis=2)
+             for x, s in zip(imgs, samples)]
+    l0m, outm, oam = _run(ctx, mixed, kw, seed=3, alphas=[_dev(a) for a in alphas])
+    assert np.array_equal(l0m, l0)
+    assert np.array_equal(outm[..., :3], out)
+    assert np.array_equal(oam, oa)

@@ -2277,10 +2277,11 @@ enb_status enb_enblend(enb_ctx* ctx, const enb_image* white, const enb_image* wh
     }
     ENB_CHECK(ctx, pixels_ok(white) && pixels_ok(black) && same_geometry(white, black),
               "enblend: white/black must be interleaved U8/U16/F32 images of one geometry");
-    if (black->dtype == ENB_F32) {
-        o.plain = 1;  // the fused level passes are fixed point
+    if (black->dtype == ENB_F32 || pixel_view(white).stride != pixel_view(black).stride) {
+        o.plain = 1;  // the fused level passes are fixed point and step both images alike
     }
-    ENB_CHECK(ctx, out && pixels_ok(out) && same_geometry(out, black), "enblend: out must match the inputs");
+    ENB_CHECK(ctx, out && pixels_ok(out) && same_geometry(out, black) && pixel_view(out).stride == pixel_view(black).stride,
+              "enblend: out must match the black image");
     ENB_CHECK(ctx, mask && bytes_ok(mask, black->width, black->height), "enblend: mask must be U8 of the image size");
     ENB_CHECK(ctx, black->width > 1 && black->height > 1, "enblend: image too small");
     ENB_CHECK(ctx, o.dither == ENB_DITHER_HASH || o.dither == ENB_DITHER_NEAREST, "enblend: unknown dither mode");

@@ -340,8 +340,10 @@ enb_status enb_nft_mask(enb_ctx* ctx, const enb_image* white_alpha, const enb_im
  * `black` under the 0/255 seam mask over the whole canvas.  out receives the
  * black image with the blended pixels where the union alpha is set (for RGBA
  * images the 4th component becomes the union alpha, 0 or the type maximum,
- * 1.0 for F32); out may be the black image itself.  F32 images always take
- * the per-operation pass structure (the fused passes are fixed point). */
+ * 1.0 for F32); out has the black image's samples per pixel and may be that
+ * image itself.  F32 images, and a white image of other samples per pixel than
+ * the black one, always take the per-operation pass structure (the fused
+ * passes are fixed point and of one layout). */
 enb_status enb_enblend(enb_ctx* ctx, const enb_image* white, const enb_image* white_alpha,
                        const enb_image* black, const enb_image* black_alpha, const enb_image* mask,
                        const enb_image* out, const enb_image* out_alpha, const enb_fuse_options* opt);

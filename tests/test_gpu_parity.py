@@ -488,3 +488,26 @@ def test_enblend_host_bands(ctx, orc, dt, planes):
     assert np.array_equal(l0, ref["level0"])
     assert np.array_equal(out, ref["out"])
     assert np.array_equal(oa, ref["alpha"])
+
+
+@pytest.mark.parametrize("dt", [np.uint8, np.uint16])
+@pytest.mark.parametrize("wide", ["white", "black"])
+@pytest.mark.parametrize("host", [False, True])
+def test_enblend_of_rgb_and_rgba(ctx, dt, wide, host):
+    """One RGB and one RGBA image with alpha planes: the blend of their RGB samples (bit for bit), and an output of
+    another number of samples than the black image's is refused."""
+    import enbgpu
+    from enbgpu import synthetic
+    white, black, mask = synthetic.panorama_pair(80, 200, 120, dt, seed=5)
+    wa, ba = (np.where(x[..., 3] != 0, 255, 0).astype(np.uint8) for x in (white, black))
+    rgb = [np.ascontiguousarray(x[..., :3]) for x in (white, black)]
+    pair = [white if wide == "white" else rgb[0], black if wide == "black" else rgb[1]]
+    put = (lambda a: a) if host else _dev
+    get = (lambda a: a) if host else (lambda t: t.cpu().numpy())
+    want, want_alpha = ctx.enblend(*map(put, rgb), put(mask), put(wa), put(ba), seed=7)
+    got, got_alpha = ctx.enblend(*map(put, pair), put(mask), put(wa), put(ba), seed=7)
+    assert np.array_equal(get(got)[..., :3], get(want))
+    assert np.array_equal(get(got_alpha), get(want_alpha))
+    other = put(np.zeros_like(rgb[0] if wide == "black" else white))
+    with pytest.raises(enbgpu.EnbError):
+        ctx.enblend(*map(put, pair), put(mask), put(wa), put(ba), out=other)

@@ -2742,8 +2742,8 @@ enb_status enb_fuse_grad(enb_ctx* ctx, const enb_enfuse_params* prm, int K, cons
                        target->height == h,
               "fuse_grad: target must be an F32 RGB image of the inputs' size");
     if (out) {
-        ENB_CHECK(ctx, pixels_ok(out) && out->dtype == ENB_F32 && out->width == w && out->height == h,
-                  "fuse_grad: out must be an F32 image of the inputs' size");
+        ENB_CHECK(ctx, pixels_ok(out) && out->dtype == ENB_F32 && out->channels == 3 && out->width == w && out->height == h,
+                  "fuse_grad: out must be an F32 RGB image of the inputs' size");
     }
     for (int k = 0; k < K; ++k) {
         if (logits) {

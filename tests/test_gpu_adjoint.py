@@ -99,6 +99,15 @@ def test_adjoint_rejects_entropy(ctx):
         ctx.fuse_grad(dev, torch.from_numpy(target).cuda(), params=enbgpu.enfuse_params(entropy_weight=0.3))
 
 
+def test_adjoint_rejects_gray_output(ctx):
+    """An output of one channel cannot take the three that the pass writes."""
+    import enbgpu
+    imgs, target = _scene(K=2, h=24, w=24)
+    dev = [torch.from_numpy(x).cuda() for x in imgs]
+    with pytest.raises(enbgpu.EnbError):
+        ctx.fuse_grad(dev, torch.from_numpy(target).cuda(), out=torch.zeros((24, 24), device="cuda"))
+
+
 @pytest.mark.parametrize("K,h,w,cwin,chans,with_logits", [
     (2, 33, 47, 5, 3, True), (3, 65, 64, 3, 3, True), (4, 16, 130, 5, 4, False), (5, 129, 67, 7, 3, True),
     (9, 70, 95, 5, 3, True), (8, 7, 8, 3, 3, True), (2, 200, 33, 5, 4, True)])

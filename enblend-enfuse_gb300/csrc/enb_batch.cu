@@ -897,6 +897,11 @@ __global__ void __launch_bounds__(256, 3) k_batch_up0(ENB_BATCH_JOBS(J), int l, 
         for (int c = 0; c < C; ++c) {
             o[c] = on ? from_pyramid_value(top ? acc[q][c] : __fadd_rn(acc[q][c], e[q][c])) : 0.0f;
         }
+        if (J::kOne) {  // enb_enfuse clears the components that it has no value for
+            for (int c = C; c < 3 && c < s.ostride; ++c) {
+                o[c] = 0.0f;
+            }
+        }
         if (s.ostride == 4) {
             o[3] = on ? 1.0f : 0.0f;  // AlphaTraits<float>::max()
         }

@@ -405,3 +405,34 @@ def test_enfuse_mask_f32_repeats_by_distance(ctx, orc, ew, filled):
     out = torch.zeros((h, w), dtype=torch.float32, device="cuda")
     ctx.enfuse_mask(_dev(img), _dev(alpha), out, enbgpu.enfuse_params(float_range=1.0, **kw))
     _close(out.cpu().numpy().astype(np.float64), ref.astype(np.float64), WEIGHT_RTOL, 1e-7 * np.abs(ref).max(), f"repeats {ew}")
+
+
+@pytest.mark.parametrize("host", [False, True])
+@pytest.mark.parametrize("samples", [2, 3, 4])
+def test_enfuse_gray_clears_other_components(ctx, host, samples):
+    """One colour sample in pixels of more: the output's other components are 0 (the 4th the alpha), whatever they
+    held, and the colour sample is that of the dense image."""
+    import ctypes
+    import enbgpu
+    from enbgpu import synthetic
+    h, w = 37, 50
+    gray = [np.ascontiguousarray(x[..., 1]) for x in synthetic.exposure_stack(h, w, [-1.0, 0.0, 1.0], np.float32, 8.0, seed=9)]
+    want, _ = ctx.enfuse(gray, params=enbgpu.enfuse_params(contrast_weight=0.5, float_range=1.0))
+    wide = [np.concatenate([x[..., None], np.ones((h, w, samples - 1), np.float32)], axis=2) for x in gray]
+    arrays = wide if host else [_dev(x) for x in wide]
+    out = np.full((h, w, samples), 7.0, np.float32)
+    out = out if host else _dev(out)
+    # freed staging memory of the pool holds something else than zeros
+    junk = torch.full((8 << 20,), 3.0, device="cuda")
+    ctx.enfuse([junk[: 3 * h * w].reshape(h, w, 3)] * 2, params=enbgpu.enfuse_params(float_range=1.0))
+    prm = enbgpu.enfuse_params(contrast_weight=0.5, float_range=1.0)
+    o = ctx._options(0, False, False, "hash", 0, host, None)
+    imgs = (enbgpu.EnbImage * 3)(*[enbgpu.pixel_image(x, channels=1) for x in arrays])
+    ctx._check(ctx.lib.enb_enfuse(ctx.handle, ctypes.byref(prm), 3, imgs, None, None,
+                                  ctypes.byref(enbgpu.pixel_image(out, channels=1)), None, ctypes.byref(o)))
+    ctx.synchronize()
+    got = out if host else out.cpu().numpy()
+    assert np.array_equal(got[..., 0], want)
+    assert not got[..., 1:3].any()
+    if samples == 4:
+        assert (got[..., 3] == 1.0).all()

@@ -66,7 +66,7 @@ struct BatchStack {
     float* g;     // K * 3 * s1 (C planes used)
     uint8_t* a;   // K * s1
     float* r;     // 3 * s1
-    float* g0;    // K * 3 * s0 (level 0 of the image pyramids, written by the weights kernel)
+    float* g0;    // K * 3 * pitch[0] * h (level 0 of the image pyramids, written by the weights kernel)
     int64_t s0, s1;
     int64_t off0[kMaxLevels], off1[kMaxLevels];
     int pitch[kMaxLevels], lw[kMaxLevels], lh[kMaxLevels];
@@ -154,7 +154,7 @@ __device__ __forceinline__ float* r_level(const BatchStack& s, int l, int C)
 // Level 0 of exposure k's image pyramid (planes of pitch[0] * h).
 __device__ __forceinline__ float* g0_level(const BatchStack& s, int k, int C)
 {
-    return s.g0 + (int64_t)k * C * s.s0;
+    return s.g0 + (int64_t)k * C * s.pitch[0] * s.h;
 }
 
 // Level 0 of an exposure's image pyramid (planar floats) with the input's
@@ -1105,7 +1105,7 @@ static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 static size_t stack_bytes(const BatchStack& s, int C)
 {
     return align256((size_t)s.K * s.s0 * 4) + align256((size_t)s.s0) + align256((size_t)s.K * C * s.s1 * 4) +
-           align256((size_t)s.K * s.s1) + align256((size_t)C * s.s1 * 4) + align256((size_t)s.K * C * s.s0 * 4);
+           align256((size_t)s.K * s.s1) + align256((size_t)C * s.s1 * 4) + align256((size_t)s.K * C * s.pitch[0] * s.h * 4);
 }
 
 static void stack_buffers(BatchStack& s, int C, char* q)

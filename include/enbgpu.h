@@ -316,7 +316,10 @@ enb_status enb_enfuse_mask(enb_ctx* ctx, const enb_enfuse_params* params, const 
  * thresholded 4th component as imported by src/assemble.h:240-253, else fully
  * opaque).  masks_in: K F32 weight planes replacing enfuseMask (--load-masks),
  * or NULL.  out: interleaved image of the input type (zero where out_alpha is
- * 0); out_alpha: U8 union alpha, may be NULL. */
+ * 0); out_alpha: U8 union alpha, may be NULL.  F32 RGB stacks of up to 16
+ * exposures take about 22 K + 5 bytes of device memory a pixel while they run
+ * (every exposure's pyramids at once); where that cannot be allocated, and with
+ * opt->plain = 1, 4 K + 41 (one exposure's). */
 enb_status enb_enfuse(enb_ctx* ctx, const enb_enfuse_params* params, int K, const enb_image* images,
                       const enb_image* alphas, const enb_image* masks_in, const enb_image* out,
                       const enb_image* out_alpha, const enb_fuse_options* opt);

@@ -436,3 +436,29 @@ def test_enfuse_gray_clears_other_components(ctx, host, samples):
     assert not got[..., 1:3].any()
     if samples == 4:
         assert (got[..., 3] == 1.0).all()
+
+
+def test_enfuse_workspace(ctx):
+    """The device memory that a float stack takes while it is fused: 32-bit masks and image levels of every exposure
+    (levels of a third of level 0's size together), alpha levels, one result pyramid and the union alpha."""
+    import ctypes
+    import enbgpu
+    K, h, w = 8, 1024, 2048  # row pitches without padding but on the last levels
+    img = torch.rand((h, w, 3), device="cuda")
+    prm = enbgpu.enfuse_params(contrast_weight=0.5, float_range=1.0)
+    out, alpha = torch.zeros_like(img), torch.zeros((h, w), dtype=torch.uint8, device="cuda")
+    ctx.enfuse([img] * K, params=prm, out=out, out_alpha=alpha)  # weight tables are made here
+    torch.cuda.synchronize()
+    cu = ctypes.CDLL("libcuda.so.1")
+    pool, used, peak, zero = ctypes.c_void_p(), ctypes.c_uint64(), ctypes.c_uint64(), ctypes.c_uint64(0)
+    current, high = 7, 8  # CU_MEMPOOL_ATTR_USED_MEM_CURRENT, CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert cu.cuMemPoolGetAttribute(pool, current, ctypes.byref(used)) == 0
+    assert cu.cuMemPoolSetAttribute(pool, high, ctypes.byref(zero)) == 0
+    ctx.enfuse([img] * K, params=prm, out=out, out_alpha=alpha)
+    torch.cuda.synchronize()
+    assert cu.cuMemPoolGetAttribute(pool, high, ctypes.byref(peak)) == 0
+    px = h * w
+    masks, level0, levels = 4 * 4 / 3 * px, 12 * px, (12 + 1) / 3 * px
+    bound = K * (masks + level0 + levels) + (4 / 3 + 12 / 3) * px
+    assert 0 < peak.value - used.value <= 1.01 * bound

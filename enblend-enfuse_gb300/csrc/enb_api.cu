@@ -54,10 +54,13 @@ struct enb_ctx {
     // batched stacks: plan (workspace, job tables) and graph of the last
     // batch geometry (key) and the addresses it is set to (buffers), staging
     // buffers of host-buffer batches; ev: the graph's start and end, the end of
-    // the last call
+    // the last call; captured: a graph of the caller's holds the plan, which
+    // then keeps its addresses and, once another plan takes its place, is kept
     struct BatchCache {
         std::string key, buffers;
         BatchPlan* plan = nullptr;
+        bool captured = false;
+        std::vector<BatchPlan*> kept;
         cudaGraphExec_t exec = nullptr;
         cudaStream_t gs = nullptr;
         cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
@@ -68,6 +71,9 @@ struct enb_ctx {
                 cudaGraphExecDestroy(exec);
             }
             batch_plan_destroy(plan);
+            for (BatchPlan* p : kept) {
+                batch_plan_destroy(p);
+            }
             cudaFree(stage);
             for (cudaEvent_t e : ev) {
                 if (e) {
@@ -2529,8 +2535,8 @@ enb_status enb_fuse_stacks(enb_ctx* ctx, const enb_enfuse_params* prm, int n, co
         return ENB_OK;
     };
     // work of the call before, also on another stream, uses the same plan (a
-    // stream being captured can neither wait for that nor take other buffers:
-    // the table of addresses is no part of a capture)
+    // stream being captured can neither wait for that nor make a plan or move
+    // one to other buffers: the table of addresses is no part of a capture)
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     ENB_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
     const bool capturing = capture != cudaStreamCaptureStatusNone;
@@ -2538,7 +2544,10 @@ enb_status enb_fuse_stacks(enb_ctx* ctx, const enb_enfuse_params* prm, int n, co
         ENB_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, bc.ev[2], 0));
     }
     const bool moved = !o.host_buffers && bc.buffers != buffers;
-    if (bc.key == key && bc.plan && moved && !capturing) {
+    const bool planned = bc.plan && bc.key == key;
+    ENB_CHECK(ctx, !capturing || (planned && !moved && !o.graph && !o.host_buffers),
+              "fuse_stacks: a call being captured takes device buffers, graph = 0, and a call on the same buffers before it");
+    if (planned && moved && !bc.captured) {
         // the same work on other buffers: only the stacks' addresses change
         // (a new plan, its tables and its graph took 6 ms of a 23.3 ms call of
         // 16 stacks; the new addresses take 0.03 ms of the host's time)
@@ -2547,15 +2556,20 @@ enb_status enb_fuse_stacks(enb_ctx* ctx, const enb_enfuse_params* prm, int n, co
         ENB_CUDA(ctx, batch_plan_rebind(bc.plan, hs, ctx->stream));
         bc.buffers = buffers;
     }
-    if (bc.key != key || !bc.plan || (moved && capturing)) {
+    if (!planned || (moved && bc.captured)) {
         if (bc.exec) {
             cudaGraphExecDestroy(bc.exec);
             bc.exec = nullptr;
         }
         ENB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         ENB_CUDA(ctx, cudaStreamSynchronize(bc.gs));
-        batch_plan_destroy(bc.plan);
+        if (bc.captured) {
+            bc.kept.push_back(bc.plan);
+        } else {
+            batch_plan_destroy(bc.plan);
+        }
         bc.plan = nullptr;
+        bc.captured = false;
         cudaFree(bc.stage);
         bc.stage = nullptr;
         bc.key.clear();
@@ -2626,6 +2640,7 @@ enb_status enb_fuse_stacks(enb_ctx* ctx, const enb_enfuse_params* prm, int n, co
             ENB_LAUNCH(ctx, batch_plan_launch(bc.plan, i, ctx->stream));
         }
     }
+    bc.captured = bc.captured || capturing;
     if (!capturing) {
         ENB_CUDA(ctx, cudaEventRecord(bc.ev[2], ctx->stream));
     }

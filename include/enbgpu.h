@@ -371,7 +371,12 @@ typedef struct {
  * it (same FP32 arithmetic up to the order of float additions).  masks are
  * computed (no --load-masks); opt->plain = 1 runs enb_enfuse stack by stack
  * instead, one kernel per operation (for comparisons).  The workspace and graph of the last batch
- * geometry stay cached in the context. */
+ * geometry stay cached in the context.  A caller's stream capture takes a call with device buffers and
+ * opt->graph = 0 whose batch, buffers included, is that of the last call before the capture
+ * (ENB_ERR_INVALID else, the capture goes on).  The captured work keeps its own buffers and workspace
+ * until the context is destroyed; it uses the context's weight tables, so no call with other weight
+ * parameters may come before its last replay, and replays are the caller's to order with calls on the
+ * same batch. */
 enb_status enb_fuse_stacks(enb_ctx* ctx, const enb_enfuse_params* params, int n_stacks, const enb_stack* stacks,
                            const enb_fuse_options* opt);
 

@@ -210,3 +210,45 @@ def test_batch_on_other_buffers(ctx, graph):
         for i, outs in got:
             for o, w in zip(outs, sets[i][2 if use_alpha else 3]):
                 assert torch.equal(o, w), i
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_captured_batch_keeps_its_buffers(ctx, graph):
+    """A call that the caller captures replays on its own buffers, whatever batches of the geometry run afterwards;
+    a capture on other buffers than the call before's, or of the library's own graph, is refused and leaves the
+    caller's capture usable."""
+    import enbgpu
+    shapes = [(37, 53, 3), (64, 40, 2)]
+    p = _params()
+    a, b = ([[_dev(x) for x in st] for st in _batch(seed=s, shapes=shapes)] for s in (81, 95))
+    oa, ob = ([torch.zeros_like(st[0]) for st in s] for s in (a, b))
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    ctx.set_stream(side.cuda_stream)
+    try:
+        ctx.fuse_stacks(a, params=p, outs=oa, graph=graph)
+        ctx.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            for s, o, own in ((b, ob, False), (a, oa, True)):
+                with pytest.raises(enbgpu.EnbError, match="being captured"):
+                    ctx.fuse_stacks(s, params=p, outs=o, graph=own)
+            ctx.fuse_stacks(a, params=p, outs=oa, graph=False)
+        for _ in range(2):
+            ctx.fuse_stacks(b, params=p, outs=ob, graph=graph)
+        ctx.fuse_stacks([b[0]], params=p, graph=graph)
+        ctx.synchronize()
+        for st in a:
+            for x in st:
+                x.mul_(0.75)
+        want = ctx.fuse_stacks(a, params=p, plain=True)
+        for x in oa + ob:
+            x.fill_(-1.0)
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+    finally:
+        ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+    for x, y in zip(oa, want):
+        assert torch.equal(x, y)
+    assert all((x == -1.0).all() for x in ob)

@@ -21,7 +21,8 @@ input pixels blended per second (2 x 4096 x 3072 = 25.17 Mpx per step).
          forward, loss and all gradients through enb_fuse_grad
   batched_fuse  the batched uneven-stack workload (64 FP32 stacks of
          uneven sizes and exposure counts): enb_fuse_stacks replayed as one
-         CUDA graph against the plain per-stack path on the same GPU
+         CUDA graph against enb_enfuse stack by stack and against single
+         operations on the same GPU
   enfuse_small / enfuse_large  enfuse of 3 x 1024x768 RGB u8 and of
          9 x 6000x4000 RGB u16 (contrast and entropy 5x5 windows) through the
          fused integer driver: value, e2e, roofline, kernels, CPU oracle
@@ -262,9 +263,9 @@ def batched_fuse(ctx, stream, n_stacks: int, reps: int = 3) -> dict:
     log-uniform in [512, 4096], 3..7 exposures, EVs evenly spaced over
     +-(count - 1) stops, weights exposure 1.0 / saturation 0.2 / contrast 0.5
     (5x5) / entropy 0.3 (5x5) in normalised-float mode; enb_fuse_stacks (one
-    CUDA graph, level schedule from enb_fuse_stacks_tune) against the plain
-    per-stack path (enb_enfuse per stack) on the same GPU, device-resident
-    inputs."""
+    CUDA graph, level schedule from enb_fuse_stacks_tune) against enb_enfuse
+    stack by stack and against single operations (plain) on the same GPU,
+    device-resident inputs."""
     import torch
     import enbgpu
     from enbgpu import synthetic
@@ -293,6 +294,14 @@ def batched_fuse(ctx, stream, n_stacks: int, reps: int = 3) -> dict:
     batched_ms = timed(lambda: ctx.fuse_stacks(stacks, params=prm, outs=outs), reps)
     launches = (ctx.launches - l0) // (reps + 1)
     ref = [o.clone() for o in outs]
+    alphas = [st[0].new_zeros(st[0].shape[:2], dtype=torch.uint8) for st in stacks]
+
+    def each():
+        for st, o, a in zip(stacks, outs, alphas):
+            ctx.enfuse(st, params=prm, out=o, out_alpha=a)
+
+    each_ms = timed(each, reps)
+    each_rel = max(float(((o - r).abs() / (r.abs() + 1e-6)).max()) for o, r in zip(outs, ref))
     plain_ms = timed(lambda: ctx.fuse_stacks(stacks, params=prm, outs=outs, plain=True), max(1, reps - 1))
     max_rel = max(float(((o - r).abs() / (r.abs() + 1e-6)).max()) for o, r in zip(outs, ref))
     ctx.profile(True)
@@ -312,9 +321,12 @@ def batched_fuse(ctx, stream, n_stacks: int, reps: int = 3) -> dict:
         "batched": {"value": units / (batched_ms / 1e3), "ms_per_step": batched_ms, "graph": True,
                     "launches_per_step": launches, "coarse_pixels": tune["best"],
                     "tuned_ms": {str(k): round(v, 3) for k, v in tune["ms"].items()}},
+        "per_stack": {"value": units / (each_ms / 1e3), "ms_per_step": each_ms,
+                      "what": "enb_enfuse stack by stack", "max_rel_diff_of_batched": each_rel},
         "plain": {"value": units / (plain_ms / 1e3), "ms_per_step": plain_ms,
-                  "what": "enb_enfuse stack by stack (the per-stack path)"},
-        "speedup": plain_ms / batched_ms,
+                  "what": "single operations, stack by stack (enb_fuse_options.plain)"},
+        "speedup": each_ms / batched_ms,
+        "speedup_vs_plain": plain_ms / batched_ms,
         "weights_ms": {"batched": weights_b, "plain": weights_p},
         "excluding_weights_ms": {"batched": batched_ms - weights_b, "plain": plain_ms - weights_p,
                                  "speedup": (plain_ms - weights_p) / max(batched_ms - weights_b, 1e-9)},

@@ -226,17 +226,17 @@ __device__ __forceinline__ void batch_normalise(const BatchStack& s, const float
     }
 }
 
-// Weights of window sizes that the pair kernel does not take: one output
-// pixel per thread on 16x16 tiles (enb_fweights.cuh).
-template <int CW, int EW, class J>
-__global__ void __launch_bounds__(256, 4) k_batch_weights(ENB_BATCH_JOBS(J), FloatWeightParams wp,
+// Weights of window sizes that the pair kernel does not take, in a batch (a
+// single stack takes the per-image kernel): one output pixel per thread on
+// 16x16 tiles (enb_fweights.cuh).
+template <int CW, int EW>
+__global__ void __launch_bounds__(256, 4) k_batch_weights(const BatchStack* __restrict__ stacks,
+                                                       const int4* __restrict__ jobs, FloatWeightParams wp,
                                                        WeightTables tab, int hard, int C)
 {
     extern __shared__ __align__(16) unsigned char bsmem[];
-    griddep_wait();
-    griddep_launch();
-    const int2 tile = job_tile<J>(jobs);
-    const BatchStack& s = job_stack(stacks, jobs, one);
+    const int2 tile = job_tile<BatchTable>(jobs);
+    const BatchStack& s = stacks[jobs[blockIdx.x].x];
     const int halo = fweight_halo(wp);
     const FTile t = ftile_carve(bsmem, BWT + 2 * halo, wp.repeat_slots, wp.ent_cut);
     float* wk = reinterpret_cast<float*>(bsmem + align16(ftile_bytes(t.TW, t.slots, wp.ent_cut))) + threadIdx.x;  // [K][BWT * BWT]
@@ -1449,34 +1449,37 @@ static cudaError_t launch_batch(void (*kernel)(KArgs...), dim3 grid, int block, 
 }
 
 template <int C, class J>
-static cudaError_t launch_weights(const BatchJobs<J>& j, dim3 grid, bool pair, const FloatWeightParams& wp, const WeightTables& tab,
-                                  int hard, size_t smem, cudaStream_t st)
+static cudaError_t launch_weights_pair(const BatchJobs<J>& j, dim3 grid, const FloatWeightParams& wp, const WeightTables& tab,
+                                       size_t smem, cudaStream_t st)
 {
     cudaError_t e = cudaErrorInvalidValue;
-    if (pair) {
-        ENB_FPAIR_DISPATCH(wp, {
-            auto k = k_batch_weights_pair<CWV, EWV, C, J>;
-            // as many CTAs per SM as the shared memory holds
-            cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-            e = launch_batch<J>(k, grid, FPT, smem, st, j, wp, tab);
-        });
-        return e;
-    }
+    ENB_FPAIR_DISPATCH(wp, {
+        auto k = k_batch_weights_pair<CWV, EWV, C, J>;
+        // as many CTAs per SM as the shared memory holds
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        e = launch_batch<J>(k, grid, FPT, smem, st, j, wp, tab);
+    });
+    return e;
+}
+
+static cudaError_t launch_weights(const BatchJobs<BatchTable>& j, dim3 grid, int C, const FloatWeightParams& wp,
+                                  const WeightTables& tab, int hard, size_t smem, cudaStream_t st)
+{
     const int cw = wp.use_contrast ? wp.contrast_window : 5;
     const int ew = wp.use_entropy ? wp.entropy_window : 5;
-    void (*k)(const BatchStack*, const int4*, const J, FloatWeightParams, WeightTables, int, int) = k_batch_weights<0, 0, J>;
+    void (*k)(const BatchStack*, const int4*, FloatWeightParams, WeightTables, int, int) = k_batch_weights<0, 0>;
     if (cw == 5 && ew == 5) {
-        k = k_batch_weights<5, 5, J>;
+        k = k_batch_weights<5, 5>;
     } else if (cw == 5 && ew == 3) {
-        k = k_batch_weights<5, 3, J>;
+        k = k_batch_weights<5, 3>;
     } else if (cw == 3 && ew == 3) {
-        k = k_batch_weights<3, 3, J>;
+        k = k_batch_weights<3, 3>;
     } else if (ew == 5) {
-        k = k_batch_weights<0, 5, J>;
+        k = k_batch_weights<0, 5>;
     } else if (ew == 3) {
-        k = k_batch_weights<0, 3, J>;
+        k = k_batch_weights<0, 3>;
     }
-    return launch_batch<J>(k, grid, BWT * BWT, smem, st, j.stacks, j.jobs, j.one, wp, tab, hard, C);
+    return launch_batch<BatchTable>(k, grid, BWT * BWT, smem, st, j.stacks, j.jobs, wp, tab, hard, C);
 }
 
 template <int C, class J>
@@ -1498,8 +1501,8 @@ static cudaError_t launch_step(const BatchPlan* p, const BatchPlan::Step& s, cud
     switch (s.kind) {
     case 0:
         note_launch("batch_weights", s.bytes);
-        return launch_weights<C>(j, dim3(grid.x, p->pair_weights ? (unsigned)p->maxK : 1u), p->pair_weights, p->wp, p->tab,
-                                 p->hard, p->wsmem, st);
+        return p->pair_weights ? launch_weights_pair<C>(j, dim3(grid.x, (unsigned)p->maxK), p->wp, p->tab, p->wsmem, st)
+                               : launch_weights(j, grid, C, p->wp, p->tab, p->hard, p->wsmem, st);
     case 5:
         note_launch("batch_normalise", s.bytes);
         return launch_batch<BatchTable>(k_batch_normalise<BatchTable>, grid, 256, 0, st, j.stacks, j.jobs, j.one, p->hard);
@@ -1543,10 +1546,11 @@ cudaError_t batch_plan_launch(const BatchPlan* p, int i, cudaStream_t st)
 // ---------------------------------------------------------------------------
 //
 // The launches of a batch of one, without its tables, graph and plan: the
-// stack goes in the kernels' parameters.  Steps in order: the weights, their
-// normalisation (pair kernel only), per level the image and the mask reduces
-// (one launch where both fit the GPU at once), the merges from the top level
-// down to the output.
+// stack goes in the kernels' parameters.  Steps in order: the weights (windows
+// of the pair kernel; of others the caller makes them and level 0 of the image
+// pyramids, exposure by exposure), their normalisation, per level the image and
+// the mask reduces (one launch where both fit the GPU at once), the merges from
+// the top level down to the output.
 
 struct BatchSingle {
     BatchStack s;
@@ -1571,10 +1575,10 @@ BatchSingle* batch_single_create(const BatchStackHost& h, const FloatWeightParam
     BatchSingle* p = new BatchSingle{stack_of(h, levels, 0), h.C, wrap, hard, wp, tab, WeightsStep(wp, h.K), {}};
     const BatchStack& s = p->s;
     p->wp.repeat_slots = p->ws.slots;
-    p->steps.push_back({0, 0});
     if (p->ws.pair) {
-        p->steps.push_back({1, 0});
+        p->steps.push_back({0, 0});
     }
+    p->steps.push_back({1, 0});
     for (int l = 0; l + 1 < s.L; ++l) {
         const int64_t tiles = (int64_t)((s.lw[l + 1] + RDW - 1) / RDW) * ((s.lh[l + 1] + RDH - 1) / RDH);
         if (2 * s.K * tiles <= kJointReduceTiles) {
@@ -1595,6 +1599,16 @@ size_t batch_single_bytes(const BatchSingle* p) { return stack_bytes(p->s, p->C)
 void batch_single_workspace(BatchSingle* p, void* work) { stack_buffers(p->s, p->C, (char*)work); }
 int batch_single_steps(const BatchSingle* p) { return (int)p->steps.size(); }
 
+bool batch_single_weighs(const BatchSingle* p) { return p->ws.pair; }
+
+void batch_single_level0(const BatchSingle* p, int k, FloatPlane* weights, PlanarView* image)
+{
+    const BatchStack& s = p->s;
+    const int64_t plane = (int64_t)s.pitch[0] * s.h;
+    *weights = FloatPlane{(float*)(s.m + (int64_t)k * s.s0 + s.off0[0]), s.pitch[0], s.w, s.h};
+    *image = PlanarView{s.g0 + (int64_t)k * p->C * plane, s.pitch[0], plane, s.w, s.h, p->C, ENB_F32};
+}
+
 template <int C>
 static cudaError_t single_step(const BatchSingle* p, int i, cudaStream_t st)
 {
@@ -1609,7 +1623,7 @@ static cudaError_t single_step(const BatchSingle* p, int i, cudaStream_t st)
     switch (p->steps[(size_t)i].kind) {
     case 0:
         note_launch("batch_weights", K * px * (4.0 * s.istride[0] + 4.0 * C + 4.0) + px);
-        return launch_weights<C>(j, tiles(s.w, s.h, p->ws.tx, p->ws.ty, p->ws.pair ? K : 1), p->ws.pair, p->wp, p->tab, p->hard, p->ws.smem, st);
+        return launch_weights_pair<C>(j, tiles(s.w, s.h, p->ws.tx, p->ws.ty, K), p->wp, p->tab, p->ws.smem, st);
     case 1:
         note_launch("batch_normalise", K * px * 12.0);
         return launch_batch<BatchOne>(k_batch_normalise<BatchOne>, tiles(s.w, s.h, FPX, FPY, 1), 256, 0, st, j.stacks, j.jobs, j.one,

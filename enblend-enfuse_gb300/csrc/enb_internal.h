@@ -362,6 +362,10 @@ BatchSingle* batch_single_create(const BatchStackHost& h, const FloatWeightParam
 void batch_single_destroy(BatchSingle* p);
 size_t batch_single_bytes(const BatchSingle* p);
 void batch_single_workspace(BatchSingle* p, void* work);
+// Whether the steps make the weights; if not, the caller first writes each
+// exposure's weights and level 0 of its image pyramid (the log mapping).
+bool batch_single_weighs(const BatchSingle* p);
+void batch_single_level0(const BatchSingle* p, int k, FloatPlane* weights, PlanarView* image);
 int batch_single_steps(const BatchSingle* p);
 cudaError_t batch_single_launch(const BatchSingle* p, int step, cudaStream_t st);
 

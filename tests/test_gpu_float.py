@@ -462,3 +462,31 @@ def test_enfuse_workspace(ctx):
     masks, level0, levels = 4 * 4 / 3 * px, 12 * px, (12 + 1) / 3 * px
     bound = K * (masks + level0 + levels) + (4 / 3 + 12 / 3) * px
     assert 0 < peak.value - used.value <= 1.01 * bound
+
+
+@pytest.mark.parametrize("windows", [(7, 0), (5, 7), (9, 3)])
+@pytest.mark.parametrize("variant", ["opaque", "alpha", "hard", "gray"])
+def test_enfuse_windows_outside_the_pair_kernel(ctx, windows, variant):
+    """Window sizes that take one pixel a thread: each exposure is weighted by the per-image kernel, the rest in the
+    passes over all exposures; bit for bit the per-operation result."""
+    import enbgpu
+    from enbgpu import synthetic
+    con, ent = windows
+    h, w, K = 43, 70, 3
+    imgs = synthetic.exposure_stack(h, w, list(np.linspace(-2.0, 2.0, K)), np.float32, 8.0, seed=21)
+    if variant == "gray":
+        imgs = [np.ascontiguousarray(x[..., 1]) for x in imgs]
+    rng = np.random.default_rng(4)
+    alphas = [_dev(np.where(rng.random((h, w)) < 0.9, 255, 0).astype(np.uint8)) for _ in imgs] if variant == "alpha" else None
+    prm = enbgpu.enfuse_params(saturation_weight=0.2, contrast_weight=0.5, contrast_window_size=con,
+                               entropy_weight=0.3 if ent else 0.0, entropy_window_size=ent or 3, float_range=1.0)
+    dev = [_dev(x) for x in imgs]
+    ctx.profile(True)
+    out, oa = ctx.enfuse(dev, alphas, params=prm, hard_mask=variant == "hard")
+    ctx.synchronize()
+    names = ctx.profile_report()
+    ctx.profile(False)
+    want, wa = ctx.enfuse(dev, alphas, params=prm, hard_mask=variant == "hard", plain=True)
+    assert names["f_enfuse_mask"]["launches"] == K and "batch_up0" in names, names
+    assert torch.equal(oa, wa)
+    assert torch.equal(out, want)

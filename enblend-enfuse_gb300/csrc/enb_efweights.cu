@@ -334,10 +334,11 @@ struct EfQuadTile {
 };
 
 // Loads exposure k's tile at (x0, y0): gray (0 where transparent), the samples
-// and the opaque flags; zero outside the image.  Ends with a barrier; nonzero when every pixel of
+// (0xffff where transparent, when there are entropy windows) and the opaque
+// flags; the image's outside is transparent.  Ends with a barrier; nonzero when every pixel of
 // the tile inside the image is opaque (then every window that counts, which
 // lies inside the image, is).
-template <typename TIn, int S, int CW, int EW, typename TM>
+template <typename TIn, int S, int CW, int EW, bool ALPHA, typename TM>
 __device__ __forceinline__ int ef_quad_load(const ITile& t, const EfWeightsArgs<TM>& a, int k, int x0, int y0)
 {
     typedef EfQuadTile<CW, EW> Q;
@@ -362,7 +363,7 @@ __device__ __forceinline__ int ef_quad_load(const ITile& t, const EfWeightsArgs<
         for (int q = 0; q < 2; ++q) {
             const int x = x0 + c + q, y = y0 + r;
             const bool in = x >= 0 && x < a.w && y >= 0 && y < a.h;
-            al[q] = in ? ef_alpha<TIn, S>(a.alpha[k], px[j][q], x, y) : 0;
+            al[q] = in ? (ALPHA ? ef_alpha<TIn, S>(a.alpha[k], px[j][q], x, y) : 1) : 0;
             mine &= al[q] || !in;
             g[q] = al[q] ? gray_of(a.wp, px[j][q][0], px[j][q][1], px[j][q][2]) : 0;
         }
@@ -371,8 +372,16 @@ __device__ __forceinline__ int ef_quad_load(const ITile& t, const EfWeightsArgs<
         *reinterpret_cast<uchar2*>(t.a + p) = make_uchar2((unsigned char)al[0], (unsigned char)al[1]);
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
-            *reinterpret_cast<uint32_t*>(t.raw + s * Q::TT + p) = (uint32_t)px[j][0][s] | ((uint32_t)px[j][1][s] << 16);
+            uint32_t v = (uint32_t)px[j][0][s] | ((uint32_t)px[j][1][s] << 16);
+            if (ALPHA && EW > 0) {
+                v |= (al[0] ? 0u : 0xffffu) | (al[1] ? 0u : 0xffff0000u);
+            }
+            *reinterpret_cast<uint32_t*>(t.raw + s * Q::TT + p) = v;
         }
+    }
+    if (!ALPHA) {
+        __syncthreads();
+        return 1;
     }
     return __syncthreads_and(mine);
 }
@@ -384,7 +393,13 @@ __device__ __forceinline__ int ef_quad_load(const ITile& t, const EfWeightsArgs<
 // contrast alone: 0.21 ms (0.45 ms).  Four CTAs an SM (64 registers) beat three
 // (8.7 ms) and two (9.4 ms).  Not kept: the next exposure's pixels in flight
 // while one is weighted, as unaligned words (8.8 ms; 0.25 ms).
-template <typename TIn, typename TM, int CW, int EW>
+// ALPHA: some exposure has alpha.  Tiles with transparent pixels weight their
+// quads too, with the taps of each window counted; evaluating their entropy
+// windows one by one had taken 2.5 times as long as a pixel a thread does on
+// images of a few tiles (9 x 400x300 u8 with holes everywhere, entropy 5x5: 0.92
+// ms, now 0.33).  Stacks without alpha have a kernel without that code: in one
+// kernel it cost them 1.5%.
+template <typename TIn, typename TM, int CW, int EW, bool ALPHA>
 __global__ void __launch_bounds__(256, kQuadBlocks) k_ef_weights_quad(const __grid_constant__ EfWeightsArgs<TM> a)
 {
     typedef EfQuadTile<CW, EW> Q;
@@ -408,8 +423,9 @@ __global__ void __launch_bounds__(256, kQuadBlocks) k_ef_weights_quad(const __gr
     uint32_t ua = 0;
     for (int k = 0; k < a.K; ++k) {
         const int x0 = blockIdx.x * EQX - Q::HX, y0 = blockIdx.y * EQY - Q::HALO;
-        const int opaque = a.img[k].stride == 3 ? ef_quad_load<TIn, 3, CW, EW, TM>(t, a, k, x0, y0)
-                                                : ef_quad_load<TIn, 4, CW, EW, TM>(t, a, k, x0, y0);
+        const int loaded = a.img[k].stride == 3 ? ef_quad_load<TIn, 3, CW, EW, ALPHA, TM>(t, a, k, x0, y0)
+                                                : ef_quad_load<TIn, 4, CW, EW, ALPHA, TM>(t, a, k, x0, y0);
+        const bool opaque = !ALPHA || loaded;
         float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (x < a.w && y < a.h) {
             const auto inside = [&](int q, int b) {  // q's window of half-width b lies in the image
@@ -443,24 +459,27 @@ __global__ void __launch_bounds__(256, kQuadBlocks) k_ef_weights_quad(const __gr
             }
             if constexpr (EW > 0) {
                 uint64_t v[4] = {~0ull, ~0ull, ~0ull, ~0ull};
-                if (opaque) {
+                uint32_t counts = 0u;  // opaque taps of the four windows, 0: all
+                if (!opaque) {
+                    int n[4];
+                    opaque_quad<EW>(t.a, Q::TW, cx, cy, n);
+                    counts = (uint32_t)(n[0] | n[1] << 8 | n[2] << 16 | n[3] << 24);
+                }
 #pragma unroll 1
-                    for (int c = 0; c < 3; ++c) {
-                        entropy_quad<EW>(t.raw + c * Q::TT, Q::TW, cx, cy, et, v);
-                    }
+                for (int c = 0; c < 3; ++c) {
+                    entropy_quad<EW>(t.raw + c * Q::TT, Q::TW, cx, cy, et, counts, a.tab, v);
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     // the rounding is monotone, so that of the least value is the least of the roundings
-                    // (entropy_fx_round); near a half-integer every channel's exact value decides, and in
-                    // tiles with transparent pixels everywhere
+                    // (entropy_fx_round); near a half-integer every channel's exact value decides
                     const uint32_t frac = (uint32_t)v[q];
                     const uint32_t dist = frac >= 0x80000000u ? frac - 0x80000000u : 0x80000000u - frac;
                     uint32_t m = min((uint32_t)(v[q] >> 32) + (frac >> 31), a.wp.maxv);
                     const int cq = ci + (q >> 1) * Q::TW + (q & 1);
                     if (!inside(q, EW / 2)) {
                         m = 0u;
-                    } else if (!opaque || dist <= (uint32_t)(EW * EW + 8)) {
+                    } else if (dist <= (uint32_t)((counts ? (int)((counts >> (8 * q)) & 255u) : EW * EW) + 8)) {
                         m = a.wp.maxv;
                         for (int c = 0; c < 3 && t.a[cq]; ++c) {
                             m = min(m, entropy_exact<EW>(t.raw + c * Q::TT, t.a, Q::TW, cq, a.tab, a.wp.maxv));
@@ -544,10 +563,14 @@ static cudaError_t ef_weights_rgb(EfWeightsArgs<TM>& a, const EfuseHost& h, cuda
     const dim3 g((unsigned)((h.w + EQX - 1) / EQX), (unsigned)((h.h + EQY - 1) / EQY));
 #define ENB_EQ(CWV, EWV)                                                                                    \
     if (cw == CWV && ew == EWV) {                                                                           \
-        auto k = k_ef_weights_quad<TIn, TM, CWV, EWV>;                                                      \
+        auto k = alpha ? k_ef_weights_quad<TIn, TM, CWV, EWV, true> : k_ef_weights_quad<TIn, TM, CWV, EWV, false>; \
         const size_t smem = EfQuadTile<CWV, EWV>::TILE + (size_t)h.K * 1024 * sizeof(float);                \
         allow_smem(k, smem);                                                                                \
         return launch_pdl_smem(k, g, dim3(256), smem, st, a);                                               \
+    }
+    bool alpha = false;
+    for (int k = 0; k < h.K; ++k) {
+        alpha = alpha || h.alpha[k].mode != kAlphaOpaque;
     }
     ENB_EQ(5, 5) ENB_EQ(5, 3) ENB_EQ(3, 5) ENB_EQ(3, 3) ENB_EQ(0, 5) ENB_EQ(0, 3) ENB_EQ(5, 0) ENB_EQ(3, 0)
 #undef ENB_EQ

@@ -768,6 +768,30 @@ __device__ __forceinline__ uint64_t entropy_scaled(uint32_t bnd, const EntropyTa
     return __umul64hi((unsigned long long)(-acc), t.scale[bins]);
 }
 
+// The same of a window with n opaque taps, the first n of the sorted keys
+// (transparent taps carry the largest key), from its boundaries run by run; out
+// of line, for tiles with transparent pixels.
+template <int M>
+static __device__ __noinline__ uint64_t entropy_scaled_alpha(uint32_t bnd, int n, const WeightTables& tab)
+{
+    const uint32_t live = (1u << n) - 1u, b = bnd & live;
+    const int bins = __popc(b) + 1;
+    if (bins <= 1) {
+        return 0ull;
+    }
+    const long long* fx = tab.plogp_fx + (int64_t)n * (M + 1);
+    const long long one = fx[1];
+    long long acc = (long long)bins * one;
+    uint32_t eq = ~b & live & ~1u;
+    while (eq) {
+        const int s0 = __ffs(eq) - 1;
+        const int len = __ffs(~(eq >> s0)) - 1;
+        acc += fx[len + 1] - one;
+        eq &= ~(((1u << len) - 1u) << s0);
+    }
+    return __umul64hi((unsigned long long)(-acc), tab.scale_fx[bins]);
+}
+
 // Boundary masks of two windows sorted in the halves of k (as in entropy_pair).
 template <int M>
 __device__ __forceinline__ void pair_boundaries(const uint32_t (&k)[M], uint32_t& b0, uint32_t& b1)
@@ -789,13 +813,15 @@ __device__ __forceinline__ void pair_boundaries(const uint32_t (&k)[M], uint32_t
 }
 
 // Least H * max (2^-32 fixed point) over the channel's windows of the 2x2
-// pixels at (cx, cy), cx even: v[q] is lowered.  Horizontally adjacent windows
+// pixels at (cx, cy), cx even: v[q] is lowered.  counts: 0 where every window
+// that counts is opaque, else byte q holds the opaque taps of window q, and
+// transparent taps hold 0xffff in the tile.  Horizontally adjacent windows
 // are the halves of the words, vertically adjacent ones share all but one
 // row: the W - 1 common rows are sorted once (the network's comparators per
 // quad: 207 instead of 280 for W = 5).
 template <int W>
 __device__ __forceinline__ void entropy_quad(const uint16_t* plane, int TW, int cx, int cy, const EntropyTables& t,
-                                             uint64_t (&v)[4])
+                                             uint32_t counts, const WeightTables& tab, uint64_t (&v)[4])
 {
     constexpr int B = W / 2;
     uint32_t r[W + 1][W];
@@ -831,8 +857,14 @@ __device__ __forceinline__ void entropy_quad(const uint16_t* plane, int TW, int 
         merge_sorted(r[q == 0 ? 0 : W], common, k, CeU16x2());
         uint32_t b0, b1;
         pair_boundaries<W * W>(k, b0, b1);
-        v[2 * q] = min(v[2 * q], entropy_scaled<W * W>(b0, t));
-        v[2 * q + 1] = min(v[2 * q + 1], entropy_scaled<W * W>(b1, t));
+        if (counts == 0u) {
+            v[2 * q] = min(v[2 * q], entropy_scaled<W * W>(b0, t));
+            v[2 * q + 1] = min(v[2 * q + 1], entropy_scaled<W * W>(b1, t));
+        } else {
+            const uint32_t n = counts >> (16 * q);
+            v[2 * q] = min(v[2 * q], entropy_scaled_alpha<W * W>(b0, (int)(n & 255u), tab));
+            v[2 * q + 1] = min(v[2 * q + 1], entropy_scaled_alpha<W * W>(b1, (int)((n >> 8) & 255u), tab));
+        }
     }
 }
 

@@ -226,3 +226,22 @@ def test_exposures_of_rgb_and_rgba_mixed(ctx, dt, samples, windows):
     assert np.array_equal(l0m, l0)
     assert np.array_equal(outm[..., :3], out)
     assert np.array_equal(oam, oa)
+
+
+@pytest.mark.parametrize("dt", [np.uint8, np.uint16])
+@pytest.mark.parametrize("window", [3, 5])
+@pytest.mark.parametrize("holes", [0.02, 0.3, 0.9])
+def test_entropy_windows_with_transparent_taps(ctx, orc, dt, window, holes):
+    """Entropy of windows with transparent taps, whose keys sort as the largest sample: few distinct samples with the
+    type's maximum among them, from a few holes to a few opaque pixels, against the oracle bit for bit."""
+    h, w, K = 39, 71, 2
+    rng = np.random.default_rng(window)
+    top = np.iinfo(dt).max
+    imgs = [rng.choice(np.array([0, 1, top // 2, top - 1, top], dt), (h, w, 3)) for _ in range(K)]
+    alphas = [np.where(rng.random((h, w)) < holes, 0, 255).astype(np.uint8) for _ in range(K)]
+    kw = dict(exposure_weight=0.2, entropy_weight=1.0, entropy_window_size=window, contrast_weight=0.3, contrast_window_size=5)
+    ref = orc.enfuse(imgs, alphas, orc.params(**kw), seed=9, want_level0=True)
+    l0, out, oa = _run(ctx, imgs, kw, seed=9, alphas=[_dev(a) for a in alphas])
+    assert np.array_equal(l0, ref["level0"])
+    assert np.array_equal(oa, ref["alpha"])
+    assert np.array_equal(out, ref["out"])

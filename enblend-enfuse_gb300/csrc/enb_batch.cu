@@ -7,14 +7,18 @@
 // conversion back.  The whole batch runs as one short sequence of launches,
 // each covering every stack and exposure at one pyramid level:
 //
-//   weights   one CTA per 16x16 tile of a stack: the K weights of each pixel
-//             (enb_fweights.cuh), their sum, the soft (or hard) masks as
-//             level 0 of the mask pyramids, the union alpha, and level 0 of
-//             the image pyramids;
+//   weights   one CTA per exposure of a 32x16 tile: the weights
+//             (enb_fpair.cuh), left as float bits in the level-0 mask plane,
+//             and level 0 of the image pyramid; windows outside the pair
+//             kernel have a kernel of their own (k_batch_weights), which
+//             normalises as well;
+//   normalise per 32x16 tile of a stack: the weights' sum, the soft (or hard)
+//             masks as level 0 of the mask pyramids, the union alpha;
 //   down l    one CTA per 64x16 destination tile of level l+1 of one
-//             exposure's image or mask pyramid (reduce with alpha); level 0
-//             of each image pyramid (the log mapping) is written by the
-//             weights kernel, which reads the input anyway;
+//             exposure's image or mask pyramid (reduce with alpha, or the
+//             opaque reduce of a stack without); level 0 of each image pyramid
+//             (the log mapping) is written by the weights kernel, which reads
+//             the input anyway;
 //   coarse    a persistent kernel walking a device work queue of (stack,
 //             level, tile) items: every reduce tile of the levels below
 //             ~64x64 of every stack and exposure, then every up tile, each
@@ -708,7 +712,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
 // Issues the copies of exposure k's level-0 tile (C planes) and mask tile.

@@ -140,24 +140,6 @@ __device__ __forceinline__ uint32_t load_sample(const void* p, int dtype, int64_
                            : (uint32_t)reinterpret_cast<const uint16_t*>(p)[i];
 }
 
-template <typename TIn, int S>
-__device__ __forceinline__ void load_pixel(const TIn* px, TIn (&p)[S])
-{
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-        p[c] = px[c];
-    }
-}
-
-template <typename TIn, int S>
-__device__ __forceinline__ void store_pixel(TIn* px, const TIn (&p)[S])
-{
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-        px[c] = p[c];
-    }
-}
-
 static inline dim3 grid2d(int w, int h, int tw, int th)
 {
     return dim3((unsigned)((w + tw - 1) / tw), (unsigned)((h + th - 1) / th));
@@ -307,17 +289,6 @@ __device__ __forceinline__ int32_t div_any(int32_t num, int32_t den)
     const uint64_t e = __ldg(&g_div_table.e[den]);
     const uint32_t q = (uint32_t)(((uint64_t)a * (uint32_t)e) >> (uint32_t)(e >> 32));
     return num < 0 ? -(int32_t)q : (int32_t)q;
-}
-
-__device__ __forceinline__ int32_t div_den(int32_t num, int den)
-{
-    if (den == 64) {
-        return num / 64;
-    }
-    if (den == 16) {
-        return num / 16;
-    }
-    return div_any(num, den);
 }
 
 // Programmatic dependent launch: a kernel launched with the programmatic

@@ -82,7 +82,7 @@ __device__ __forceinline__ void ld_pair(const T* p, int32_t& a, int32_t& b)
 
 template <typename T, typename TM>
 struct EfLevelArgs {
-    int K, C, dw, dh, cw, ch, wrap, mfrac;
+    int K, dw, dh, cw, ch, wrap;
     const T* g[kEfuseMaxK];   // level l of the image pyramids
     const T* gc[kEfuseMaxK];  // level l + 1
     const TM* m[kEfuseMaxK];  // level l of the mask pyramids
@@ -611,13 +611,11 @@ static EfLevelArgs<T, TM> level_args(const EfuseHost& h, int l)
 {
     EfLevelArgs<T, TM> a{};
     a.K = h.K;
-    a.C = h.C;
     a.dw = h.lw[l];
     a.dh = h.lh[l];
     a.cw = h.lw[l + 1];
     a.ch = h.lh[l + 1];
     a.wrap = h.wrap;
-    a.mfrac = h.dtype == ENB_U8 ? 7 : 15;
     for (int k = 0; k < h.K; ++k) {
         a.g[k] = (const T*)h.g[k][l];
         a.gc[k] = (const T*)h.g[k][l + 1];

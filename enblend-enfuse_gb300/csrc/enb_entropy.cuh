@@ -172,15 +172,16 @@ namespace enb {
 //
 // Float samples rarely repeat except at the clip values 0 and 1.  The
 // samples equal to 0.0 or 1.0 are counted per window (two bins whose sizes
-// are those counts); all other opaque samples go through the repeat marks
-// below, and a window without marks has only singletons besides the two
-// clip bins, so its H follows from three counts.  Every opaque sample of the
-// tile (halo included) goes into a shared-memory hash table per channel; a
-// second insertion of an equal key flags the slot.  A sample whose slot is
-// flagged occurs more than once in the tile and gets a repeat mark.  A
-// window with no mark in channel c has all-distinct keys in that channel
-// (marks from matches elsewhere in the tile only send a window down the
-// exact sorting path, they never change a result).
+// are those counts); all other opaque samples go through repeat marks, and a
+// window without marks has only singletons besides the two clip bins, so its
+// H follows from three counts.  Here is the search of the one-pixel-a-thread
+// kernels (the pair kernels search by rounds of plain stores, enb_fpair.cuh):
+// every opaque sample of the tile (halo included) goes into a shared-memory
+// hash table per channel; a second insertion of an equal key flags the slot.
+// A sample whose slot is flagged occurs more than once in the tile and gets a
+// repeat mark.  A window with no mark in channel c has all-distinct keys in
+// that channel (marks from matches elsewhere in the tile only send a window
+// down the exact sorting path, they never change a result).
 //
 // Per-pixel counters (one 64-bit word per tile pixel, summed over a window):
 //   bits  0..14  samples equal to 1.0, channels 0..2 (5 bits each)

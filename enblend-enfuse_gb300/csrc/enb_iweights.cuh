@@ -199,7 +199,6 @@ struct ITile {
     int TT;          // plane size: TW * rows
 };
 
-__host__ __device__ inline size_t itile_bytes(int TW) { return (size_t)TW * TW * (sizeof(int32_t) + 3 * sizeof(uint16_t) + 1); }
 __host__ __device__ inline size_t itile_bytes_rect(int TW, int TH)
 {
     return (size_t)TW * TH * (sizeof(int32_t) + 3 * sizeof(uint16_t) + 1);
@@ -209,51 +208,6 @@ __host__ __device__ inline int iweight_halo(const WeightParams& wp)
 {
     const int hc = wp.use_contrast ? wp.contrast_window / 2 : 0, he = wp.use_entropy ? wp.entropy_window / 2 : 0;
     return hc > he ? hc : he;
-}
-
-__device__ __forceinline__ ITile itile_carve(unsigned char* smem, int TW)
-{
-    ITile t;
-    t.TW = TW;
-    t.gray = reinterpret_cast<int32_t*>(smem);
-    t.TT = TW * TW;
-    t.raw = reinterpret_cast<uint16_t*>(t.gray + TW * TW);
-    t.a = reinterpret_cast<uint8_t*>(t.raw + 3 * TW * TW);
-    return t;
-}
-
-// Loads the tile whose top-left input pixel is (x0, y0): zero and
-// transparent outside the image.  All threads call; the caller syncs.
-__device__ __forceinline__ void itile_load(const ITile& t, const WeightParams& wp, const PixelView& img,
-                                           const AlphaSrc& alpha, int x0, int y0)
-{
-    const int TW = t.TW, TT = TW * TW;
-    const int w = img.w, h = img.h, C = img.C;
-    for (int k = threadIdx.x; k < TT; k += blockDim.x) {
-        const int r = k / TW, c = k - r * TW;
-        const int gx = x0 + c, gy = y0 + r;
-        int32_t g = 0;
-        uint8_t a = 0;
-        uint32_t rgb[3] = {0, 0, 0};
-        if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-            const int64_t base = (int64_t)gy * img.pitch + (int64_t)gx * img.stride;
-            for (int ch = 0; ch < C; ++ch) {
-                rgb[ch] = load_sample(img.p, img.dtype, base + ch);
-            }
-            g = C == 1 ? (int32_t)rgb[0] : gray_of(wp, rgb[0], rgb[1], rgb[2]);
-            a = (uint8_t)alpha_at(alpha, gx, gy);
-            if (wp.ent_cut) {
-                // the tile's samples feed only the entropy windows then; the
-                // saturation reloads its pixel
-                entropy_clamp(wp, rgb, C);
-            }
-        }
-        t.gray[k] = g;
-        t.a[k] = a;
-        for (int ch = 0; ch < 3; ++ch) {
-            t.raw[ch * TT + k] = (uint16_t)rgb[ch];
-        }
-    }
 }
 
 // The enfuseMask weight of the output pixel (x, y) at tile index ci:
@@ -381,9 +335,9 @@ __device__ __forceinline__ ITile itile_carve_rect(unsigned char* smem, int TW, i
     return t;
 }
 
-// Loads the TW x TH tile whose top-left input pixel is (x0, y0) as
-// itile_load does (all threads call); ends with a barrier and returns
-// nonzero when every tile pixel lies in the image and is opaque.
+// Loads the TW x TH tile whose top-left input pixel is (x0, y0), zero and
+// transparent outside the image (all threads call); ends with a barrier and
+// returns nonzero when every tile pixel lies in the image and is opaque.
 __device__ __forceinline__ int itile_load_rect(const ITile& t, const WeightParams& wp, const PixelView& img,
                                                const AlphaSrc& alpha, int x0, int y0)
 {

@@ -15,8 +15,8 @@
 // Columns of at most 4096 rows: q^2 and every other number of the column
 // envelope is an integer below 2^24, exact in float, so the envelope of a
 // 0 / FLT_MAX column is the distance to the nearest feature above or below
-// (FLT_MAX without one) and k_nft_near scans for it with bit masks, one warp
-// per 32 columns x 1/32 of the rows.  Taller columns round and keep the
+// (FLT_MAX without one) and k_nft_near scans for it with bit masks, half a warp
+// per 16 columns x 1/32 of the rows.  Taller columns round and keep the
 // sequential envelope (k_nft_columns, one thread a line).
 //
 // Rows: the sums round (q^2 beyond 2^24) and which vertex survives depends on
@@ -122,13 +122,13 @@ __global__ void __launch_bounds__(128) k_nft_columns(const NftArgs a)
 
 constexpr int kNearRows = 4096;
 constexpr uint16_t kNoFeature = 0xffff;
-constexpr int kNearWords = kNearRows / 32 / 32;  // feature words of a warp's rows
+constexpr int kNearWords = kNearRows / 32 / 32;  // feature words of a half warp's rows
 
 struct NearArgs {
     const uint8_t* white;
     const uint8_t* black;
     int64_t wpitch, bpitch;
-    int w, h, rows;      // rows: rows of one warp
+    int w, h, rows;      // rows: rows of one half warp
     uint16_t* g;         // [2][h][pitch]: rows to the nearest feature, kNoFeature
     int64_t pitch;
     unsigned int* tally; // [2]
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(32 * kNearCols, 3) k_nft_near(const NearArgs a
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-        int above = INT_MIN / 2, below = INT_MAX / 2;  // nearest feature outside the warp's rows
+        int above = INT_MIN / 2, below = INT_MAX / 2;  // nearest feature outside the half warp's rows
         for (int q = 0; q < r; ++q) {
             above = max(above, last[t][q][lane]);
         }

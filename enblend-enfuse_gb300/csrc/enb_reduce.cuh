@@ -21,8 +21,9 @@
 //               no alpha is read, summed or written;
 //   zeros:      taps outside the image dropped, times a constant (the
 //               transposed expand, enb_adjoint.cu).
-// blockIdx.z selects one of up to two jobs of the same geometry (the white and
-// black pyramids of a level), so a level of both images is one launch.
+// blockIdx.z selects one of several jobs of the same geometry (the white and
+// black pyramids of a level and the seam mask's, the exposures of a stack and
+// their masks), so a level of all of them is one launch.
 #pragma once
 
 #include "enb_device.cuh"

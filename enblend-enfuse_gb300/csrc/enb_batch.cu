@@ -70,8 +70,8 @@ struct BatchStack {
     float* g;     // K * 3 * s1 (C planes used)
     uint8_t* a;   // K * s1
     float* r;     // 3 * s1
-    float* g0;    // K * 3 * pitch[0] * h (level 0 of the image pyramids, written by the weights kernel)
-    int64_t s0, s1;
+    float* g0;    // K * 3 * p0 (level 0 of the image pyramids, written by the weights kernel)
+    int64_t s0, s1, p0;  // p0: pitch[0] * h
     int64_t off0[kMaxLevels], off1[kMaxLevels];
     int pitch[kMaxLevels], lw[kMaxLevels], lh[kMaxLevels];
 };
@@ -158,7 +158,7 @@ __device__ __forceinline__ float* r_level(const BatchStack& s, int l, int C)
 // Level 0 of exposure k's image pyramid (planes of pitch[0] * h).
 __device__ __forceinline__ float* g0_level(const BatchStack& s, int k, int C)
 {
-    return s.g0 + (int64_t)k * C * s.pitch[0] * s.h;
+    return s.g0 + (int64_t)k * C * s.p0;
 }
 
 // Level 0 of an exposure's image pyramid (planar floats) with the input's
@@ -1062,6 +1062,7 @@ void level_geometry(BatchStack& s, int64_t coarse_pixels)
         lh = (lh + 1) >> 1;
     }
     s.s0 = o0;
+    s.p0 = (int64_t)s.pitch[0] * s.h;
     s.s1 = o1 > 0 ? o1 : 1;
 }
 
@@ -1108,7 +1109,7 @@ static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 static size_t stack_bytes(const BatchStack& s, int C)
 {
     return align256((size_t)s.K * s.s0 * 4) + align256((size_t)s.s0) + align256((size_t)s.K * C * s.s1 * 4) +
-           align256((size_t)s.K * s.s1) + align256((size_t)C * s.s1 * 4) + align256((size_t)s.K * C * s.pitch[0] * s.h * 4);
+           align256((size_t)s.K * s.s1) + align256((size_t)C * s.s1 * 4) + align256((size_t)s.K * C * s.p0 * 4);
 }
 
 static void stack_buffers(BatchStack& s, int C, char* q)
@@ -1607,9 +1608,8 @@ bool batch_single_weighs(const BatchSingle* p) { return p->ws.pair; }
 void batch_single_level0(const BatchSingle* p, int k, FloatPlane* weights, PlanarView* image)
 {
     const BatchStack& s = p->s;
-    const int64_t plane = (int64_t)s.pitch[0] * s.h;
     *weights = FloatPlane{(float*)(s.m + (int64_t)k * s.s0 + s.off0[0]), s.pitch[0], s.w, s.h};
-    *image = PlanarView{s.g0 + (int64_t)k * p->C * plane, s.pitch[0], plane, s.w, s.h, p->C, ENB_F32};
+    *image = PlanarView{s.g0 + (int64_t)k * p->C * s.p0, s.pitch[0], s.p0, s.w, s.h, p->C, ENB_F32};
 }
 
 template <int C>

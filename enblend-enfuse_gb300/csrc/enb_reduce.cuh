@@ -465,20 +465,32 @@ __device__ __forceinline__ void reduce_tail(const TailGeometry& g, T* const* p, 
     AC* lev = smem;                              // [NV][h][w]
     AC* sums = smem + NV * kTailPixels;          // [NV][dh][w]
     {
+        // all loads before the first store, which they might not pass
+        constexpr int N = kTailPixels / kTailThreads;
         const int w = g.w[0], n = w * g.h[0];
         const int64_t plane = g.pitch[0] * g.h[0];
-#pragma unroll 4
-        for (int i = threadIdx.x; i < n; i += kTailThreads) {
-            const int y = i / w, x = i - y * w;
-            const int64_t o = (int64_t)y * g.pitch[0] + x;
-            const int al = A ? ld_dep(&ap[0][(int64_t)y * g.apitch[0] + x]) != 0 : 1;
+        AC v[N][C];
+        int al[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const int i = min((int)threadIdx.x + u * kTailThreads, n - 1), y = i / w, x = i - y * w;
+            al[u] = A ? ld_dep(&ap[0][(int64_t)y * g.apitch[0] + x]) != 0 : 1;
 #pragma unroll
             for (int c = 0; c < C; ++c) {
-                const AC v = (AC)ld_dep(&p[0][c * plane + o]);
-                lev[c * n + i] = al ? v : (AC)0;
+                v[u][c] = (AC)ld_dep(&p[0][c * plane + (int64_t)y * g.pitch[0] + x]);
             }
-            if (A) {
-                lev[(NV - 1) * n + i] = (AC)al;
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const int i = threadIdx.x + u * kTailThreads;
+            if (i < n) {
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    lev[c * n + i] = al[u] ? v[u][c] : (AC)0;
+                }
+                if (A) {
+                    lev[(NV - 1) * n + i] = (AC)al[u];
+                }
             }
         }
     }

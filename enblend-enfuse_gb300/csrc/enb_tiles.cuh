@@ -31,32 +31,40 @@ struct CoarseLevels {
 };
 
 // Stage the 34x10 coarse neighbourhoods of a 64x16 destination tile for NP
-// planes; loads unrolled and independent of each other.
+// planes; all loads before the first store, which they might not pass.
 template <int NP, typename T, bool EARLIER, int NT>
 __device__ __forceinline__ void stage_coarse(int32_t (*ss)[ESH][ESW], const CoarseLevels& cl, int I0, int J0,
                                              int dw, int wrap)
 {
     constexpr int N = ESH * ESW;
     constexpr int IT = (N + NT - 1) / NT;
+    int32_t v[IT][NP], f[IT];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+        const int k = min((int)threadIdx.x + it * NT, N - 1);
+        const int r = k / ESW, c = k - r * ESW;
+        const int j = J0 - 1 + r;
+        int i = I0 - 1 + c;
+        f[it] = wrap && (dw & 1) && (i == -1 || i == cl.w) ? 4 : 1;  // as TileWindow
+        if (wrap) {
+            i = imod(i, cl.w);
+        }
+        f[it] = j >= 0 && j < cl.h && i >= 0 && i < cl.w ? f[it] : 0;
+        // clamped position: the loads are unconditional, the taps outside
+        // the level are zeroed afterwards
+        const int64_t o = (int64_t)min(max(j, 0), cl.h - 1) * cl.pitch + min(max(i, 0), cl.w - 1);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            v[it][p] = (int32_t)ld_src<EARLIER>(&reinterpret_cast<const T*>(cl.p[p])[o]);
+        }
+    }
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
         const int k = threadIdx.x + it * NT;
         if (k < N) {
-            const int r = k / ESW, c = k - r * ESW;
-            const int j = J0 - 1 + r;
-            int i = I0 - 1 + c;
-            const int32_t f = wrap && (dw & 1) && (i == -1 || i == cl.w) ? 4 : 1;  // as TileWindow
-            if (wrap) {
-                i = imod(i, cl.w);
-            }
-            const bool in = j >= 0 && j < cl.h && i >= 0 && i < cl.w;
-            // clamped position: the loads are unconditional, the taps outside
-            // the level are zeroed afterwards
-            const int64_t o = (int64_t)min(max(j, 0), cl.h - 1) * cl.pitch + min(max(i, 0), cl.w - 1);
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
-                const int32_t v = (int32_t)ld_src<EARLIER>(&reinterpret_cast<const T*>(cl.p[p])[o]);
-                ss[p][r][c] = in ? v * f : 0;
+                (&ss[p][0][0])[k] = v[it][p] * f[it];
             }
         }
     }
@@ -76,16 +84,23 @@ __device__ __forceinline__ void stage_coarse4_interior(int4 (*s4)[ESH][ESW], con
     for (int p = 0; p < 3 * C; ++p) {
         base[p] = reinterpret_cast<const T*>(cl.p[p]) + (int64_t)(J0 - 1) * cl.pitch + (I0 - 1);
     }
+    int32_t v[IT][3 * C];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+        const int k = min((int)threadIdx.x + it * NT, N - 1);
+        const int r = k / ESW, o = r * (int)cl.pitch + k - r * ESW;
+#pragma unroll
+        for (int p = 0; p < 3 * C; ++p) {
+            v[it][p] = (int32_t)ld_src<EARLIER>(&base[p][o]);
+        }
+    }
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
         const int k = threadIdx.x + it * NT;
         if (k < N) {
-            const int r = k / ESW, c = k - r * ESW;
-            const int o = r * (int)cl.pitch + c;
 #pragma unroll
             for (int ch = 0; ch < C; ++ch) {
-                s4[ch][r][c] = make_int4((int32_t)ld_src<EARLIER>(&base[ch][o]), (int32_t)ld_src<EARLIER>(&base[C + ch][o]),
-                                         (int32_t)ld_src<EARLIER>(&base[2 * C + ch][o]), 0);
+                (&s4[ch][0][0])[k] = make_int4(v[it][ch], v[it][C + ch], v[it][2 * C + ch], 0);
             }
         }
     }

@@ -1337,7 +1337,7 @@ enb_status enfuse_fused(enb_ctx* ctx, const enb_enfuse_params* prm, int K, const
 // stored, with the values of the per-operation passes.  It keeps the
 // pyramids of every exposure at once; done is false when they do not fit the
 // device's memory (the per-operation passes, which keep one, then run).
-// 4 x 1601x1203 RGB, all weights: 22 launches and 0.66 ms, against 165
+// 4 x 1601x1203 RGB, all weights: 22 launches and 0.46 ms, against 165
 // launches and 1.43 ms one operation at a time.
 enb_status enfuse_float(enb_ctx* ctx, const enb_enfuse_params* prm, int K, const enb_image* images,
                         const enb_image* alphas, const enb_image* out, const enb_image* out_alpha,
@@ -2571,8 +2571,8 @@ enb_status enb_fuse_stacks(enb_ctx* ctx, const enb_enfuse_params* prm, int n, co
               "fuse_stacks: a call being captured takes device buffers, graph = 0, and a call on the same buffers before it");
     if (planned && moved && !bc.captured) {
         // the same work on other buffers: only the stacks' addresses change
-        // (a new plan, its tables and its graph took 6 ms of a 23.3 ms call of
-        // 16 stacks; the new addresses take 0.03 ms of the host's time)
+        // (16 stacks: a new plan, its tables and its graph take 5 ms, the new
+        // addresses 7 us of the host's time)
         std::vector<BatchStackHost> hs;
         ENB_TRY(stack_hosts(hs));
         ENB_CUDA(ctx, batch_plan_rebind(bc.plan, hs, ctx->stream));

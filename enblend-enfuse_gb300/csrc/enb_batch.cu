@@ -278,8 +278,8 @@ __global__ void __launch_bounds__(256, 4) k_batch_weights(const BatchStack* __re
 // windows fits five times): the warps hide the kernel's latencies better than
 // more registers would.  For the same reason the tables come inside a struct,
 // not as restrict parameters: reading the stack's fields again after every
-// store costs less than the registers that keep them (16 stacks: 10.9 against
-// 11.5 ms).  A block is one exposure of a tile (blockIdx.z, in a batch
+// store costs less than the registers that keep them (10.9 against 11.5 ms on
+// 16 stacks, with all exposures of a tile in a block).  A block is one exposure of a tile (blockIdx.z, in a batch
 // blockIdx.y, where those past a stack's exposures leave at once): a tile's
 // exposures in turn made blocks several times as long, and a single stack's
 // last wave of them kept the chip busy to 73 % (with the search for repeats of

@@ -387,18 +387,19 @@ __device__ __forceinline__ int ef_quad_load(const ITile& t, const EfWeightsArgs<
 }
 
 // Bound by instructions, the min/max pairs of the sorting networks first.
-// 9 x 6000x4000 u16, all weights, 5x5 windows: 8.4 ms, 850 instructions a pixel
-// and exposure (12.7 ms and 1,550 with pairs of pixels, each window sorted by
+// 9 x 6000x4000 u16, all weights, 5x5 windows: 8.0 ms, 911 instructions a pixel
+// and exposure (12.7 ms and 1,546 with pairs of pixels, each window sorted by
 // itself and every channel's entropy rounded); 5 x 2047x1535 u16 with alpha,
-// contrast alone: 0.21 ms (0.45 ms).  Four CTAs an SM (64 registers) beat three
-// (8.7 ms) and two (9.4 ms).  Not kept: the next exposure's pixels in flight
-// while one is weighted, as unaligned words (8.8 ms; 0.25 ms).
+// contrast alone: 0.21 ms (0.45 ms).  Before the two instances below, at 8.4
+// ms: four CTAs an SM (64 registers) beat three (8.7 ms) and two (9.4 ms); not
+// kept: the next exposure's pixels in flight while one is weighted, as
+// unaligned words (8.8 ms; 0.25 ms).
 // ALPHA: some exposure has alpha.  Tiles with transparent pixels weight their
 // quads too, with the taps of each window counted; evaluating their entropy
 // windows one by one had taken 2.5 times as long as a pixel a thread does on
 // images of a few tiles (9 x 400x300 u8 with holes everywhere, entropy 5x5: 0.92
-// ms, now 0.33).  Stacks without alpha have a kernel without that code: in one
-// kernel it cost them 1.5%.
+// ms a call, now 0.33).  Stacks without alpha have an instance without that
+// code: in one kernel for both they took 8.7 ms.
 template <typename TIn, typename TM, int CW, int EW, bool ALPHA>
 __global__ void __launch_bounds__(256, kQuadBlocks) k_ef_weights_quad(const __grid_constant__ EfWeightsArgs<TM> a)
 {

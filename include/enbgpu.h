@@ -414,9 +414,10 @@ typedef struct {
  * the scalars in `res` and, when grad_logits is given, dL/d logit_k per
  * pixel.  logits: K F32 planes or NULL (all 0).  out: optional F32 image
  * receiving the forward result.  Entropy weights, the exposure cutoff, hard
- * masks and wrap-around are not differentiated (ENB_ERR_UNSUPPORTED).  The backward rebuilds each
- * exposure's Laplacian pyramid instead of keeping K of them, so the memory
- * held is one pyramid per kind whatever K.  Device buffers; synchronous. */
+ * masks and wrap-around are not differentiated (ENB_ERR_UNSUPPORTED).  No Laplacian
+ * pyramid is kept: both sweeps form Laplacians from the Gaussian pyramids of
+ * all K images, which stay in memory with the K mask pyramids and weights,
+ * about 25 K + 32 bytes a pixel.  Device buffers; synchronous. */
 enb_status enb_fuse_grad(enb_ctx* ctx, const enb_enfuse_params* params, int K, const enb_image* images,
                          const enb_image* logits, const enb_image* target, const enb_image* out,
                          const enb_image* grad_logits, enb_fuse_grad_result* res, const enb_fuse_options* opt);
